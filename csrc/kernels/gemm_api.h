@@ -33,8 +33,8 @@ int gemmBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, in
 
 // D[M,N] = (A * B^T) .* gelu_tanh'(pre[M,N]) in bf16, and colsum[n] += sum_m D[m,n] (fp32, may be null): the
 // backward of "linear -> GELU -> linear" between the second layer's input gradient and the first layer's output
-// gradient, with the first layer's bias gradient as a by-product.  `pre` has D's row stride.  CTA pairs; M a multiple
-// of 256 and N a multiple of 256; flags: GEMM_A_MN / GEMM_B_MN only.
+// gradient, with the first layer's bias gradient as a by-product.  `pre` has D's row stride.  CTA pairs; N a
+// multiple of 32; flags: GEMM_A_MN / GEMM_B_MN only.
 int gemmBf16Dgelu(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, int64_t ldd, const void* pre, float* colsum,
                   int M, int N, int K, uint32_t flags, int sms, uint32_t* status, cudaStream_t stream);
 

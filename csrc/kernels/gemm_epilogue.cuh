@@ -93,7 +93,8 @@ __device__ __forceinline__ void patch_load_bf16(uint8_t* P, int lane, const __nv
 
 // Backward of a GELU that sits between two linear layers, fused into the GEMM that produces the gradient of the
 // activation: D = (A * B^T) .* gelu'(pre), and the column sums of D (the bias gradient of the first layer) are added
-// to `colsum` (fp32, zeroed by the caller).  Full tiles only (M % 128 == 0, N % 256 == 0); `pre` has D's layout.
+// to `colsum` (fp32, zeroed by the caller).  N % 32 == 0; `pre` has D's layout.  Runs on the CTA-pair kernels (eight epilogue
+// warps, coalescing patch).
 struct DgeluEpi {
   static constexpr bool kRow128 = false;
   __nv_bfloat16* D;
@@ -101,62 +102,52 @@ struct DgeluEpi {
   float* colsum;
   long long ldd;
   int M, N;
-  uint8_t* patch = nullptr;      // kPatchBytesPerCta of shared memory when the pipeline provides it (see above)
+  int bn = BN;
+  uint8_t* patch = nullptr;      // kPatchBytesPerCta of shared memory (see above)
 
+  __device__ __forceinline__ int width() const { return bn; }
   __device__ __forceinline__ int a_row0(const TileCoord& t) const { return t.m * BM; }
-  __device__ __forceinline__ int b_row0(const TileCoord& t) const { return t.n * BN; }
+  __device__ __forceinline__ int b_row0(const TileCoord& t) const { return t.n * bn; }
   __device__ __forceinline__ void attach_smem(uint8_t*) {}
-  __device__ __forceinline__ void attach_patch(uint8_t* p) {
-    if ((ldd & 7) == 0 && ((reinterpret_cast<uintptr_t>(D) | reinterpret_cast<uintptr_t>(pre)) & 15) == 0) patch = p;
-  }
+  __device__ __forceinline__ void attach_patch(uint8_t* p) { patch = p; }
   // The pre-activations of a strip are fetched one strip ahead (four 16-byte loads per lane, eight rows per instruction)
   // and parked in registers: their latency passes behind the previous strip's arithmetic instead of in front of this one's.
   dev::Vec16 ahead[4];
   __device__ __forceinline__ void fetch_ahead(const TileCoord& t, int quarter, int lane, int col_in_tile) {
-    const __nv_bfloat16* g0 = pre + static_cast<long long>(t.m * BM + quarter * 32) * ldd + t.n * BN + col_in_tile + (lane & 3) * 8;
+    const int row0 = t.m * BM + quarter * 32, col = t.n * bn + col_in_tile;
+    const __nv_bfloat16* g0 = pre + static_cast<long long>(row0) * ldd + col + (lane & 3) * 8;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) ahead[j] = dev::ld16(g0 + ((lane >> 2) + 8 * j) * ldd);
+    for (int j = 0; j < 4; ++j) {
+      const int rr = (lane >> 2) + 8 * j;
+      ahead[j] = (col < N && row0 + rr < M) ? dev::ld16(g0 + rr * ldd) : dev::Vec16{{0u, 0u, 0u, 0u}};
+    }
   }
-  // columns that one epilogue warp walks through: the whole tile, or half of it where two warps share a lane quarter
-  __device__ __forceinline__ int span() const { return blockDim.x > 192 ? BN / 2 : BN; }
+  // the strips of a tile are split over the two warps of a lane quarter: the first takes [0, split), the second the rest
+  __device__ __forceinline__ int split() const { return (bn / 32 + 1) / 2 * 32; }
   __device__ __forceinline__ void tile_begin(const TileCoord& t) {
-    if (patch) fetch_ahead(t, (threadIdx.x >> 5) & 3, threadIdx.x & 31, (((threadIdx.x >> 5) - 2) >> 2) * span());
+    fetch_ahead(t, (threadIdx.x >> 5) & 3, threadIdx.x & 31, (((threadIdx.x >> 5) - 2) >> 2) * split());
   }
   __device__ __forceinline__ void tile_done(const TileCoord&, const volatile uint32_t*) {}
 
   __device__ __forceinline__ void strip(const TileCoord& t, int row_in_tile, int col_in_tile, uint32_t* r) {
-    const int row = t.m * BM + row_in_tile, col = t.n * BN + col_in_tile;
-    const long long at = static_cast<long long>(row) * ldd + col;
-    float v[32];
-    if (patch) {
-      const int lane = row_in_tile & 31, quarter = (row_in_tile >> 5) & 3;
-      uint8_t* P = my_patch(patch);
-      const long long at0 = static_cast<long long>(row - lane) * ldd + col;
-      float x[32];
+    const int row = t.m * BM + row_in_tile, col = t.n * bn + col_in_tile;
+    const int lane = row_in_tile & 31, quarter = (row_in_tile >> 5) & 3, row0 = row - lane;
+    if (col >= N || row0 >= M) return;       // uniform over the warp
+    uint8_t* P = my_patch(patch);
+    float v[32], x[32];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        *reinterpret_cast<dev::Vec16*>(P + ((lane >> 2) + 8 * j) * kPatchRowBytes + (lane & 3) * 16) = ahead[j];
-      __syncwarp();
+    for (int j = 0; j < 4; ++j)
+      *reinterpret_cast<dev::Vec16*>(P + ((lane >> 2) + 8 * j) * kPatchRowBytes + (lane & 3) * 16) = ahead[j];
+    __syncwarp();
 #pragma unroll
-      for (int i = 0; i < 4; ++i) dev::unpack<DT_BF16>(*reinterpret_cast<const dev::Vec16*>(P + lane * kPatchRowBytes + i * 16), x + 8 * i);
-      __syncwarp();
-      if (((col_in_tile + 32) & (span() - 1)) != 0) fetch_ahead(t, quarter, lane, col_in_tile + 32);
+    for (int i = 0; i < 4; ++i) dev::unpack<DT_BF16>(*reinterpret_cast<const dev::Vec16*>(P + lane * kPatchRowBytes + i * 16), x + 8 * i);
+    __syncwarp();
+    if (col_in_tile + 32 < ((threadIdx.x >> 5) - 2 < 4 ? split() : bn)) fetch_ahead(t, quarter, lane, col_in_tile + 32);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * dgelu_tanh(x[i]);
-      patch_store_bf16(P, lane, D + at0, ldd, v, 32);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 32; i += 8) {
-        float x[8];
-        dev::unpack<DT_BF16>(dev::ld16(pre + at + i), x);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[i + j] = __uint_as_float(r[i + j]) * dgelu_tanh(x[j]);
-      }
-#pragma unroll
-      for (int i = 0; i < 32; i += 8) dev::st16(D + at + i, dev::pack<DT_BF16>(v + i));
-    }
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * dgelu_tanh(x[i]);
+    patch_store_bf16(P, lane, D + static_cast<long long>(row0) * ldd + col, ldd, v, M - row0);
     if (colsum) {
-      const int lane = threadIdx.x & 31;       // an epilogue warp holds 32 consecutive rows, one per lane
+      // an epilogue warp holds 32 consecutive rows, one per lane; rows past M were multiplied from zero fill, so they add 0
       warp_transpose_sum32(v, lane);
       atomicAdd(colsum + col + lane, v[0]);
     }
@@ -171,10 +162,12 @@ struct StoreEpi {
   long long ldd;
   int M, N;
   uint32_t flags;
+  int bn = BN;                   // tile width in columns (CTA-pair kernels choose it per launch, the others use BN)
   uint8_t* patch = nullptr;      // kPatchBytesPerCta of shared memory when the pipeline provides it (see above)
 
+  __device__ __forceinline__ int width() const { return bn; }
   __device__ __forceinline__ int a_row0(const TileCoord& t) const { return t.m * BM; }
-  __device__ __forceinline__ int b_row0(const TileCoord& t) const { return t.n * BN; }
+  __device__ __forceinline__ int b_row0(const TileCoord& t) const { return t.n * bn; }
   __device__ __forceinline__ void attach_smem(uint8_t*) {}
   __device__ __forceinline__ void attach_patch(uint8_t* p) { patch = p; }
   __device__ __forceinline__ void tile_begin(const TileCoord&) {}
@@ -224,7 +217,7 @@ struct StoreEpi {
   }
 
   __device__ __forceinline__ void strip(const TileCoord& t, int row_in_tile, int col_in_tile, uint32_t* r) {
-    const int row = t.m * BM + row_in_tile, col = t.n * BN + col_in_tile;
+    const int row = t.m * BM + row_in_tile, col = t.n * bn + col_in_tile;
     if (col >= N) return;
     float v[32];
 #pragma unroll

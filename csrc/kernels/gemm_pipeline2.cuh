@@ -15,6 +15,7 @@
 #include <utility>
 
 #include "gemm_pipeline.cuh"
+#include "launch.h"
 
 namespace pccl {
 namespace gemm2 {
@@ -40,7 +41,7 @@ struct Barriers {
   uint64_t tmem_full[2];        // per CTA: accumulator ready
   uint64_t tmem_empty[2];       // used in the leader: both CTAs' epilogues have drained the accumulator
   uint64_t drain;
-  uint64_t sched_full[SCHED_SLOTS];    // per CTA: the slot holds the tile index of iteration it (it % SCHED_SLOTS)
+  uint64_t sched_full[SCHED_SLOTS];    // per CTA: the slot holds the tile index of iteration it ((it - 1) % SCHED_SLOTS; the first tile is static)
   uint64_t sched_empty[SCHED_SLOTS];   // used in the leader: every role of both CTAs has read the slot
   uint64_t inbox_full[SCHED_SLOTS];    // used in the peer: the leader has stored the index into `inbox`
   int32_t sched_tile[SCHED_SLOTS];     // per CTA: tile index, or -1 for "no more tiles"; written by this CTA's producer
@@ -59,6 +60,11 @@ static_assert(sizeof(Barriers) <= BAR_BYTES, "barriers overrun their area");
 // kernel was launched with SMEM_BYTES of this header and the epilogue's own staging, if any, does not live there).
 template <class E, class = void> struct HasPatch : std::false_type {};
 template <class E> struct HasPatch<E, std::void_t<decltype(std::declval<E&>().attach_patch(nullptr))>> : std::true_type {};
+// An epilogue with `int width()` runs the whole problem on tiles of that many columns (a multiple of 32, at most BN): the MMA
+// is issued with N = width and each CTA loads width / 2 rows of B (rounded up to whole 64-column boxes where B is MN-major).
+// The launch picks the width so that the tiles fill the last round of CTA pairs (gemm_tc05.cu: pickTileN).
+template <class E, class = void> struct HasWidth : std::false_type {};
+template <class E> struct HasWidth<E, std::void_t<decltype(std::declval<const E&>().width())>> : std::true_type {};
 template <class E, class = void> struct HasVarN : std::false_type {};
 template <class E> struct HasVarN<E, std::void_t<decltype(E::kVarN)>> : std::true_type {};
 
@@ -88,6 +94,9 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
   const bool leader = cta == 0;
   const int num_kb = (K + BK - 1) / BK;
   volatile uint32_t* abort = &bar->abort;
+  int width = BN;
+  if constexpr (HasWidth<Epi>::value) width = epi.width();
+  const int b_boxes = B_MN ? (width / 2 + 63) / 64 : 1;        // MN-major B: 64-column boxes per CTA and k-block
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NSTAGES; ++s) {
@@ -121,6 +130,8 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = bar->tmem_base;
+  dev::pdl_launch();
+  dev::pdl_wait();                    // nothing above touched global memory
   epi.attach_smem(smem + NSTAGES * STAGE_BYTES + BAR_BYTES);
   if constexpr (HasPatch<Epi>::value && NSTAGES == STAGES) epi.attach_patch(smem + NSTAGES * STAGE_BYTES + BAR_BYTES);
 
@@ -128,8 +139,9 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
   // of a warp call this together and lane 0 releases the slot.  Returns 1 (tile), 0 (end of the list) or -1 (gave up).
   auto ring_tile = [&](int it, TileCoord* t, bool warp_wide) -> int {
     if constexpr (DYN) {
-      const int q = it & (SCHED_SLOTS - 1);
-      if (!tc::mbar_wait(&bar->sched_full[q], (it / SCHED_SLOTS) & 1, abort)) return -1;     // published inside this CTA
+      if (it == 0) return sched.at(static_cast<int>(blockIdx.x >> 1), t) ? 1 : 0;
+      const int q = (it - 1) & (SCHED_SLOTS - 1);
+      if (!tc::mbar_wait(&bar->sched_full[q], ((it - 1) / SCHED_SLOTS) & 1, abort)) return -1;     // published inside this CTA
       const int32_t v = *reinterpret_cast<volatile int32_t*>(&bar->sched_tile[q]);
       if (warp_wide) __syncwarp();
       // the slot goes back to the leader; the zero that is added to the address is computed from the value read (in a
@@ -153,9 +165,10 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
       uint32_t phase = 0;
       bool ok = true;
       TileCoord t;
-      // dynamic scheduling, leader: the index for the next iteration is drawn one iteration ahead, so the atomic's latency
-      // hides behind this tile's loads.  Every producer draws exactly one index past the end; whoever draws the very last
-      // one of the launch (total + pairs - 1) puts the counter back to zero for the next launch on this stream.
+      // dynamic scheduling: a pair's first tile is its own index, so no load waits for an atomic; the leader draws the index
+      // of the next iteration one iteration ahead, so the atomic's latency hides behind this tile's loads.  Every pair draws
+      // exactly one index past the end: `total` draws in all, and whoever makes the last of them puts the counter back to
+      // zero for the next launch on this stream.
       uint32_t drawn = 0;
       const uint32_t n_pairs = gridDim.x >> 1;
       if constexpr (DYN) {
@@ -163,12 +176,14 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
       }
       for (int it = 0; ok; ++it) {
         if constexpr (DYN) {
-          if (leader) {
-            const int q = it & (SCHED_SLOTS - 1);
-            if (!tc::mbar_wait(&bar->sched_empty[q], ((it / SCHED_SLOTS) & 1) ^ 1, abort)) { ok = false; break; }   // no data comes with it
+          if (it == 0) {
+            if (!sched.at(static_cast<int>(blockIdx.x >> 1), &t)) break;
+          } else if (leader) {
+            const int q = (it - 1) & (SCHED_SLOTS - 1);
+            if (!tc::mbar_wait(&bar->sched_empty[q], (((it - 1) / SCHED_SLOTS) & 1) ^ 1, abort)) { ok = false; break; }   // no data comes with it
             const uint32_t cur = drawn;        // drawn one iteration ago: nothing has waited for the atomic until here
-            if (cur == sched.total + n_pairs - 1) atomicExch(sched.counter, 0u);
-            const int32_t v = cur < sched.total ? static_cast<int32_t>(cur) : -1;
+            if (cur == sched.total - 1) atomicExch(sched.counter, 0u);
+            const int32_t v = cur + n_pairs < sched.total ? static_cast<int32_t>(cur + n_pairs) : -1;
             bar->sched_tile[q] = v;
             tc::mbar_arrive(&bar->sched_full[q]);                                          // this CTA's readers
             tc::st_shared_cluster_u32(tc::mapa(tc::smem_u32(&bar->inbox[q]), 1), static_cast<uint32_t>(v));
@@ -177,8 +192,8 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
             drawn = atomicAdd(sched.counter, 1u);
           } else {
             // the peer's producer: index out of the inbox (cluster-scope acquire), into this CTA's slot for its epilogue warps
-            const int q = it & (SCHED_SLOTS - 1);
-            if (!tc::mbar_wait_cluster(&bar->inbox_full[q], (it / SCHED_SLOTS) & 1, abort)) { ok = false; break; }
+            const int q = (it - 1) & (SCHED_SLOTS - 1);
+            if (!tc::mbar_wait_cluster(&bar->inbox_full[q], ((it - 1) / SCHED_SLOTS) & 1, abort)) { ok = false; break; }
             const int32_t v = *reinterpret_cast<volatile int32_t*>(&bar->inbox[q]);
             bar->sched_tile[q] = v;
             tc::mbar_arrive(&bar->sched_full[q]);
@@ -196,7 +211,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         const int row0 = epi.a_row0(t), col0 = epi.b_row0(t);        // already offset by this CTA's half
         const CUtensorMap* const tmA_t = NPROB > 1 ? tmA + t.extra : tmA;
         const CUtensorMap* tmB_t = NPROB > 1 ? tmB + t.extra : tmB;
-        uint32_t stage_tx = 2 * STAGE_BYTES;
+        uint32_t stage_tx = 2u * (A_BYTES + static_cast<uint32_t>(B_MN ? b_boxes * 64 : width / 2) * (BK * 2));
         if constexpr (HasVarN<Epi>::value) {
           const int sel = epi.b_box(t);
           tmB_t = tmB + sel;
@@ -218,8 +233,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
           if constexpr (!B_MN) {
             tc::tma_load_2d_pair(sb, tmB_t, full_leader, k0, col0);
           } else {
-#pragma unroll
-            for (int j = 0; j < HALF_N / 64; ++j) tc::tma_load_2d_pair(sb + j * (64 * BK * 2), tmB_t, full_leader, col0 + j * 64, k0);
+            for (int j = 0; j < b_boxes; ++j) tc::tma_load_2d_pair(sb + j * (64 * BK * 2), tmB_t, full_leader, col0 + j * 64, k0);
           }
           if (++stage == NSTAGES) { stage = 0; phase ^= 1; }
         }
@@ -229,7 +243,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
     if (leader && tc::elect_one()) {
-      constexpr uint32_t idesc = tc::make_idesc(1, 1, A_MN, B_MN, PAIR_M, BN);
+      const uint32_t idesc = tc::make_idesc(1, 1, A_MN, B_MN, PAIR_M, static_cast<uint32_t>(width));
       constexpr uint32_t A_LBO = A_MN ? 64 * BK * 2 : 16, B_LBO = B_MN ? 64 * BK * 2 : 16, SBO = 1024;
       constexpr uint32_t A_KSTEP = A_MN ? (UMMA_K / 8) * 1024 : UMMA_K * 2;
       constexpr uint32_t B_KSTEP = B_MN ? (UMMA_K / 8) * 1024 : UMMA_K * 2;
@@ -282,7 +296,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
       tc::tc_fence_after();
       const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
       epi.tile_begin(t);
-      int n_strips = BN / 32;
+      int n_strips = width / 32;
       if constexpr (HasVarN<Epi>::value) n_strips = (epi.tile_n(t) + 31) / 32;
       // with eight epilogue warps the two warps of a lane quarter take the lower and the upper half of the strips
       constexpr int kSplit = EPI_WARPS / 4;
@@ -323,7 +337,11 @@ struct PairEpi {
   Epi& e;
   int cta;
   __device__ __forceinline__ int a_row0(const TileCoord& t) const { return e.a_row0(half_tile(t, cta)); }
-  __device__ __forceinline__ int b_row0(const TileCoord& t) const { return e.b_row0(half_tile(t, cta)) + cta * HALF_N; }
+  __device__ __forceinline__ int b_row0(const TileCoord& t) const { return e.b_row0(half_tile(t, cta)) + cta * (width() / 2); }
+  __device__ __forceinline__ int width() const {
+    if constexpr (HasWidth<Epi>::value) return e.width();
+    else return BN;
+  }
   __device__ __forceinline__ void attach_smem(uint8_t* p) { e.attach_smem(p); }
   __device__ __forceinline__ void attach_patch(uint8_t* p) {
     if constexpr (HasPatch<Epi>::value) e.attach_patch(p);

@@ -14,6 +14,7 @@
 #include "gemm_epilogue.cuh"
 #include "gemm_pipeline.cuh"
 #include "gemm_pipeline2.cuh"
+#include "launch.h"
 #include "tensormap.h"
 
 namespace pccl {
@@ -53,7 +54,7 @@ template <bool A_MN, bool B_MN, class Epi = StoreEpi, bool DYN = false>
 __global__ void __launch_bounds__(gemm2::NUM_THREADS_WIDE, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Epi epi, int K,
                       uint32_t* status, uint32_t* counter) {
-  const int tiles_m = (epi.M + gemm2::PAIR_M - 1) / gemm2::PAIR_M, tiles_n = (epi.N + gemm2::BN - 1) / gemm2::BN;
+  const int tiles_m = (epi.M + gemm2::PAIR_M - 1) / gemm2::PAIR_M, tiles_n = (epi.N + epi.bn - 1) / epi.bn;
   NoGate gate;
   const int cta = static_cast<int>(tc::cluster_ctarank());
   gemm2::PairEpi<Epi> pe{epi, cta};
@@ -93,6 +94,7 @@ struct DualSched {
 struct DualEpi {
   static constexpr bool kRow128 = false;
   StoreEpi e[2];
+  __device__ __forceinline__ int width() const { return e[0].bn; }        // one width for both problems
   __device__ __forceinline__ int a_row0(const TileCoord& t) const { return e[t.extra].a_row0(t); }
   __device__ __forceinline__ int b_row0(const TileCoord& t) const { return e[t.extra].b_row0(t); }
   __device__ __forceinline__ void attach_smem(uint8_t*) {}
@@ -106,7 +108,7 @@ template <bool A_MN, bool B_MN, bool DYN>
 __global__ void __launch_bounds__(gemm2::NUM_THREADS_WIDE, 1)
 gemm_bf16_pair_dual_kernel(const __grid_constant__ DualMaps maps, DualEpi epi, int K, uint32_t* status, uint32_t* counter) {
   DualSched sched{{(epi.e[0].M + gemm2::PAIR_M - 1) / gemm2::PAIR_M, (epi.e[1].M + gemm2::PAIR_M - 1) / gemm2::PAIR_M},
-                  {(epi.e[0].N + gemm2::BN - 1) / gemm2::BN, (epi.e[1].N + gemm2::BN - 1) / gemm2::BN},
+                  {(epi.e[0].N + epi.e[0].bn - 1) / epi.e[0].bn, (epi.e[1].N + epi.e[1].bn - 1) / epi.e[1].bn},
                   static_cast<int>(blockIdx.x >> 1), static_cast<int>(gridDim.x >> 1), counter, 0u};
   sched.total = static_cast<uint32_t>(sched.tiles_m[0] * sched.tiles_n[0] + sched.tiles_m[1] * sched.tiles_n[1]);
   NoGate gate;
@@ -152,57 +154,44 @@ uint32_t* tileCounterFor(cudaStream_t stream) {
   return p;
 }
 
-template <class Kern>
-int setPairSmem(Kern kern, bool* done) {
-  if (*done) return 0;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm2::SMEM_BYTES);
-  if (e != cudaSuccess) return static_cast<int>(e);
-  *done = true;
-  return 0;
+// Tile width of a CTA-pair launch: 256 columns unless a narrower tile fills the last round of pairs better.  A round of
+// narrower tiles is not cheaper in proportion -- every k-block still loads the pair's 256 rows of A, and L2 -> SM is what
+// bounds it -- so the candidates are weighed with the measured time of a full round relative to a round of 256-wide tiles
+// (16384 x 8192 x 2048 and 16384 x 2048 x 2048, one B200: 12.4 us at 256, 11.3 / 10.0 / 9.1 / 7.9 / 7.0 / 6.7 / 6.0 us at
+// 224 ... 32).  Measured both ways (us, 256 wide -> chosen): 1531 x 2048 x 8192 53 -> 47 (48 tiles on 74 pairs -> 66),
+// 2331 x 768 x 3072 28.6 -> 22.6, 8192 x 3584 x 8192 328 -> 316 (448 tiles = 6.05 rounds -> 512 = 6.9); 1531 x 6144 x 2048
+// (144 tiles, 1.95 rounds) stays at 256: 40 against 44 at 192.  Two problems (gemmBf16Dual) share one width.
+int pickTileN(int tiles_m0, int n0, int tiles_m1, int n1, int pairs) {
+  static const struct { int bn; float round; } kWidths[] = {{256, 1.f}, {224, .91f}, {192, .80f}, {160, .725f},
+                                                            {128, .62f}, {96, .56f}, {64, .53f}, {32, .48f}};
+  if (pairs < 1) pairs = 1;
+  int best = 256;
+  float best_cost = 0.f;
+  for (const auto& w : kWidths) {
+    const long long tiles = static_cast<long long>(tiles_m0) * ((n0 + w.bn - 1) / w.bn) + static_cast<long long>(tiles_m1) * ((n1 + w.bn - 1) / w.bn);
+    const float cost = static_cast<float>((tiles + pairs - 1) / pairs) * w.round;
+    if (w.bn == 256 || cost < best_cost * 0.999f) { best = w.bn; best_cost = cost; }
+  }
+  return best;
+}
+
+// One CTA pair per cluster, allowed to start before the previous kernel of the stream has ended (launch.h).
+template <class... KArgs, class... Args>
+int launchPairKernel(void (*kern)(KArgs...), int grid, cudaStream_t stream, bool* attr_set, Args... args) {
+  if (!*attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm2::SMEM_BYTES);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    *attr_set = true;
+  }
+  return static_cast<int>(launchOverlapped(kern, dim3(grid), dim3(gemm2::NUM_THREADS_WIDE), gemm2::SMEM_BYTES, stream, 2, args...));
 }
 
 template <bool A_MN, bool B_MN, class Epi = StoreEpi>
 int launchPair(const CUtensorMap& ta, const CUtensorMap& tb, const Epi& epi, int K, int grid, uint32_t* status, cudaStream_t stream) {
   static bool attr_set = false, attr_set_dyn = false;
   uint32_t* counter = tileCounterFor(stream);
-  if (counter) {
-    auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, Epi, true>;
-    if (int e = setPairSmem(kern, &attr_set_dyn)) return e;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(gemm2::NUM_THREADS_WIDE);
-    cfg.dynamicSmemBytes = gemm2::SMEM_BYTES;
-    cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int Kc = K;
-    return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, ta, tb, epi, Kc, status, counter));
-  }
-  auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, Epi, false>;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm2::SMEM_BYTES);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    attr_set = true;
-  }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(gemm2::NUM_THREADS_WIDE);
-  cfg.dynamicSmemBytes = gemm2::SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  int Kc = K;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, ta, tb, epi, Kc, status, static_cast<uint32_t*>(nullptr)));
+  return counter ? launchPairKernel(gemm_bf16_pair_kernel<A_MN, B_MN, Epi, true>, grid, stream, &attr_set_dyn, ta, tb, epi, K, status, counter)
+                 : launchPairKernel(gemm_bf16_pair_kernel<A_MN, B_MN, Epi, false>, grid, stream, &attr_set, ta, tb, epi, K, status, counter);
 }
 
 template <bool A_MN, bool B_MN>
@@ -250,27 +239,29 @@ int gemmBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, in
     return static_cast<int>(cudaErrorInvalidValue);
   }
   const bool a_mn = flags & GEMM_A_MN, b_mn = flags & GEMM_B_MN;
-  CUtensorMap ta, tb;
-  // K-major: dims {K, rows}; MN-major: dims {rows, K}
-  if (!a_mn ? !makeTensorMap2D(&ta, A, TM_BF16, K, M, lda, BK, BM, &g_err) : !makeTensorMap2D(&ta, A, TM_BF16, M, K, lda, 64, BK, &g_err))
-    return static_cast<int>(cudaErrorInvalidValue);
-  if (!b_mn ? !makeTensorMap2D(&tb, B, TM_BF16, K, N, ldb, BK, BN, &g_err) : !makeTensorMap2D(&tb, B, TM_BF16, N, K, ldb, 64, BK, &g_err))
-    return static_cast<int>(cudaErrorInvalidValue);
+  // tensor maps: a K-major operand has dims {K, rows}, an MN-major one {rows, K}
   StoreEpi epi{D, D2, static_cast<const __nv_bfloat16*>(bias), ldd, M, N, flags};
   if (flags & GEMM_PAIR) {
-    // per-CTA boxes: 128 rows of A and 128 rows (half of N) of B
+    int n_sm2 = deviceSmCount();
+    if (sms > 0 && sms < n_sm2) n_sm2 = sms;
+    const int bn = pickTileN((M + 255) / 256, N, 0, 0, n_sm2 / 2);
+    epi.bn = bn;
+    // per-CTA boxes: 128 rows of A and half of the tile's columns of B
     CUtensorMap pa, pb;
     if (!a_mn ? !makeTensorMap2D(&pa, A, TM_BF16, K, M, lda, BK, 128, &g_err) : !makeTensorMap2D(&pa, A, TM_BF16, M, K, lda, 64, BK, &g_err))
       return static_cast<int>(cudaErrorInvalidValue);
-    if (!b_mn ? !makeTensorMap2D(&pb, B, TM_BF16, K, N, ldb, BK, 128, &g_err) : !makeTensorMap2D(&pb, B, TM_BF16, N, K, ldb, 64, BK, &g_err))
+    if (!b_mn ? !makeTensorMap2D(&pb, B, TM_BF16, K, N, ldb, BK, bn / 2, &g_err) : !makeTensorMap2D(&pb, B, TM_BF16, N, K, ldb, 64, BK, &g_err))
       return static_cast<int>(cudaErrorInvalidValue);
-    int pair_tiles = ((M + 255) / 256) * ((N + 255) / 256);
-    int n_sm2 = deviceSmCount();
-    if (sms > 0 && sms < n_sm2) n_sm2 = sms;
+    int pair_tiles = ((M + 255) / 256) * ((N + bn - 1) / bn);
     int grid2 = 2 * (pair_tiles < n_sm2 / 2 ? pair_tiles : n_sm2 / 2);
     if (a_mn) return b_mn ? launchPair<true, true>(pa, pb, epi, K, grid2, status, stream) : launchPair<true, false>(pa, pb, epi, K, grid2, status, stream);
     return b_mn ? launchPair<false, true>(pa, pb, epi, K, grid2, status, stream) : launchPair<false, false>(pa, pb, epi, K, grid2, status, stream);
   }
+  CUtensorMap ta, tb;
+  if (!a_mn ? !makeTensorMap2D(&ta, A, TM_BF16, K, M, lda, BK, BM, &g_err) : !makeTensorMap2D(&ta, A, TM_BF16, M, K, lda, 64, BK, &g_err))
+    return static_cast<int>(cudaErrorInvalidValue);
+  if (!b_mn ? !makeTensorMap2D(&tb, B, TM_BF16, K, N, ldb, BK, BN, &g_err) : !makeTensorMap2D(&tb, B, TM_BF16, N, K, ldb, 64, BK, &g_err))
+    return static_cast<int>(cudaErrorInvalidValue);
   int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   int n_sm = deviceSmCount();
   if (sms > 0 && sms < n_sm) n_sm = sms;
@@ -282,9 +273,9 @@ int gemmBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, in
 int gemmBf16Dgelu(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, int64_t ldd, const void* pre, float* colsum,
                   int M, int N, int K, uint32_t flags, int sms, uint32_t* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if ((lda | ldb | ldd) % 8 || M % 256 || N % 256 ||
+  if ((lda | ldb | ldd) % 8 || N % 32 ||
       (reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(D) | reinterpret_cast<uintptr_t>(pre)) % 16) {
-    g_err = "gemmBf16Dgelu: M and N must be multiples of 256, strides multiples of 8 elements, pointers 16-byte aligned";
+    g_err = "gemmBf16Dgelu: N must be a multiple of 32, strides multiples of 8 elements, pointers 16-byte aligned";
     return static_cast<int>(cudaErrorInvalidValue);
   }
   const bool a_mn = flags & GEMM_A_MN, b_mn = flags & GEMM_B_MN;
@@ -292,14 +283,15 @@ int gemmBf16Dgelu(const void* A, int64_t lda, const void* B, int64_t ldb, void* 
     g_err = "gemmBf16Dgelu: an MN-major A operand is not built";
     return static_cast<int>(cudaErrorInvalidValue);
   }
-  CUtensorMap pa, pb;
-  if (!makeTensorMap2D(&pa, A, TM_BF16, K, M, lda, BK, 128, &g_err)) return static_cast<int>(cudaErrorInvalidValue);
-  if (!b_mn ? !makeTensorMap2D(&pb, B, TM_BF16, K, N, ldb, BK, 128, &g_err) : !makeTensorMap2D(&pb, B, TM_BF16, N, K, ldb, 64, BK, &g_err))
-    return static_cast<int>(cudaErrorInvalidValue);
-  DgeluEpi epi{static_cast<__nv_bfloat16*>(D), static_cast<const __nv_bfloat16*>(pre), colsum, ldd, M, N};
-  int pair_tiles = (M / 256) * (N / 256);
   int n_sm = deviceSmCount();
   if (sms > 0 && sms < n_sm) n_sm = sms;
+  const int bn = pickTileN((M + 255) / 256, N, 0, 0, n_sm / 2);
+  CUtensorMap pa, pb;
+  if (!makeTensorMap2D(&pa, A, TM_BF16, K, M, lda, BK, 128, &g_err)) return static_cast<int>(cudaErrorInvalidValue);
+  if (!b_mn ? !makeTensorMap2D(&pb, B, TM_BF16, K, N, ldb, BK, bn / 2, &g_err) : !makeTensorMap2D(&pb, B, TM_BF16, N, K, ldb, 64, BK, &g_err))
+    return static_cast<int>(cudaErrorInvalidValue);
+  DgeluEpi epi{static_cast<__nv_bfloat16*>(D), static_cast<const __nv_bfloat16*>(pre), colsum, ldd, M, N, bn};
+  int pair_tiles = ((M + 255) / 256) * ((N + bn - 1) / bn);
   int grid = 2 * (pair_tiles < n_sm / 2 ? pair_tiles : n_sm / 2);
   return b_mn ? launchPair<false, true, DgeluEpi>(pa, pb, epi, K, grid, status, stream)
               : launchPair<false, false, DgeluEpi>(pa, pb, epi, K, grid, status, stream);
@@ -309,6 +301,9 @@ int gemmBf16Dual(const GemmProblem& p0, const GemmProblem& p1, int K, uint32_t f
   const GemmProblem* ps[2] = {&p0, &p1};
   const bool a_mn = flags & GEMM_A_MN, b_mn = flags & GEMM_B_MN;
   if (K <= 0) return 0;
+  int n_sm = deviceSmCount();
+  if (sms > 0 && sms < n_sm) n_sm = sms;
+  const int bn = pickTileN((p0.M + 255) / 256, p0.N, (p1.M + 255) / 256, p1.N, n_sm / 2);
   DualMaps maps;
   DualEpi epi;
   for (int q = 0; q < 2; ++q) {
@@ -320,34 +315,16 @@ int gemmBf16Dual(const GemmProblem& p0, const GemmProblem& p1, int K, uint32_t f
     }
     if (!a_mn ? !makeTensorMap2D(&maps.a[q], p.A, TM_BF16, K, p.M, p.lda, BK, 128, &g_err) : !makeTensorMap2D(&maps.a[q], p.A, TM_BF16, p.M, K, p.lda, 64, BK, &g_err))
       return static_cast<int>(cudaErrorInvalidValue);
-    if (!b_mn ? !makeTensorMap2D(&maps.b[q], p.B, TM_BF16, K, p.N, p.ldb, BK, 128, &g_err) : !makeTensorMap2D(&maps.b[q], p.B, TM_BF16, p.N, K, p.ldb, 64, BK, &g_err))
+    if (!b_mn ? !makeTensorMap2D(&maps.b[q], p.B, TM_BF16, K, p.N, p.ldb, BK, bn / 2, &g_err) : !makeTensorMap2D(&maps.b[q], p.B, TM_BF16, p.N, K, p.ldb, 64, BK, &g_err))
       return static_cast<int>(cudaErrorInvalidValue);
-    epi.e[q] = StoreEpi{p.D, nullptr, nullptr, p.ldd, p.M, p.N, (flags & GEMM_OUT_F32) | (p.accumulate ? GEMM_ACCUMULATE : 0u)};
+    epi.e[q] = StoreEpi{p.D, nullptr, nullptr, p.ldd, p.M, p.N, (flags & GEMM_OUT_F32) | (p.accumulate ? GEMM_ACCUMULATE : 0u), bn};
   }
-  const long long tiles = static_cast<long long>((p0.M + 255) / 256) * ((p0.N + 255) / 256) + static_cast<long long>((p1.M + 255) / 256) * ((p1.N + 255) / 256);
-  int n_sm = deviceSmCount();
-  if (sms > 0 && sms < n_sm) n_sm = sms;
+  const long long tiles = static_cast<long long>((p0.M + 255) / 256) * ((p0.N + bn - 1) / bn) + static_cast<long long>((p1.M + 255) / 256) * ((p1.N + bn - 1) / bn);
   const int grid = 2 * static_cast<int>(tiles < n_sm / 2 ? tiles : n_sm / 2);
   static bool attr_set[8] = {false, false, false, false, false, false, false, false};   // per kernel: the instantiations share one function type
   uint32_t* counter = tileCounterFor(stream);
   bool& attr = attr_set[(counter ? 4 : 0) | (a_mn ? 2 : 0) | (b_mn ? 1 : 0)];
-  auto go = [&](auto kern) {
-    if (int e = setPairSmem(kern, &attr)) return e;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(gemm2::NUM_THREADS_WIDE);
-    cfg.dynamicSmemBytes = gemm2::SMEM_BYTES;
-    cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int Kc = K;
-    return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, maps, epi, Kc, status, counter));
-  };
+  auto go = [&](auto kern) { return launchPairKernel(kern, grid, stream, &attr, maps, epi, K, status, counter); };
   if (counter) {
     if (a_mn) return b_mn ? go(gemm_bf16_pair_dual_kernel<true, true, true>) : go(gemm_bf16_pair_dual_kernel<true, false, true>);
     return b_mn ? go(gemm_bf16_pair_dual_kernel<false, true, true>) : go(gemm_bf16_pair_dual_kernel<false, false, true>);

@@ -152,7 +152,7 @@ class _MlpFn(torch.autograd.Function):
         x2, w1, b1, w2, b2, pre, act = ctx.saved_tensors
         dz2 = _as_operand(dz)
         rows, n1 = pre.shape
-        if rows % 256 == 0 and n1 % 256 == 0:
+        if n1 % 32 == 0:
             sums = torch.zeros(n1, dtype=torch.float32, device=pre.device) if b1 is not None else None
             dy2 = gemm_dgelu(dz2, w2, pre, b_t=True, colsum=sums)
             db1 = _deliver_bias(b1, sums.to(b1.dtype)) if b1 is not None else None

@@ -62,7 +62,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     """``out = op(a) @ op(b)`` with ``op(a) = a.T if a_t else a`` (a: [M,K] or [K,M]) and
     ``op(b) = b if b_t else b.T`` (b: [N,K], or [K,N] when ``b_t``).  So the default is the linear
     layer form ``a @ b.T``.  ``bias`` (bf16 [N]) is added; ``gelu_out`` receives gelu_tanh(out).
-    ``pair`` selects the CTA-pair kernel (cta_group::2, 256 x 256 tiles); default from PCCL_GEMM_PAIR.
+    ``pair`` selects the CTA-pair kernel (cta_group::2, tiles of 256 rows); default from PCCL_GEMM_PAIR.
     ``residual`` (bf16, out's shape and strides) is added in the epilogue: ``out = a @ b.T + bias + residual``.
     ``row_stores`` turns the epilogue's coalescing patch off (comparison runs)."""
     _check(a, "a")
@@ -142,7 +142,7 @@ def gemm_dgelu(a: torch.Tensor, b: torch.Tensor, pre: torch.Tensor, *, b_t: bool
     """``out = (a @ op(b)) * gelu_tanh'(pre)`` in one kernel (the GELU derivative is applied in the GEMM epilogue), and,
     when ``colsum`` (fp32 [N], zeroed by the caller) is given, ``colsum += out.sum(0)``.  This is the step of an MLP's
     backward pass that turns the gradient of the second layer's input into the gradient of the first layer's output;
-    the column sums are the first layer's bias gradient.  M and N must be multiples of 256."""
+    the column sums are the first layer's bias gradient.  N must be a multiple of 32."""
     _check(a, "a")
     _check(b, "b")
     M, K = a.shape

@@ -166,6 +166,47 @@ def test_gemm_residual_epilogue_adds_the_residual_stream():
         assert (out.float() - ref).abs().max().item() <= 2e-2 * max(1.0, ref.abs().max().item())
 
 
+# The CTA-pair kernel picks its tile width per launch: these sizes select 64, 64, 192, 128, 224, 160 and 256 columns, with
+# rows and columns that end inside a tile and (1416, 2056, 3000) inside a 32-column strip.
+@pytest.mark.parametrize("M,N,K", [(257, 40, 72), (300, 1416, 200), (1531, 2056, 136), (2331, 776, 264), (4096, 3576, 128), (1999, 1416, 328), (1531, 6152, 64)])
+@pytest.mark.parametrize("a_t,b_t", [(False, False), (False, True), (True, True)])
+def test_cta_pair_gemm_tile_widths(M, N, K, a_t, b_t):
+    from pccl_b200.ops import gemm, check_status
+    if a_t:
+        M = (M + 7) // 8 * 8
+    a = _rand((K, M) if a_t else (M, K), 61)
+    b = _rand((K, N) if b_t else (N, K), 62)
+    ref = _ref(a, b, a_t, b_t)
+    out32 = gemm(a, b, a_t=a_t, b_t=b_t, out_dtype=torch.float32, pair=True)
+    bias = _rand((N,), 63)
+    act = torch.full((M, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    pre = torch.empty_like(act)
+    gemm(a, b, a_t=a_t, b_t=b_t, out=pre, bias=bias, gelu_out=act, pair=True)
+    check_status("pair gemm widths")
+    # fp32 sums of K exact products in another order: K * 2^-24 of the absolute sum, far below 1e-3 of the largest result
+    assert (out32 - ref).abs().max().item() <= 1e-3 * max(1.0, ref.abs().max().item())
+    full = ref + bias.float()
+    assert (pre.float() - full).abs().max().item() <= 2 ** -8 * full.abs().max().item()           # one bf16 rounding
+    gelu = torch.nn.functional.gelu(full, approximate="tanh")
+    assert ((act.float() - gelu).abs() <= 0.01 + 0.01 * gelu.abs()).all()                            # hardware tanh, then bf16
+
+
+@pytest.mark.parametrize("M", [1, 40, 1531])
+def test_gemm_dgelu_ragged_rows(M):
+    from pccl_b200.ops import check_status
+    from pccl_b200.ops.gemm import gemm_dgelu
+    N, K = 1056, 136
+    a, b, pre = _rand((M, K), 64), _rand((K, N), 65, 0.05), _rand((M, N), 66, 1.5)
+    sums = torch.zeros(N, dtype=torch.float32, device="cuda")
+    out = gemm_dgelu(a, b, pre, b_t=True, colsum=sums)
+    check_status("gemm dgelu ragged")
+    x = pre.float().requires_grad_(True)
+    torch.nn.functional.gelu(x, approximate="tanh").backward(a.float() @ b.float())
+    ref = x.grad
+    assert (out.float() - ref).abs().max().item() <= 2e-2 * max(1.0, ref.abs().max().item())
+    assert (sums - ref.sum(0)).abs().max().item() <= 2e-2 * max(1.0, ref.sum(0).abs().max().item())
+
+
 @pytest.mark.parametrize("b_t", [True, False])
 def test_gemm_dgelu_epilogue_and_column_sums(b_t):
     """(a @ op(b)) * gelu_tanh'(pre) with the column sums of the result, against fp32 PyTorch."""

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <string>
 
 #include "api.h"
 
@@ -21,6 +22,7 @@ enum GemmFlags : uint32_t {
   GEMM_ADD_D2 = 1u << 8,      // D = A*B^T (+bias) + D2 (bf16, D's layout, read only): a residual connection; not with GEMM_GELU
   GEMM_ROW_STORES = 1u << 9,  // epilogue stores straight from the accumulator layout (a row per lane) instead of through the
                               // coalescing patch: for comparison runs
+  GEMM_SKINNY = 1u << 10,     // few rows (M <= 256, A K-major): weights on the tile's M side, K split over a cluster (gemm_skinny.cu)
 };
 
 // D[M,N] (ldd) = A * B^T.  K-major operands: A is [M,K] with row stride lda, B is [N,K] with row
@@ -30,6 +32,9 @@ enum GemmFlags : uint32_t {
 // null) receives ST_TIMEOUT if a pipeline wait runs out.
 int gemmBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, int64_t ldd, int M, int N, int K,
              uint32_t flags, const void* bias, void* D2, int sms, uint32_t* status, cudaStream_t stream);
+
+int gemmSkinnyBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, int64_t ldd, int M, int N, int K, uint32_t flags,
+                   const void* bias, void* D2, uint32_t* status, cudaStream_t stream, std::string* err);   // gemmBf16 with GEMM_SKINNY
 
 // D[M,N] = (A * B^T) .* gelu_tanh'(pre[M,N]) in bf16, and colsum[n] += sum_m D[m,n] (fp32, may be null): the
 // backward of "linear -> GELU -> linear" between the second layer's input gradient and the first layer's output

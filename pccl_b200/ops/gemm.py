@@ -15,6 +15,8 @@ from .._native import C
 import os
 
 _PAIR_DEFAULT = os.environ.get("PCCL_GEMM_PAIR", "1") != "0"      # CTA pairs unless switched off
+# up to this many rows (of a K-major a) the weights are streamed by the few-row kernel (csrc/kernels/gemm_skinny.cu says why)
+_SKINNY_ROWS = 128
 _status: Dict[int, torch.Tensor] = {}
 _launches = 0
 
@@ -62,7 +64,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     """``out = op(a) @ op(b)`` with ``op(a) = a.T if a_t else a`` (a: [M,K] or [K,M]) and
     ``op(b) = b if b_t else b.T`` (b: [N,K], or [K,N] when ``b_t``).  So the default is the linear
     layer form ``a @ b.T``.  ``bias`` (bf16 [N]) is added; ``gelu_out`` receives gelu_tanh(out).
-    ``pair`` selects the CTA-pair kernel (cta_group::2, tiles of 256 rows); default from PCCL_GEMM_PAIR.
+    ``pair`` selects the CTA-pair kernel (cta_group::2, tiles of 256 rows); default: up to 128 rows of a K-major ``a`` take
+    the few-row kernel, more the CTA pairs (PCCL_GEMM_PAIR).
     ``residual`` (bf16, out's shape and strides) is added in the epilogue: ``out = a @ b.T + bias + residual``.
     ``row_stores`` turns the epilogue's coalescing patch off (comparison runs)."""
     _check(a, "a")
@@ -86,7 +89,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
         flags |= C.GEMM_OUT_F32
     if accumulate:
         flags |= C.GEMM_ACCUMULATE
-    if (_PAIR_DEFAULT and M > 128) if pair is None else pair:
+    if pair is None and M <= _SKINNY_ROWS and not (a_t or sms or row_stores):
+        flags |= C.GEMM_SKINNY
+    elif (_PAIR_DEFAULT and M > 128) if pair is None else pair:
         flags |= C.GEMM_PAIR
     if row_stores:
         flags |= C.GEMM_ROW_STORES

@@ -207,6 +207,35 @@ def test_gemm_dgelu_ragged_rows(M):
     assert (sums - ref.sum(0)).abs().max().item() <= 2e-2 * max(1.0, ref.sum(0).abs().max().item())
 
 
+@pytest.mark.parametrize("M", [1, 15, 17, 33, 100, 128])
+@pytest.mark.parametrize("N,K", [(40, 72), (1001, 200), (512, 2048), (8200, 520)])
+@pytest.mark.parametrize("b_t", [False, True])
+def test_few_row_gemm(M, N, K, b_t):
+    """Weights on the tile's M side, K split over a cluster of 1, 4 or 8 CTAs, with every epilogue."""
+    from pccl_b200.ops import gemm, check_status
+    ld = (N + 7) // 8 * 8
+    a = _rand((M, K), 71)
+    b = _rand((K, ld), 72)[:, :N] if b_t else _rand((N, K), 72)
+    ref = _ref(a, b, False, b_t)
+    big = max(1.0, ref.abs().max().item())
+    acc = torch.ones((M, ld), dtype=torch.float32, device="cuda")[:, :N]
+    gemm(a, b, b_t=b_t, out=acc, accumulate=True)
+    bias, res = _rand((N,), 73), _rand((M, ld), 74)[:, :N]
+    act = torch.full((M, ld), 9.0, dtype=torch.bfloat16, device="cuda")
+    pre = torch.full((M, ld), 9.0, dtype=torch.bfloat16, device="cuda")
+    gemm(a, b, b_t=b_t, bias=bias, gelu_out=act[:, :N], out=pre[:, :N])
+    out = torch.empty((M, ld), dtype=torch.bfloat16, device="cuda")[:, :N]
+    gemm(a, b, b_t=b_t, bias=bias, residual=res, out=out)
+    check_status("few-row gemm")
+    assert (acc - ref - 1).abs().max().item() <= 1e-3 * big                   # fp32, sums in another order
+    full = ref + bias.float()
+    assert (pre[:, :N].float() - full).abs().max().item() <= 2 ** -8 * full.abs().max().item()      # one bf16 rounding
+    gelu = torch.nn.functional.gelu(full, approximate="tanh")
+    assert ((act[:, :N].float() - gelu).abs() <= 0.01 + 0.01 * gelu.abs()).all()
+    assert (out.float() - full - res.float()).abs().max().item() <= 2 ** -8 * (full + res.float()).abs().max().item()
+    assert (act[:, N:] == 9.0).all() and (pre[:, N:] == 9.0).all()             # nothing past the last column
+
+
 @pytest.mark.parametrize("b_t", [True, False])
 def test_gemm_dgelu_epilogue_and_column_sums(b_t):
     """(a @ op(b)) * gelu_tanh'(pre) with the column sums of the result, against fp32 PyTorch."""

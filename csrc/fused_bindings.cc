@@ -4,6 +4,7 @@
 
 #include <stdexcept>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "engine.h"
@@ -116,11 +117,24 @@ void bindFused(py::module_& m) {
                                reinterpret_cast<cudaStream_t>(stream)), "quant_fp8_blocks");
   });
   m.def("gemm_grouped", [](uint64_t a, int64_t lda, uint64_t b, int64_t ldb, uint64_t d, int64_t ldd, uint64_t row_off, int groups,
-                           int max_rows, int N, int K, uint32_t flags, int sms, uint64_t status, uint64_t stream) {
+                           int max_rows, int N, int K, uint32_t flags, int sms, uint64_t status, uint64_t stream, uint64_t d2) {
     check(gemmGroupedBf16(reinterpret_cast<const void*>(a), lda, reinterpret_cast<const void*>(b), ldb, reinterpret_cast<void*>(d), ldd,
-                          reinterpret_cast<const int*>(row_off), groups, max_rows, N, K, flags, sms,
+                          reinterpret_cast<const int*>(row_off), groups, max_rows, N, K, flags, reinterpret_cast<void*>(d2), sms,
                           reinterpret_cast<uint32_t*>(status), reinterpret_cast<cudaStream_t>(stream)), "gemm_grouped");
+  }, py::arg("a"), py::arg("lda"), py::arg("b"), py::arg("ldb"), py::arg("d"), py::arg("ldd"), py::arg("row_off"), py::arg("groups"),
+     py::arg("max_rows"), py::arg("N"), py::arg("K"), py::arg("flags"), py::arg("sms"), py::arg("status"), py::arg("stream"), py::arg("d2") = 0);
+  // problem: (a, lda, b, ldb, d, ldd, M, N)
+  using Problem = std::tuple<uint64_t, int64_t, uint64_t, int64_t, uint64_t, int64_t, int, int>;
+  m.def("gemm_grouped_wgrad", [](const Problem& p0, const Problem& p1, uint64_t row_off, int groups, int max_rows, uint64_t maps,
+                                 uint64_t status, uint64_t stream) {
+    auto problem = [](const Problem& p) {
+      return GemmProblem{reinterpret_cast<const void*>(std::get<0>(p)), std::get<1>(p), reinterpret_cast<const void*>(std::get<2>(p)),
+                         std::get<3>(p), reinterpret_cast<void*>(std::get<4>(p)), std::get<5>(p), std::get<6>(p), std::get<7>(p), false};
+    };
+    check(gemmGroupedWgrad(problem(p0), problem(p1), reinterpret_cast<const int*>(row_off), groups, max_rows, reinterpret_cast<void*>(maps),
+                           reinterpret_cast<uint32_t*>(status), reinterpret_cast<cudaStream_t>(stream)), "gemm_grouped_wgrad");
   });
+  m.attr("GEMM_DGELU") = static_cast<uint32_t>(GEMM_DGELU);
   m.attr("GEMM_GELU_INPLACE") = static_cast<uint32_t>(GEMM_GELU_INPLACE);
 
   // ---- production: this process is one rank -------------------------------------------------------

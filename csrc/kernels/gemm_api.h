@@ -23,6 +23,7 @@ enum GemmFlags : uint32_t {
   GEMM_ROW_STORES = 1u << 9,  // epilogue stores straight from the accumulator layout (a row per lane) instead of through the
                               // coalescing patch: for comparison runs
   GEMM_SKINNY = 1u << 10,     // few rows (M <= 256, A K-major): weights on the tile's M side, K split over a cluster (gemm_skinny.cu)
+  GEMM_DGELU = 1u << 11,      // grouped GEMM: D = A*B^T .* gelu_tanh'(D2) (D2 bf16, D's layout, read only)
 };
 
 // D[M,N] (ldd) = A * B^T.  K-major operands: A is [M,K] with row stride lda, B is [N,K] with row
@@ -58,9 +59,16 @@ int gemmBf16Dual(const GemmProblem& p0, const GemmProblem& p1, int K, uint32_t f
 // Grouped GEMM for expert layers: group g multiplies rows [row_off[g], row_off[g+1]) of A [*, K] with
 // the g-th [N, K] block of B (stacked [groups*N, K]) into the same rows of D [*, N].  `row_off`
 // (groups+1 int32) lives on the device, so no host synchronisation is needed to know the sizes.
-// flags: GEMM_GELU_INPLACE.
+// flags: GEMM_B_MN (the blocks of B are [K, N], K % 64 == 0), GEMM_GELU_INPLACE, GEMM_GELU and GEMM_DGELU (with D2, D's layout);
+// all but GEMM_GELU_INPLACE need N % 4 == 0.
 int gemmGroupedBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, int64_t ldd, const int* row_off,
-                    int groups, int max_rows, int N, int K, uint32_t flags, int sms, uint32_t* status, cudaStream_t stream);
+                    int groups, int max_rows, int N, int K, uint32_t flags, void* D2, int sms, uint32_t* status, cudaStream_t stream);
+
+// Weight gradients of two grouped layers over the same groups as one launch: for both problems and every group g,
+//   D[g * M .. +M, N] = A[rows of g, M]^T * B[rows of g, N]       (A, B bf16 with `max_rows` rows, D bf16 [groups * M, N])
+// with zeros for a group without rows.  `maps`: 512 bytes per group of device scratch (128-byte aligned) for descriptors.
+int gemmGroupedWgrad(const GemmProblem& p0, const GemmProblem& p1, const int* row_off, int groups, int max_rows, void* maps, uint32_t* status,
+                     cudaStream_t stream);
 
 // Block-scaled fp8: A is e4m3 [M, K] (row stride lda bytes = elements) with fp32 scales sa [M, ld_sa], one per row and
 // 128 values of K; B is e4m3 [N, K] with fp32 scales sb [ceil(N/128), ld_sb], one per 128 x 128 block.

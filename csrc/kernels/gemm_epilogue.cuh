@@ -30,6 +30,19 @@ __device__ __forceinline__ float dgelu_tanh(float x) {
   return fmaf(q, fmaf(-t, t, 1.0f), fmaf(0.5f, t, 0.5f));
 }
 
+// The same two functions to full fp32 accuracy, through the logistic function (0.5 (1 + tanh u) = 1 / (1 + exp(-2u))): for
+// results that replaced ones computed with an accurate tanh.
+__device__ __forceinline__ float gelu_logistic(float x) {
+  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+  return x * __fdividef(1.0f, 1.0f + __expf(-2.0f * k0 * (x + k1 * x * x * x)));
+}
+__device__ __forceinline__ float dgelu_logistic(float x) {
+  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+  const float a = x * x;
+  const float s = __fdividef(1.0f, 1.0f + __expf(-2.0f * k0 * x * fmaf(k1, a, 1.0f)));
+  return fmaf(x * s * (1.0f - s), 2.0f * k0 * fmaf(3.0f * k1, a, 1.0f), s);
+}
+
 // Sums v[0..31] of the 32 lanes column by column: afterwards lane l holds (in v[0]) the sum over the warp of v[l].
 // A butterfly that halves the number of live values per step: 31 shuffles instead of 32 five-step reductions.
 __device__ __forceinline__ void warp_transpose_sum32(float* v, int lane) {

@@ -66,6 +66,16 @@ template <class E> struct HasPatch<E, std::void_t<decltype(std::declval<E&>().at
 template <class E, class = void> struct HasWidth : std::false_type {};
 template <class E> struct HasWidth<E, std::void_t<decltype(std::declval<const E&>().width())>> : std::true_type {};
 template <class E, class = void> struct HasVarN : std::false_type {};
+// An epilogue with `int a_k0(const TileCoord&)` adds that to A's k coordinate: an MN-major A whose tiles come from one of
+// several [K, rows] matrices stacked along k (the weights of the experts).
+template <class E, class = void> struct HasAK0 : std::false_type {};
+template <class E> struct HasAK0<E, std::void_t<decltype(std::declval<const E&>().a_k0(std::declval<const TileCoord&>()))>> : std::true_type {};
+// An epilogue with `static constexpr bool kRaggedK = true` gives every tile its own reduction range (k_begin(t), k_blocks(t),
+// possibly no block at all) and its own descriptors (a_map(t), b_map(t)), which lie in global memory, written by an earlier
+// kernel of the stream: their outer extent ends where the tile's range ends, so the last k-block is filled up with zeros
+// where the next group's rows would follow.
+template <class E, class = void> struct HasRaggedK : std::false_type {};
+template <class E> struct HasRaggedK<E, std::void_t<decltype(E::kRaggedK)>> : std::true_type {};
 template <class E> struct HasVarN<E, std::void_t<decltype(E::kVarN)>> : std::true_type {};
 
 // `sched` enumerates pair tiles: t.m indexes 256-row blocks.  Epi sees per-CTA coordinates through
@@ -115,9 +125,11 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
     }
     bar->abort = 0;
     tc::fence_barrier_init();
-    for (int q = 0; q < NPROB; ++q) {
-      tc::tma_prefetch_desc(tmA + q);
-      tc::tma_prefetch_desc(tmB + q);
+    if constexpr (!HasRaggedK<Epi>::value) {
+      for (int q = 0; q < NPROB; ++q) {
+        tc::tma_prefetch_desc(tmA + q);
+        tc::tma_prefetch_desc(tmB + q);
+      }
     }
   }
   __syncthreads();
@@ -209,7 +221,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         }
         if (!gate.wait(t, abort)) { ok = false; break; }
         const int row0 = epi.a_row0(t), col0 = epi.b_row0(t);        // already offset by this CTA's half
-        const CUtensorMap* const tmA_t = NPROB > 1 ? tmA + t.extra : tmA;
+        const CUtensorMap* tmA_t = NPROB > 1 ? tmA + t.extra : tmA;
         const CUtensorMap* tmB_t = NPROB > 1 ? tmB + t.extra : tmB;
         uint32_t stage_tx = 2u * (A_BYTES + static_cast<uint32_t>(B_MN ? b_boxes * 64 : width / 2) * (BK * 2));
         if constexpr (HasVarN<Epi>::value) {
@@ -217,18 +229,28 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
           tmB_t = tmB + sel;
           stage_tx = 2 * (A_BYTES + (B_BYTES >> sel));
         }
-        for (int kb = 0; kb < num_kb; ++kb) {
+        int blocks = num_kb, ka0 = 0, kb0 = 0;
+        if constexpr (HasAK0<Epi>::value) ka0 = epi.a_k0(t);
+        if constexpr (HasRaggedK<Epi>::value) {
+          blocks = epi.k_blocks(t);
+          ka0 = kb0 = epi.k_begin(t);
+          tmA_t = epi.a_map(t);
+          tmB_t = epi.b_map(t);
+          tc::tensormap_acquire(tmA_t);
+          tc::tensormap_acquire(tmB_t);
+        }
+        for (int kb = 0; kb < blocks; ++kb) {
           if (!tc::mbar_wait(&bar->empty[stage], phase ^ 1, abort)) { ok = false; break; }
           uint8_t* sa = smem + stage * STAGE_BYTES;
           uint8_t* sb = sa + A_BYTES;
           const uint32_t full_leader = tc::mapa(tc::smem_u32(&bar->full[stage]), 0);
           if (leader) tc::mbar_arrive_expect_tx(&bar->full[stage], stage_tx);   // both CTAs' bytes
-          const int k0 = kb * BK;
+          const int k0 = kb0 + kb * BK, ka = ka0 + kb * BK;
           if constexpr (!A_MN) {
-            tc::tma_load_2d_pair(sa, tmA_t, full_leader, k0, row0);
+            tc::tma_load_2d_pair(sa, tmA_t, full_leader, ka, row0);
           } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j) tc::tma_load_2d_pair(sa + j * (64 * BK * 2), tmA_t, full_leader, row0 + j * 64, k0);
+            for (int j = 0; j < BM / 64; ++j) tc::tma_load_2d_pair(sa + j * (64 * BK * 2), tmA_t, full_leader, row0 + j * 64, ka);
           }
           if constexpr (!B_MN) {
             tc::tma_load_2d_pair(sb, tmB_t, full_leader, k0, col0);
@@ -260,7 +282,9 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         const uint32_t d_tmem = tmem + acc * BN;
         uint32_t idesc_t = idesc;
         if constexpr (HasVarN<Epi>::value) idesc_t = tc::make_idesc(1, 1, A_MN, B_MN, PAIR_M, static_cast<uint32_t>(epi.tile_n(t)));
-        for (int kb = 0; kb < num_kb; ++kb) {
+        int blocks = num_kb;
+        if constexpr (HasRaggedK<Epi>::value) blocks = epi.k_blocks(t);
+        for (int kb = 0; kb < blocks; ++kb) {
           if (!tc::mbar_wait(&bar->full[stage], phase, abort)) { ok = false; break; }
           tc::tc_fence_after();
           const uint32_t sa = tc::smem_u32(smem + stage * STAGE_BYTES), sb = sa + A_BYTES;

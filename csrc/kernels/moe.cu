@@ -16,6 +16,7 @@
 #include "gemm_epilogue.cuh"
 #include "gemm_pipeline.cuh"
 #include "gemm_pipeline2.cuh"
+#include "launch.h"
 #include "moe_api.h"
 #include "prims.cuh"
 #include "tensormap.h"
@@ -426,7 +427,7 @@ using namespace gemm;
 struct GroupedSched {
   const int* row_off;    // groups + 1
   int groups, tiles_n, first, stride;
-  int tile_rows;         // 128 (single CTA) or 256 (CTA pair)
+  int tile_rows;
   mutable int cur_g = 0;
   mutable long long cur_base = 0;
   // Tile `idx` of the concatenated per-group tile lists -> (group, m-tile inside group, n-tile).
@@ -492,25 +493,15 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   run<false, false>(&tmA, &tmB, K, sched, gate, epi, status);
 }
 
-__global__ void __launch_bounds__(NUM_THREADS, 1)
-gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GroupedEpi epi, int groups, int K,
-                         uint32_t* status) {
-  GroupedSched sched{epi.row_off, groups, (epi.N + BN - 1) / BN, static_cast<int>(blockIdx.x >> 1), static_cast<int>(gridDim.x >> 1), 2 * BM};
-  NoGate gate;
-  const int cta = static_cast<int>(tc::cluster_ctarank());
-  gemm2::PairEpi<GroupedEpi> pe{epi, cta};
-  gemm2::PairGate<NoGate> pg{gate, cta};
-  gemm2::run<false, false>(&tmA, &tmB, K, sched, pg, pe, status);
-}
-
-// The same product with the operands exchanged: the weights of a group are the M side of the tile (whole 256-row tiles, their
-// count is a multiple of 256) and the group's rows are the N side, whose extent the MMA instruction takes per tile in steps
+// The same product with the operands exchanged: the weights of a group are the M side of the tile (256 output features; the
+// last tile of a group may reach into the next group's weights, its surplus rows are not stored) and the group's rows are the
+// N side, whose extent the MMA instruction takes per tile in steps
 // of 16.  A group of 520 rows then costs 2 + 8/256 tiles of tensor time per weight tile, where the row-major form above pays
 // for 3: with a few hundred rows per expert that is a fifth of the whole product.  The accumulator arrives transposed (lane =
 // output feature, column = row of the group), so a warp stores 32 consecutive features of one row per instruction.
 struct RaggedSched {
   const int* row_off;
-  int groups, tiles_f, first, stride;        // tiles_f = N / 256 weight tiles per group
+  int groups, tiles_f, first, stride;        // tiles_f = ceil(N / 256) weight tiles per group
   mutable int cur_g = 0;
   mutable long long cur_base = 0;
   __device__ __forceinline__ bool get(int it, TileCoord* t) const {
@@ -533,12 +524,20 @@ struct RaggedSched {
   }
 };
 
+// The epilogue of the exchanged form, with the element-wise work of the expert MLP in it:
+//   GEMM_GELU_INPLACE  D = gelu(acc)                      (serving)
+//   GEMM_GELU          D = acc, D2 = gelu(acc)            (training: the pre-activation is kept for the backward pass)
+//   GEMM_DGELU         D = acc * gelu'(D2)                (backward, D2 = the pre-activation)
+// W_MN: the weights of a group are stored [K, N] (the backward pass multiplies by the transposed weights of the forward pass).
+template <bool W_MN>
 struct RaggedEpi {
   static constexpr bool kVarN = true;
   __nv_bfloat16* D;
+  __nv_bfloat16* D2;
   long long ldd;
   const int* row_off;
   int N;             // output features per group
+  int K;
   uint32_t flags;
   int cta;
   __device__ __forceinline__ int tile_n(const TileCoord& t) const {
@@ -551,30 +550,27 @@ struct RaggedEpi {
     const int half = tile_n(t) >> 1;
     return half > 64 ? 0 : half > 32 ? 1 : half > 16 ? 2 : half > 8 ? 3 : 4;
   }
-  __device__ __forceinline__ int a_row0(const TileCoord& t) const { return t.extra * N + t.m * 256 + cta * 128; }
+  __device__ __forceinline__ int a_row0(const TileCoord& t) const { return (W_MN ? 0 : t.extra * N) + t.m * 256 + cta * 128; }
+  __device__ __forceinline__ int a_k0(const TileCoord& t) const { return W_MN ? t.extra * K : 0; }
   __device__ __forceinline__ int b_row0(const TileCoord& t) const { return row_off[t.extra] + t.n * 256 + cta * (tile_n(t) >> 1); }
   __device__ __forceinline__ void attach_smem(uint8_t*) {}
   __device__ __forceinline__ void tile_begin(const TileCoord&) {}
   __device__ __forceinline__ void tile_done(const TileCoord&, const volatile uint32_t*) {}
+
   // The lane holds 32 rows of ONE feature; its neighbours hold the next features of the same rows.  Two exchange steps
   // (lane ^ 1, lane ^ 2) regroup that into 4 consecutive features of one row per lane, so a strip leaves as 8 stores of 8 bytes
-  // per lane instead of 32 of 2: lanes 4q..4q+3 then cover rows 4j+0..3 of features 4q..4q+3.
-  __device__ __forceinline__ void strip(const TileCoord& t, int feat_in_cta, int col0, uint32_t* r) {
-    const int lane = feat_in_cta & 31;
-    const int feat4 = t.m * 256 + cta * 128 + (feat_in_cta & ~3);
-    const int row0 = row_off[t.extra] + t.n * 256 + col0;
-    const int n_valid = row_off[t.extra + 1] - row0;          // rows of this strip that belong to the group (may exceed 32)
-    const bool gelu = flags & GEMM_GELU_INPLACE;
+  // per lane instead of 32 of 2: lanes 4q..4q+3 then cover rows 4j+0..3 of features 4q..4q+3.  `at` is row 0 of the strip at the
+  // lane's four features, null where those lie past N.
+  static __device__ __forceinline__ void put(__nv_bfloat16* at, long long ldd, int lane, int n_valid, const float* v) {
     const bool odd1 = lane & 1, odd2 = lane & 2;
     uint32_t p[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      float a = __uint_as_float(r[2 * j]), b = __uint_as_float(r[2 * j + 1]);
-      if (gelu) { a = gelu_tanh(a); b = gelu_tanh(b); }
+      const float a = v[2 * j], b = v[2 * j + 1];
       const float got = __shfl_xor_sync(0xffffffffu, odd1 ? a : b, 1);
       // even lane: row 2j, features (f, f+1) = (own a, neighbour's a); odd lane: row 2j+1, features (f-1, f) = (neighbour's b, own b)
-      const __nv_bfloat162 v = odd1 ? __floats2bfloat162_rn(got, b) : __floats2bfloat162_rn(a, got);
-      p[j] = *reinterpret_cast<const uint32_t*>(&v);
+      const __nv_bfloat162 x = odd1 ? __floats2bfloat162_rn(got, b) : __floats2bfloat162_rn(a, got);
+      p[j] = *reinterpret_cast<const uint32_t*>(&x);
     }
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
@@ -582,21 +578,148 @@ struct RaggedEpi {
       // bit 1 clear: keeps pair-row 2m, features +0..1 own, +2..3 from lane ^ 2; bit 1 set: keeps pair-row 2m+1
       const uint2 out = odd2 ? make_uint2(got, p[2 * m + 1]) : make_uint2(p[2 * m], got);
       const int row = 2 * (2 * m + (odd2 ? 1 : 0)) + (odd1 ? 1 : 0);
-      if (row < n_valid)
-        *reinterpret_cast<uint2*>(D + static_cast<long long>(row0 + row) * ldd + feat4) = out;
+      if (at && row < n_valid) *reinterpret_cast<uint2*>(at + row * ldd) = out;
+    }
+  }
+  // The same exchange the other way round: 8 loads of 8 bytes, then lane ^ 2, lane ^ 1; rows past n_valid read as zero.
+  static __device__ __forceinline__ void get(const __nv_bfloat16* at, long long ldd, int lane, int n_valid, float* v) {
+    const bool odd1 = lane & 1, odd2 = lane & 2;
+    uint2 in[8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      const int row = 2 * (2 * m + (odd2 ? 1 : 0)) + (odd1 ? 1 : 0);
+      in[m] = at && row < n_valid ? *reinterpret_cast<const uint2*>(at + row * ldd) : make_uint2(0u, 0u);
+    }
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, odd2 ? in[m].x : in[m].y, 2);
+      const uint32_t p[2] = {odd2 ? got : in[m].x, odd2 ? in[m].y : got};
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        // p = (low: feature of the even lane, high: feature of the odd lane) of row 2j (even lane) or 2j+1 (odd lane)
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, odd1 ? p[i] << 16 : p[i] & 0xffff0000u, 1);
+        const int j = 2 * m + i;
+        v[2 * j] = __uint_as_float(odd1 ? other : p[i] << 16);
+        v[2 * j + 1] = __uint_as_float(odd1 ? p[i] & 0xffff0000u : other);
+      }
+    }
+  }
+  __device__ __forceinline__ void strip(const TileCoord& t, int feat_in_cta, int col0, uint32_t* r) {
+    const int lane = feat_in_cta & 31;
+    const int feat4 = t.m * 256 + cta * 128 + (feat_in_cta & ~3);
+    const int row0 = row_off[t.extra] + t.n * 256 + col0;
+    const int n_valid = row_off[t.extra + 1] - row0;          // rows of this strip that belong to the group (may exceed 32)
+    const long long off = row0 * ldd + feat4;
+    const bool in = feat4 < N;                                // N % 4 == 0
+    float v[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+    if (flags & GEMM_DGELU) {
+      float pre[32];
+      get(in ? D2 + off : nullptr, ldd, lane, n_valid, pre);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] *= dgelu_logistic(pre[i]);
+    }
+    if (flags & GEMM_GELU_INPLACE) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
+    }
+    put(in ? D + off : nullptr, ldd, lane, n_valid, v);
+    if (flags & GEMM_GELU) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = gelu_logistic(v[i]);
+      put(in ? D2 + off : nullptr, ldd, lane, n_valid, v);
     }
   }
 };
 
 struct RaggedMaps { CUtensorMap x[5]; };     // boxes of 128, 64, 32, 16, 8 rows
 
+template <bool W_MN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-gemm_grouped_ragged_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ RaggedMaps tmX, RaggedEpi epi, int groups, int K,
-                           uint32_t* status) {
-  RaggedSched sched{epi.row_off, groups, epi.N / 256, static_cast<int>(blockIdx.x >> 1), static_cast<int>(gridDim.x >> 1)};
+gemm_grouped_ragged_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ RaggedMaps tmX, RaggedEpi<W_MN> epi, int groups,
+                           int K, uint32_t* status) {
+  RaggedSched sched{epi.row_off, groups, (epi.N + 255) / 256, static_cast<int>(blockIdx.x >> 1), static_cast<int>(gridDim.x >> 1)};
   NoGate gate;
   epi.cta = static_cast<int>(tc::cluster_ctarank());
-  gemm2::run<false, false>(&tmW, tmX.x, K, sched, gate, epi, status);
+  gemm2::run<W_MN, false>(&tmW, tmX.x, K, sched, gate, epi, status);
+}
+
+// ---------------------------------------------------------------------------------------------
+// grouped weight gradients
+// ---------------------------------------------------------------------------------------------
+// D_q[g] = A_q[rows of g]^T * B_q[rows of g] for every group g and the two projections q of the expert MLP as one tile list:
+// M_q x N_q outputs per group, reduced over the group's rows, whose number only the device knows.  Both operands are read
+// where they lie (MN-major).  The reduction of a group ends in the middle of a k-block as a rule, and what follows in memory
+// are the next group's rows; so every (group, operand) has a descriptor of its own whose outer extent is the group's end, and
+// TMA fills the rest of the block with zeros.  The descriptors are made on the device from four templates, one warp each.
+// A group without rows gets zeros.
+struct WgradTemplates { CUtensorMap m[4]; };           // A_0, B_0, A_1, B_1
+
+__global__ void __launch_bounds__(128) wgrad_maps_kernel(const __grid_constant__ WgradTemplates tmpl, const int* __restrict__ row_off,
+                                                         int groups, CUtensorMap* __restrict__ maps) {
+  __shared__ __align__(128) CUtensorMap stage[4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = blockIdx.x;
+  reinterpret_cast<uint32_t*>(&stage[warp])[lane] = reinterpret_cast<const uint32_t*>(&tmpl.m[warp])[lane];
+  __syncwarp();
+  if (lane == 0) tc::tensormap_set_outer(&stage[warp], static_cast<uint32_t>(max(1, row_off[g + 1])));
+  __syncwarp();
+  tc::tensormap_publish(maps + g * 4 + warp, &stage[warp]);
+}
+
+struct WgradSched {
+  int tiles_m[2], tiles_n[2], groups, first, stride;
+  __device__ __forceinline__ bool get(int it, TileCoord* t) const {
+    const long long idx = first + static_cast<long long>(it) * stride;
+    const int n0 = tiles_m[0] * tiles_n[0], per = n0 + tiles_m[1] * tiles_n[1];
+    const int g = static_cast<int>(idx / per);
+    if (g >= groups) return false;
+    int r = static_cast<int>(idx - static_cast<long long>(g) * per);
+    const int q = r >= n0 ? 1 : 0;
+    if (q) r -= n0;
+    t->m = r % tiles_m[q];
+    t->n = r / tiles_m[q];
+    t->extra = g * 2 + q;
+    return true;
+  }
+};
+
+struct WgradEpi {
+  static constexpr bool kRaggedK = true;
+  StoreEpi e[2];               // D: group 0
+  const int* row_off;
+  const CUtensorMap* maps;     // [groups][4]
+  int cta;
+  __device__ __forceinline__ int k_begin(const TileCoord& t) const { return row_off[t.extra >> 1]; }
+  __device__ __forceinline__ int k_blocks(const TileCoord& t) const {
+    return (row_off[(t.extra >> 1) + 1] - row_off[t.extra >> 1] + gemm2::BK - 1) / gemm2::BK;
+  }
+  __device__ __forceinline__ const CUtensorMap* a_map(const TileCoord& t) const { return maps + t.extra * 2; }
+  __device__ __forceinline__ const CUtensorMap* b_map(const TileCoord& t) const { return maps + t.extra * 2 + 1; }
+  __device__ __forceinline__ int a_row0(const TileCoord& t) const { return t.m * 256 + cta * 128; }
+  __device__ __forceinline__ int b_row0(const TileCoord& t) const { return t.n * 256 + cta * 128; }
+  __device__ __forceinline__ void attach_smem(uint8_t*) {}
+  __device__ __forceinline__ void attach_patch(uint8_t* p) { e[0].attach_patch(p); e[1].attach_patch(p); }
+  __device__ __forceinline__ void tile_begin(const TileCoord&) {}
+  __device__ __forceinline__ void tile_done(const TileCoord&, const volatile uint32_t*) {}
+  __device__ __forceinline__ void strip(const TileCoord& t, int row, int col, uint32_t* r) {
+    const int g = t.extra >> 1;
+    StoreEpi s = e[t.extra & 1];
+    s.D = static_cast<__nv_bfloat16*>(s.D) + static_cast<long long>(g) * s.M * s.ldd;
+    if (row_off[g + 1] == row_off[g]) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) r[i] = 0u;          // nothing was accumulated
+    }
+    s.strip(TileCoord{t.m * 2 + cta, t.n, 0}, row, col, r);
+  }
+};
+
+__global__ void __launch_bounds__(gemm2::NUM_THREADS_WIDE, 1) gemm_grouped_wgrad_kernel(WgradEpi epi, int groups, uint32_t* status) {
+  WgradSched sched{{(epi.e[0].M + 255) / 256, (epi.e[1].M + 255) / 256}, {(epi.e[0].N + 255) / 256, (epi.e[1].N + 255) / 256}, groups,
+                   static_cast<int>(blockIdx.x >> 1), static_cast<int>(gridDim.x >> 1)};
+  NoGate gate;
+  epi.cta = static_cast<int>(tc::cluster_ctarank());
+  gemm2::run<true, true, WgradSched, NoGate, WgradEpi, gemm2::STAGES, 1, false, 8>(nullptr, nullptr, gemm2::BK, sched, gate, epi, status);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -761,45 +884,43 @@ int launchMoePlan(const int* counts_all, const int* ids, const int* pos, int* ro
 }
 
 int gemmGroupedBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, int64_t ldd, const int* row_off,
-                    int groups, int max_rows, int N, int K, uint32_t flags, int sms, uint32_t* status, cudaStream_t stream) {
+                    int groups, int max_rows, int N, int K, uint32_t flags, void* D2, int sms, uint32_t* status, cudaStream_t stream) {
   if (groups <= 0 || max_rows <= 0) return 0;
   if ((lda | ldb | ldd) % 8) return static_cast<int>(cudaErrorInvalidValue);
+  const bool w_mn = flags & GEMM_B_MN;
+  if (((flags & (GEMM_GELU | GEMM_DGELU)) && (!D2 || reinterpret_cast<uintptr_t>(D2) % 8)) || (w_mn && K % BK)) return static_cast<int>(cudaErrorInvalidValue);
   CUtensorMap ta, tb;
   std::string err;
-  if (!makeTensorMap2D(&ta, A, TM_BF16, K, max_rows, lda, BK, BM, &err)) return static_cast<int>(cudaErrorInvalidValue);
   int n_sm = deviceSmCount();
   if (sms > 0 && sms < n_sm) n_sm = sms;
-  GroupedEpi epi{static_cast<__nv_bfloat16*>(D), ldd, row_off, N, flags};
-  static const bool ragged_on = !(std::getenv("PCCL_GROUPED_RAGGED") && std::getenv("PCCL_GROUPED_RAGGED")[0] == '0');
-  if (N % 256 == 0 && n_sm >= 2 && ragged_on) {
+  if (N % 4 == 0 && reinterpret_cast<uintptr_t>(D) % 8 == 0 && n_sm >= 2) {
     // operands exchanged: weights on the M side, the groups' rows on an N side that is cut to the rows there are
     CUtensorMap tw;
     RaggedMaps tx;
-    if (!makeTensorMap2D(&tw, B, TM_BF16, K, static_cast<uint64_t>(groups) * N, ldb, BK, 128, &err)) return static_cast<int>(cudaErrorInvalidValue);
+    if (!w_mn ? !makeTensorMap2D(&tw, B, TM_BF16, K, static_cast<uint64_t>(groups) * N, ldb, BK, 128, &err)
+              : !makeTensorMap2D(&tw, B, TM_BF16, N, static_cast<uint64_t>(groups) * K, ldb, 64, BK, &err))
+      return static_cast<int>(cudaErrorInvalidValue);
     for (int i = 0; i < 5; ++i)
       if (!makeTensorMap2D(&tx.x[i], A, TM_BF16, K, max_rows, lda, BK, 128 >> i, &err)) return static_cast<int>(cudaErrorInvalidValue);
-    static bool set3 = false;
-    if (!set3) {
-      cudaError_t e = cudaFuncSetAttribute(gemm_grouped_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm2::SMEM_BYTES);
-      if (e != cudaSuccess) return static_cast<int>(e);
-      set3 = true;
-    }
-    RaggedEpi repi{static_cast<__nv_bfloat16*>(D), ldd, row_off, N, flags, 0};
-    return static_cast<int>(gemm2::launch_pairs(gemm_grouped_ragged_kernel, dim3(n_sm & ~1), NUM_THREADS, gemm2::SMEM_BYTES, stream, false, tw, tx,
-                                                repi, groups, K, status));
+    static bool set[2] = {false, false};
+    auto go = [&](auto kern, auto epi, bool* done) {
+      if (!*done) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm2::SMEM_BYTES);
+        if (e != cudaSuccess) return static_cast<int>(e);
+        *done = true;
+      }
+      return static_cast<int>(launchOverlapped(kern, dim3(n_sm & ~1), dim3(NUM_THREADS), gemm2::SMEM_BYTES, stream, 2, tw, tx, epi, groups, K, status));
+    };
+    if (w_mn)
+      return go(gemm_grouped_ragged_kernel<true>,
+                RaggedEpi<true>{static_cast<__nv_bfloat16*>(D), static_cast<__nv_bfloat16*>(D2), ldd, row_off, N, K, flags, 0}, &set[1]);
+    return go(gemm_grouped_ragged_kernel<false>,
+              RaggedEpi<false>{static_cast<__nv_bfloat16*>(D), static_cast<__nv_bfloat16*>(D2), ldd, row_off, N, K, flags, 0}, &set[0]);
   }
-  if (N % 256 == 0 && n_sm >= 2) {       // CTA pairs: each CTA loads 128 of the 256 B rows of a tile
-    if (!makeTensorMap2D(&tb, B, TM_BF16, K, static_cast<uint64_t>(groups) * N, ldb, BK, 128, &err)) return static_cast<int>(cudaErrorInvalidValue);
-    static bool set2 = false;
-    if (!set2) {
-      cudaError_t e = cudaFuncSetAttribute(gemm_grouped_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm2::SMEM_BYTES);
-      if (e != cudaSuccess) return static_cast<int>(e);
-      set2 = true;
-    }
-    return static_cast<int>(gemm2::launch_pairs(gemm_grouped_pair_kernel, dim3(n_sm & ~1), NUM_THREADS, gemm2::SMEM_BYTES, stream, false, ta, tb,
-                                                epi, groups, K, status));
-  }
+  if (flags & ~static_cast<uint32_t>(GEMM_GELU_INPLACE)) return static_cast<int>(cudaErrorInvalidValue);
+  if (!makeTensorMap2D(&ta, A, TM_BF16, K, max_rows, lda, BK, BM, &err)) return static_cast<int>(cudaErrorInvalidValue);
   if (!makeTensorMap2D(&tb, B, TM_BF16, K, static_cast<uint64_t>(groups) * N, ldb, BK, BN, &err)) return static_cast<int>(cudaErrorInvalidValue);
+  GroupedEpi epi{static_cast<__nv_bfloat16*>(D), ldd, row_off, N, flags};
   static bool set = false;
   if (!set) {
     cudaError_t e = cudaFuncSetAttribute(gemm_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
@@ -808,6 +929,40 @@ int gemmGroupedBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void
   }
   gemm_grouped_kernel<<<n_sm, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, epi, groups, K, status);
   return static_cast<int>(cudaGetLastError());
+}
+
+int gemmGroupedWgrad(const GemmProblem& p0, const GemmProblem& p1, const int* row_off, int groups, int max_rows, void* maps, uint32_t* status,
+                     cudaStream_t stream) {
+  if (groups <= 0) return 0;
+  const GemmProblem* ps[2] = {&p0, &p1};
+  WgradTemplates tm;
+  WgradEpi epi{};
+  std::string err;
+  long long tiles = 0;
+  for (int q = 0; q < 2; ++q) {
+    const GemmProblem& p = *ps[q];
+    if (max_rows <= 0 || p.M <= 0 || p.N <= 0 || (p.lda | p.ldb | p.ldd) % 8 || p.accumulate ||
+        (reinterpret_cast<uintptr_t>(p.A) | reinterpret_cast<uintptr_t>(p.B) | reinterpret_cast<uintptr_t>(p.D)) % 16)
+      return static_cast<int>(cudaErrorInvalidValue);
+    if (!makeTensorMap2D(&tm.m[2 * q], p.A, TM_BF16, p.M, max_rows, p.lda, 64, gemm2::BK, &err) ||
+        !makeTensorMap2D(&tm.m[2 * q + 1], p.B, TM_BF16, p.N, max_rows, p.ldb, 64, gemm2::BK, &err))
+      return static_cast<int>(cudaErrorInvalidValue);
+    epi.e[q] = StoreEpi{p.D, nullptr, nullptr, p.ldd, p.M, p.N, 0u};
+    tiles += static_cast<long long>(groups) * ((p.M + 255) / 256) * ((p.N + 255) / 256);
+  }
+  if (reinterpret_cast<uintptr_t>(maps) % 128) return static_cast<int>(cudaErrorInvalidValue);
+  epi.row_off = row_off;
+  epi.maps = static_cast<const CUtensorMap*>(maps);
+  static bool set = false;
+  if (!set) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_grouped_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm2::SMEM_BYTES);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    set = true;
+  }
+  wgrad_maps_kernel<<<groups, 128, 0, stream>>>(tm, row_off, groups, static_cast<CUtensorMap*>(maps));
+  const int pairs = deviceSmCount() / 2;
+  return static_cast<int>(launchOverlapped(gemm_grouped_wgrad_kernel, dim3(2 * static_cast<int>(tiles < pairs ? tiles : pairs)),
+                                           dim3(gemm2::NUM_THREADS_WIDE), gemm2::SMEM_BYTES, stream, 2, epi, groups, status));
 }
 
 }  // namespace pccl

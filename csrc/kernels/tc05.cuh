@@ -71,6 +71,21 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
 
+// ---- descriptors written on the device -----------------------------------------------------------------
+// A descriptor in shared memory (128 bytes, 128-byte aligned): set the extent of its outer dimension.
+__device__ __forceinline__ void tensormap_set_outer(void* smem_map, uint32_t extent) {
+  asm volatile("tensormap.replace.tile.global_dim.shared::cta.b1024.b32 [%0], 1, %1;" ::"l"(static_cast<uint64_t>(smem_u32(smem_map))), "r"(extent) : "memory");
+}
+// ... publish it in global memory for TMA loads of later kernels (whole warp) ...
+__device__ __forceinline__ void tensormap_publish(CUtensorMap* gmem_map, const void* smem_map) {
+  asm volatile("tensormap.cp_fenceproxy.global.shared::cta.tensormap::generic.release.gpu.sync.aligned [%0], [%1], 128;"
+               ::"l"(gmem_map), "r"(smem_u32(smem_map)) : "memory");
+}
+// ... and what a thread executes before its first load through a descriptor published that way.
+__device__ __forceinline__ void tensormap_acquire(const CUtensorMap* gmem_map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(gmem_map) : "memory");
+}
+
 // ---- bulk (non-tensor) async copies: global -> shared (completes on an mbarrier) and shared -> global ----
 __device__ __forceinline__ void bulk_load_g2s(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"

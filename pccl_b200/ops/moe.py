@@ -36,16 +36,46 @@ def quant_fp8_blocks(w: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
 
 
 def grouped_gemm(a: torch.Tensor, b: torch.Tensor, row_off: torch.Tensor, n: int, out: Optional[torch.Tensor] = None,
-                 gelu: bool = False) -> torch.Tensor:
-    """Rows [row_off[g], row_off[g+1]) of ``a`` [*, K] times ``b[g*n:(g+1)*n]`` ([groups*n, K]) ^T -> same rows of out [*, n]."""
-    groups = row_off.numel() - 1
+                 gelu: bool = False, *, b_t: bool = False, gelu_out: Optional[torch.Tensor] = None,
+                 dgelu: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Rows [row_off[g], row_off[g+1]) of ``a`` [*, K] times ``b[g*n:(g+1)*n]`` ([groups*n, K]) ^T -> same rows of out [*, n].
+    ``b_t``: the blocks of ``b`` are [K, n] (stacked [groups*K, n]) and not transposed.  ``gelu_out`` receives gelu_tanh(out);
+    ``dgelu`` (a pre-activation) makes it ``out = product * gelu_tanh'(dgelu)``; both have ``out``'s shape and strides."""
+    groups, K = row_off.numel() - 1, a.shape[1]
+    if b_t and K % 64:                 # the kernel reads k in blocks of 64, which must not reach into the next group's weights
+        b, b_t = b.view(groups, K, n).transpose(1, 2).reshape(groups * n, K), False
     if out is None:
         out = torch.empty((a.shape[0], n), dtype=torch.bfloat16, device=a.device)
+    side = gelu_out if gelu_out is not None else dgelu
+    if side is not None and ((gelu_out is not None and dgelu is not None) or gelu or side.dtype != torch.bfloat16 or side.shape != out.shape
+                             or side.stride() != out.stride()):
+        raise ValueError("grouped_gemm: one of gelu, gelu_out and dgelu, a bf16 tensor of out's shape and strides")
+    flags = (C.GEMM_GELU_INPLACE if gelu else 0) | (C.GEMM_B_MN if b_t else 0)
+    if side is not None:
+        flags |= C.GEMM_GELU if gelu_out is not None else C.GEMM_DGELU
     C.gemm_grouped(a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), out.data_ptr(), out.stride(0), row_off.data_ptr(), groups,
-                   a.shape[0], n, a.shape[1], C.GEMM_GELU_INPLACE if gelu else 0, 0, status_words().data_ptr(),
-                   torch.cuda.current_stream().cuda_stream)
+                   a.shape[0], n, K, flags, 0, status_words().data_ptr(), torch.cuda.current_stream().cuda_stream,
+                   side.data_ptr() if side is not None else 0)
     count_launch()
     return out
+
+
+def grouped_wgrad(a0: torch.Tensor, b0: torch.Tensor, a1: torch.Tensor, b1: torch.Tensor, row_off: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``d_q[g] = a_q[rows of g]^T @ b_q[rows of g]`` for q = 0, 1 and every group, as [groups * M_q, N_q] (zeros for a group
+    without rows); a_q [rows, M_q] and b_q [rows, N_q] are bf16 over the same rows."""
+    groups, rows = row_off.numel() - 1, a0.shape[0]
+    problems, outs = [], []
+    for a, b in ((a0, b0), (a1, b1)):
+        if a.shape[0] != rows or b.shape[0] != rows or a.stride(1) != 1 or b.stride(1) != 1:
+            raise ValueError("grouped_wgrad: operands must be row-major over the same rows")
+        d = torch.empty((groups * a.shape[1], b.shape[1]), dtype=torch.bfloat16, device=a.device)
+        problems.append((a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), d.data_ptr(), d.stride(0), a.shape[1], b.shape[1]))
+        outs.append(d)
+    maps = torch.empty(groups * 512, dtype=torch.uint8, device=a0.device)          # the kernel's descriptors
+    C.gemm_grouped_wgrad(problems[0], problems[1], row_off.data_ptr(), groups, rows, maps.data_ptr(), status_words().data_ptr(),
+                         torch.cuda.current_stream().cuda_stream)
+    count_launch(2)
+    return outs[0], outs[1]
 
 
 class MoEExchange:

@@ -8,18 +8,16 @@ e4m3 payload of a row is the same for all of its destinations, only the block sc
 the experts' input gradients come back through the combine kernel; the gradients of the gate weights
 are dot products of the upstream gradient with the expert output rows, taken by a third kernel that
 pulls the rows like the combine does.  The expert GEMMs of the backward pass are the grouped kernel
-again (input gradients) and one tcgen05 GEMM per expert (weight gradients, whose reduction dimension
-is the expert's row count).  The reference has no model code; this is the EP strategy it names.
+again (input gradients, on the weights as they are stored) and one launch for the weight gradients of all
+experts, whose reduction dimension is the expert's row count.  No step waits for the host.  The reference has no model code; this is the EP strategy it names.
 """
 from __future__ import annotations
 
 import torch
 import torch.nn as nn
-import torch.nn.functional as F
 
 from ..engine import Engine
-from ..ops.gemm import gemm
-from ..ops.moe import MoEExchange, grouped_gemm
+from ..ops.moe import MoEExchange, grouped_gemm, grouped_wgrad
 
 
 class _MoEFn(torch.autograd.Function):
@@ -32,8 +30,8 @@ class _MoEFn(torch.autograd.Function):
         ex.dispatch(x, ids, plan)
         xr = ex.received(plan)                                   # what the experts see (after the e4m3 round trip)
         d_ff = w1.shape[0] // ex.epr
-        h_pre = grouped_gemm(xr, w1, plan["row_off"], d_ff)
-        h = F.gelu(h_pre, approximate="tanh")
+        h = torch.empty((xr.shape[0], d_ff), dtype=torch.bfloat16, device=xr.device)
+        h_pre = grouped_gemm(xr, w1, plan["row_off"], d_ff, gelu_out=h)
         grouped_gemm(h, w2, plan["row_off"], ex.H, out=ex.y)
         out = ex.combine(ids, probs, plan)
         ctx.save_for_backward(gate_logits, w1, w2, ids, probs, plan["rows"], plan["row_off"], plan["n_rows"], xr, h_pre, h)
@@ -53,21 +51,10 @@ class _MoEFn(torch.autograd.Function):
         # output gradients to the experts, each weighted by its gate probability
         ex.dispatch(dout, ids, plan, probs=probs)
         g = ex.received(plan)
-        # experts: input gradients with the grouped kernel (it multiplies by B^T, so the weights are laid out transposed)
-        w2t = w2.view(epr, H, d_ff).transpose(1, 2).reshape(epr * d_ff, H).contiguous()
-        dh = grouped_gemm(g, w2t, row_off, d_ff)
-        dh_pre = torch.ops.aten.gelu_backward(dh, h_pre, approximate="tanh")
-        w1t = w1.view(epr, d_ff, H).transpose(1, 2).reshape(epr * H, d_ff).contiguous()
-        grouped_gemm(dh_pre, w1t, row_off, H, out=ex.y)
-        # weight gradients: per expert, reduced over that expert's rows (the one place the host needs the row counts)
-        offs = row_off.tolist()
-        dw1 = torch.zeros_like(w1)
-        dw2 = torch.zeros_like(w2)
-        for e in range(epr):
-            r0, r1 = offs[e], offs[e + 1]
-            if r1 > r0:
-                gemm(dh_pre[r0:r1], xr[r0:r1], a_t=True, b_t=True, out=dw1[e * d_ff:(e + 1) * d_ff])
-                gemm(g[r0:r1], h[r0:r1], a_t=True, b_t=True, out=dw2[e * H:(e + 1) * H])
+        # experts: the same grouped kernel on the weights as they lie, gelu' in its epilogue, then all weight gradients at once
+        dh_pre = grouped_gemm(g, w2, row_off, d_ff, b_t=True, dgelu=h_pre)
+        grouped_gemm(dh_pre, w1, row_off, H, b_t=True, out=ex.y)
+        dw1, dw2 = grouped_wgrad(dh_pre, xr, g, h, row_off)
         # input gradients back to the tokens: a plain sum over the k assignments (the gate weight went out with dout)
         dx = ex.combine(ids, torch.ones_like(probs), plan)
         # softmax over all experts, top-k taken: chain rule through the softmax for the selected probabilities

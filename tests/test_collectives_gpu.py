@@ -485,8 +485,7 @@ def test_fp8_quantisers_match_reference(native):
 
 @pytest.mark.parametrize("N,gelu", [(384, False), (512, False), (768, True)])
 def test_grouped_gemm_matches_per_group_reference(native, N, gelu):
-    """N = 384 takes the single-CTA row-major kernel; multiples of 256 take the CTA-pair kernel with the operands exchanged,
-    whose tiles end where a group's rows end (group sizes around and off the multiples of 16 and 256)."""
+    """The CTA-pair kernel with the operands exchanged (N = 384: the last weight tile reaches past the group's features), whose tiles end where a group's rows end (group sizes around and off the multiples of 16 and 256)."""
     from pccl_b200.ops import check_status
     from pccl_b200.ops.moe import grouped_gemm
     torch.manual_seed(4)
@@ -506,6 +505,59 @@ def test_grouped_gemm_matches_per_group_reference(native, N, gelu):
             ref = torch.nn.functional.gelu(ref, approximate="tanh")
         assert (out[lo:lo + n].float() - ref).abs().max().item() < 0.05 if n else True
     assert torch.all(out[total:] == 7.0)        # rows past the last group are untouched
+
+
+@pytest.mark.parametrize("N,K,b_t", [(384, 512, False), (392, 192, False), (256, 512, True), (136, 192, True), (648, 200, True)])
+def test_grouped_gemm_gelu_forms(native, N, K, b_t):
+    """GELU side output and GELU-backward epilogue of the grouped kernel, weights as [n, K] and [K, n]: feature counts off the
+    256-row tiles (136, 392, 648), a K that ends inside a k-block (200: laid out anew for the [K, n] form), groups around the
+    multiples of 16 and 256.  fp32 sums of <= 512 terms and one bf16 rounding: 2^-8 of the value and of the largest."""
+    from pccl_b200.ops import check_status
+    from pccl_b200.ops.moe import grouped_gemm
+    torch.manual_seed(5)
+    sizes = [17, 0, 257, 1, 256, 15]
+    off = torch.tensor([0] + list(torch.tensor(sizes).cumsum(0)), dtype=torch.int32, device="cuda")
+    total, G = int(off[-1]), len(sizes)
+    a = (torch.randn(total + 40, K, device="cuda") * 0.5).bfloat16()
+    b = (torch.randn((G * K, N) if b_t else (G * N, K), device="cuda") * 0.1).bfloat16()
+    pre_in = torch.randn(total + 40, N, device="cuda").bfloat16()
+    act = torch.full((total + 40, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    pre, d = act.clone(), act.clone()
+    grouped_gemm(a, b, off, N, out=pre, gelu_out=act, b_t=b_t)
+    grouped_gemm(a, b, off, N, out=d, dgelu=pre_in, b_t=b_t)
+    check_status("grouped gemm")
+    for g, n in enumerate(sizes):
+        s = slice(int(off[g]), int(off[g]) + n)
+        w = b[g * K:(g + 1) * K].double() if b_t else b[g * N:(g + 1) * N].double().t()
+        ref = (a[s].double() @ w).requires_grad_(True)
+        x = pre_in[s].double().requires_grad_(True)
+        gx, = torch.autograd.grad(torch.nn.functional.gelu(x, approximate="tanh").sum(), x)
+        for got, want in ((pre[s], ref), (act[s], torch.nn.functional.gelu(ref, approximate="tanh")), (d[s], ref * gx)):
+            assert (got.double() - want).abs().le(2 ** -8 * want.abs() + 1e-5).all()
+    assert all((t[total:] == 7.0).all() for t in (pre, act, d))                     # rows past the last group are untouched
+
+
+@pytest.mark.parametrize("sizes", [[130, 0, 257, 1, 64, 63, 65, 0], [0, 0, 5], [512]])
+@pytest.mark.parametrize("M,N", [(256, 512), (136, 328)])
+def test_grouped_weight_gradients(native, M, N, sizes):
+    """Group ends inside and at the edges of a k-block, empty groups, feature counts off the tiles; the rows past the last group
+    hold NaN (they are uninitialised memory in use) and must not be read into any sum."""
+    from pccl_b200.ops import check_status
+    from pccl_b200.ops.moe import grouped_wgrad
+    torch.manual_seed(6)
+    off = torch.tensor([0] + list(torch.tensor(sizes).cumsum(0)), dtype=torch.int32, device="cuda")
+    total = int(off[-1])
+    ops = [torch.randn(total + 70, f, device="cuda").bfloat16() for f in (M, N, N, M)]
+    for t in ops:
+        t[total:] = float("nan")
+    d0, d1 = grouped_wgrad(*ops, off)
+    check_status("grouped weight gradients")
+    for d, a, b in ((d0, ops[0], ops[1]), (d1, ops[2], ops[3])):
+        d = d.view(len(sizes), a.shape[1], b.shape[1])
+        for g, n in enumerate(sizes):
+            s = slice(int(off[g]), int(off[g]) + n)
+            ref = a[s].double().t() @ b[s].double()
+            assert (d[g].double() - ref).abs().le(2 ** -8 * ref.abs() + 1e-4).all()
 
 
 def test_moe_dispatch_combine_emulated(native):

@@ -163,7 +163,7 @@ class MoEExchange:
         return ids, probs, {"rows": rows, "row_off": row_off, "n_rows": row_off[-1:]}
 
     # ---- kernels ----------------------------------------------------------------------------
-    def _exchange(self, kind: str, x, ids, rows, probs, out, gate=None, dedupe: bool = False) -> None:
+    def _exchange(self, kind: str, x, ids, rows, probs, out, gate=None, dedupe: bool = False, groups: bool = True) -> None:
         self.epoch += 1
         st = status_words()
         off = self.eng.heap_offset
@@ -172,7 +172,7 @@ class MoEExchange:
                        [x.data_ptr()] if x is not None else [], [ids.data_ptr()], [rows.data_ptr()],
                        [probs.data_ptr()] if probs is not None else [], [out.data_ptr()] if out is not None else [],
                        [st.data_ptr()], self.blocks, 0, torch.cuda.current_stream().cuda_stream,
-                       alias_off=off(self.alias), group_off=off(self.groups), z_off=off(self.z),
+                       alias_off=off(self.alias), group_off=off(self.groups) if groups else 0, z_off=off(self.z),
                        gate=[gate.data_ptr()] if gate is not None else [], dedupe=dedupe)
         count_launch()
 
@@ -234,6 +234,9 @@ class MoEExchange:
 
     def forward(self, x: torch.Tensor, gate_logits: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor) -> torch.Tensor:
         ids, probs, plan = self.route_and_plan(gate_logits)
-        self.dispatch(x, ids, plan, gate=probs)
+        # Adding up a token's rows on each rank before they travel saves NVLink traffic.  In a world of one nothing travels and it
+        # would be a second pass over the sums: the combine weighs the expert rows itself (the same fp32 sum in the same order).
+        grouped = self.eng.world > 1
+        self._exchange("dispatch", x, ids, plan["rows"], None, None, gate=probs, dedupe=True, groups=grouped)
         self.experts(w1, w2, plan)
-        return self.combine(ids, probs, plan, grouped=True)
+        return self.combine(ids, probs, plan, grouped=grouped)

@@ -20,7 +20,8 @@ int launchAdamW(float* p, float* m, float* v, const float* g, void* p_bf16, long
 int launchCrossEntropy(void* logits, const long long* targets, float* loss, long long rows, int vocab, long long ld,
                        float grad_scale, long long ignore_index, uint32_t* status, cudaStream_t stream);
 
-// LayerNorm over the last dimension D (multiple of 8, <= 8192) of bf16 [rows, D]; mean / rstd are fp32 [rows].
+// LayerNorm over the last dimension D (multiple of 8, <= 8192) of bf16 [rows, D]; mean / rstd are fp32 [rows], or both
+// null where no backward pass follows.
 // With `delta` (bf16 [rows, D], may be null) the norm is taken of s = x + delta and s is stored to `sum_out`:
 // the residual connection of a pre-norm block and the norm in one pass.
 int launchLayerNormFwd(const void* x, const void* delta, void* sum_out, const void* gamma, const void* beta, void* y, float* mean,

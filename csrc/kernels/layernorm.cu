@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(256) ln_fwd_kernel(const __nv_bfloat16* __rest
     }
   }
   const float rs = rsqrtf(block_sum(q, scratch) / D + eps);
-  if (threadIdx.x == 0) { mean[row] = mu; rstd[row] = rs; }
+  if (threadIdx.x == 0 && mean) { mean[row] = mu; rstd[row] = rs; }
 #pragma unroll
   for (int j = 0; j < MAXV; ++j) {
     const int v = threadIdx.x + j * 256;

@@ -13,13 +13,13 @@ import torch
 import torch.nn as nn
 
 from ..ops.elementwise import colsum
-from ..ops.gemm import gemm, gemm_dgelu, gemm_dual
+from ..ops.gemm import gemm, gemm_dgelu, gemm_dual, records_graph
 
 
 def _as_operand(t: torch.Tensor) -> torch.Tensor:
     """2-D view usable as a GEMM operand: unit inner stride, row stride % 8 == 0, 16-byte aligned
     (a column slice of a padded buffer qualifies; anything else is made contiguous)."""
-    t2 = t.reshape(-1, t.shape[-1])
+    t2 = t if t.dim() == 2 else t.reshape(-1, t.shape[-1])
     if t2.stride(1) != 1 or t2.stride(0) % 8 or t2.data_ptr() % 16:
         t2 = t2.contiguous()
     return t2
@@ -66,7 +66,11 @@ def _bias_grad(dy2: torch.Tensor, bias: Optional[torch.Tensor]) -> Optional[torc
     if bias is None:
         return None
     if dy2.shape[1] % 8 == 0 and dy2.is_cuda:
-        db = colsum(dy2)
+        out = _main_grad_out(bias, torch.bfloat16)
+        db = colsum(dy2, out=out)
+        if out is not None:
+            _finish_main_grad(bias)
+            return None
     else:
         db = dy2.sum(0, dtype=torch.float32).to(bias.dtype)
     mg = _grad_target(bias)
@@ -80,22 +84,32 @@ def _bias_grad(dy2: torch.Tensor, bias: Optional[torch.Tensor]) -> Optional[torc
     return None
 
 
+def _main_grad_out(p: torch.Tensor, dtype: torch.dtype) -> Optional[torch.Tensor]:
+    """The flat-bucket gradient of ``p`` if a kernel may write it directly: nothing is in it yet this step."""
+    mg = _grad_target(p)
+    if mg is None or mg.dtype != dtype or getattr(p, "_pccl_written", False) or not mg.is_contiguous() or mg.data_ptr() % 16:
+        return None
+    return mg
+
+
+def _linear_forward(x, weight, bias, residual):
+    x2 = _as_operand(x)
+    y = gemm(x2, weight, bias=bias, residual=residual.reshape(-1, weight.shape[0]) if residual is not None else None)
+    return x2, (y if x.dim() == 2 else y.view(*x.shape[:-1], weight.shape[0]))
+
+
 class _LinearFn(torch.autograd.Function):
     """y = x W^T + b (+ residual).  ``defer_bias_grad``: the bias gradient is produced elsewhere (by the fused
     residual-add + LayerNorm that consumes y, which sums the same rows anyway), so backward skips it."""
 
     @staticmethod
     def forward(ctx, x, weight, bias, residual=None, defer_bias_grad=False):
-        x2 = _as_operand(x)
-        res2 = None
-        if residual is not None:
-            res2 = residual.reshape(-1, weight.shape[0])
-        y = gemm(x2, weight, bias=bias, residual=res2)
+        x2, y = _linear_forward(x, weight, bias, residual)
         ctx.save_for_backward(x2, weight, bias)
         ctx.x_shape = x.shape
         ctx.defer_bias_grad = defer_bias_grad
         ctx.has_residual = residual is not None
-        return y.view(*x.shape[:-1], weight.shape[0])
+        return y
 
     @staticmethod
     def backward(ctx, dy):
@@ -139,7 +153,7 @@ class _MlpFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w1, b1, w2, b2, defer_b2_grad=False):
         x2 = _as_operand(x)
-        act = torch.empty((x2.shape[0], w1.shape[0]), dtype=torch.bfloat16, device=x.device)
+        act = x2.new_empty((x2.shape[0], w1.shape[0]))
         pre = gemm(x2, w1, bias=b1, gelu_out=act)
         out = gemm(act, w2, bias=b2)
         ctx.save_for_backward(x2, w1, b1, w2, b2, pre, act)
@@ -155,7 +169,7 @@ class _MlpFn(torch.autograd.Function):
         if n1 % 32 == 0:
             sums = torch.zeros(n1, dtype=torch.float32, device=pre.device) if b1 is not None else None
             dy2 = gemm_dgelu(dz2, w2, pre, b_t=True, colsum=sums)
-            db1 = _deliver_bias(b1, sums.to(b1.dtype)) if b1 is not None else None
+            db1 = _deliver_bias(b1, sums) if b1 is not None else None
         else:
             dact = gemm(dz2, w2, b_t=True)
             dy2 = torch.ops.aten.gelu_backward(dact, pre, approximate="tanh")
@@ -169,11 +183,11 @@ class _MlpFn(torch.autograd.Function):
 def _deliver_bias(bias: torch.Tensor, db: torch.Tensor) -> Optional[torch.Tensor]:
     mg = _grad_target(bias)
     if mg is None:
-        return db
+        return db.to(bias.dtype)
     if getattr(bias, "_pccl_written", False):
-        mg.add_(db)
+        mg.add_(db.to(bias.dtype))
     else:
-        mg.copy_(db)
+        mg.copy_(db)                       # rounds fp32 sums to the bucket's dtype
     _finish_main_grad(bias)
     return None
 
@@ -192,12 +206,20 @@ class Linear(nn.Module):
     def forward(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None, defer_bias_grad: bool = False) -> torch.Tensor:
         """``residual`` is added in the GEMM epilogue.  ``defer_bias_grad=True`` promises that the consumer of the output
         (``LayerNorm.add_norm(..., prev_bias=self.bias)``) produces this layer's bias gradient."""
-        return _LinearFn.apply(x, self.weight, self.bias, residual, defer_bias_grad)
+        if records_graph():
+            return _LinearFn.apply(x, self.weight, self.bias, residual, defer_bias_grad)
+        return _linear_forward(x, self.weight, self.bias, residual)[1]
 
 
 def mlp(x: torch.Tensor, fc1: "Linear", fc2: "Linear", defer_fc2_bias_grad: bool = False) -> torch.Tensor:
     """``fc2(gelu_tanh(fc1(x)))`` with the two layers' backward passes fused (see ``_MlpFn``)."""
-    return _MlpFn.apply(x, fc1.weight, fc1.bias, fc2.weight, fc2.bias, defer_fc2_bias_grad)
+    w1, w2 = fc1.weight, fc2.weight
+    if records_graph():
+        return _MlpFn.apply(x, w1, fc1.bias, w2, fc2.bias, defer_fc2_bias_grad)
+    x2 = _as_operand(x)
+    act = x2.new_empty((x2.shape[0], w1.shape[0]))
+    gemm(x2, w1, bias=fc1.bias, gelu_out=act)
+    return gemm(act, w2, bias=fc2.bias).view(*x.shape[:-1], w2.shape[0])
 
 
 class LinearGelu(Linear):

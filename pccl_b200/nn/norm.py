@@ -9,7 +9,39 @@ import torch
 import torch.nn as nn
 
 from .._native import C
-from ..ops.gemm import count_launch
+from ..ops.gemm import count_launch, records_graph, stream_handle
+
+
+def _finish(param: torch.Tensor) -> None:
+    param._pccl_written = True
+    cb = getattr(param, "_pccl_ready", None)
+    if cb is not None:
+        cb()
+
+
+def _writable(param: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """The flat-bucket gradient of ``param`` if the kernel may write it directly (nothing is in it yet this step)."""
+    mg = getattr(param, "main_grad", None)
+    if mg is None or mg.dtype != torch.bfloat16 or getattr(param, "_pccl_written", False) or not mg.is_contiguous() or mg.data_ptr() % 16:
+        return None
+    return mg
+
+
+def _own(param: torch.Tensor) -> Optional[torch.Tensor]:
+    """Like ``_writable`` for a parameter of the norm itself, whose gradient otherwise travels through autograd: only where
+    nobody else is to see it there, i.e. the parameter is used once this step and has no hook but the wrapper's."""
+    hooks = getattr(param, "_post_accumulate_grad_hooks", None)
+    if getattr(param, "_pccl_forwards", 0) != 1 or param._backward_hooks or (hooks is not None and len(hooks) > 1):
+        return None
+    return _writable(param)
+
+
+def _count_use(*params: torch.Tensor) -> None:
+    if torch.is_grad_enabled():
+        for p in params:
+            n = getattr(p, "_pccl_forwards", None)
+            if n is not None:
+                p._pccl_forwards = n + 1
 
 
 def _deliver(param: Optional[torch.Tensor], grad: torch.Tensor):
@@ -20,42 +52,54 @@ def _deliver(param: Optional[torch.Tensor], grad: torch.Tensor):
     mg = getattr(param, "main_grad", None)
     if mg is None:
         return grad
-    if getattr(param, "_pccl_written", False):
-        mg.add_(grad.to(mg.dtype).view_as(mg))
-    else:
-        mg.copy_(grad.view_as(mg))
-    param._pccl_written = True
-    cb = getattr(param, "_pccl_ready", None)
-    if cb is not None:
-        cb()
+    if grad is not mg:
+        if getattr(param, "_pccl_written", False):
+            mg.add_(grad.to(mg.dtype).view_as(mg))
+        else:
+            mg.copy_(grad.view_as(mg))
+    _finish(param)
     return None
 
 
-def _ln_forward(x2, delta2, weight, bias, eps):
+def _ln_forward(x2, delta2, weight, bias, eps, want_stats=True):
+    """(sum or None, y, fp32 [2, rows] with means and reciprocal deviations or None)"""
     rows, D = x2.shape
     y = torch.empty_like(x2)
     s = torch.empty_like(x2) if delta2 is not None else None
-    mean = torch.empty(rows, dtype=torch.float32, device=x2.device)
-    rstd = torch.empty(rows, dtype=torch.float32, device=x2.device)
+    stats = x2.new_empty((2, rows), dtype=torch.float32) if want_stats else None
+    at = stats.data_ptr() if want_stats else 0
     C.layernorm_fwd(x2.data_ptr(), delta2.data_ptr() if delta2 is not None else 0, s.data_ptr() if s is not None else 0,
-                    weight.data_ptr(), bias.data_ptr(), y.data_ptr(), mean.data_ptr(), rstd.data_ptr(), rows, D, eps,
-                    torch.cuda.current_stream().cuda_stream)
+                    weight.data_ptr(), bias.data_ptr(), y.data_ptr(), at, at + 4 * rows if at else 0, rows, D, eps, stream_handle())
     count_launch()
-    return s, y, mean, rstd
+    return s, y, stats
 
 
-def _ln_backward(dy2, x2, weight, mean, rstd, dres2, want_colsum):
+def _ln_backward(dy2, x2, weight, bias, stats, dres2, colsum_of):
+    """(dx, dgamma, dbeta, column sums of dx or None).  A parameter gradient that went straight into the flat bucket is the
+    bucket's view; ``colsum_of`` is the parameter whose gradient the column sums are, or None."""
     rows, D = x2.shape
     dx = torch.empty_like(x2)
-    dg = torch.empty_like(weight)
-    db = torch.empty_like(weight)
-    dc = torch.empty_like(weight) if want_colsum else None
-    partials = torch.empty(3 * C.layernorm_bwd_parts(rows) * D, dtype=torch.float32, device=x2.device)
-    C.layernorm_bwd(dy2.data_ptr(), x2.data_ptr(), weight.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
+    dg, db = _own(weight), _own(bias)
+    dg = torch.empty_like(weight) if dg is None else dg
+    db = torch.empty_like(bias) if db is None else db
+    dc = None
+    if colsum_of is not None:
+        dc = _writable(colsum_of)
+        dc = torch.empty_like(weight) if dc is None else dc
+    partials = x2.new_empty(3 * C.layernorm_bwd_parts(rows) * D, dtype=torch.float32)
+    at = stats.data_ptr()
+    C.layernorm_bwd(dy2.data_ptr(), x2.data_ptr(), weight.data_ptr(), at, at + 4 * rows,
                     dres2.data_ptr() if dres2 is not None else 0, dx.data_ptr(), dg.data_ptr(), db.data_ptr(),
-                    dc.data_ptr() if dc is not None else 0, partials.data_ptr(), rows, D, torch.cuda.current_stream().cuda_stream)
+                    dc.data_ptr() if dc is not None else 0, partials.data_ptr(), rows, D, stream_handle())
     count_launch(2)
-    return dx, dg, db, dc
+    return dx, _own_result(weight, dg), _own_result(bias, db), dc
+
+
+def _own_result(param, grad):
+    if grad is not getattr(param, "main_grad", None):
+        return grad                        # autograd accumulates it
+    _finish(param)
+    return None
 
 
 def _rows(t: torch.Tensor, D: int) -> torch.Tensor:
@@ -67,15 +111,15 @@ class _LayerNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, eps):
         x2 = _rows(x, x.shape[-1])
-        _, y, mean, rstd = _ln_forward(x2, None, weight, bias, eps)
-        ctx.save_for_backward(x2, weight, mean, rstd)
+        _, y, stats = _ln_forward(x2, None, weight, bias, eps)
+        ctx.save_for_backward(x2, weight, bias, stats)
         ctx.shape = x.shape
         return y.view(x.shape)
 
     @staticmethod
     def backward(ctx, dy):
-        x2, weight, mean, rstd = ctx.saved_tensors
-        dx, dg, db, _ = _ln_backward(_rows(dy, x2.shape[1]), x2, weight, mean, rstd, None, False)
+        x2, weight, bias, stats = ctx.saved_tensors
+        dx, dg, db, _ = _ln_backward(_rows(dy, x2.shape[1]), x2, weight, bias, stats, None, None)
         return dx.view(ctx.shape), dg, db, None
 
 
@@ -88,21 +132,21 @@ class _AddLayerNormFn(torch.autograd.Function):
     def forward(ctx, x, delta, weight, bias, prev_bias, eps):
         D = x.shape[-1]
         x2, d2 = _rows(x, D), _rows(delta, D)
-        s, y, mean, rstd = _ln_forward(x2, d2, weight, bias, eps)
-        ctx.save_for_backward(s, weight, mean, rstd)
+        s, y, stats = _ln_forward(x2, d2, weight, bias, eps)
+        ctx.save_for_backward(s, weight, bias, stats)
         ctx.prev_bias = prev_bias
         ctx.shape = x.shape
         return s.view(x.shape), y.view(x.shape)
 
     @staticmethod
     def backward(ctx, ds, dy):
-        s, weight, mean, rstd = ctx.saved_tensors
+        s, weight, bias, stats = ctx.saved_tensors
         D = s.shape[1]
         if dy is None:
             dy = torch.zeros_like(s)
         dres = _rows(ds, D) if ds is not None else None
         want = ctx.prev_bias is not None and ctx.needs_input_grad[4]
-        dx, dg, db, dc = _ln_backward(_rows(dy, D), s, weight, mean, rstd, dres, want)
+        dx, dg, db, dc = _ln_backward(_rows(dy, D), s, weight, bias, stats, dres, ctx.prev_bias if want else None)
         dxv = dx.view(ctx.shape)
         return dxv, dxv, dg, db, (_deliver(ctx.prev_bias, dc) if want else None), None
 
@@ -117,9 +161,19 @@ class LayerNorm(nn.Module):
         self.bias = nn.Parameter(torch.zeros(dim, device=device, dtype=dtype))
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        return _LayerNormFn.apply(x, self.weight, self.bias, self.eps)
+        weight, bias = self.weight, self.bias
+        if records_graph():
+            _count_use(weight, bias)
+            return _LayerNormFn.apply(x, weight, bias, self.eps)
+        return _ln_forward(_rows(x, x.shape[-1]), None, weight, bias, self.eps, False)[1].view(x.shape)
 
     def add_norm(self, x: torch.Tensor, delta: torch.Tensor, prev_bias: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
         """Returns ``(x + delta, LayerNorm(x + delta))``.  Pass the bias of the linear layer that produced ``delta`` as
         ``prev_bias`` when that layer was told to leave its bias gradient to this norm (``Linear(..., defer_bias_grad=True)``)."""
-        return _AddLayerNormFn.apply(x, delta, self.weight, self.bias, prev_bias, self.eps)
+        weight, bias = self.weight, self.bias
+        if records_graph():
+            _count_use(weight, bias)
+            return _AddLayerNormFn.apply(x, delta, weight, bias, prev_bias, self.eps)
+        D = x.shape[-1]
+        s, y, _ = _ln_forward(_rows(x, D), _rows(delta, D), weight, bias, self.eps, False)
+        return s.view(x.shape), y.view(x.shape)

@@ -13,7 +13,7 @@ import torch
 
 from .._native import C
 from ..engine import Engine, dtype_name
-from .gemm import count_launch
+from .gemm import count_launch, stream_handle
 
 _NVLS_OK = {("f32", "sum"), ("bf16", "sum"), ("bf16", "max"), ("bf16", "min"), ("f16", "sum"), ("f16", "max"), ("f16", "min")}
 
@@ -49,7 +49,7 @@ def all_reduce(eng: Engine, inp: torch.Tensor, out: Optional[torch.Tensor] = Non
     dt = dtype_name(inp.dtype)
     nbytes = inp.numel() * inp.element_size()
     a = _algo(eng, algo, dt, op, nbytes)
-    s = (stream or torch.cuda.current_stream()).cuda_stream
+    s = stream.cuda_stream if stream is not None else stream_handle()
     C.collective(eng.raw, "allreduce", a, dt, op, eng.heap_offset(inp), eng.heap_offset(out), inp.numel(), lane, 1.0, "",
                  _blocks(nbytes if (nbytes <= ((64 << 10) if a == "nvls" else (256 << 10)) and out is not inp) else nbytes // eng.world, blocks),
                  threads, s, 0, 0, 0)
@@ -66,7 +66,7 @@ def reduce_scatter(eng: Engine, inp: torch.Tensor, out: torch.Tensor, op: str = 
     if inp.numel() != n * eng.world:
         raise ValueError("reduce_scatter: inp must hold world * out.numel() elements")
     a = _algo(eng, algo, dt, op, n * inp.element_size(), "reduce_scatter")
-    s = (stream or torch.cuda.current_stream()).cuda_stream
+    s = stream.cuda_stream if stream is not None else stream_handle()
     sym_out = eng.is_symmetric(out)
     C.collective(eng.raw, "reduce_scatter", a, dt, op, eng.heap_offset(inp), eng.heap_offset(out) if sym_out else 0, n, lane,
                  float(scale), dtype_name(out.dtype), _blocks(n * inp.element_size(), blocks), threads, s, 0,
@@ -86,7 +86,7 @@ def reduce_scatter_adamw(eng: Engine, grads: torch.Tensor, master: torch.Tensor,
     if grads.dtype != torch.bfloat16 or grads.numel() != n * eng.world or n % 8:
         raise ValueError("reduce_scatter_adamw: bf16 bucket of world * n elements with n % 8 == 0 expected")
     a = _algo(eng, algo, "bf16", "sum", n * 2)
-    s = (stream or torch.cuda.current_stream()).cuda_stream
+    s = stream.cuda_stream if stream is not None else stream_handle()
     C.reduce_scatter_adamw(eng.raw, a, eng.heap_offset(grads), n, lane, float(scale), master.data_ptr(), exp_avg.data_ptr(),
                            exp_avg_sq.data_ptr(), param_bf16.data_ptr(), lr, betas[0], betas[1], eps, weight_decay, step,
                            _blocks(n * 2, blocks), threads, s)
@@ -105,7 +105,7 @@ def all_reduce_fp8(eng: Engine, q: torch.Tensor, s: torch.Tensor, out_q: Optiona
     n = q.numel()
     if q.element_size() != 1 or n % 128 or s.dtype != torch.float32 or s.numel() != n // 128:
         raise ValueError("all_reduce_fp8: q must be one-byte elements (n % 128 == 0) and s fp32 with n / 128 entries")
-    st = (stream or torch.cuda.current_stream()).cuda_stream
+    st = stream.cuda_stream if stream is not None else stream_handle()
     C.collective(eng.raw, "allreduce_fp8", "p2p", "e4m3", op, eng.heap_offset(q), eng.heap_offset(out_q), n, lane, 1.0, "",
                  _blocks(n // eng.world, blocks), threads, st, 0, 0, 0, eng.heap_offset(s), eng.heap_offset(out_s))
     count_launch()
@@ -119,7 +119,7 @@ def reduce_scatter_fp8(eng: Engine, q: torch.Tensor, s: torch.Tensor, out_q: tor
     m = out_q.numel()
     if q.element_size() != 1 or m % 128 or q.numel() != m * eng.world or s.numel() != q.numel() // 128 or out_s.numel() != m // 128:
         raise ValueError("reduce_scatter_fp8: shapes do not match world * shard with 128-value blocks")
-    st = (stream or torch.cuda.current_stream()).cuda_stream
+    st = stream.cuda_stream if stream is not None else stream_handle()
     C.collective(eng.raw, "reduce_scatter_fp8", "p2p", "e4m3", op, eng.heap_offset(q), eng.heap_offset(out_q), m, lane, 1.0, "",
                  _blocks(m, blocks), threads, st, 0, 0, 0, eng.heap_offset(s), eng.heap_offset(out_s))
     count_launch()
@@ -135,7 +135,7 @@ def all_gather(eng: Engine, inp: torch.Tensor, out: torch.Tensor, algo: str = "a
     # better than the multicast store (which also comes back to the sender)
     if algo == "auto" and nbytes >= (4 << 20):
         a = "p2p"
-    s = (stream or torch.cuda.current_stream()).cuda_stream
+    s = stream.cuda_stream if stream is not None else stream_handle()
     C.collective(eng.raw, "allgather", a, "u8", "sum", 0, eng.heap_offset(out), nbytes, lane, 1.0, "",
                  _blocks(nbytes, blocks), threads, s, inp.data_ptr(), 0, 0)
     count_launch()
@@ -146,7 +146,7 @@ def all_to_all(eng: Engine, inp: torch.Tensor, out: torch.Tensor, blocks: Option
                lane: int = 0, stream=None) -> torch.Tensor:
     """Block d of ``inp`` goes to rank d; ``out`` (symmetric) receives block s from rank s."""
     nbytes = inp.numel() * inp.element_size() // eng.world
-    s = (stream or torch.cuda.current_stream()).cuda_stream
+    s = stream.cuda_stream if stream is not None else stream_handle()
     C.collective(eng.raw, "alltoall", "p2p", "u8", "sum", 0, eng.heap_offset(out), nbytes, lane, 1.0, "",
                  _blocks(nbytes * eng.world, blocks), threads, s, inp.data_ptr(), 0, 0)
     count_launch()

@@ -4,7 +4,7 @@ from __future__ import annotations
 import torch
 
 from .._native import C
-from .gemm import count_launch, status_words
+from .gemm import count_launch, status_words, stream_handle
 
 
 def adamw_step(master: torch.Tensor, exp_avg: torch.Tensor, exp_avg_sq: torch.Tensor, grad: torch.Tensor,
@@ -17,7 +17,7 @@ def adamw_step(master: torch.Tensor, exp_avg: torch.Tensor, exp_avg_sq: torch.Te
             raise ValueError("adamw_step: fp32 contiguous tensors of one length expected")
     if param_bf16.dtype != torch.bfloat16 or param_bf16.numel() != n or not param_bf16.is_contiguous():
         raise ValueError("adamw_step: param_bf16 must be a contiguous bf16 tensor of the same length")
-    s = (stream or torch.cuda.current_stream()).cuda_stream
+    s = stream.cuda_stream if stream is not None else stream_handle()
     C.adamw(master.data_ptr(), exp_avg.data_ptr(), exp_avg_sq.data_ptr(), grad.data_ptr(), param_bf16.data_ptr(), n,
             lr, betas[0], betas[1], eps, weight_decay, step, grad_scale, s)
     count_launch()
@@ -37,7 +37,7 @@ def cross_entropy_(logits: torch.Tensor, targets: torch.Tensor, *, grad_scale: f
         raise ValueError("cross_entropy_: int64 targets, one per row")
     loss = torch.empty(rows, dtype=torch.float32, device=logits.device)
     C.cross_entropy(logits.data_ptr(), targets.data_ptr(), loss.data_ptr(), rows, vocab, logits.stride(0), grad_scale,
-                    ignore_index, status_words(logits.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+                    ignore_index, status_words(logits.device).data_ptr(), stream_handle())
     count_launch()
     return loss
 
@@ -51,6 +51,6 @@ def colsum(x: torch.Tensor, out: torch.Tensor = None) -> torch.Tensor:
     if out is None:
         out = torch.empty(n, dtype=torch.bfloat16, device=x.device)
     partials = torch.empty(C.colsum_parts(rows) * n, dtype=torch.float32, device=x.device)
-    C.colsum(x.data_ptr(), x.stride(0), rows, n, out.data_ptr(), partials.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    C.colsum(x.data_ptr(), x.stride(0), rows, n, out.data_ptr(), partials.data_ptr(), stream_handle())
     count_launch(2)
     return out

@@ -12,7 +12,7 @@ import torch
 
 from .._native import C
 from ..engine import Engine
-from .gemm import count_launch, status_words
+from .gemm import count_launch, status_words, stream_handle
 
 
 def default_copy_ctas(world: int) -> int:
@@ -57,7 +57,7 @@ class AllGatherGemm:
         self.epoch += 1
         C.ag_gemm(self.eng.raw, self.eng.heap_offset(self.x_full), self.M, n, self.K, w.data_ptr(), w.stride(0), out.data_ptr(),
                   out.stride(0), bias.data_ptr() if bias is not None else 0, self.eng.heap_offset(self.ready), self.epoch, self.n_copy,
-                  self.ctas, self.flag_lane, status_words().data_ptr(), torch.cuda.current_stream().cuda_stream, w_t)
+                  self.ctas, self.flag_lane, status_words().data_ptr(), stream_handle(), w_t)
         count_launch()
         return out
 
@@ -88,7 +88,7 @@ class GemmReduceScatter:
         self.epoch += 1
         C.gemm_rs(self.eng.raw, y.data_ptr(), y.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), self.M, self.N,
                   y.shape[1], self.eng.heap_offset(self.stage), self.eng.heap_offset(self.flags), self.epoch, self.ctas,
-                  status_words().data_ptr(), torch.cuda.current_stream().cuda_stream, w_t)
+                  status_words().data_ptr(), stream_handle(), w_t)
         count_launch()
         return out
 
@@ -128,7 +128,7 @@ class AllGatherGemmFp8:
             raise ValueError("AllGatherGemmFp8.quantize_local: contiguous bf16 [M/world, K]")
         quant = C.quant_mx8_rows if self.mx else C.quant_fp8_rows
         quant(x.data_ptr(), self.xq_local.data_ptr(), self.xs_local.data_ptr(), self.m_local, self.K,
-              torch.cuda.current_stream().cuda_stream)
+              stream_handle())
         count_launch()
 
     def __call__(self, wq: torch.Tensor, ws: torch.Tensor, bias: Optional[torch.Tensor] = None, gelu: bool = False,
@@ -151,7 +151,7 @@ class AllGatherGemmFp8:
                       [wq.data_ptr()], wq.stride(0), [ws.data_ptr()], ws.stride(0), d, ldd, dq, ds, ldq,
                       bias.data_ptr() if bias is not None else 0, C.GEMM_GELU_INPLACE if gelu else 0, self.eng.heap_offset(self.ready),
                       self.epoch, self.n_copy, self.ctas, self.flag_lane, [status_words().data_ptr()], 0,
-                      torch.cuda.current_stream().cuda_stream, self.mx)
+                      stream_handle(), self.mx)
         count_launch()
         return result
 
@@ -184,6 +184,6 @@ class GemmReduceScatterFp8:
         C.gemm_rs_fp8(self.eng.raw, [], [yq.data_ptr()], yq.stride(0), [ys.data_ptr()], ys.stride(0), [wq.data_ptr()], wq.stride(0),
                       [ws.data_ptr()], ws.stride(0), [out.data_ptr()], out.stride(0), self.M, self.N, k,
                       self.eng.heap_offset(self.stage), self.eng.heap_offset(self.flags), self.epoch, self.ctas,
-                      [status_words().data_ptr()], 0, torch.cuda.current_stream().cuda_stream)
+                      [status_words().data_ptr()], 0, stream_handle())
         count_launch()
         return out

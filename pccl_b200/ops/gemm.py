@@ -9,6 +9,7 @@ from __future__ import annotations
 from typing import Dict, Optional
 
 import torch
+from torch.autograd import forward_ad as _forward_ad
 
 from .._native import C
 
@@ -17,7 +18,9 @@ import os
 _PAIR_DEFAULT = os.environ.get("PCCL_GEMM_PAIR", "1") != "0"      # CTA pairs unless switched off
 # up to this many rows (of a K-major a) the weights are streamed by the few-row kernel (csrc/kernels/gemm_skinny.cu says why)
 _SKINNY_ROWS = 128
+_functorch_active, _tracing = torch._C._are_functorch_transforms_active, torch._C._get_tracing_state
 _status: Dict[int, torch.Tensor] = {}
+_status_ptr: Dict[int, int] = {}
 _launches = 0
 
 
@@ -27,6 +30,30 @@ def status_words(device=None) -> torch.Tensor:
     if idx not in _status:
         _status[idx] = torch.zeros(64, dtype=torch.int32, device=f"cuda:{idx}")
     return _status[idx]
+
+
+_raw_stream, _device_index = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+
+
+def stream_handle() -> int:
+    """``cudaStream_t`` of the calling thread's current stream on its current device.  ``torch.cuda.current_stream()`` builds
+    two Python objects for the same number: 3.3 us of every launch against 0.3."""
+    return _raw_stream(_device_index())
+
+
+def records_graph() -> bool:
+    """Whether an operation must go through ``autograd.Function.apply``: gradients are recorded, or a transform, a forward-mode
+    level or a tracer wants to see it.  Otherwise its forward runs directly (apply() alone is 7 us)."""
+    return (torch.is_grad_enabled() or _functorch_active() or _forward_ad._current_level >= 0 or _tracing() is not None)
+
+
+def _status_of(t: torch.Tensor) -> int:
+    """Address of the status words of a CUDA tensor's device."""
+    idx = t.get_device()
+    ptr = _status_ptr.get(idx)
+    if ptr is None:
+        ptr = _status_ptr[idx] = status_words(t.device).data_ptr()
+    return ptr
 
 
 def check_status(what: str = "kernel") -> None:
@@ -49,11 +76,15 @@ def count_launch(n: int = 1) -> None:
     _launches += n
 
 
-def _check(t: torch.Tensor, name: str) -> None:
-    if not t.is_cuda or t.dtype != torch.bfloat16 or t.dim() != 2 or t.stride(1) != 1:
+def _check(t: torch.Tensor, name: str):
+    """Checks a GEMM operand; returns its row stride and address."""
+    st = t.stride()
+    if len(st) != 2 or st[1] != 1 or t.dtype is not torch.bfloat16 or not t.is_cuda:
         raise ValueError(f"gemm: {name} must be a 2-D CUDA bf16 tensor with unit inner stride")
-    if t.stride(0) % 8 or t.data_ptr() % 16:
+    ptr = t.data_ptr()
+    if st[0] % 8 or ptr % 16:
         raise ValueError(f"gemm: {name} needs a row stride that is a multiple of 8 and a 16-byte aligned base")
+    return st[0], ptr
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = False,
@@ -68,25 +99,26 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     the few-row kernel, more the CTA pairs (PCCL_GEMM_PAIR).
     ``residual`` (bf16, out's shape and strides) is added in the epilogue: ``out = a @ b.T + bias + residual``.
     ``row_stores`` turns the epilogue's coalescing patch off (comparison runs)."""
-    _check(a, "a")
-    _check(b, "b")
-    M, K = (a.shape[1], a.shape[0]) if a_t else (a.shape[0], a.shape[1])
-    N, Kb = (b.shape[1], b.shape[0]) if b_t else (b.shape[0], b.shape[1])
+    lda, a_ptr = _check(a, "a")
+    ldb, b_ptr = _check(b, "b")
+    M, K = a.shape
+    if a_t:
+        M, K = K, M
+    N, Kb = b.shape
+    if b_t:
+        N, Kb = Kb, N
     if K != Kb:
         raise ValueError(f"gemm: inner dimensions differ ({K} vs {Kb})")
     if out is None:
         ldd = (N + 7) // 8 * 8
-        store = torch.empty((M, ldd), dtype=out_dtype, device=a.device)
-        out = store[:, :N] if ldd != N else store
-    if out.dtype not in (torch.bfloat16, torch.float32) or out.shape != (M, N) or out.stride(1) != 1:
+        out = a.new_empty((M, ldd), dtype=out_dtype)
+        if ldd != N:
+            out = out[:, :N]
+    ldd, inner = out.stride() if out.dim() == 2 else (0, 0)
+    f32 = out.dtype is torch.float32
+    if not (f32 or out.dtype is torch.bfloat16) or out.shape != (M, N) or inner != 1:
         raise ValueError("gemm: out must be [M,N] bf16/fp32 with unit inner stride")
-    flags = 0
-    if a_t:
-        flags |= C.GEMM_A_MN
-    if b_t:
-        flags |= C.GEMM_B_MN
-    if out.dtype == torch.float32:
-        flags |= C.GEMM_OUT_F32
+    flags = (C.GEMM_A_MN if a_t else 0) | (C.GEMM_B_MN if b_t else 0) | (C.GEMM_OUT_F32 if f32 else 0)
     if accumulate:
         flags |= C.GEMM_ACCUMULATE
     if pair is None and M <= _SKINNY_ROWS and not (a_t or sms or row_stores):
@@ -113,8 +145,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
             raise ValueError("gemm: residual must be bf16 with out's shape and strides (and excludes gelu_out)")
         flags |= C.GEMM_ADD_D2
         d2 = residual.data_ptr()
-    C.gemm_bf16(a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), out.data_ptr(), out.stride(0), M, N, K, flags,
-                bias_ptr, d2, sms, status_words(a.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+    C.gemm_bf16(a_ptr, lda, b_ptr, ldb, out.data_ptr(), ldd, M, N, K, flags, bias_ptr, d2, sms, _status_of(a), stream_handle())
     count_launch()
     return out
 
@@ -138,7 +169,7 @@ def gemm_dual(a0: torch.Tensor, b0: torch.Tensor, out0: torch.Tensor, a1: torch.
     flags = (C.GEMM_A_MN if a_t else 0) | (C.GEMM_B_MN if b_t else 0) | (C.GEMM_OUT_F32 if out0.dtype == torch.float32 else 0)
     C.gemm_bf16_dual(a0.data_ptr(), a0.stride(0), b0.data_ptr(), b0.stride(0), out0.data_ptr(), out0.stride(0), dims[0][0], dims[0][1], accumulate0,
                      a1.data_ptr(), a1.stride(0), b1.data_ptr(), b1.stride(0), out1.data_ptr(), out1.stride(0), dims[1][0], dims[1][1], accumulate1,
-                     dims[0][2], flags, sms, status_words(a0.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+                     dims[0][2], flags, sms, _status_of(a0), stream_handle())
     count_launch()
 
 
@@ -162,7 +193,7 @@ def gemm_dgelu(a: torch.Tensor, b: torch.Tensor, pre: torch.Tensor, *, b_t: bool
         raise ValueError("gemm_dgelu: colsum must be a contiguous fp32 vector of length N")
     C.gemm_bf16_dgelu(a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), out.data_ptr(), out.stride(0), pre.data_ptr(),
                       colsum.data_ptr() if colsum is not None else 0, M, N, K, C.GEMM_B_MN if b_t else 0, sms,
-                      status_words(a.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+                      _status_of(a), stream_handle())
     count_launch()
     return out
 
@@ -174,7 +205,7 @@ def quant_rows(x: torch.Tensor):
         raise ValueError("quant_rows: contiguous bf16 with K % 128 == 0")
     q = torch.empty((rows, k), dtype=torch.uint8, device=x.device)
     s = torch.empty((rows, k // 128), dtype=torch.float32, device=x.device)
-    C.quant_fp8_rows(x.data_ptr(), q.data_ptr(), s.data_ptr(), rows, k, torch.cuda.current_stream().cuda_stream)
+    C.quant_fp8_rows(x.data_ptr(), q.data_ptr(), s.data_ptr(), rows, k, stream_handle())
     count_launch()
     return q, s
 
@@ -186,7 +217,7 @@ def quant_blocks(w: torch.Tensor):
         raise ValueError("quant_blocks: contiguous bf16 with both sizes multiples of 128")
     q = torch.empty((n, k), dtype=torch.uint8, device=w.device)
     s = torch.empty((n // 128, k // 128), dtype=torch.float32, device=w.device)
-    C.quant_fp8_blocks(w.data_ptr(), q.data_ptr(), s.data_ptr(), n, k, torch.cuda.current_stream().cuda_stream)
+    C.quant_fp8_blocks(w.data_ptr(), q.data_ptr(), s.data_ptr(), n, k, stream_handle())
     count_launch()
     return q, s
 
@@ -230,7 +261,7 @@ def gemm_fp8(a_q: torch.Tensor, a_s: torch.Tensor, b_q: torch.Tensor, b_s: torch
         bias_ptr = bias.data_ptr()
     C.gemm_fp8(a_q.data_ptr(), a_q.stride(0), a_s.data_ptr(), a_s.stride(0), b_q.data_ptr(), b_q.stride(0), b_s.data_ptr(),
                b_s.stride(0), out.data_ptr(), out.stride(0), M, N, K, flags, bias_ptr, 0, sms,
-               status_words(a_q.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+               _status_of(a_q), stream_handle())
     count_launch()
     return out
 
@@ -243,7 +274,7 @@ def quant_rows_mx(x: torch.Tensor):
         raise ValueError("quant_rows_mx: contiguous bf16 with K % 128 == 0")
     q = torch.empty((rows, k), dtype=torch.uint8, device=x.device)
     s = torch.empty((rows, k // 128), dtype=torch.uint8, device=x.device)
-    C.quant_mx8_rows(x.data_ptr(), q.data_ptr(), s.data_ptr(), rows, k, torch.cuda.current_stream().cuda_stream)
+    C.quant_mx8_rows(x.data_ptr(), q.data_ptr(), s.data_ptr(), rows, k, stream_handle())
     count_launch()
     return q, s
 
@@ -255,7 +286,7 @@ def quant_blocks_mx(w: torch.Tensor):
         raise ValueError("quant_blocks_mx: contiguous bf16 with both sizes multiples of 128")
     q = torch.empty((n, k), dtype=torch.uint8, device=w.device)
     s = torch.empty((n // 128, k // 128), dtype=torch.uint8, device=w.device)
-    C.quant_mx8_blocks(w.data_ptr(), q.data_ptr(), s.data_ptr(), n, k, torch.cuda.current_stream().cuda_stream)
+    C.quant_mx8_blocks(w.data_ptr(), q.data_ptr(), s.data_ptr(), n, k, stream_handle())
     count_launch()
     return q, s
 
@@ -304,7 +335,7 @@ def gemm_mx8(a_q: torch.Tensor, a_s: torch.Tensor, b_q: torch.Tensor, b_s: torch
         bias_ptr = bias.data_ptr()
     C.gemm_mx8(a_q.data_ptr(), a_q.stride(0), a_s.data_ptr(), a_s.stride(0), b_q.data_ptr(), b_q.stride(0), b_s.data_ptr(),
                b_s.stride(0), out.data_ptr(), out.stride(0), M, N, K, flags, bias_ptr, 0, sms,
-               status_words(a_q.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+               _status_of(a_q), stream_handle())
     count_launch()
     return out
 

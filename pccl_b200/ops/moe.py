@@ -12,7 +12,7 @@ import torch
 from .._native import C
 from ..engine import Engine
 from . import collectives as coll
-from .gemm import count_launch, status_words
+from .gemm import count_launch, status_words, stream_handle
 
 
 def quant_fp8_rows(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -20,7 +20,7 @@ def quant_fp8_rows(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     rows, hidden = x.shape
     q = torch.empty((rows, hidden), dtype=torch.uint8, device=x.device)
     s = torch.empty((rows, hidden // 128), dtype=torch.float32, device=x.device)
-    C.quant_fp8_rows(x.data_ptr(), q.data_ptr(), s.data_ptr(), rows, hidden, torch.cuda.current_stream().cuda_stream)
+    C.quant_fp8_rows(x.data_ptr(), q.data_ptr(), s.data_ptr(), rows, hidden, stream_handle())
     count_launch()
     return q, s
 
@@ -30,7 +30,7 @@ def quant_fp8_blocks(w: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     rows, cols = w.shape
     q = torch.empty((rows, cols), dtype=torch.uint8, device=w.device)
     s = torch.empty((rows // 128, cols // 128), dtype=torch.float32, device=w.device)
-    C.quant_fp8_blocks(w.data_ptr(), q.data_ptr(), s.data_ptr(), rows, cols, torch.cuda.current_stream().cuda_stream)
+    C.quant_fp8_blocks(w.data_ptr(), q.data_ptr(), s.data_ptr(), rows, cols, stream_handle())
     count_launch()
     return q, s
 
@@ -54,7 +54,7 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, row_off: torch.Tensor, n: int
     if side is not None:
         flags |= C.GEMM_GELU if gelu_out is not None else C.GEMM_DGELU
     C.gemm_grouped(a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), out.data_ptr(), out.stride(0), row_off.data_ptr(), groups,
-                   a.shape[0], n, K, flags, 0, status_words().data_ptr(), torch.cuda.current_stream().cuda_stream,
+                   a.shape[0], n, K, flags, 0, status_words().data_ptr(), stream_handle(),
                    side.data_ptr() if side is not None else 0)
     count_launch()
     return out
@@ -73,7 +73,7 @@ def grouped_wgrad(a0: torch.Tensor, b0: torch.Tensor, a1: torch.Tensor, b1: torc
         outs.append(d)
     maps = torch.empty(groups * 512, dtype=torch.uint8, device=a0.device)          # the kernel's descriptors
     C.gemm_grouped_wgrad(problems[0], problems[1], row_off.data_ptr(), groups, rows, maps.data_ptr(), status_words().data_ptr(),
-                         torch.cuda.current_stream().cuda_stream)
+                         stream_handle())
     count_launch(2)
     return outs[0], outs[1]
 
@@ -148,7 +148,7 @@ class MoEExchange:
         probs = torch.empty((T, K), dtype=torch.float32, device=dev)
         pos = torch.empty((T, K), dtype=torch.int32, device=dev)
         counts = torch.zeros(E, dtype=torch.int32, device=dev)
-        s = torch.cuda.current_stream().cuda_stream
+        s = stream_handle()
         C.moe_route(lg.data_ptr(), ids.data_ptr(), probs.data_ptr(), pos.data_ptr(), counts.data_ptr(), T, E, K, s)
         if eng.world > 1:
             coll.all_gather(eng, counts, self.counts_all.view(-1), lane=self.flag_lane)
@@ -171,7 +171,7 @@ class MoEExchange:
                        off(self.recv_s), off(self.y), self.epoch, self.flag_lane,
                        [x.data_ptr()] if x is not None else [], [ids.data_ptr()], [rows.data_ptr()],
                        [probs.data_ptr()] if probs is not None else [], [out.data_ptr()] if out is not None else [],
-                       [st.data_ptr()], self.blocks, 0, torch.cuda.current_stream().cuda_stream,
+                       [st.data_ptr()], self.blocks, 0, stream_handle(),
                        alias_off=off(self.alias), group_off=off(self.groups) if groups else 0, z_off=off(self.z),
                        gate=[gate.data_ptr()] if gate is not None else [], dedupe=dedupe)
         count_launch()
@@ -197,7 +197,7 @@ class MoEExchange:
         if out is None:
             out = torch.empty((self.cap, self.H), dtype=torch.bfloat16, device="cuda")
         C.moe_dequant(self.recv_q.data_ptr(), self.recv_s.data_ptr(), out.data_ptr(), plan["n_rows"].data_ptr(), self.cap,
-                      self.H, torch.cuda.current_stream().cuda_stream, alias=self.alias.data_ptr())
+                      self.H, stream_handle(), alias=self.alias.data_ptr())
         count_launch()
         return out
 
@@ -211,7 +211,7 @@ class MoEExchange:
     def experts(self, w1: torch.Tensor, w2: torch.Tensor, plan: Dict[str, torch.Tensor]) -> None:
         """w1: [experts_per_rank * d_ff, hidden], w2: [experts_per_rank * hidden, d_ff]; result in self.y."""
         C.moe_dequant(self.recv_q.data_ptr(), self.recv_s.data_ptr(), self.x_bf16.data_ptr(), plan["n_rows"].data_ptr(), self.cap,
-                      self.H, torch.cuda.current_stream().cuda_stream, alias=self.alias.data_ptr())
+                      self.H, stream_handle(), alias=self.alias.data_ptr())
         count_launch()
         d_ff = w1.shape[0] // self.epr
         h = grouped_gemm(self.x_bf16, w1, plan["row_off"], d_ff, gelu=True)
@@ -227,7 +227,7 @@ class MoEExchange:
             out = torch.empty((self.T, self.H), dtype=torch.bfloat16, device="cuda")
         if grouped:
             C.moe_reduce_groups(self.y.data_ptr(), self.z.data_ptr(), self.alias.data_ptr(), self.groups.data_ptr(),
-                                plan["n_rows"].data_ptr(), self.cap, self.H, torch.cuda.current_stream().cuda_stream)
+                                plan["n_rows"].data_ptr(), self.cap, self.H, stream_handle())
             count_launch()
         self._exchange("combine", None, ids, plan["rows"], probs, out, dedupe=grouped)
         return out

@@ -38,6 +38,7 @@ class _Bucket:
         self.exp_avg: torch.Tensor = None
         self.exp_avg_sq: torch.Tensor = None
         self.decay = True
+        self.event: torch.cuda.Event = None  # "the last gradient is written", recorded anew every step
 
 
 class ShardedDataParallel:
@@ -153,6 +154,7 @@ class ShardedDataParallel:
                 p.main_grad = b.grads[off:off + p.numel()].view(p.shape)
                 p._pccl_written = False
                 p._pccl_seen = 0
+                p._pccl_forwards = 0       # recorded uses since zero_grad (norms: nn/norm.py)
                 if not hasattr(p, "_pccl_uses"):
                     p._pccl_uses = 1           # a model sets 2 on a weight it uses twice (tied embeddings)
                 p._pccl_ready = self._make_ready(b, p)
@@ -194,8 +196,13 @@ class ShardedDataParallel:
         p._pccl_ready()
 
     def _launch_reduce(self, b: _Bucket) -> None:
-        ev = torch.cuda.Event(enable_timing=self._timing)
-        ev.record(torch.cuda.current_stream())
+        if self._timing:
+            ev = torch.cuda.Event(enable_timing=True)
+        else:
+            if b.event is None:
+                b.event = torch.cuda.Event()
+            ev = b.event
+        ev.record()
         self.comm_stream.wait_event(ev)
         if self._timing:
             marks = {"ready": ev, "start": torch.cuda.Event(enable_timing=True), "reduced": torch.cuda.Event(enable_timing=True),
@@ -241,6 +248,7 @@ class ShardedDataParallel:
             for p in b.params:
                 p._pccl_written = False
                 p._pccl_seen = 0
+                p._pccl_forwards = 0
                 p.grad = None
 
     def optimizer_step(self) -> None:

@@ -286,3 +286,54 @@ def test_fused_mlp_backward_matches_fp32_reference():
     fc2.bias.grad = None
     mlp(x, fc1, fc2, defer_fc2_bias_grad=True).backward(g)
     assert fc2.bias.grad is None
+
+
+def test_norm_gradients_reach_the_buckets_by_either_way():
+    """A norm used once is written into the flat bucket by the kernel; one that is used twice, or whose weight has a hook,
+    travels through autograd.  Both end in the gradient that plain autograd gives (bf16 sums of two terms: 2^-7)."""
+    import torch
+    import torch.nn as nn
+    from pccl_b200.nn import LayerNorm, Linear
+    from pccl_b200.parallel.dp import ShardedDataParallel
+
+    class Net(nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.once, self.twice, self.hooked = (LayerNorm(64, device="cuda") for _ in range(3))
+            self.lin = Linear(64, 64, device="cuda", init_std=0.3)
+
+        def forward(self, x, t):
+            h = self.twice(self.lin(self.once(x)))
+            return (self.hooked(self.twice(h + x)) * t).float().mean()
+
+    torch.manual_seed(3)
+    net = Net()
+    x, t = torch.randn(40, 64, device="cuda").bfloat16(), torch.randn(40, 64, device="cuda").bfloat16()
+    ref = torch.autograd.grad(net(x, t), list(net.parameters()))
+    seen = []
+    net.hooked.weight.register_hook(lambda g: seen.append(g.shape))
+    dp = ShardedDataParallel(net, heap_bytes=64 << 20)
+    for step in range(2):
+        dp.zero_grad()
+        net(x, t).backward()
+        if step == 0:                                     # before the update changes the parameters
+            for p, g in zip(net.parameters(), ref):
+                assert (p.main_grad.float() - g.float()).abs().max().item() <= 2 ** -7 * g.float().abs().max().item() + 1e-6
+        dp.optimizer_step()
+    assert len(seen) == 2 and all(p.grad is None for p in net.parameters())
+
+
+def test_forward_without_gradients_is_the_same_forward():
+    """Without gradients the layers run outside autograd.Function: same kernels, same bits, and transforms still refuse."""
+    import torch
+    from pccl_b200.nn import LayerNorm, Linear, LinearGelu, mlp
+    torch.manual_seed(4)
+    x, d = (torch.randn(3, 50, 72, device="cuda").bfloat16() for _ in range(2))
+    fc1, fc2, ln = LinearGelu(72, 96, device="cuda"), Linear(96, 72, device="cuda"), LayerNorm(72, device="cuda")
+    calls = [lambda: fc2(fc1(x), residual=d), lambda: mlp(x, fc1, fc2), lambda: ln(x), lambda: ln.add_norm(x, d)[0], lambda: ln.add_norm(x, d)[1]]
+    for f in calls:
+        with torch.no_grad():
+            plain = f()
+        assert torch.equal(plain, f().detach())
+    with torch.no_grad(), pytest.raises(RuntimeError):
+        torch.vmap(lambda v: ln(v))(x)

@@ -65,8 +65,7 @@ int gemmFp8(const void* A, int64_t lda, const float* sa, int ld_sa, const void* 
   int n_sm = deviceSmCount();
   if (sms > 0 && sms < n_sm) n_sm = sms;
   int grid = tiles < n_sm ? tiles : n_sm;
-  gemm_fp8_kernel<<<grid, gemm8::NUM_THREADS, gemm8::SMEM_BYTES, stream>>>(ta, tb, epi, sc, K, status);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launchOverlapped(gemm_fp8_kernel, dim3(grid), dim3(gemm8::NUM_THREADS), gemm8::SMEM_BYTES, stream, 1, ta, tb, epi, sc, K, status));
 }
 
 }  // namespace pccl

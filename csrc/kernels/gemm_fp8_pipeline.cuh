@@ -28,6 +28,7 @@
 
 #include "../base/instr.h"
 #include "gemm_pipeline.cuh"
+#include "launch.h"
 #include "prims.cuh"
 #include "tc05.cuh"
 
@@ -112,6 +113,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = bar->tmem_base;
+  dev::pdl_wait();
   epi.attach_smem(smem + STAGES * STAGE_BYTES + 256);
 
   if (warp == 0) {
@@ -141,6 +143,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
           if (armed & (1u << s))
             for (uint32_t i = 0; i < (1u << 16) && !tc::mbar_try_wait(&bar->full[s], (armed_par >> s) & 1); ++i) {}
       }
+      dev::pdl_launch();                // the last load is on its way: the next kernel of the stream may move in
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer

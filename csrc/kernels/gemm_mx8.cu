@@ -18,10 +18,10 @@ namespace {
 __global__ void __launch_bounds__(gemmx::NUM_THREADS, 1)
 gemm_mx8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, gemm::StoreEpi epi,
                 gemmx::Scales sc, int K, uint32_t* status) {
-  gemm::GroupedSched sched{(epi.M + gemmx::BM - 1) / gemmx::BM, (epi.N + gemmx::BN - 1) / gemmx::BN, static_cast<int>(blockIdx.x),
+  gemm::GroupedSched sched{(epi.M + gemmx::BM - 1) / gemmx::BM, (epi.N + epi.bn - 1) / epi.bn, static_cast<int>(blockIdx.x),
                            static_cast<int>(gridDim.x)};
   gemm::NoGate gate;
-  gemmx::run(&tmA, &tmB, K, sc, sched, gate, epi, status);
+  gemmx::run(&tmA, &tmB, K, sc, sched, gate, epi, status, epi.bn);
 }
 
 // Smallest power of two >= amax / 448 (so that the scaled block fits e4m3), as a float and as its UE8M0 byte.
@@ -47,16 +47,24 @@ __device__ __forceinline__ uint2 quant8_mx(const float* f, float inv) {
   return make_uint2(w[0], w[1]);
 }
 
-// 16 consecutive lanes own one 1 x 128 block (8 values each)
+// 16 consecutive lanes own one 1 x 128 block (8 values each); rows are whole blocks, so the matrix is one list of blocks.  Four
+// loads in flight per thread.  A CTA per row took 61 us at 8192 x 8192 (its fp32-scale twin in moe.cu), this form 41: 201 MB at 4.9 TB/s.
 __global__ void __launch_bounds__(256) quant_rows_mx_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q,
-                                                            uint8_t* __restrict__ scales, long long rows, int k) {
-  const int nvec = k >> 3, G = k >> 7;
-  for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
-    for (int v = threadIdx.x; v < ((nvec + 31) & ~31); v += blockDim.x) {
+                                                            uint8_t* __restrict__ scales, long long nvec) {
+  dev::pdl_launch();
+  dev::pdl_wait();
+  for (long long v0 = static_cast<long long>(blockIdx.x) * 1024 + threadIdx.x; v0 - (threadIdx.x & 31) < nvec; v0 += static_cast<long long>(gridDim.x) * 1024) {
+    dev::Vec16 in[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (v0 + j * 256 < nvec) in[j] = dev::ld16(x + (v0 + j * 256) * 8);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const long long v = v0 + j * 256;
       float f[8];
       float amax = 0.f;
       if (v < nvec) {
-        dev::unpack<DT_BF16>(dev::ld16(x + r * k + v * 8), f);
+        dev::unpack<DT_BF16>(in[j], f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
       }
@@ -65,8 +73,8 @@ __global__ void __launch_bounds__(256) quant_rows_mx_kernel(const __nv_bfloat16*
       uint8_t byte;
       const float scale = pow2_scale(amax, &byte);
       if (v < nvec) {
-        *reinterpret_cast<uint2*>(q + r * k + v * 8) = quant8_mx(f, 1.0f / scale);
-        if ((v & 15) == 0) scales[r * G + (v >> 4)] = byte;
+        *reinterpret_cast<uint2*>(q + v * 8) = quant8_mx(f, 1.0f / scale);
+        if ((v & 15) == 0) scales[v >> 4] = byte;
       }
     }
   }
@@ -107,15 +115,30 @@ __global__ void __launch_bounds__(256) quant_blocks_mx_kernel(const __nv_bfloat1
 
 thread_local std::string g_errx;
 
+// Columns per tile: 224 unless narrower tiles fill the last round of CTAs better.  Measured time of a full round relative to
+// 224 columns (148 tiles of 128 rows each, K = 2048 and 8192, one B200, mean of the two): a round is bound by the operands
+// that an SM gets from L2, of which A's 128 rows stay.  1531 x 8192 x 3584: 192 tiles of 224 in two rounds, 276 of 160 in two.
+int pickWidthMx(int tiles_m, int n, int sms) {
+  static const struct { int bn; float round; } kWidths[] = {{224, 1.f}, {192, .89f}, {160, .83f}, {128, .78f}, {96, .75f}, {64, .70f}, {32, .68f}};
+  int best = gemmx::BN;
+  float best_cost = 0.f;
+  for (const auto& w : kWidths) {
+    const long long tiles = static_cast<long long>(tiles_m) * ((n + w.bn - 1) / w.bn);
+    const float cost = static_cast<float>((tiles + sms - 1) / sms) * w.round;
+    if (w.bn == gemmx::BN || cost < best_cost * 0.999f) { best = w.bn; best_cost = cost; }
+  }
+  return best;
+}
+
 }  // namespace
 
 const char* gemmMx8LastError() { return g_errx.c_str(); }
 
 int launchQuantMx8Rows(const void* x, void* q, uint8_t* scales, long long rows, int k, cudaStream_t stream) {
   if (k % 128 || rows <= 0) return static_cast<int>(cudaErrorInvalidValue);
-  const long long blocks = rows < 4096 ? rows : 4096;
-  quant_rows_mx_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scales, rows, k);
-  return static_cast<int>(cudaGetLastError());
+  const long long nvec = rows * (k >> 3), blocks = (nvec + 1023) / 1024, most = deviceSmCount() * 8ll;
+  return static_cast<int>(launchOverlapped(quant_rows_mx_kernel, dim3(static_cast<unsigned>(blocks < most ? blocks : most)), dim3(256), 0, stream, 1,
+                                           static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scales, nvec));
 }
 
 int launchQuantMx8Blocks(const void* w, void* q, uint8_t* scales, int rows, int cols, cudaStream_t stream) {
@@ -148,8 +171,11 @@ int gemmMx8(const void* A, int64_t lda, const uint8_t* sa, int ld_sa, const void
   }
   CUtensorMap ta, tb;
   if (!makeTensorMap2D(&ta, A, TM_U8, K, M, lda, gemmx::BK, gemmx::BM, &g_errx)) return static_cast<int>(cudaErrorInvalidValue);
-  if (!makeTensorMap2D(&tb, B, TM_U8, K, N, ldb, gemmx::BK, gemmx::BN, &g_errx)) return static_cast<int>(cudaErrorInvalidValue);
-  gemm::StoreEpi epi{D, D2, static_cast<const __nv_bfloat16*>(bias), ldd, M, N, flags};
+  int n_sm = deviceSmCount();
+  if (sms > 0 && sms < n_sm) n_sm = sms;
+  const int bn = pickWidthMx((M + gemmx::BM - 1) / gemmx::BM, N, n_sm);
+  if (!makeTensorMap2D(&tb, B, TM_U8, K, N, ldb, gemmx::BK, bn, &g_errx)) return static_cast<int>(cudaErrorInvalidValue);
+  gemm::StoreEpi epi{D, D2, static_cast<const __nv_bfloat16*>(bias), ldd, M, N, flags, bn};
   gemmx::Scales sc{sa, sb, ld_sa, ld_sb, M, N};
   static bool attr_set = false;
   if (!attr_set) {
@@ -157,12 +183,9 @@ int gemmMx8(const void* A, int64_t lda, const uint8_t* sa, int ld_sa, const void
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_set = true;
   }
-  int tiles = ((M + gemmx::BM - 1) / gemmx::BM) * ((N + gemmx::BN - 1) / gemmx::BN);
-  int n_sm = deviceSmCount();
-  if (sms > 0 && sms < n_sm) n_sm = sms;
-  int grid = tiles < n_sm ? tiles : n_sm;
-  gemm_mx8_kernel<<<grid, gemmx::NUM_THREADS, gemmx::SMEM_BYTES, stream>>>(ta, tb, epi, sc, K, status);
-  return static_cast<int>(cudaGetLastError());
+  const int tiles = ((M + gemmx::BM - 1) / gemmx::BM) * ((N + bn - 1) / bn);
+  return static_cast<int>(launchOverlapped(gemm_mx8_kernel, dim3(tiles < n_sm ? tiles : n_sm), dim3(gemmx::NUM_THREADS), gemmx::SMEM_BYTES, stream, 1,
+                                           ta, tb, epi, sc, K, status));
 }
 
 }  // namespace pccl

@@ -5,7 +5,7 @@
 // and nothing is promoted in registers (the exact-fp32-scale kernel of gemm_fp8_pipeline.cuh pays twice
 // the MMA time for that).
 //
-//   warp 0      TMA producer: 128 x 128 A and 224 x 128 B tiles (128-byte swizzle), 5 stages; `Gate` as in
+//   warp 0      TMA producer: 128 x 128 A and (up to) 224 x 128 B tiles (128-byte swizzle), 5 stages; `Gate` as in
 //               the other pipelines
 //   warp 1      MMA issuer: per stage four MMAs 128 x 224 x 32; every fourth stage it first copies the
 //               scale images of the next 512 values of K from shared memory into TMEM (tcgen05.cp
@@ -27,6 +27,7 @@
 
 #include "../base/instr.h"
 #include "gemm_pipeline.cuh"
+#include "launch.h"
 #include "prims.cuh"
 #include "tc05.cuh"
 
@@ -92,9 +93,10 @@ __device__ __forceinline__ void mma_mx8(uint32_t d_tmem, uint64_t a_desc, uint64
 // [15]/[16] A/B MN-major, [17,23) N>>3, [23] scale format (1 = UE8M0), [24,29) M>>4, [29,31) A scale id.
 __host__ __device__ constexpr uint32_t make_idesc_mx(uint32_t m, uint32_t n) { return ((n >> 3) << 17) | (1u << 23) | ((m >> 4) << 24); }
 
+// `width` (a multiple of 32, at most BN): columns of a tile.
 template <class Sched, class Gate, class Epi>
 __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* tmB, int K, const Scales& sc, const Sched& sched,
-                                    const Gate& gate, Epi& epi, uint32_t* status) {
+                                    const Gate& gate, Epi& epi, uint32_t* status, int width = BN) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* sf_smem = smem + STAGES * STAGE_BYTES;
@@ -103,6 +105,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
   const int num_kb = (K + BK - 1) / BK;
   const int num_kg = (num_kb + 3) / 4;
   volatile uint32_t* abort = &bar->abort;
+  const uint32_t stage_tx = static_cast<uint32_t>(A_BYTES + width * BK);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -131,6 +134,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = bar->tmem_base;
+  dev::pdl_wait();
   epi.attach_smem(nullptr);
 
   if (warp == 0) {
@@ -142,11 +146,11 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
       TileCoord t;
       for (int it = 0; ok && sched.get(it, &t); ++it) {
         if (!gate.wait(t, abort)) { ok = false; break; }
-        const int row0 = t.m * BM, col0 = t.n * BN;
+        const int row0 = t.m * BM, col0 = t.n * width;
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!tc::mbar_wait(&bar->empty[stage], phase ^ 1, abort)) { ok = false; break; }
           uint8_t* sa = smem + stage * STAGE_BYTES;
-          tc::mbar_arrive_expect_tx(&bar->full[stage], STAGE_BYTES);
+          tc::mbar_arrive_expect_tx(&bar->full[stage], stage_tx);
           armed |= 1u << stage;
           armed_par = (armed_par & ~(1u << stage)) | (phase << stage);
           tc::tma_load_2d(sa, tmA, &bar->full[stage], kb * BK, row0);
@@ -160,11 +164,12 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
           if (armed & (1u << s))
             for (uint32_t i = 0; i < (1u << 16) && !tc::mbar_try_wait(&bar->full[s], (armed_par >> s) & 1); ++i) {}
       }
+      dev::pdl_launch();                // the last load is on its way: the next kernel of the stream may move in
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (tc::elect_one()) {
-      constexpr uint32_t idesc0 = make_idesc_mx(BM, BN);
+      const uint32_t idesc0 = make_idesc_mx(BM, static_cast<uint32_t>(width));
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0, g = 0;       // g: 512-wide K groups issued so far
       bool ok = true;
@@ -221,7 +226,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
     const bool aligned4 = ((sc.ld_sa | sc.ld_sb) & 3) == 0 && ((reinterpret_cast<uintptr_t>(sc.sa) | reinterpret_cast<uintptr_t>(sc.sb)) & 3) == 0;
     uint32_t wa[4], wb[8];
     auto fetch = [&](const TileCoord& tt, int kg) {
-      const int row0 = tt.m * BM, col0 = tt.n * BN, kb0 = kg * 4;
+      const int row0 = tt.m * BM, col0 = tt.n * width, kb0 = kg * 4;
       const bool wide = aligned4 && kb0 + 4 <= num_kb;     // four scale bytes in one load
 #pragma unroll
       for (int q = 0; q < 4; ++q) {               // A: rows 32 q + lane
@@ -305,11 +310,11 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
       const TileCoord t0{t.m, 0, t.extra};           // the adapter gets absolute columns
       epi.tile_begin(t0);
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = 0; c < width / 32; ++c) {
         uint32_t r[32];
         tc::tmem_ld_32x32(taddr + c * 32, r);
         tc::tmem_ld_wait();
-        epi.strip(t0, quarter * 32 + lane, t.n * BN + c * 32, r);
+        epi.strip(t0, quarter * 32 + lane, t.n * width + c * 32, r);
       }
       tc::tc_fence_before();
       __syncwarp();

@@ -298,3 +298,22 @@ def test_colsum_kernel_matches_torch(rows, N):
     view = _rand((rows, N + 24), 42)[:, 8:8 + N] if N % 8 == 0 and N > 8 else None     # a column slice of a wider buffer
     if view is not None and view.data_ptr() % 16 == 0:
         assert (colsum(view).float() - view.float().sum(0)).abs().max().item() <= 1e-2 * max(1.0, view.float().sum(0).abs().max().item())
+
+
+@pytest.mark.parametrize("M,N", [(1, 40), (130, 1000), (300, 4104), (1531, 3584), (2000, 520), (19000, 232), (9000, 448)])
+def test_mx8_tile_widths(M, N):
+    """Sizes over which the launch picks tiles of 32 ... 224 columns, with ragged last tiles and scale blocks that a tile straddles.
+    fp32 output against the product of the dequantised operands: the sums differ in their order only."""
+    from pccl_b200.ops import check_status
+    from pccl_b200.ops.gemm import dequant_rows, gemm_mx8, quant_rows_mx, ue8m0_to_float
+    K = 384
+    a, w = _rand((M, K), 81), _rand((N, K), 82)
+    aq, a_s = quant_rows_mx(a)
+    wq, w_rows = quant_rows_mx(w)
+    w_s = w_rows[::128].contiguous()                      # one scale byte per 128 rows: any byte is as good as another here
+    out = gemm_mx8(aq, a_s, wq, w_s, out_dtype=torch.float32)
+    check_status("gemm_mx8")
+    af = dequant_rows(aq, ue8m0_to_float(a_s))
+    wf = wq.view(torch.float8_e4m3fn).float() * ue8m0_to_float(w_s).repeat_interleave(128, 1).repeat_interleave(128, 0)[:N]
+    ref = af.double() @ wf.double().t()
+    assert (out.double() - ref).abs().max().item() <= 2e-3 * max(1.0, ref.abs().max().item())      # a wrong scale or tile is off by O(1)

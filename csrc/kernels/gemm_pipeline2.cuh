@@ -142,7 +142,6 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = bar->tmem_base;
-  dev::pdl_launch();
   dev::pdl_wait();                    // nothing above touched global memory
   epi.attach_smem(smem + NSTAGES * STAGE_BYTES + BAR_BYTES);
   if constexpr (HasPatch<Epi>::value && NSTAGES == STAGES) epi.attach_patch(smem + NSTAGES * STAGE_BYTES + BAR_BYTES);
@@ -261,6 +260,9 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         }
       }
       if (!ok && atomicExch(const_cast<uint32_t*>(&bar->abort), 1u) == 0) dev::report(status, ST_TIMEOUT, blockIdx.x, 0, 0);
+      // The last load is on its way: the next kernel of the stream may move in.  Not earlier: its CTAs would wait on the SMs for
+      // the whole of this kernel, in the places that a kernel of another stream (the optimizer's) could work in.
+      dev::pdl_launch();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)

@@ -337,3 +337,51 @@ def test_forward_without_gradients_is_the_same_forward():
         assert torch.equal(plain, f().detach())
     with torch.no_grad(), pytest.raises(RuntimeError):
         torch.vmap(lambda v: ln(v))(x)
+
+
+@pytest.mark.parametrize("D", [8, 64, 256, 264, 768, 1544, 2048, 2056, 4096, 8192])
+@pytest.mark.parametrize("rows", [1, 5, 700])
+def test_layer_norm_backward_over_widths(D, rows):
+    """One to eight warps per row, one to eight rows side by side in a CTA, widths off the vector counts, fewer rows than a trip
+    takes; against fp64 on the same bf16 inputs.  dx is rounded once (2^-8 of its terms), column sums are fp32 sums of `rows`
+    terms rounded once."""
+    import torch
+    from pccl_b200.nn import LayerNorm
+    torch.manual_seed(D + rows)
+    ln = LayerNorm(D, device="cuda")
+    ln.weight.data.copy_(torch.randn(D, device="cuda").bfloat16())
+    x, d, gs, gy = (torch.randn(rows, D, device="cuda").bfloat16() for _ in range(4))
+    xr, dr = x.clone().requires_grad_(True), d.clone().requires_grad_(True)
+    prev = torch.nn.Parameter(torch.zeros(D, device="cuda").bfloat16())
+    s, y = ln.add_norm(xr, dr, prev)
+    got = torch.autograd.grad([s, y], [xr, ln.weight, ln.bias, prev], [gs, gy])
+    s64 = s.detach().double().requires_grad_(True)
+    w64, b64 = ln.weight.detach().double().requires_grad_(True), torch.zeros(D, device="cuda", dtype=torch.float64, requires_grad=True)
+    y64 = F.layer_norm(s64, (D,), w64, b64, ln.eps)
+    dx, dw, db = torch.autograd.grad(y64, [s64, w64, b64], gy.double())
+    dx = dx + gs.double()
+    for a, b in zip(got, (dx, dw, db, dx.sum(0))):
+        assert (a.double() - b).abs().max().item() <= 2 ** -8 * b.abs().max().item() + 1e-4
+
+
+@pytest.mark.parametrize("vocab", [7, 1001, 50257])
+def test_cross_entropy_with_masked_and_large_logits(vocab):
+    """Logits of -inf (masked classes, whole stretches of them), of the type's lowest value and of +-3e4: the running maximum starts
+    at -inf and grows late in the row."""
+    import torch
+    from pccl_b200.ops.elementwise import cross_entropy_
+    torch.manual_seed(vocab)
+    ld = (vocab + 7) // 8 * 8
+    lg = (torch.randn(6, ld, device="cuda") * 4).bfloat16()[:, :vocab]
+    lg[1, : vocab // 2] = float("-inf")
+    lg[2, vocab // 2:] = float("-inf")
+    lg[3] = torch.finfo(torch.bfloat16).min
+    lg[4] = torch.linspace(-3e4, 3e4, vocab, device="cuda").bfloat16()
+    lg[5, : vocab - 1] = float("-inf")
+    tgt = torch.tensor([0, vocab - 1, 0, 3, vocab - 1, vocab - 1], device="cuda")
+    ref = lg.double().requires_grad_(True)
+    loss64 = F.cross_entropy(ref, tgt, reduction="none")
+    g64, = torch.autograd.grad(loss64.sum(), ref)
+    loss = cross_entropy_(lg, tgt)
+    assert ((loss.double() - loss64).abs() <= 1e-5 * loss64.abs() + 1e-5).all()      # 3e4 in fp32: 2^-24 relative, a few roundings
+    assert (lg.double() - g64).abs().max().item() <= 2 ** -8

@@ -134,13 +134,14 @@ void bindFused(py::module_& m) {
     check(gemmGroupedWgrad(problem(p0), problem(p1), reinterpret_cast<const int*>(row_off), groups, max_rows, reinterpret_cast<void*>(maps),
                            reinterpret_cast<uint32_t*>(status), reinterpret_cast<cudaStream_t>(stream)), "gemm_grouped_wgrad");
   });
+  m.attr("GEMM_GELU_FULL") = static_cast<uint32_t>(GEMM_GELU_FULL);
   m.attr("GEMM_DGELU") = static_cast<uint32_t>(GEMM_DGELU);
   m.attr("GEMM_GELU_INPLACE") = static_cast<uint32_t>(GEMM_GELU_INPLACE);
 
   // ---- production: this process is one rank -------------------------------------------------------
   m.def("ag_gemm", [](Engine& e, uint64_t x_off, int M, int N, int K, uint64_t w, int64_t ldw, uint64_t d, int64_t ldd,
                       uint64_t bias, uint64_t ready, uint64_t epoch, int n_copy, int ctas, int flag_lane, uint64_t status,
-                      uint64_t stream, bool b_mn) {
+                      uint64_t stream, bool b_mn, uint32_t flags, uint64_t d2, uint64_t colsum) {
     AgGemmArgs A{};
     A.w = e.worldTable();
     A.nvirt = 1;
@@ -148,7 +149,8 @@ void bindFused(py::module_& m) {
     A.x_off = x_off; A.epoch = epoch; A.bar_epoch = e.nextEpoch(flag_lane); A.n_copy = n_copy; A.flag_lane = flag_lane;
     A.spin_ns = kDefaultSpinLimit;
     A.tail_tiles = static_cast<int>(LaunchEnvironments::getInt("PCCL_AG_TAIL", -1));     // -1: from the cost model
-    A.flags = bias ? GEMM_BIAS : 0;
+    A.flags = flags | (bias ? GEMM_BIAS : 0);
+    A.r[0].D2 = reinterpret_cast<void*>(d2); A.r[0].colsum = reinterpret_cast<float*>(colsum);
     A.r[0].D = reinterpret_cast<void*>(d); A.r[0].ldd = ldd; A.r[0].bias = reinterpret_cast<const void*>(bias);
     A.ready_off = ready; A.r[0].status = reinterpret_cast<uint32_t*>(status);
     A.r[0].rank = e.rank();
@@ -156,10 +158,12 @@ void bindFused(py::module_& m) {
     check(launchAgGemm(A, &h, ctas, reinterpret_cast<cudaStream_t>(stream)), "ag_gemm");
   }, py::arg("engine"), py::arg("x_off"), py::arg("M"), py::arg("N"), py::arg("K"), py::arg("w"), py::arg("ldw"), py::arg("d"), py::arg("ldd"),
      py::arg("bias"), py::arg("ready"), py::arg("epoch"), py::arg("n_copy"), py::arg("ctas"), py::arg("flag_lane"), py::arg("status"),
-     py::arg("stream"), py::arg("b_mn") = false);
+     py::arg("stream"), py::arg("b_mn") = false, py::arg("flags") = 0, py::arg("d2") = 0, py::arg("colsum") = 0);
   m.def("gemm_rs", [](Engine& e, uint64_t y, int64_t ldy, uint64_t w, int64_t ldw, uint64_t out, int64_t ldo, int M, int N, int K,
-                      uint64_t stage_off, uint64_t flag_off2, uint64_t epoch, int ctas, uint64_t status, uint64_t stream, bool b_mn) {
+                      uint64_t stage_off, uint64_t flag_off2, uint64_t epoch, int ctas, uint64_t status, uint64_t stream, bool b_mn,
+                      uint64_t bias) {
     GemmRsArgs A{};
+    A.r[0].bias = reinterpret_cast<const void*>(bias);
     A.w = e.worldTable();
     A.nvirt = 1;
     A.M = M; A.N = N; A.K = K; A.M_local = M / e.world();
@@ -170,7 +174,7 @@ void bindFused(py::module_& m) {
     check(launchGemmRs(A, &h, ctas, reinterpret_cast<cudaStream_t>(stream)), "gemm_rs");
   }, py::arg("engine"), py::arg("y"), py::arg("ldy"), py::arg("w"), py::arg("ldw"), py::arg("out"), py::arg("ldo"), py::arg("M"), py::arg("N"),
      py::arg("K"), py::arg("stage_off"), py::arg("flag_off2"), py::arg("epoch"), py::arg("ctas"), py::arg("status"), py::arg("stream"),
-     py::arg("b_mn") = false);
+     py::arg("b_mn") = false, py::arg("bias") = 0);
   // ---- block-scaled fp8 forms ------------------------------------------------------------------------
   // One entry per (virtual) rank in the lists; with an engine the lists have one entry and the world is the engine's.
   m.def("ag_gemm_fp8", [](Engine* e, const std::vector<uint64_t>& heaps, uint64_t flag_off, uint64_t x_off, uint64_t xs_off, int M, int N,

@@ -38,6 +38,10 @@ struct AgGemmRank {
   void* Dq;                   // when set, the output is quantised instead: e4m3 [M, ldq] ...
   float* Ds;                  // ... with fp32 1 x 128 scales [M, N/128]
   long long ldq;
+  // bf16 CTA-pair form, D's layout: GELU of the output (flags GEMM_GELU), or the pre-activation of GEMM_DGELU, which also adds
+  // the column sums of D to `colsum` (fp32 [N], or null)
+  void* D2;
+  float* colsum;
 };
 
 struct AgGemmArgs {
@@ -52,7 +56,7 @@ struct AgGemmArgs {
   int n_copy;                 // CTAs that pull peer rows (the rest compute)
   int flag_lane;
   uint64_t spin_ns;
-  uint32_t flags;             // GEMM_BIAS, GEMM_GELU_INPLACE (fp8 path)
+  uint32_t flags;             // GEMM_BIAS; bf16: GEMM_GELU (| GEMM_GELU_FULL), GEMM_DGELU; fp8: GEMM_GELU_INPLACE
   int elem_bytes;             // 2 (bf16 X) or 1 (e4m3 X with scales at xs_off); 0 is read as 2
   uint64_t xs_off;            // fp8: heap offset of the symmetric gathered scales [M, K/128]: fp32, or UE8M0 bytes (scale_bytes 1)
   int scale_bytes;            // 4 (fp32 scales; 0 is read as 4) or 1 (UE8M0 bytes, hardware block scaling)
@@ -76,6 +80,7 @@ struct GemmRsRank {
   const float* y_scale;       // fp32 [M, ld_ys]
   const float* w_scale;       // fp32 [N/128, ld_ws]
   int ld_ys, ld_ws;
+  const void* bias;           // bf16 [N], added to this rank's rows, or null (16-byte aligned)
 };
 
 struct GemmRsArgs {

@@ -39,8 +39,9 @@ __device__ __forceinline__ void probe_stamp(unsigned long long* p, int word) {
   if (p && threadIdx.x == 0) p[word] = dev::global_timer_ns();
 }
 
-template <bool B_MN, bool PAIR>
-__global__ void __launch_bounds__(NUM_THREADS, 1) ag_gemm_kernel(const __grid_constant__ AgGemmArgs A) {
+// DGELU (CTA pairs): the product is multiplied by gelu'(pre) and its column sums taken in the epilogue, with eight epilogue warps.
+template <bool B_MN, bool PAIR, bool DGELU = false>
+__global__ void __launch_bounds__(DGELU ? gemm2::NUM_THREADS_WIDE : NUM_THREADS, 1) ag_gemm_kernel(const __grid_constant__ AgGemmArgs A) {
   const AgGemmRank& R = A.r[blockIdx.y];
   unsigned long long* const probe = cta_probe(A.probe);
   probe_stamp(probe, 4);
@@ -63,8 +64,15 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) ag_gemm_kernel(const __grid_co
   AgSched sched{R.rank, A.w.world, tiles_ml / unit, tiles_n, group_first, group_size, copier ? total - tail : 0, copier ? total : total - tail};
   AgGate gate{reinterpret_cast<const uint32_t*>(A.w.heap[R.rank] + A.ready_off), R.rank,
               static_cast<uint32_t>(A.epoch) * static_cast<uint32_t>(A.n_copy), A.spin_ns, probe};
-  StoreEpi epi{R.D, nullptr, static_cast<const __nv_bfloat16*>(R.bias), R.ldd, A.M, A.N, A.flags};
-  if constexpr (PAIR) {
+  StoreEpi epi{R.D, R.D2, static_cast<const __nv_bfloat16*>(R.bias), R.ldd, A.M, A.N, A.flags};
+  if constexpr (DGELU) {
+    DgeluEpiT<true> de{static_cast<__nv_bfloat16*>(R.D), static_cast<const __nv_bfloat16*>(R.D2), R.colsum, R.ldd, A.M, A.N};
+    const int cta = static_cast<int>(tc::cluster_ctarank());
+    gemm2::PairEpi<DgeluEpiT<true>> pe{de, cta};
+    gemm2::PairGate<AgGate> pg{gate, cta};
+    gemm2::run<false, B_MN, AgSched, gemm2::PairGate<AgGate>, gemm2::PairEpi<DgeluEpiT<true>>, gemm2::STAGES, 1, false, 8>(&R.tmA, &R.tmB, A.K, sched, pg, pe,
+                                                                                                                   R.status);
+  } else if constexpr (PAIR) {
     const int cta = static_cast<int>(tc::cluster_ctarank());
     gemm2::PairEpi<StoreEpi> pe{epi, cta};
     gemm2::PairGate<AgGate> pg{gate, cta};
@@ -133,6 +141,13 @@ int launchAgGemm(AgGemmArgs& A, const AgGemmHost* host, int ctas, cudaStream_t s
   const bool pair = A.M_local % 256 == 0 && ctas % 2 == 0;
   if (pair && (A.n_copy & 1)) A.n_copy += 1;
   A.probe = g_probe;
+  const bool dgelu = A.flags & GEMM_DGELU;
+  for (int v = 0; v < nv; ++v) {
+    if (((A.flags & (GEMM_GELU | GEMM_DGELU)) && (!A.r[v].D2 || reinterpret_cast<uintptr_t>(A.r[v].D2) % 16)) || (dgelu && (!pair || A.N % 32 || A.r[v].ldd % 8))) {
+      g_err = "ag_gemm: the GELU forms need a 16-byte aligned D2; the GELU-backward form 256 rows per rank and N a multiple of 32";
+      return static_cast<int>(cudaErrorInvalidValue);
+    }
+  }
   if (A.tail_tiles < 0 && A.n_copy > 0) {
     // Size of the tail from a cost model: the copy CTAs are busy for about t_copy (a copy CTA was measured to push about
     // 6.6 GB/s: 24 KiB in flight against a few microseconds of store round trip), a tile takes t_tile at ~1.5 PFLOP/s over
@@ -157,18 +172,19 @@ int launchAgGemm(AgGemmArgs& A, const AgGemmHost* host, int ctas, cudaStream_t s
     }
   }
   dim3 grid(ctas, nv);
-  const int which = (host[0].b_mn ? 1 : 0) + (pair ? 2 : 0);
-  static bool set[4] = {false, false, false, false};
+  const int which = dgelu ? (host[0].b_mn ? 5 : 4) : (host[0].b_mn ? 1 : 0) + (pair ? 2 : 0);
+  static bool set[6] = {false, false, false, false, false, false};
   auto k00 = ag_gemm_kernel<false, false>; auto k10 = ag_gemm_kernel<true, false>;
   auto k01 = ag_gemm_kernel<false, true>;  auto k11 = ag_gemm_kernel<true, true>;
-  auto kern = which == 0 ? k00 : which == 1 ? k10 : which == 2 ? k01 : k11;
+  auto d0 = ag_gemm_kernel<false, true, true>; auto d1 = ag_gemm_kernel<true, true, true>;
+  auto kern = which == 0 ? k00 : which == 1 ? k10 : which == 2 ? k01 : which == 3 ? k11 : which == 4 ? d0 : d1;
   const int smem_bytes = pair ? gemm2::SMEM_BYTES : SMEM_BYTES;      // the pair pipeline's ring and barrier area are its own
   if (!set[which]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     if (e != cudaSuccess) return static_cast<int>(e);
     set[which] = true;
   }
-  if (pair) return static_cast<int>(gemm2::launch_pairs(kern, grid, NUM_THREADS, smem_bytes, stream, true, A));
+  if (pair) return static_cast<int>(gemm2::launch_pairs(kern, grid, dgelu ? gemm2::NUM_THREADS_WIDE : NUM_THREADS, smem_bytes, stream, true, A));
   void* args[] = {&A};
   return static_cast<int>(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kern), grid, dim3(NUM_THREADS), args, SMEM_BYTES, stream));
 }
@@ -181,6 +197,7 @@ int launchGemmRs(GemmRsArgs& A, const GemmRsHost* host, int ctas, cudaStream_t s
     return static_cast<int>(cudaErrorInvalidValue);
   }
   for (int v = 0; v < nv; ++v) {
+    if (reinterpret_cast<uintptr_t>(A.r[v].bias) % 16) { g_err = "gemm_rs: the bias must be 16-byte aligned"; return static_cast<int>(cudaErrorInvalidValue); }
     if (!makeTensorMap2D(&A.r[v].tmA, host[v].Y, TM_BF16, A.K, A.M, host[v].ldy, BK, BM, &g_err)) return static_cast<int>(cudaErrorInvalidValue);
     if (host[v].b_mn != host[0].b_mn) { g_err = "gemm_rs: all ranks must use the same operand form"; return static_cast<int>(cudaErrorInvalidValue); }
     const bool okB = host[v].b_mn ? makeTensorMap2D(&A.r[v].tmB, host[v].W, TM_BF16, A.N, A.K, host[v].ldw, 64, BK, &g_err)

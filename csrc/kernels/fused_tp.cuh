@@ -291,6 +291,16 @@ struct RsEpiT {
         for (int k = 0; k < 8; ++k) v[i + k] += f[k];
       }
     }
+    if (R->bias) {
+      const __nv_bfloat16* b = static_cast<const __nv_bfloat16*>(R->bias) + col;      // the same for all lanes
+#pragma unroll
+      for (int i = 0; i < 32; i += 8) {
+        float f[8];
+        dev::unpack<DT_BF16>(dev::ld16(b + i), f);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[i + k] += f[k];
+      }
+    }
     __nv_bfloat16* out = static_cast<__nv_bfloat16*>(R->out) + row_local * R->ldo + col;
 #pragma unroll
     for (int i = 0; i < 32; i += 8) dev::st16(out + i, dev::pack<DT_BF16>(v + i));

@@ -23,7 +23,8 @@ enum GemmFlags : uint32_t {
   GEMM_ROW_STORES = 1u << 9,  // epilogue stores straight from the accumulator layout (a row per lane) instead of through the
                               // coalescing patch: for comparison runs
   GEMM_SKINNY = 1u << 10,     // few rows (M <= 256, A K-major): weights on the tile's M side, K split over a cluster (gemm_skinny.cu)
-  GEMM_DGELU = 1u << 11,      // grouped GEMM: D = A*B^T .* gelu_tanh'(D2) (D2 bf16, D's layout, read only)
+  GEMM_DGELU = 1u << 11,      // grouped and all-gather GEMM: D = A*B^T .* gelu_tanh'(D2) (D2 bf16, D's layout, read only)
+  GEMM_GELU_FULL = 1u << 12,  // GEMM_GELU to full fp32 accuracy instead of through the hardware tanh (relative error 2^-11)
 };
 
 // D[M,N] (ldd) = A * B^T.  K-major operands: A is [M,K] with row stride lda, B is [N,K] with row

@@ -108,7 +108,9 @@ __device__ __forceinline__ void patch_load_bf16(uint8_t* P, int lane, const __nv
 // activation: D = (A * B^T) .* gelu'(pre), and the column sums of D (the bias gradient of the first layer) are added
 // to `colsum` (fp32, zeroed by the caller).  N % 32 == 0; `pre` has D's layout.  Runs on the CTA-pair kernels (eight epilogue
 // warps, coalescing patch).
-struct DgeluEpi {
+// FULL: gelu' to full fp32 accuracy (dgelu_logistic) instead of through the hardware tanh.
+template <bool FULL = false>
+struct DgeluEpiT {
   static constexpr bool kRow128 = false;
   __nv_bfloat16* D;
   const __nv_bfloat16* pre;
@@ -157,7 +159,7 @@ struct DgeluEpi {
     __syncwarp();
     if (col_in_tile + 32 < ((threadIdx.x >> 5) - 2 < 4 ? split() : bn)) fetch_ahead(t, quarter, lane, col_in_tile + 32);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * dgelu_tanh(x[i]);
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * (FULL ? dgelu_logistic(x[i]) : dgelu_tanh(x[i]));
     patch_store_bf16(P, lane, D + static_cast<long long>(row0) * ldd + col, ldd, v, M - row0);
     if (colsum) {
       // an epilogue warp holds 32 consecutive rows, one per lane; rows past M were multiplied from zero fill, so they add 0
@@ -166,6 +168,8 @@ struct DgeluEpi {
     }
   }
 };
+
+using DgeluEpi = DgeluEpiT<false>;
 
 struct StoreEpi {
   static constexpr bool kRow128 = false;   // takes 32-column strips
@@ -223,8 +227,13 @@ struct StoreEpi {
     }
     patch_store_bf16(P, lane, static_cast<__nv_bfloat16*>(D) + at0, ldd, v, rows_valid);
     if (flags & GEMM_GELU) {
+      if (flags & GEMM_GELU_FULL) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
+        for (int i = 0; i < 32; ++i) v[i] = gelu_logistic(v[i]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
+      }
       patch_store_bf16(P, lane, static_cast<__nv_bfloat16*>(D2) + at0, ldd, v, rows_valid);
     }
   }
@@ -298,7 +307,7 @@ struct StoreEpi {
       if (flags & GEMM_GELU) {
         __nv_bfloat16* d2 = static_cast<__nv_bfloat16*>(D2) + static_cast<long long>(row) * ldd + col;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
+        for (int i = 0; i < 32; ++i) v[i] = flags & GEMM_GELU_FULL ? gelu_logistic(v[i]) : gelu_tanh(v[i]);
 #pragma unroll
         for (int i = 0; i < 32; i += 8) dev::st16(d2 + i, dev::pack<DT_BF16>(v + i));
       }
@@ -310,7 +319,7 @@ struct StoreEpi {
         float x = (flags & GEMM_ACCUMULATE) ? v[i] + __bfloat162float(d[i]) : v[i];
         d[i] = __float2bfloat16_rn(x);
         if (flags & GEMM_GELU)
-          (static_cast<__nv_bfloat16*>(D2) + static_cast<long long>(row) * ldd + col)[i] = __float2bfloat16_rn(gelu_tanh(x));
+          (static_cast<__nv_bfloat16*>(D2) + static_cast<long long>(row) * ldd + col)[i] = __float2bfloat16_rn(flags & GEMM_GELU_FULL ? gelu_logistic(x) : gelu_tanh(x));
       }
     }
   }

@@ -47,17 +47,27 @@ class AllGatherGemm:
         self.flag_lane = flag_lane
 
     def __call__(self, w: torch.Tensor, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
-                 w_t: bool = False) -> torch.Tensor:
-        """``w`` is [N, K]; with ``w_t`` it is stored [K, N] and consumed transposed (no copy)."""
+                 w_t: bool = False, *, gelu_out: Optional[torch.Tensor] = None, dgelu: Optional[torch.Tensor] = None,
+                 colsum: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """``w`` is [N, K]; with ``w_t`` it is stored [K, N] and consumed transposed (no copy).  ``gelu_out`` (out's shape,
+        contiguous like it) receives gelu_tanh(out).  ``dgelu`` (a pre-activation of that shape; rows per rank a multiple of
+        256, N of 32) makes it ``out = product * gelu_tanh'(dgelu)``, and ``colsum`` (fp32 [N]) grows by its column sums."""
         n = w.shape[1] if w_t else w.shape[0]
         if w.dtype != torch.bfloat16 or w.shape[0 if w_t else 1] != self.K or w.stride(1) != 1:
             raise ValueError("AllGatherGemm: w must be bf16 [N, K] (or [K, N] with w_t)")
         if out is None:
             out = torch.empty((self.M, n), dtype=torch.bfloat16, device="cuda")
+        side, flags = (gelu_out, C.GEMM_GELU | C.GEMM_GELU_FULL) if gelu_out is not None else (dgelu, C.GEMM_DGELU if dgelu is not None else 0)
+        if side is not None and (side.dtype != torch.bfloat16 or side.shape != out.shape or side.stride() != out.stride()
+                                 or (gelu_out is not None and dgelu is not None)):
+            raise ValueError("AllGatherGemm: one of gelu_out and dgelu, bf16 with out's shape and strides")
+        if colsum is not None and (dgelu is None or colsum.dtype != torch.float32 or colsum.numel() != n or not colsum.is_contiguous()):
+            raise ValueError("AllGatherGemm: colsum goes with dgelu and is a contiguous fp32 vector of length N")
         self.epoch += 1
         C.ag_gemm(self.eng.raw, self.eng.heap_offset(self.x_full), self.M, n, self.K, w.data_ptr(), w.stride(0), out.data_ptr(),
                   out.stride(0), bias.data_ptr() if bias is not None else 0, self.eng.heap_offset(self.ready), self.epoch, self.n_copy,
-                  self.ctas, self.flag_lane, status_words().data_ptr(), stream_handle(), w_t)
+                  self.ctas, self.flag_lane, status_words().data_ptr(), stream_handle(), w_t, flags,
+                  side.data_ptr() if side is not None else 0, colsum.data_ptr() if colsum is not None else 0)
         count_launch()
         return out
 
@@ -78,8 +88,12 @@ class GemmReduceScatter:
         self.epoch = 0
         self.ctas = ctas or C.sm_count()
 
-    def __call__(self, y: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, w_t: bool = False) -> torch.Tensor:
-        """``w`` is [N, K]; with ``w_t`` it is stored [K, N] and consumed transposed (no copy)."""
+    def __call__(self, y: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, w_t: bool = False,
+                 bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """``w`` is [N, K]; with ``w_t`` it is stored [K, N] and consumed transposed (no copy).  ``bias`` (bf16 [N], 16-byte
+        aligned) is added to this rank's rows."""
+        if bias is not None and (bias.dtype != torch.bfloat16 or bias.numel() != self.N or not bias.is_contiguous()):
+            raise ValueError("GemmReduceScatter: bias must be a contiguous bf16 vector of length N")
         wn, wk = (w.shape[1], w.shape[0]) if w_t else (w.shape[0], w.shape[1])
         if y.shape[0] != self.M or wn != self.N or y.shape[1] != wk:
             raise ValueError("GemmReduceScatter: shape mismatch")
@@ -88,7 +102,7 @@ class GemmReduceScatter:
         self.epoch += 1
         C.gemm_rs(self.eng.raw, y.data_ptr(), y.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), self.M, self.N,
                   y.shape[1], self.eng.heap_offset(self.stage), self.eng.heap_offset(self.flags), self.epoch, self.ctas,
-                  status_words().data_ptr(), stream_handle(), w_t)
+                  status_words().data_ptr(), stream_handle(), w_t, bias.data_ptr() if bias is not None else 0)
         count_launch()
         return out
 

@@ -16,7 +16,14 @@ import torch.nn as nn
 
 from ..engine import Engine
 from ..ops.fused_tp import AllGatherGemm, GemmReduceScatter
-from ..ops.gemm import gemm
+from ..ops.elementwise import colsum
+from ..ops.gemm import gemm, gemm_dual
+
+
+def _column_sums(dy: torch.Tensor) -> torch.Tensor:
+    if dy.shape[1] % 8 == 0 and dy.data_ptr() % 16 == 0:
+        return colsum(dy)
+    return dy.sum(0, dtype=torch.float32).to(dy.dtype)
 
 
 class _ColumnFn(torch.autograd.Function):
@@ -37,16 +44,16 @@ class _ColumnFn(torch.autograd.Function):
         # dx_local = reduce_scatter_rows(dy @ W): W is [N1, K] = the [K_gemm, N_gemm] form -> w_t
         dx = layer.rs_bwd(dy, weight, w_t=True)
         dw = gemm(dy, layer.ag.x_full, a_t=True, b_t=True)            # [N1, K]
-        db = dy.sum(0, dtype=torch.float32).to(dy.dtype) if ctx.has_bias else None
-        return dx, dw, db, None
+        return dx, dw, _column_sums(dy) if ctx.has_bias else None, None
 
 
 class _RowFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, h, weight, layer):
-        z = layer.rs(h, weight)
+    def forward(ctx, h, weight, bias, layer):
+        z = layer.rs(h, weight, bias=bias)
         ctx.layer = layer
         ctx.save_for_backward(h, weight)
+        ctx.has_bias = bias is not None
         return z
 
     @staticmethod
@@ -56,7 +63,38 @@ class _RowFn(torch.autograd.Function):
         layer.ag_bwd.x_local.copy_(dz_local)
         dh = layer.ag_bwd(weight, w_t=True)                           # all_gather(dz) @ W2, W2 is [D, N1]
         dw = gemm(layer.ag_bwd.x_full, h, a_t=True, b_t=True)         # [D, N1]
-        return dh, dw, None
+        return dh, dw, _column_sums(dz_local.contiguous()) if ctx.has_bias else None, None
+
+
+class _MlpFn(torch.autograd.Function):
+    """Column-parallel layer, GELU and row-parallel layer as one node: GELU and its derivative run in the epilogues of the two
+    all-gather GEMMs (the derivative's also sums the first layer's bias gradient), the second bias in the reduce-scatter's,
+    and both weight gradients are one launch."""
+
+    @staticmethod
+    def forward(ctx, x_local, w1, b1, w2, b2, fc1, fc2):
+        fc1.ag.x_local.copy_(x_local)
+        act = torch.empty((fc1.ag.M, w1.shape[0]), dtype=torch.bfloat16, device=w1.device)
+        pre = fc1.ag(w1, b1, gelu_out=act)
+        z = fc2.rs(act, w2, bias=b2)
+        ctx.save_for_backward(w1, w2, pre, act)
+        ctx.layers, ctx.has_bias = (fc1, fc2), (b1 is not None, b2 is not None)
+        return z
+
+    @staticmethod
+    def backward(ctx, dz_local):
+        w1, w2, pre, act = ctx.saved_tensors
+        fc1, fc2 = ctx.layers
+        n1, d = w1.shape
+        dz_local = dz_local.contiguous()
+        fc2.ag_bwd.x_local.copy_(dz_local)
+        sums = torch.zeros(n1, dtype=torch.float32, device=w1.device) if ctx.has_bias[0] else None
+        dpre = fc2.ag_bwd(w2, w_t=True, dgelu=pre, colsum=sums)
+        dx = fc1.rs_bwd(dpre, w1, w_t=True)
+        dw1, dw2 = torch.empty_like(w1, memory_format=torch.contiguous_format), torch.empty_like(w2, memory_format=torch.contiguous_format)
+        gemm_dual(dpre, fc1.ag.x_full, dw1, fc2.ag_bwd.x_full, act, dw2, a_t=True, b_t=True)
+        return (dx, dw1, sums.to(torch.bfloat16) if sums is not None else None, dw2, _column_sums(dz_local) if ctx.has_bias[1] else None,
+                None, None)
 
 
 class ColumnParallelLinear(nn.Module):
@@ -96,8 +134,7 @@ class RowParallelLinear(nn.Module):
         self.ag_bwd = AllGatherGemm(eng, tokens, out_features, n_copy=n_copy, flag_lane=6)
 
     def forward(self, h: torch.Tensor) -> torch.Tensor:
-        z = _RowFn.apply(h, self.weight, self)
-        return z if self.bias is None else z + self.bias
+        return _RowFn.apply(h, self.weight, self.bias, self)
 
 
 class TensorParallelMLP(nn.Module):
@@ -109,4 +146,9 @@ class TensorParallelMLP(nn.Module):
         self.fc2 = RowParallelLinear(eng, tokens, d_ff, d_model, n_copy=n_copy)
 
     def forward(self, x_local: torch.Tensor) -> torch.Tensor:
-        return self.fc2(torch.nn.functional.gelu(self.fc1(x_local), approximate="tanh"))
+        fc1, fc2 = self.fc1, self.fc2
+        # One node where the GELU-backward epilogue fits (CTA pairs: 256 rows per rank; 32 columns) and nobody listens in between.
+        fits = (fc1.ag.M // fc1.eng.world) % 256 == 0 and fc1.weight.shape[0] % 32 == 0 and fc2.ag_bwd.ctas % 2 == 0
+        if fits and not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in (fc1, fc2)):
+            return _MlpFn.apply(x_local, fc1.weight, fc1.bias, fc2.weight, fc2.bias, fc1, fc2)
+        return fc2(torch.nn.functional.gelu(fc1(x_local), approximate="tanh"))

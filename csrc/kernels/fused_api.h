@@ -62,6 +62,7 @@ struct AgGemmArgs {
   int scale_bytes;            // 4 (fp32 scales; 0 is read as 4) or 1 (UE8M0 bytes, hardware block scaling)
   int tail_tiles;             // tiles at the end of the tile order that the copy CTAs compute once their rows are sent
   unsigned long long* probe;  // null, or kProbeWords x u64 per CTA (see setFusedProbe)
+  int bn;                     // tile width in columns (bf16 form; set by launchAgGemm)
   AgGemmRank r[kMaxVirt];
 };
 

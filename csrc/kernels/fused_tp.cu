@@ -21,6 +21,7 @@
 #include <string>
 
 #include "fused_api.h"
+#include "gemm_api.h"
 #include "fused_tp.cuh"
 #include "gemm_pipeline2.cuh"
 #include "tensormap.h"
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(DGELU ? gemm2::NUM_THREADS_WIDE : NUM_THREADS,
   }
   // The tile order is cut in two: the GEMM CTAs take all but the last tail_tiles, the copy CTAs take those once their
   // rows are on their way (otherwise their SMs would sit idle for the rest of the kernel).
-  const int tiles_ml = A.M_local / BM, tiles_n = (A.N + BN - 1) / BN;
+  const int tiles_ml = A.M_local / BM, tiles_n = (A.N + A.bn - 1) / A.bn;
   const int unit = PAIR ? 2 : 1;
   const long long total = static_cast<long long>(A.w.world) * (tiles_ml / unit) * tiles_n;
   const long long tail = A.n_copy > 0 ? (A.tail_tiles < total ? A.tail_tiles : total) : 0;
@@ -64,9 +65,9 @@ __global__ void __launch_bounds__(DGELU ? gemm2::NUM_THREADS_WIDE : NUM_THREADS,
   AgSched sched{R.rank, A.w.world, tiles_ml / unit, tiles_n, group_first, group_size, copier ? total - tail : 0, copier ? total : total - tail};
   AgGate gate{reinterpret_cast<const uint32_t*>(A.w.heap[R.rank] + A.ready_off), R.rank,
               static_cast<uint32_t>(A.epoch) * static_cast<uint32_t>(A.n_copy), A.spin_ns, probe};
-  StoreEpi epi{R.D, R.D2, static_cast<const __nv_bfloat16*>(R.bias), R.ldd, A.M, A.N, A.flags};
+  StoreEpi epi{R.D, R.D2, static_cast<const __nv_bfloat16*>(R.bias), R.ldd, A.M, A.N, A.flags, A.bn};
   if constexpr (DGELU) {
-    DgeluEpiT<true> de{static_cast<__nv_bfloat16*>(R.D), static_cast<const __nv_bfloat16*>(R.D2), R.colsum, R.ldd, A.M, A.N};
+    DgeluEpiT<true> de{static_cast<__nv_bfloat16*>(R.D), static_cast<const __nv_bfloat16*>(R.D2), R.colsum, R.ldd, A.M, A.N, A.bn};
     const int cta = static_cast<int>(tc::cluster_ctarank());
     gemm2::PairEpi<DgeluEpiT<true>> pe{de, cta};
     gemm2::PairGate<AgGate> pg{gate, cta};
@@ -141,6 +142,8 @@ int launchAgGemm(AgGemmArgs& A, const AgGemmHost* host, int ctas, cudaStream_t s
   const bool pair = A.M_local % 256 == 0 && ctas % 2 == 0;
   if (pair && (A.n_copy & 1)) A.n_copy += 1;
   A.probe = g_probe;
+  // single CTAs multiply 256-column tiles; pairs take the width that fills their last round (all tiles of a rank count)
+  A.bn = pair ? gemmPairTileN(A.M / 256, A.N, 0, 0, ctas / 2) : BN;
   const bool dgelu = A.flags & GEMM_DGELU;
   for (int v = 0; v < nv; ++v) {
     if (((A.flags & (GEMM_GELU | GEMM_DGELU)) && (!A.r[v].D2 || reinterpret_cast<uintptr_t>(A.r[v].D2) % 16)) || (dgelu && (!pair || A.N % 32 || A.r[v].ldd % 8))) {
@@ -154,9 +157,9 @@ int launchAgGemm(AgGemmArgs& A, const AgGemmHost* host, int ctas, cudaStream_t s
     // the whole GPU; the tail makes both groups finish together:
     //   (T - R) / G = t_copy / t_tile + R / C   with T tiles, G GEMM groups, C copy groups.
     const int unit = pair ? 2 : 1;
-    const double T = static_cast<double>(A.w.world) * (A.M_local / (BM * unit)) * ((A.N + BN - 1) / BN);
+    const double T = static_cast<double>(A.w.world) * (A.M_local / (BM * unit)) * ((A.N + A.bn - 1) / A.bn);
     const double C = A.n_copy / unit, G = (ctas - A.n_copy) / unit;
-    const double t_tile = 2.0 * BM * unit * BN * A.K / (1.5e15 / (148.0 / unit));
+    const double t_tile = 2.0 * BM * unit * A.bn * A.K / (1.5e15 / (148.0 / unit));
     const bool mc = A.w.mc_heap != nullptr && A.nvirt <= 1;      // one multicast store reaches every peer
     const double bytes = static_cast<double>(mc ? 1 : A.w.world - 1) * A.M_local * A.K * (A.elem_bytes ? A.elem_bytes : 2);
     const double t_copy = bytes / (6.6e9 * A.n_copy) + 20e-6;
@@ -164,10 +167,10 @@ int launchAgGemm(AgGemmArgs& A, const AgGemmHost* host, int ctas, cudaStream_t s
     A.tail_tiles = Rt > 0 ? static_cast<int>(Rt) : 0;
   }
   if (A.tail_tiles < 0) A.tail_tiles = 0;
-  // per-CTA TMA boxes: 128 rows of A; 256 rows of B (single CTA) or 128 (pair)
+  // per-CTA TMA boxes: 128 rows of A; 256 rows of B (single CTA) or half a tile's columns (pair)
   if (pair) {
     for (int v = 0; v < nv; ++v) {
-      const bool okB = host[v].b_mn ? true : makeTensorMap2D(&A.r[v].tmB, host[v].W, TM_BF16, A.K, A.N, host[v].ldw, BK, 128, &g_err);
+      const bool okB = host[v].b_mn ? true : makeTensorMap2D(&A.r[v].tmB, host[v].W, TM_BF16, A.K, A.N, host[v].ldw, BK, A.bn / 2, &g_err);
       if (!okB) return static_cast<int>(cudaErrorInvalidValue);
     }
   }

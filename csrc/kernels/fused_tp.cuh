@@ -48,6 +48,16 @@ __device__ __forceinline__ bool cta_peer_barrier(const World& W, int me, int lan
 // Within a row block consecutive tiles share the B panel (same n, different source rank).
 // [begin, end) is the slice of that order which this group of CTAs works through (`first` + it * `stride` inside it):
 // the GEMM CTAs take everything but the last `tail` tiles, the copy CTAs take the tail once their rows are sent.
+// Tile r of a panel of tiles_m x tiles_n: 16 rows of tiles at a time, column by column, so that their A rows stay in L2 while the
+// columns go by.  Down whole columns an A of 8192 x 8192 (134 MB) came from memory again for every two or three columns, which
+// a launch at the power limit pays for in clock.
+__device__ __forceinline__ void panel_tile(int r, int tiles_m, int tiles_n, int* m, int* n) {
+  const int per_group = GroupedSched::GROUP_M * tiles_n, g = r / per_group;
+  const int rr = r - g * per_group, gm = min(GroupedSched::GROUP_M, tiles_m - g * GroupedSched::GROUP_M);
+  *m = g * GroupedSched::GROUP_M + rr % gm;
+  *n = rr / gm;
+}
+
 struct AgSched {
   int me, world, tiles_ml, tiles_n, first, stride;
   long long begin, end;
@@ -56,9 +66,8 @@ struct AgSched {
     const int per_panel = tiles_ml * tiles_n;
     if (idx >= end || idx >= static_cast<long long>(world) * per_panel) return false;
     if (idx < per_panel) {
-      const int r = static_cast<int>(idx);
-      t->m = me * tiles_ml + r % tiles_ml;
-      t->n = r / tiles_ml;
+      panel_tile(static_cast<int>(idx), tiles_ml, tiles_n, &t->m, &t->n);
+      t->m += me * tiles_ml;
       t->extra = me;
       return true;
     }
@@ -207,8 +216,8 @@ struct RsSched {
     const int panel = static_cast<int>(idx / per_panel), r = static_cast<int>(idx % per_panel);
     int owner = me + 1 + panel;          // peers first, own rows last
     if (owner >= world) owner -= world;
-    t->m = owner * tiles_ml + r % tiles_ml;
-    t->n = r / tiles_ml;
+    panel_tile(r, tiles_ml, tiles_n, &t->m, &t->n);
+    t->m += owner * tiles_ml;
     t->extra = owner;
     return true;
   }

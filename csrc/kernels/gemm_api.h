@@ -91,6 +91,8 @@ int launchQuantMx8Blocks(const void* w, void* q, uint8_t* scales, int rows, int 
 const char* gemmMx8LastError();
 
 const char* gemmLastError();
+// Tile width (columns) of a CTA-pair launch over up to two problems of `tiles` 256-row tiles and n columns each.
+int gemmPairTileN(int tiles_m0, int n0, int tiles_m1, int n1, int pairs);
 // Tile scheduling of the CTA-pair kernels: 1 = tiles are handed out at run time (an atomic counter per stream), 0 = fixed
 // round-robin lists, -1 = what the environment says (PCCL_GEMM_DYNAMIC, default 1).
 void gemmSetDynamic(int mode);

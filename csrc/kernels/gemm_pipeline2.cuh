@@ -62,7 +62,7 @@ template <class E, class = void> struct HasPatch : std::false_type {};
 template <class E> struct HasPatch<E, std::void_t<decltype(std::declval<E&>().attach_patch(nullptr))>> : std::true_type {};
 // An epilogue with `int width()` runs the whole problem on tiles of that many columns (a multiple of 32, at most BN): the MMA
 // is issued with N = width and each CTA loads width / 2 rows of B (rounded up to whole 64-column boxes where B is MN-major).
-// The launch picks the width so that the tiles fill the last round of CTA pairs (gemm_tc05.cu: pickTileN).
+// The launch picks the width so that the tiles fill the last round of CTA pairs (gemm_tc05.cu: gemmPairTileN).
 template <class E, class = void> struct HasWidth : std::false_type {};
 template <class E> struct HasWidth<E, std::void_t<decltype(std::declval<const E&>().width())>> : std::true_type {};
 template <class E, class = void> struct HasVarN : std::false_type {};

@@ -154,27 +154,6 @@ uint32_t* tileCounterFor(cudaStream_t stream) {
   return p;
 }
 
-// Tile width of a CTA-pair launch: 256 columns unless a narrower tile fills the last round of pairs better.  A round of
-// narrower tiles is not cheaper in proportion -- every k-block still loads the pair's 256 rows of A, and L2 -> SM is what
-// bounds it -- so the candidates are weighed with the measured time of a full round relative to a round of 256-wide tiles
-// (16384 x 8192 x 2048 and 16384 x 2048 x 2048, one B200: 12.4 us at 256, 11.3 / 10.0 / 9.1 / 7.9 / 7.0 / 6.7 / 6.0 us at
-// 224 ... 32).  Measured both ways (us, 256 wide -> chosen): 1531 x 2048 x 8192 53 -> 47 (48 tiles on 74 pairs -> 66),
-// 2331 x 768 x 3072 28.6 -> 22.6, 8192 x 3584 x 8192 328 -> 316 (448 tiles = 6.05 rounds -> 512 = 6.9); 1531 x 6144 x 2048
-// (144 tiles, 1.95 rounds) stays at 256: 40 against 44 at 192.  Two problems (gemmBf16Dual) share one width.
-int pickTileN(int tiles_m0, int n0, int tiles_m1, int n1, int pairs) {
-  static const struct { int bn; float round; } kWidths[] = {{256, 1.f}, {224, .91f}, {192, .80f}, {160, .725f},
-                                                            {128, .62f}, {96, .56f}, {64, .53f}, {32, .48f}};
-  if (pairs < 1) pairs = 1;
-  int best = 256;
-  float best_cost = 0.f;
-  for (const auto& w : kWidths) {
-    const long long tiles = static_cast<long long>(tiles_m0) * ((n0 + w.bn - 1) / w.bn) + static_cast<long long>(tiles_m1) * ((n1 + w.bn - 1) / w.bn);
-    const float cost = static_cast<float>((tiles + pairs - 1) / pairs) * w.round;
-    if (w.bn == 256 || cost < best_cost * 0.999f) { best = w.bn; best_cost = cost; }
-  }
-  return best;
-}
-
 // One CTA pair per cluster, allowed to start before the previous kernel of the stream has ended (launch.h).
 template <class... KArgs, class... Args>
 int launchPairKernel(void (*kern)(KArgs...), int grid, cudaStream_t stream, bool* attr_set, Args... args) {
@@ -211,6 +190,27 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const StoreEpi& epi, in
 
 const char* gemmLastError() { return g_err.c_str(); }
 
+// Tile width of a CTA-pair launch: 256 columns unless a narrower tile fills the last round of pairs better.  A round of
+// narrower tiles is not cheaper in proportion -- every k-block still loads the pair's 256 rows of A, and L2 -> SM is what
+// bounds it -- so the candidates are weighed with the measured time of a full round relative to a round of 256-wide tiles
+// (16384 x 8192 x 2048 and 16384 x 2048 x 2048, one B200: 12.4 us at 256, 11.3 / 10.0 / 9.1 / 7.9 / 7.0 / 6.7 / 6.0 us at
+// 224 ... 32).  Measured both ways (us, 256 wide -> chosen): 1531 x 2048 x 8192 53 -> 47 (48 tiles on 74 pairs -> 66),
+// 2331 x 768 x 3072 28.6 -> 22.6, 8192 x 3584 x 8192 328 -> 316 (448 tiles = 6.05 rounds -> 512 = 6.9); 1531 x 6144 x 2048
+// (144 tiles, 1.95 rounds) stays at 256: 40 against 44 at 192.  Two problems (gemmBf16Dual) share one width.
+int gemmPairTileN(int tiles_m0, int n0, int tiles_m1, int n1, int pairs) {
+  static const struct { int bn; float round; } kWidths[] = {{256, 1.f}, {224, .91f}, {192, .80f}, {160, .725f},
+                                                            {128, .62f}, {96, .56f}, {64, .53f}, {32, .48f}};
+  if (pairs < 1) pairs = 1;
+  int best = 256;
+  float best_cost = 0.f;
+  for (const auto& w : kWidths) {
+    const long long tiles = static_cast<long long>(tiles_m0) * ((n0 + w.bn - 1) / w.bn) + static_cast<long long>(tiles_m1) * ((n1 + w.bn - 1) / w.bn);
+    const float cost = static_cast<float>((tiles + pairs - 1) / pairs) * w.round;
+    if (w.bn == 256 || cost < best_cost * 0.999f) { best = w.bn; best_cost = cost; }
+  }
+  return best;
+}
+
 void gemmSetDynamic(int mode) { g_dynamic = mode < 0 ? -1 : (mode ? 1 : 0); }
 
 int gemmResetTileCounters() {
@@ -246,7 +246,7 @@ int gemmBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, in
   if (flags & GEMM_PAIR) {
     int n_sm2 = deviceSmCount();
     if (sms > 0 && sms < n_sm2) n_sm2 = sms;
-    const int bn = pickTileN((M + 255) / 256, N, 0, 0, n_sm2 / 2);
+    const int bn = gemmPairTileN((M + 255) / 256, N, 0, 0, n_sm2 / 2);
     epi.bn = bn;
     // per-CTA boxes: 128 rows of A and half of the tile's columns of B
     CUtensorMap pa, pb;
@@ -287,7 +287,7 @@ int gemmBf16Dgelu(const void* A, int64_t lda, const void* B, int64_t ldb, void* 
   }
   int n_sm = deviceSmCount();
   if (sms > 0 && sms < n_sm) n_sm = sms;
-  const int bn = pickTileN((M + 255) / 256, N, 0, 0, n_sm / 2);
+  const int bn = gemmPairTileN((M + 255) / 256, N, 0, 0, n_sm / 2);
   CUtensorMap pa, pb;
   if (!makeTensorMap2D(&pa, A, TM_BF16, K, M, lda, BK, 128, &g_err)) return static_cast<int>(cudaErrorInvalidValue);
   if (!b_mn ? !makeTensorMap2D(&pb, B, TM_BF16, K, N, ldb, BK, bn / 2, &g_err) : !makeTensorMap2D(&pb, B, TM_BF16, N, K, ldb, 64, BK, &g_err))
@@ -305,7 +305,7 @@ int gemmBf16Dual(const GemmProblem& p0, const GemmProblem& p1, int K, uint32_t f
   if (K <= 0) return 0;
   int n_sm = deviceSmCount();
   if (sms > 0 && sms < n_sm) n_sm = sms;
-  const int bn = pickTileN((p0.M + 255) / 256, p0.N, (p1.M + 255) / 256, p1.N, n_sm / 2);
+  const int bn = gemmPairTileN((p0.M + 255) / 256, p0.N, (p1.M + 255) / 256, p1.N, n_sm / 2);
   DualMaps maps;
   DualEpi epi;
   for (int q = 0; q < 2; ++q) {

@@ -2,6 +2,7 @@
 #include <pybind11/pybind11.h>
 #include <pybind11/stl.h>
 
+#include <array>
 #include <stdexcept>
 #include <string>
 
@@ -100,6 +101,13 @@ void bindGemm(py::module_& m) {
                                  reinterpret_cast<float*>(mean), reinterpret_cast<float*>(rstd), rows, D, eps,
                                  reinterpret_cast<cudaStream_t>(stream));
     if (err != 0) throw std::runtime_error(std::string("layernorm_fwd: ") + cudaErrorName(err));
+  });
+  m.def("qkv_pack", [](const std::array<uint64_t, 3>& grads, const std::array<long long, 9>& strides, uint64_t out, int batch, int seq, int heads,
+                       int hd, uint64_t colsum, uint64_t partials, uint64_t stream) {
+    const void* g[3] = {reinterpret_cast<const void*>(grads[0]), reinterpret_cast<const void*>(grads[1]), reinterpret_cast<const void*>(grads[2])};
+    int err = launchQkvPack(g, strides.data(), reinterpret_cast<void*>(out), batch, seq, heads, hd, reinterpret_cast<void*>(colsum),
+                            reinterpret_cast<float*>(partials), reinterpret_cast<cudaStream_t>(stream));
+    if (err != 0) throw std::runtime_error(std::string("qkv_pack: ") + cudaErrorName(err));
   });
   m.def("layernorm_bwd_parts", &layerNormBwdParts);
   m.def("layernorm_bwd", [](uint64_t dy, uint64_t x, uint64_t g, uint64_t mean, uint64_t rstd, uint64_t dres, uint64_t dx, uint64_t dg,

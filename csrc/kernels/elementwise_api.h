@@ -39,4 +39,10 @@ int launchLayerNormBwd(const void* dy, const void* x, const void* gamma, const f
 int colSumParts(long long rows);
 int launchColSum(const void* x, long long ld, long long rows, int N, void* out_bf16, float* partials, cudaStream_t stream);
 
+// Gradients of q, k, v (grads[3], bf16 [batch, heads, seq, hd] with strides[3 i ..] = batch, head, position in elements, multiples
+// of 8; the last dimension contiguous) packed into out [batch * seq, 3, heads, hd], and its column sums as bf16 [3 * heads * hd].
+// `partials`: fp32 scratch of colSumParts(batch * seq) * 3 * heads * hd elements.
+int launchQkvPack(const void* const* grads, const long long* strides, void* out, int batch, int seq, int heads, int hd, void* colsum_bf16,
+                  float* partials, cudaStream_t stream);
+
 }  // namespace pccl

@@ -307,6 +307,62 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16
   }
 }
 
+// The gradients of q, k and v, each [batch, heads, seq, hd] with the given strides, become the gradient of the packed
+// projection output [batch * seq, 3, heads, hd] in one pass that also sums its columns (the projection's bias gradient): a copy
+// and a column-sum kernel otherwise read the 3 x rows x width values once more.  A CTA owns 256 output columns (one vector of
+// eight per lane, hd % 8 == 0, so a vector lies in one head of one of the three) and a block of rows, eight at a time.
+struct QkvGrads {
+  const __nv_bfloat16* g[3];
+  long long sb[3], sh[3], st[3];           // strides in elements: batch, head, position
+};
+
+__global__ void __launch_bounds__(256) qkv_pack_kernel(QkvGrads in, __nv_bfloat16* __restrict__ out, long long rows, int seq, int heads, int hd,
+                                                       int rows_per_part, float* __restrict__ part) {
+  __shared__ float sm[8][256 + 8];
+  dev::pdl_launch();
+  dev::pdl_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int width = heads * hd, N = 3 * width;
+  const int col = blockIdx.x * 256 + lane * 8;
+  const long long r0 = static_cast<long long>(blockIdx.y) * rows_per_part;
+  const long long r1 = r0 + rows_per_part < rows ? r0 + rows_per_part : rows;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (col < N) {
+    const int which = col / width, h = (col - which * width) / hd, d = col - which * width - h * hd;
+    const __nv_bfloat16* g = (which == 0 ? in.g[0] : which == 1 ? in.g[1] : in.g[2]) + (which == 0 ? in.sh[0] : which == 1 ? in.sh[1] : in.sh[2]) * h + d;
+    const long long sb = which == 0 ? in.sb[0] : which == 1 ? in.sb[1] : in.sb[2], st = which == 0 ? in.st[0] : which == 1 ? in.st[1] : in.st[2];
+    for (long long r = r0 + warp; r < r1; r += 64) {
+      Vec16 v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const long long row = r + 8 * i;
+        const long long b = row / seq;
+        if (row < r1) v[i] = ld16(g + b * sb + (row - b * seq) * st);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const long long row = r + 8 * i;
+        if (row >= r1) break;
+        st16(out + row * N + col, v[i]);
+        float f[8];
+        unpack<DT_BF16>(v[i], f);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[k] += f[k];
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) sm[warp][lane * 8 + k] = acc[k];
+  __syncthreads();
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c < N) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += sm[w][threadIdx.x];
+    part[static_cast<long long>(blockIdx.y) * N + c] = t;
+  }
+}
+
 }  // namespace
 
 int launchLayerNormFwd(const void* x, const void* delta, void* sum_out, const void* gamma, const void* beta, void* y, float* mean,
@@ -351,20 +407,44 @@ int launchLayerNormBwd(const void* dy, const void* x, const void* gamma, const f
 
 int colSumParts(long long rows) { return static_cast<int>((rows + 255) / 256 < 64 ? (rows + 255) / 256 : 64); }
 
+// Row blocks of a column-sum launch: about four CTAs per SM in one go.  With 64 row blocks whatever the width, 16384 x 6144 had 1536
+// CTAs for 1184 places and took 54 us; now 50 (201 MB).
+static int colSumGrid(long long rows, int N) {
+  const int cols = (N + 255) / 256, fit = deviceSmCount() * 4 / cols, parts = colSumParts(rows);
+  return fit < 1 ? 1 : parts > fit ? fit : parts;
+}
+
 int launchColSum(const void* x, long long ld, long long rows, int N, void* out_bf16, float* partials, cudaStream_t stream) {
   if (rows <= 0 || N <= 0) return 0;
   if (N % 8 || ld % 8 || reinterpret_cast<uintptr_t>(x) % 16) return static_cast<int>(cudaErrorInvalidValue);
-  // About four CTAs per SM in one go: with 64 row blocks whatever the width, 16384 x 6144 had 1536 CTAs for 1184 places and took
-  // 54 us; now 50 (201 MB).
-  const int cols = (N + 255) / 256, fit = deviceSmCount() * 4 / cols;
-  int parts = colSumParts(rows);
-  if (parts > fit && fit >= 1) parts = fit;
-  else if (fit < 1) parts = 1;
+  const int cols = (N + 255) / 256, parts = colSumGrid(rows, N);
   const int rows_per_part = static_cast<int>((rows + parts - 1) / parts);
   const int e = static_cast<int>(launchOverlapped(colsum_partial_kernel, dim3(cols, parts), dim3(256), 0, stream, 1,
                                                   static_cast<const __nv_bfloat16*>(x), ld, rows, N, rows_per_part, partials));
   if (e != 0) return e;
   ReduceJob job{{partials, nullptr, nullptr}, {static_cast<__nv_bfloat16*>(out_bf16), nullptr, nullptr}};
+  return static_cast<int>(launchOverlapped(partial_rows_reduce_kernel, dim3((N + 31) / 32, 1), dim3(1024), 0, stream, 1, job, parts, N));
+}
+
+int launchQkvPack(const void* const* grads, const long long* strides, void* out, int batch, int seq, int heads, int hd, void* colsum_bf16,
+                  float* partials, cudaStream_t stream) {
+  const long long rows = static_cast<long long>(batch) * seq;
+  if (rows <= 0) return 0;
+  QkvGrads in;
+  for (int i = 0; i < 3; ++i) {
+    in.g[i] = static_cast<const __nv_bfloat16*>(grads[i]);
+    in.sb[i] = strides[3 * i];
+    in.sh[i] = strides[3 * i + 1];
+    in.st[i] = strides[3 * i + 2];
+    if ((in.sb[i] | in.sh[i] | in.st[i]) % 8 || reinterpret_cast<uintptr_t>(grads[i]) % 16) return static_cast<int>(cudaErrorInvalidValue);
+  }
+  if (hd % 8 || reinterpret_cast<uintptr_t>(out) % 16) return static_cast<int>(cudaErrorInvalidValue);
+  const int N = 3 * heads * hd, parts = colSumGrid(rows, N);
+  const int rows_per_part = static_cast<int>((rows + parts - 1) / parts);
+  const int e = static_cast<int>(launchOverlapped(qkv_pack_kernel, dim3((N + 255) / 256, parts), dim3(256), 0, stream, 1, in,
+                                                  static_cast<__nv_bfloat16*>(out), rows, seq, heads, hd, rows_per_part, partials));
+  if (e != 0) return e;
+  ReduceJob job{{partials, nullptr, nullptr}, {static_cast<__nv_bfloat16*>(colsum_bf16), nullptr, nullptr}};
   return static_cast<int>(launchOverlapped(partial_rows_reduce_kernel, dim3((N + 31) / 32, 1), dim3(1024), 0, stream, 1, job, parts, N));
 }
 

@@ -16,7 +16,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from ..nn.linear import Embedding, Linear, LinearGelu, _LinearFn, mlp
+from ..nn.linear import Embedding, Linear, LinearGelu, _LinearFn, mlp, split_qkv
 from ..nn.loss import fused_cross_entropy
 from ..nn.norm import LayerNorm
 
@@ -84,8 +84,11 @@ class Block(nn.Module):
             h = self.ln1(x)
         else:
             x, h = self.ln1.add_norm(x, delta, prev_bias)
-        qkv = self.qkv(h).view(B, T, 3, self.n_head, D // self.n_head)
-        q, k, v = (t.transpose(1, 2) for t in qkv.unbind(2))    # unbind: one stacked gradient, no zero-fills
+        if (D // self.n_head) % 8 == 0:
+            q, k, v = split_qkv(self.qkv(h, defer_bias_grad=True), self.n_head, self.qkv.bias)
+        else:
+            qkv = self.qkv(h).view(B, T, 3, self.n_head, D // self.n_head)
+            q, k, v = (t.transpose(1, 2) for t in qkv.unbind(2))    # unbind: one stacked gradient, no zero-fills
         a = F.scaled_dot_product_attention(q, k, v, is_causal=True)
         d_attn = self.proj(a.transpose(1, 2).reshape(B, T, D), defer_bias_grad=True)
         x, h = self.ln2.add_norm(x, d_attn, self.proj.bias)

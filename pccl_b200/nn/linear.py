@@ -12,8 +12,9 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
+from .._native import C
 from ..ops.elementwise import colsum
-from ..ops.gemm import gemm, gemm_dgelu, gemm_dual, records_graph
+from ..ops.gemm import count_launch, gemm, gemm_dgelu, gemm_dual, records_graph, stream_handle
 
 
 def _as_operand(t: torch.Tensor) -> torch.Tensor:
@@ -190,6 +191,47 @@ def _deliver_bias(bias: torch.Tensor, db: torch.Tensor) -> Optional[torch.Tensor
         mg.copy_(db)                       # rounds fp32 sums to the bucket's dtype
     _finish_main_grad(bias)
     return None
+
+
+class _SplitQkvFn(torch.autograd.Function):
+    """The packed projection output [B, T, 3, heads, hd] as q, k, v [B, heads, T, hd] (views).  Backward packs their gradients and
+    sums the packed rows' columns in one pass: ``bias``, the bias of the layer that made the projection, gets that as its gradient."""
+
+    @staticmethod
+    def forward(ctx, qkv, bias):
+        ctx.bias, ctx.shape = bias, qkv.shape
+        return tuple(t.transpose(1, 2) for t in qkv.unbind(2))
+
+    @staticmethod
+    def backward(ctx, *grads):
+        B, T, _, heads, hd = ctx.shape
+        bias = ctx.bias
+        gs = []
+        for g in grads:
+            g = g if g is not None else bias.new_zeros((B, heads, T, hd))
+            gs.append(g if g.stride(3) == 1 and not any(s % 8 for s in g.stride()[:3]) and g.data_ptr() % 16 == 0 else g.contiguous())
+        N = 3 * heads * hd
+        out = gs[0].new_empty((B, T, 3, heads, hd))
+        mg = _main_grad_out(bias, torch.bfloat16)
+        db = mg if mg is not None else bias.new_empty(N)
+        partials = gs[0].new_empty(C.colsum_parts(B * T) * N, dtype=torch.float32)
+        C.qkv_pack([g.data_ptr() for g in gs], [s for g in gs for s in g.stride()[:3]], out.data_ptr(), B, T, heads, hd, db.data_ptr(),
+                   partials.data_ptr(), stream_handle())
+        count_launch(2)
+        if mg is not None:
+            _finish_main_grad(bias)
+            return out, None
+        return out, _deliver_bias(bias, db)
+
+
+def split_qkv(qkv: torch.Tensor, heads: int, bias: torch.Tensor):
+    """q, k, v [B, heads, T, hd] of a packed projection output [B, T, 3 * heads * hd], made by a layer with ``defer_bias_grad=True``
+    whose ``bias`` gets its gradient here."""
+    B, T, width = qkv.shape
+    packed = qkv.view(B, T, 3, heads, width // (3 * heads))
+    if records_graph():
+        return _SplitQkvFn.apply(packed, bias)
+    return tuple(t.transpose(1, 2) for t in packed.unbind(2))
 
 
 class Linear(nn.Module):

@@ -385,3 +385,29 @@ def test_cross_entropy_with_masked_and_large_logits(vocab):
     loss = cross_entropy_(lg, tgt)
     assert ((loss.double() - loss64).abs() <= 1e-5 * loss64.abs() + 1e-5).all()      # 3e4 in fp32: 2^-24 relative, a few roundings
     assert (lg.double() - g64).abs().max().item() <= 2 ** -8
+
+
+@pytest.mark.parametrize("B,T,heads,hd", [(1, 1, 1, 8), (2, 77, 3, 24), (3, 130, 2, 64), (1, 300, 5, 128)])
+@pytest.mark.parametrize("layout", ["bthd", "bhtd", "odd"])
+def test_split_qkv_packs_gradients_and_sums_columns(B, T, heads, hd, layout):
+    """Gradients in the layouts that attention kernels return, and one (head dimension not innermost) that is copied first; the
+    packed gradient is a copy (exact), its column sums fp32 sums of bf16 values rounded once."""
+    import torch
+    from pccl_b200.nn.linear import split_qkv
+    torch.manual_seed(T)
+    qkv = torch.randn(B, T, 3 * heads * hd, device="cuda").bfloat16().requires_grad_(True)
+    bias = torch.nn.Parameter(torch.zeros(3 * heads * hd, device="cuda").bfloat16())
+    q, k, v = split_qkv(qkv, heads, bias)
+    ref = qkv.detach().view(B, T, 3, heads, hd)
+    for i, t in enumerate((q, k, v)):
+        assert torch.equal(t, ref[:, :, i].transpose(1, 2))
+    gs = [torch.randn(B, heads, T, hd, device="cuda").bfloat16() for _ in range(3)]
+    if layout == "bthd":
+        gs = [g.transpose(1, 2).contiguous().transpose(1, 2) for g in gs]
+    elif layout == "odd":
+        gs = [g.transpose(2, 3).contiguous().transpose(2, 3) for g in gs]
+    dq, db = torch.autograd.grad([q, k, v], [qkv, bias], gs)
+    want = torch.stack([g.transpose(1, 2) for g in gs], 2).reshape(B, T, -1)
+    assert torch.equal(dq, want)
+    sums = want.double().sum((0, 1))
+    assert ((db.double() - sums).abs() <= 2 ** -8 * sums.abs() + 1e-4).all()

@@ -17,10 +17,10 @@ namespace {
 __global__ void __launch_bounds__(gemm8::NUM_THREADS, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, gemm::StoreEpi epi,
                 gemm8::Scales sc, int K, uint32_t* status) {
-  gemm::GroupedSched sched{(epi.M + gemm8::BM - 1) / gemm8::BM, (epi.N + gemm8::BN - 1) / gemm8::BN, static_cast<int>(blockIdx.x),
+  gemm::GroupedSched sched{(epi.M + gemm8::BM - 1) / gemm8::BM, (epi.N + gemm8::NARROW_BN - 1) / gemm8::NARROW_BN, static_cast<int>(blockIdx.x),
                            static_cast<int>(gridDim.x)};
   gemm::NoGate gate;
-  gemm8::run(&tmA, &tmB, K, sc, sched, gate, epi, status);
+  gemm8::run<gemm8::NARROW_STAGES, gemm8::NARROW_BN>(&tmA, &tmB, K, sc, sched, gate, epi, status);
 }
 
 thread_local std::string g_err8;
@@ -52,20 +52,20 @@ int gemmFp8(const void* A, int64_t lda, const float* sa, int ld_sa, const void* 
   }
   CUtensorMap ta, tb;
   if (!makeTensorMap2D(&ta, A, TM_U8, K, M, lda, gemm8::BK, gemm8::BM, &g_err8)) return static_cast<int>(cudaErrorInvalidValue);
-  if (!makeTensorMap2D(&tb, B, TM_U8, K, N, ldb, gemm8::BK, gemm8::BN, &g_err8)) return static_cast<int>(cudaErrorInvalidValue);
-  gemm::StoreEpi epi{D, D2, static_cast<const __nv_bfloat16*>(bias), ldd, M, N, flags};
+  if (!makeTensorMap2D(&tb, B, TM_U8, K, N, ldb, gemm8::BK, gemm8::NARROW_BN, &g_err8)) return static_cast<int>(cudaErrorInvalidValue);
+  gemm::StoreEpi epi{D, D2, static_cast<const __nv_bfloat16*>(bias), ldd, M, N, flags, gemm8::NARROW_BN};
   gemm8::Scales sc{sa, sb, ld_sa, ld_sb, M, N};
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm8::SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm8::NARROW_SMEM_BYTES);
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_set = true;
   }
-  int tiles = ((M + gemm8::BM - 1) / gemm8::BM) * ((N + gemm8::BN - 1) / gemm8::BN);
+  int tiles = ((M + gemm8::BM - 1) / gemm8::BM) * ((N + gemm8::NARROW_BN - 1) / gemm8::NARROW_BN);
   int n_sm = deviceSmCount();
   if (sms > 0 && sms < n_sm) n_sm = sms;
   int grid = tiles < n_sm ? tiles : n_sm;
-  return static_cast<int>(launchOverlapped(gemm_fp8_kernel, dim3(grid), dim3(gemm8::NUM_THREADS), gemm8::SMEM_BYTES, stream, 1, ta, tb, epi, sc, K, status));
+  return static_cast<int>(launchOverlapped(gemm_fp8_kernel, dim3(grid), dim3(gemm8::NUM_THREADS), gemm8::NARROW_SMEM_BYTES, stream, 1, ta, tb, epi, sc, K, status));
 }
 
 }  // namespace pccl

@@ -3,10 +3,10 @@
 // i.e. activations carry one fp32 scale per row and 128 values of K (1 x 128), weights one per
 // 128 x 128 block.  The tensor cores cannot apply fp32 scales, so the sum is built in two levels:
 //
-//   warp 0       TMA producer: 128 x 128 A and 256 x 128 B fp8 tiles (128-byte swizzle; one stage is one
+//   warp 0       TMA producer: 128 x 128 A and 256 (or 128) x 128 B fp8 tiles (128-byte swizzle; one stage is one
 //                K block) through a 4-stage ring; `Gate` as in the bf16 pipeline
 //   warp 1       MMA issuer: four tcgen05.mma kind::f8f6f4 128x256x32 per stage into a FRESH TMEM
-//                accumulator; the two 256-column accumulators alternate per K block
+//                accumulator; the two 256-column (or four 128-column) accumulators are taken in turn
 //   warps 2..9   promotion + epilogue: every K block, tcgen05.ld the block's partial products and
 //                fold them, times sa*sb, into 128 fp32 registers per thread (warp w and w+4 share
 //                a 32-lane quarter of TMEM and split the 256 columns; packed fma.rn.f32x2); after
@@ -14,10 +14,8 @@
 //                bf16 pipeline's
 //
 // so the same epilogue adapters (plain store, reduce-scatter) serve both precisions.
-// Cost model: the promotion reads 128 KiB of TMEM per K block through the load/store data path
-// (128 B per clock and SM, ~1024 clocks) while the four MMAs of the block need ~512, so this
-// exact-fp32-scale scheme tops out near half of the fp8 tensor peak -- about the bf16 peak -- and
-// its gain over bf16 is the halved operand traffic (HBM, L2 and NVLink).
+// What bounds it: the chain of a K block (see run below), not the tensor cores (28 % busy at 4096 x 4096 x 3584 with 128-column
+// tiles), not TMEM reads and not L2.  Its gain over bf16 is the halved operand traffic and storage.
 // All waits are bounded; on a time-out the CTA flags the error, drains its copies, frees TMEM
 // and returns.  No TMA load uses cluster multicast.
 //
@@ -42,18 +40,23 @@ constexpr int MAX_STAGES = 4;
 constexpr int A_BYTES = BM * BK;            // 16 KiB
 constexpr int B_BYTES = BN * BK;            // 32 KiB
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int TMEM_COLS = 512;              // two 128 x 256 fp32 accumulators, alternating per K block
+constexpr int MAX_RING = 6;                 // stages of 128-column tiles
+constexpr int TMEM_COLS = 512;              // two 128 x 256 (or four 128 x 128) fp32 accumulators, taken in turn per K block
+constexpr int MAX_ACC = 4;
 constexpr int EPI_WARPS = 8;
 constexpr int NUM_THREADS = 64 + EPI_WARPS * 32;   // 320
 constexpr int smem_bytes(int stages) { return stages * STAGE_BYTES + 1024 + 256; }
 constexpr int SMEM_BYTES = smem_bytes(MAX_STAGES);   // epilogues that stage through shared memory start at stages * STAGE_BYTES + 256
 constexpr int CW = BN / 2;                  // columns per epilogue warp
+// ... of tiles of 128 columns (run<NARROW_STAGES, 128>)
+constexpr int NARROW_BN = 128, NARROW_STAGES = 6;
+constexpr int NARROW_SMEM_BYTES = NARROW_STAGES * (A_BYTES + NARROW_BN * BK) + 1024 + 256;
 
 struct Barriers {
-  uint64_t full[MAX_STAGES];
-  uint64_t empty[MAX_STAGES];
-  uint64_t tmem_full[2];
-  uint64_t tmem_empty[2];
+  uint64_t full[MAX_RING];
+  uint64_t empty[MAX_RING];
+  uint64_t tmem_full[MAX_ACC];
+  uint64_t tmem_empty[MAX_ACC];
   uint64_t drain;
   uint32_t tmem_base;
   uint32_t abort;
@@ -80,9 +83,18 @@ __device__ __forceinline__ void ffma2(float& acc0, float& acc1, uint32_t r0, uin
 }
 
 // STAGES (<= 4) operand stages of 48 KiB; an epilogue that needs shared memory of its own runs with three.
-template <int STAGES = MAX_STAGES, class Sched, class Gate, class Epi>
+// BNT = 128 (up to six stages of 32 KiB): a K block is a chain MMA -> commit -> tcgen05.ld -> fold -> accumulator free -> MMA, about
+// 2900 clocks long at 256 columns, and with two accumulators in turn half of that is what a block takes, whatever the tensor
+// cores and TMEM could do (eight warps read TMEM at 880 bytes per clock and SM: 150 clocks per block).  128 columns leave room for
+// four accumulators, and the 64 sums per thread no longer spill: 8192 x 8192 x 3584 372 -> 320 us, 1531 x 8192 x 3584 117 -> 80,
+// 128 x 8192 x 3584 66 -> 31, 18944 x 8192 x 1024 (whole rounds) 218 -> 203.  The fused kernels keep 256 columns: their epilogues
+// quantise or stage whole 128-column halves.
+template <int STAGES = MAX_STAGES, int BNT = BN, class Sched, class Gate, class Epi>
 __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* tmB, int K, const Scales& sc, const Sched& sched,
                                     const Gate& gate, Epi& epi, uint32_t* status) {
+  constexpr int ACC = TMEM_COLS / BNT, CW = BNT / 2, STAGE_BYTES = A_BYTES + BNT * BK;
+  static_assert(ACC <= MAX_ACC && STAGES <= MAX_RING, "barriers");
+  static_assert(!Epi::kRow128 || BNT == 256, "a thread's 128 columns are half of a 256-column tile");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   Barriers* bar = reinterpret_cast<Barriers*>(smem + STAGES * STAGE_BYTES);
@@ -95,7 +107,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
       tc::mbar_init(&bar->full[s], 1);
       tc::mbar_init(&bar->empty[s], 1);
     }
-    for (int a = 0; a < 2; ++a) {
+    for (int a = 0; a < ACC; ++a) {
       tc::mbar_init(&bar->tmem_full[a], 1);
       tc::mbar_init(&bar->tmem_empty[a], EPI_WARPS);
     }
@@ -148,7 +160,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (tc::elect_one()) {
-      constexpr uint32_t idesc = tc::make_idesc(0, 0, false, false, BM, BN);   // e4m3 x e4m3 -> f32
+      constexpr uint32_t idesc = tc::make_idesc(0, 0, false, false, BM, BNT);   // e4m3 x e4m3 -> f32
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
@@ -158,7 +170,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
           if (!tc::mbar_wait(&bar->tmem_empty[acc], acc_phase ^ 1, abort)) { ok = false; break; }
           if (!tc::mbar_wait(&bar->full[stage], phase, abort)) { ok = false; break; }
           tc::tc_fence_after();
-          const uint32_t d_tmem = tmem + acc * BN;
+          const uint32_t d_tmem = tmem + acc * BNT;
           const uint32_t sa = tc::smem_u32(smem + stage * STAGE_BYTES), sb = sa + A_BYTES;
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
@@ -169,7 +181,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
           tc::mma_commit(&bar->empty[stage]);
           tc::mma_commit(&bar->tmem_full[acc]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
-          if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+          if (++acc == ACC) { acc = 0; acc_phase ^= 1; }
         }
       }
       if (!ok && atomicExch(const_cast<uint32_t*>(&bar->abort), 1u) == 0) dev::report(status, ST_TIMEOUT, blockIdx.x, 1, 0);
@@ -215,7 +227,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         }
         if (!tc::mbar_wait(&bar->tmem_full[acc], acc_phase, abort)) { ok = false; break; }
         tc::tc_fence_after();
-        const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN + half * CW;
+        const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BNT + half * CW;
 #pragma unroll
         for (int c = 0; c < CW / 32; c += 2) {
           uint32_t r0[32], r1[32];
@@ -230,7 +242,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         tc::tc_fence_before();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&bar->tmem_empty[acc]);
-        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        if (++acc == ACC) { acc = 0; acc_phase ^= 1; }
       }
       if (!ok) break;
       epi.tile_begin(t);

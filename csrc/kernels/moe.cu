@@ -720,12 +720,12 @@ gemm_grouped_ragged_kernel(const __grid_constant__ CUtensorMap tmW, const __grid
 struct WgradTemplates { CUtensorMap m[4]; };           // A_0, B_0, A_1, B_1
 
 __global__ void __launch_bounds__(128) wgrad_maps_kernel(const __grid_constant__ WgradTemplates tmpl, const int* __restrict__ row_off,
-                                                         int groups, CUtensorMap* __restrict__ maps) {
+                                                         int max_rows, CUtensorMap* __restrict__ maps) {
   __shared__ __align__(128) CUtensorMap stage[4];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = blockIdx.x;
   reinterpret_cast<uint32_t*>(&stage[warp])[lane] = reinterpret_cast<const uint32_t*>(&tmpl.m[warp])[lane];
   __syncwarp();
-  if (lane == 0) tc::tensormap_set_outer(&stage[warp], static_cast<uint32_t>(max(1, row_off[g + 1])));
+  if (lane == 0) tc::tensormap_set_outer(&stage[warp], static_cast<uint32_t>(max(1, min(row_off[g + 1], max_rows))));     // never past the operands
   __syncwarp();
   tc::tensormap_publish(maps + g * 4 + warp, &stage[warp]);
 }
@@ -1063,7 +1063,7 @@ int gemmGroupedWgrad(const GemmProblem& p0, const GemmProblem& p1, const int* ro
     if (e != cudaSuccess) return static_cast<int>(e);
     set = true;
   }
-  wgrad_maps_kernel<<<groups, 128, 0, stream>>>(tm, row_off, groups, static_cast<CUtensorMap*>(maps));
+  wgrad_maps_kernel<<<groups, 128, 0, stream>>>(tm, row_off, max_rows, static_cast<CUtensorMap*>(maps));
   const int pairs = deviceSmCount() / 2;
   return static_cast<int>(launchOverlapped(gemm_grouped_wgrad_kernel, dim3(2 * static_cast<int>(tiles < pairs ? tiles : pairs)),
                                            dim3(gemm2::NUM_THREADS_WIDE), gemm2::SMEM_BYTES, stream, 2, epi, groups, status));

@@ -317,3 +317,20 @@ def test_mx8_tile_widths(M, N):
     wf = wq.view(torch.float8_e4m3fn).float() * ue8m0_to_float(w_s).repeat_interleave(128, 1).repeat_interleave(128, 0)[:N]
     ref = af.double() @ wf.double().t()
     assert (out.double() - ref).abs().max().item() <= 2e-3 * max(1.0, ref.abs().max().item())      # a wrong scale or tile is off by O(1)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 128), (127, 136, 256), (129, 264, 640), (260, 1000, 1152), (3000, 128, 384)])
+def test_fp8_gemm_at_the_edges_of_its_tiles(M, N, K):
+    """Ragged rows and columns around 128, one to nine K blocks (four accumulators are taken in turn), scales that differ per block;
+    fp32 output against the product of the dequantised operands (2e-3, as for the other fp8 forms)."""
+    from pccl_b200.ops import check_status
+    from pccl_b200.ops.gemm import dequant_rows, gemm_fp8, quant_rows
+    a = (_rand((M, K), 91).float() * torch.logspace(-1, 1, K // 128, device="cuda").repeat_interleave(128)).bfloat16()
+    wq, w_rows = quant_rows(_rand((N, K), 92))
+    aq, a_s = quant_rows(a)
+    w_s = (w_rows[::128] * (1.0 + torch.arange((N + 127) // 128, device="cuda")[:, None])).contiguous()
+    out = gemm_fp8(aq, a_s, wq, w_s, out_dtype=torch.float32)
+    check_status("gemm_fp8")
+    wf = wq.view(torch.float8_e4m3fn).double() * w_s.double().repeat_interleave(128, 1).repeat_interleave(128, 0)[:N]
+    ref = dequant_rows(aq, a_s).double() @ wf.t()
+    assert (out.double() - ref).abs().max().item() <= 2e-3 * max(1.0, ref.abs().max().item())

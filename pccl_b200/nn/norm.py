@@ -12,13 +12,6 @@ from .._native import C
 from ..ops.gemm import count_launch, records_graph, stream_handle
 
 
-def _finish(param: torch.Tensor) -> None:
-    param._pccl_written = True
-    cb = getattr(param, "_pccl_ready", None)
-    if cb is not None:
-        cb()
-
-
 def _writable(param: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     """The flat-bucket gradient of ``param`` if the kernel may write it directly (nothing is in it yet this step)."""
     mg = getattr(param, "main_grad", None)
@@ -27,21 +20,28 @@ def _writable(param: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     return mg
 
 
-def _own(param: torch.Tensor) -> Optional[torch.Tensor]:
-    """Like ``_writable`` for a parameter of the norm itself, whose gradient otherwise travels through autograd: only where
-    nobody else is to see it there, i.e. the parameter is used once this step and has no hook but the wrapper's."""
-    hooks = getattr(param, "_post_accumulate_grad_hooks", None)
-    if getattr(param, "_pccl_forwards", 0) != 1 or param._backward_hooks or (hooks is not None and len(hooks) > 1):
-        return None
-    return _writable(param)
+def _accumulates(ctx, param: torch.Tensor) -> bool:
+    """Whether the running backward pass will accumulate a gradient of this node into ``param``: false for a frozen parameter and
+    for an ``autograd.grad`` call, whether it asks for the parameter or for something else."""
+    for node, _ in ctx.next_functions:
+        if node is not None and getattr(node, "variable", None) is param:
+            try:
+                return torch._C._will_engine_execute_node(node)
+            except RuntimeError:               # autograd.grad asked for this very leaf
+                return False
+    return False
 
 
-def _count_use(*params: torch.Tensor) -> None:
-    if torch.is_grad_enabled():
-        for p in params:
-            n = getattr(p, "_pccl_forwards", None)
-            if n is not None:
-                p._pccl_forwards = n + 1
+def _grad_buffer(ctx, param: torch.Tensor) -> torch.Tensor:
+    """Where a kernel puts the gradient of a parameter of the norm.  It always goes back to autograd, which knows who else
+    contributes to it and which hooks see it; but where it will end in the flat bucket anyway it is written there to begin with,
+    and the wrapper's hook finds nothing to copy.  The bucket is lent once per step: a second contribution gets memory of
+    its own, and autograd adds the two."""
+    mg = _writable(param)
+    if mg is None or getattr(param, "_pccl_lent", True) or not _accumulates(ctx, param):
+        return torch.empty_like(param)
+    param._pccl_lent = True
+    return mg.view(mg.shape)                   # a tensor of its own: autograd keeps it as ``.grad`` without a copy
 
 
 def _deliver(param: Optional[torch.Tensor], grad: torch.Tensor):
@@ -57,7 +57,10 @@ def _deliver(param: Optional[torch.Tensor], grad: torch.Tensor):
             mg.add_(grad.to(mg.dtype).view_as(mg))
         else:
             mg.copy_(grad.view_as(mg))
-    _finish(param)
+    param._pccl_written = True
+    cb = getattr(param, "_pccl_ready", None)
+    if cb is not None:
+        cb()
     return None
 
 
@@ -74,32 +77,17 @@ def _ln_forward(x2, delta2, weight, bias, eps, want_stats=True):
     return s, y, stats
 
 
-def _ln_backward(dy2, x2, weight, bias, stats, dres2, colsum_of):
-    """(dx, dgamma, dbeta, column sums of dx or None).  A parameter gradient that went straight into the flat bucket is the
-    bucket's view; ``colsum_of`` is the parameter whose gradient the column sums are, or None."""
+def _ln_backward(dy2, x2, weight, stats, dres2, dg, db, dc=None):
+    """dx.  Writes the gradients of weight and bias to ``dg`` and ``db`` and, if given, the column sums of dx to ``dc``."""
     rows, D = x2.shape
     dx = torch.empty_like(x2)
-    dg, db = _own(weight), _own(bias)
-    dg = torch.empty_like(weight) if dg is None else dg
-    db = torch.empty_like(bias) if db is None else db
-    dc = None
-    if colsum_of is not None:
-        dc = _writable(colsum_of)
-        dc = torch.empty_like(weight) if dc is None else dc
     partials = x2.new_empty(3 * C.layernorm_bwd_parts(rows) * D, dtype=torch.float32)
     at = stats.data_ptr()
     C.layernorm_bwd(dy2.data_ptr(), x2.data_ptr(), weight.data_ptr(), at, at + 4 * rows,
                     dres2.data_ptr() if dres2 is not None else 0, dx.data_ptr(), dg.data_ptr(), db.data_ptr(),
                     dc.data_ptr() if dc is not None else 0, partials.data_ptr(), rows, D, stream_handle())
     count_launch(2)
-    return dx, _own_result(weight, dg), _own_result(bias, db), dc
-
-
-def _own_result(param, grad):
-    if grad is not getattr(param, "main_grad", None):
-        return grad                        # autograd accumulates it
-    _finish(param)
-    return None
+    return dx
 
 
 def _rows(t: torch.Tensor, D: int) -> torch.Tensor:
@@ -112,14 +100,16 @@ class _LayerNormFn(torch.autograd.Function):
     def forward(ctx, x, weight, bias, eps):
         x2 = _rows(x, x.shape[-1])
         _, y, stats = _ln_forward(x2, None, weight, bias, eps)
-        ctx.save_for_backward(x2, weight, bias, stats)
+        ctx.save_for_backward(x2, weight, stats)
+        ctx.params = (weight, bias)
         ctx.shape = x.shape
         return y.view(x.shape)
 
     @staticmethod
     def backward(ctx, dy):
-        x2, weight, bias, stats = ctx.saved_tensors
-        dx, dg, db, _ = _ln_backward(_rows(dy, x2.shape[1]), x2, weight, bias, stats, None, None)
+        x2, weight, stats = ctx.saved_tensors
+        dg, db = (_grad_buffer(ctx, p) for p in ctx.params)
+        dx = _ln_backward(_rows(dy, x2.shape[1]), x2, weight, stats, None, dg, db)
         return dx.view(ctx.shape), dg, db, None
 
 
@@ -133,20 +123,25 @@ class _AddLayerNormFn(torch.autograd.Function):
         D = x.shape[-1]
         x2, d2 = _rows(x, D), _rows(delta, D)
         s, y, stats = _ln_forward(x2, d2, weight, bias, eps)
-        ctx.save_for_backward(s, weight, bias, stats)
-        ctx.prev_bias = prev_bias
+        ctx.save_for_backward(s, weight, stats)
+        ctx.params, ctx.prev_bias = (weight, bias), prev_bias
         ctx.shape = x.shape
         return s.view(x.shape), y.view(x.shape)
 
     @staticmethod
     def backward(ctx, ds, dy):
-        s, weight, bias, stats = ctx.saved_tensors
+        s, weight, stats = ctx.saved_tensors
         D = s.shape[1]
         if dy is None:
             dy = torch.zeros_like(s)
         dres = _rows(ds, D) if ds is not None else None
         want = ctx.prev_bias is not None and ctx.needs_input_grad[4]
-        dx, dg, db, dc = _ln_backward(_rows(dy, D), s, weight, bias, stats, dres, ctx.prev_bias if want else None)
+        dg, db = (_grad_buffer(ctx, p) for p in ctx.params)
+        dc = None
+        if want:
+            dc = _writable(ctx.prev_bias)
+            dc = torch.empty_like(weight) if dc is None else dc
+        dx = _ln_backward(_rows(dy, D), s, weight, stats, dres, dg, db, dc)
         dxv = dx.view(ctx.shape)
         return dxv, dxv, dg, db, (_deliver(ctx.prev_bias, dc) if want else None), None
 
@@ -163,7 +158,6 @@ class LayerNorm(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         weight, bias = self.weight, self.bias
         if records_graph():
-            _count_use(weight, bias)
             return _LayerNormFn.apply(x, weight, bias, self.eps)
         return _ln_forward(_rows(x, x.shape[-1]), None, weight, bias, self.eps, False)[1].view(x.shape)
 
@@ -172,7 +166,6 @@ class LayerNorm(nn.Module):
         ``prev_bias`` when that layer was told to leave its bias gradient to this norm (``Linear(..., defer_bias_grad=True)``)."""
         weight, bias = self.weight, self.bias
         if records_graph():
-            _count_use(weight, bias)
             return _AddLayerNormFn.apply(x, delta, weight, bias, prev_bias, self.eps)
         D = x.shape[-1]
         s, y, _ = _ln_forward(_rows(x, D), _rows(delta, D), weight, bias, self.eps, False)

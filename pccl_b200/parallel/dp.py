@@ -154,7 +154,7 @@ class ShardedDataParallel:
                 p.main_grad = b.grads[off:off + p.numel()].view(p.shape)
                 p._pccl_written = False
                 p._pccl_seen = 0
-                p._pccl_forwards = 0       # recorded uses since zero_grad (norms: nn/norm.py)
+                p._pccl_lent = False       # whether a kernel has been given main_grad to write to since zero_grad (nn/norm.py)
                 if not hasattr(p, "_pccl_uses"):
                     p._pccl_uses = 1           # a model sets 2 on a weight it uses twice (tied embeddings)
                 p._pccl_ready = self._make_ready(b, p)
@@ -189,7 +189,7 @@ class ShardedDataParallel:
             return
         if p._pccl_written:
             p.main_grad.add_(g.to(p.main_grad.dtype))
-        else:
+        elif g.data_ptr() != p.main_grad.data_ptr():         # equal: the kernel was given the bucket (nn/norm.py)
             p.main_grad.copy_(g)
         p.grad = None
         p._pccl_written = True
@@ -248,7 +248,7 @@ class ShardedDataParallel:
             for p in b.params:
                 p._pccl_written = False
                 p._pccl_seen = 0
-                p._pccl_forwards = 0
+                p._pccl_lent = False
                 p.grad = None
 
     def optimizer_step(self) -> None:

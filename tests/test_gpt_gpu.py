@@ -411,3 +411,78 @@ def test_split_qkv_packs_gradients_and_sums_columns(B, T, heads, hd, layout):
     assert torch.equal(dq, want)
     sums = want.double().sum((0, 1))
     assert ((db.double() - sums).abs() <= 2 ** -8 * sums.abs() + 1e-4).all()
+
+
+def _wrapped_norms():
+    """x -> norm -> norm under the data-parallel wrapper, inputs, and the gradients that plain autograd gives."""
+    import torch.nn as nn
+    from pccl_b200.nn import LayerNorm
+    from pccl_b200.parallel.dp import ShardedDataParallel
+
+    class Net(nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.a, self.b = (LayerNorm(64, device="cuda") for _ in range(2))
+
+        def forward(self, x, t):
+            return (self.b(self.a(x)) * t).float().mean()
+
+    torch.manual_seed(9)
+    net = Net()
+    for p in net.parameters():
+        p.data.add_(torch.randn(64, device="cuda").bfloat16() * 0.3)
+    x, t = (torch.randn(40, 64, device="cuda").bfloat16() for _ in range(2))
+    x.requires_grad_(True)
+    ref = torch.autograd.grad(net(x, t), [x] + list(net.parameters()))
+    dp = ShardedDataParallel(net, heap_bytes=64 << 20)
+    dp.zero_grad()
+    return net, dp, x, t, ref
+
+
+def test_frozen_norm_is_not_trained():
+    net, dp, x, t, _ = _wrapped_norms()
+    net.a.weight.requires_grad_(False)
+    before = [p.detach().clone() for p in net.parameters()]
+    net(x, t).backward()
+    assert not net.a.weight._pccl_written and dp.buckets[0].pending == 1
+    with pytest.raises(RuntimeError, match="never arrived"):
+        dp.optimizer_step()
+    torch.cuda.synchronize()
+    assert all(torch.equal(p, q) for p, q in zip(net.parameters(), before))
+
+
+def test_autograd_grad_over_a_wrapped_norm():
+    """``autograd.grad`` returns the gradients (in memory of their own) and leaves buckets and their counters alone; the step
+    that follows is as if it had not been."""
+    net, dp, x, t, ref = _wrapped_norms()
+    params = list(net.parameters())
+    got = torch.autograd.grad(net(x, t), [x] + params)
+    alone, = torch.autograd.grad(net(x, t), [x])
+    assert all(torch.equal(a, b) for a, b in zip(got, ref)) and torch.equal(alone, ref[0])
+    assert dp.buckets[0].pending == 4 and not dp.flat_grads.any() and not any(p._pccl_written for p in params)
+    net(x, t).backward()
+    assert all(torch.equal(p.main_grad, g) for p, g in zip(params, ref[1:])) and dp.buckets[0].pending == 0
+    dp.optimizer_step()
+    assert all(torch.equal(a, b) for a, b in zip(got, ref))
+
+
+def test_norm_weight_that_the_loss_uses_once_more():
+    """A penalty on a norm's weight: the bucket gets the sum of both contributions, once."""
+    net, dp, x, t, ref = _wrapped_norms()
+    w = net.a.weight.detach().clone()
+    (net(x, t) + net.a.weight.float().pow(2).sum()).backward()
+    assert [p._pccl_seen for p in net.parameters()] == [1, 1, 1, 1]
+    want = ref[1].float() + 2 * w.float()
+    assert (net.a.weight.main_grad.float() - want).abs().max().item() <= 2 ** -7 * want.abs().max().item()      # two bf16 terms
+    assert all(torch.equal(p.main_grad, g) for p, g in zip(list(net.parameters())[1:], ref[2:]))
+
+
+def test_norm_bias_may_change_between_forward_and_backward():
+    from pccl_b200.nn import LayerNorm
+    ln = LayerNorm(64, device="cuda")
+    x = torch.randn(5, 64, device="cuda").bfloat16()
+    y = ln(x)
+    with torch.no_grad():
+        ln.bias.add_(1)
+    y.backward(torch.ones_like(y))
+    assert torch.equal(ln.bias.grad, torch.full_like(ln.bias, 5.0))

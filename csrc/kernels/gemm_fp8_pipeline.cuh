@@ -215,15 +215,15 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
       const float* pb = sc.sb + static_cast<long long>(gblk) * sc.ld_sb;
       // raw scales travel two K blocks ahead of their use, so that no load latency is exposed
       // (A's scales may have been written by a peer during this launch: read them past L1)
-      float a0 = __ldcg(pa), b0 = __ldg(pb);
-      float a1 = num_kb > 1 ? __ldcg(pa + 1) : 0.f, b1 = num_kb > 1 ? __ldg(pb + 1) : 0.f;
+      float a0 = dev::ld_cg_f32(pa), b0 = dev::ld_f32(pb);
+      float a1 = num_kb > 1 ? dev::ld_cg_f32(pa + 1) : 0.f, b1 = num_kb > 1 ? dev::ld_f32(pb + 1) : 0.f;
       for (int kb = 0; kb < num_kb; ++kb) {
         const float s = a0 * b0;
         a0 = a1;
         b0 = b1;
         if (kb + 2 < num_kb) {
-          a1 = __ldcg(pa + kb + 2);
-          b1 = __ldg(pb + kb + 2);
+          a1 = dev::ld_cg_f32(pa + kb + 2);
+          b1 = dev::ld_f32(pb + kb + 2);
         }
         if (!tc::mbar_wait(&bar->tmem_full[acc], acc_phase, abort)) { ok = false; break; }
         tc::tc_fence_after();

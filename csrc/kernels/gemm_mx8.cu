@@ -49,8 +49,8 @@ __device__ __forceinline__ uint2 quant8_mx(const float* f, float inv) {
 
 // 16 consecutive lanes own one 1 x 128 block (8 values each); rows are whole blocks, so the matrix is one list of blocks.  Four
 // loads in flight per thread.  A CTA per row took 61 us at 8192 x 8192 (its fp32-scale twin in moe.cu), this form 41: 201 MB at 4.9 TB/s.
-__global__ void __launch_bounds__(256) quant_rows_mx_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q,
-                                                            uint8_t* __restrict__ scales, long long nvec) {
+__global__ void __launch_bounds__(256) quant_rows_mx_kernel(const __nv_bfloat16* x, uint8_t* q,
+                                                            uint8_t* scales, long long nvec) {
   dev::pdl_launch();
   dev::pdl_wait();
   for (long long v0 = static_cast<long long>(blockIdx.x) * 1024 + threadIdx.x; v0 - (threadIdx.x & 31) < nvec; v0 += static_cast<long long>(gridDim.x) * 1024) {

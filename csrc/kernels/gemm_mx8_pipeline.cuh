@@ -234,11 +234,11 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         const uint8_t* p = sc.sa + static_cast<long long>(row) * sc.ld_sa;
         uint32_t w = 0;
         if (wide) {
-          w = __ldcg(reinterpret_cast<const uint32_t*>(p + kb0));     // may have been written by a peer: past L1
+          w = dev::ld_cg_u32(p + kb0);     // may have been written by a peer: past L1
         } else {
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            if (kb0 + j < num_kb) w |= static_cast<uint32_t>(__ldcg(p + kb0 + j)) << (8 * j);
+            if (kb0 + j < num_kb) w |= dev::ld_cg_u8(p + kb0 + j) << (8 * j);
         }
         wa[q] = w;
       }
@@ -248,11 +248,11 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         const uint8_t* p = sc.sb + static_cast<long long>(blk) * sc.ld_sb;
         uint32_t w = 0;
         if (wide) {
-          w = __ldg(reinterpret_cast<const uint32_t*>(p + kb0));
+          w = dev::ld_u32(p + kb0);
         } else {
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            if (kb0 + j < num_kb) w |= static_cast<uint32_t>(__ldg(p + kb0 + j)) << (8 * j);
+            if (kb0 + j < num_kb) w |= dev::ld_u8(p + kb0 + j) << (8 * j);
         }
         wb[q] = w;
       }

@@ -3,9 +3,14 @@
 // A short kernel spends a few microseconds on its launch, on barriers, TMEM and descriptors before it touches memory, and
 // the SMs sit idle meanwhile.  A kernel launched through launchOverlapped() may be placed on SMs while its predecessor's
 // last CTAs are still running; it calls pdl_wait() before its first access to global memory, which returns when the
-// predecessor has completed and its writes are visible, and pdl_launch() once it holds its resources, which lets its own
-// successor do the same.  Both are no-ops in a kernel that was launched the ordinary way, and an ordinary launch behind such
-// a kernel waits for its end as usual.
+// predecessor has completed and its writes are visible, and pdl_launch(), which lets its own successor do the same: a short
+// kernel once it holds its resources, a GEMM with its last operand load.  Both are no-ops in a kernel that was launched the
+// ordinary way, and an ordinary launch behind such a kernel waits for its end as usual.
+//
+// What a kernel reads after pdl_wait() may have been written after the kernel started.  So its pointers are not `__restrict__`
+// (a `const` one would promise data that nobody writes during the kernel: the compiler could read it through the non-coherent
+// path, or above the wait, which orders nothing that cannot alias) and it uses neither __ldg nor __ldcg, whose place in the
+// program is not fixed either (prims.cuh: ld_f32 and the like).
 #pragma once
 #include <cuda_runtime.h>
 

@@ -36,10 +36,10 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 }
 
 template <int MAXV>
-__global__ void __launch_bounds__(256) ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
-                                                     __nv_bfloat16* __restrict__ sum_out, const __nv_bfloat16* __restrict__ gamma,
-                                                     const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
-                                                     float* __restrict__ mean, float* __restrict__ rstd, int D, float eps) {
+__global__ void __launch_bounds__(256) ln_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* delta,
+                                                     __nv_bfloat16* sum_out, const __nv_bfloat16* gamma,
+                                                     const __nv_bfloat16* beta, __nv_bfloat16* y,
+                                                     float* mean, float* rstd, int D, float eps) {
   __shared__ float scratch[8];
   dev::pdl_launch();
   dev::pdl_wait();
@@ -100,11 +100,11 @@ __global__ void __launch_bounds__(256) ln_fwd_kernel(const __nv_bfloat16* __rest
 // 4096 x 8192 218 -> 83; 16384 x 2048 77 -> 79 (3.4 TB/s; before, a form of its own for D = 256, 512, 1024 and 2048 with one warp per
 // row and its sums in shared memory).
 template <int VPT, int R>
-__global__ void __launch_bounds__(256, VPT == 1 ? 2 : 1) ln_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                                                                       const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean,
-                                                                       const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dres,
-                                                                       __nv_bfloat16* __restrict__ dx, float* __restrict__ part_g,
-                                                                       float* __restrict__ part_b, float* __restrict__ part_c, long long rows,
+__global__ void __launch_bounds__(256, VPT == 1 ? 2 : 1) ln_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
+                                                                       const __nv_bfloat16* gamma, const float* mean,
+                                                                       const float* rstd, const __nv_bfloat16* dres,
+                                                                       __nv_bfloat16* dx, float* part_g,
+                                                                       float* part_b, float* part_c, long long rows,
                                                                        int D, int gw) {
   __shared__ float2 stat[2][8][R];                          // [parity][warp][row]: partial sums of a warp
   extern __shared__ __align__(16) float group_sums[];       // [groups][arrays][D], with more than one group
@@ -263,8 +263,8 @@ __global__ void __launch_bounds__(1024) partial_rows_reduce_kernel(ReduceJob job
 // Column sums of a bf16 matrix [rows, N] (row stride ld): the bias gradient of a linear layer whose output gradient
 // comes from elsewhere.  A CTA owns 256 columns (one 16-byte vector per lane, 8 warps = 8 rows at a time) and a block
 // of rows; it writes one partial row, which partial_rows_reduce_kernel adds up.
-__global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16* __restrict__ x, long long ld, long long rows, int N,
-                                                             int rows_per_part, float* __restrict__ part) {
+__global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16* x, long long ld, long long rows, int N,
+                                                             int rows_per_part, float* part) {
   __shared__ float sm[8][256 + 8];
   dev::pdl_launch();
   dev::pdl_wait();
@@ -316,8 +316,8 @@ struct QkvGrads {
   long long sb[3], sh[3], st[3];           // strides in elements: batch, head, position
 };
 
-__global__ void __launch_bounds__(256) qkv_pack_kernel(QkvGrads in, __nv_bfloat16* __restrict__ out, long long rows, int seq, int heads, int hd,
-                                                       int rows_per_part, float* __restrict__ part) {
+__global__ void __launch_bounds__(256) qkv_pack_kernel(QkvGrads in, __nv_bfloat16* out, long long rows, int seq, int heads, int hd,
+                                                       int rows_per_part, float* part) {
   __shared__ float sm[8][256 + 8];
   dev::pdl_launch();
   dev::pdl_wait();

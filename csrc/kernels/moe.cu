@@ -329,9 +329,9 @@ __global__ void __launch_bounds__(256 * kCombineSubs) moe_combine_dot_kernel(con
 // One warp per row, eight values per lane and step (a warp stores 512 consecutive bytes), four steps in flight, the next row's
 // alias fetched behind this row.  The stores bound it (the e4m3 rows of a de-duplicated exchange come out of L2): 32768 rows of
 // 7168 take 110 us, 470 MB at 4.3 TB/s (a CTA per row and half-filled second trips: 167).
-__global__ void __launch_bounds__(256) moe_dequant_kernel(const uint8_t* __restrict__ q, const float* __restrict__ scales,
-                                                          __nv_bfloat16* __restrict__ out, const int* __restrict__ n_rows,
-                                                          int max_rows, int hidden, const int* __restrict__ alias) {
+__global__ void __launch_bounds__(256) moe_dequant_kernel(const uint8_t* q, const float* scales,
+                                                          __nv_bfloat16* out, const int* n_rows,
+                                                          int max_rows, int hidden, const int* alias) {
   dev::pdl_launch();
   dev::pdl_wait();
   const int rows = min(*n_rows, max_rows);
@@ -373,9 +373,9 @@ __global__ void __launch_bounds__(256) moe_dequant_kernel(const uint8_t* __restr
 
 // z[r] = sum_j weight_j * y[row_j] over the group record of primary row r, for groups of two or more (a group of one stays in y
 // and gets its weight in the combine).  Element-wise over the row, accumulated in fp32.
-__global__ void __launch_bounds__(256) moe_reduce_groups_kernel(const __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ z,
-                                                                const int* __restrict__ alias, const uint32_t* __restrict__ groups,
-                                                                const int* __restrict__ n_rows, int max_rows, int hidden) {
+__global__ void __launch_bounds__(256) moe_reduce_groups_kernel(const __nv_bfloat16* y, __nv_bfloat16* z,
+                                                                const int* alias, const uint32_t* groups,
+                                                                const int* n_rows, int max_rows, int hidden) {
   dev::pdl_launch();
   dev::pdl_wait();
   const int rows = min(*n_rows, max_rows);
@@ -416,8 +416,8 @@ __global__ void __launch_bounds__(256) moe_reduce_groups_kernel(const __nv_bfloa
 
 // Rows are whole 128-value blocks, so the matrix is one list of blocks, 16 lanes to each; four loads in flight per thread.
 // 8192 x 8192: 61 -> 41 us (a CTA per row, staged in shared memory, before).
-__global__ void __launch_bounds__(256) quant_rows_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q,
-                                                         float* __restrict__ scales, long long nvec) {
+__global__ void __launch_bounds__(256) quant_rows_kernel(const __nv_bfloat16* x, uint8_t* q,
+                                                         float* scales, long long nvec) {
   dev::pdl_launch();
   dev::pdl_wait();
   for (long long v0 = static_cast<long long>(blockIdx.x) * 1024 + threadIdx.x; v0 - (threadIdx.x & 31) < nvec; v0 += static_cast<long long>(gridDim.x) * 1024) {
@@ -789,7 +789,7 @@ __global__ void __launch_bounds__(gemm2::NUM_THREADS_WIDE, 1) gemm_grouped_wgrad
 // routing and placement
 // ---------------------------------------------------------------------------------------------
 template <int PER_LANE>
-__device__ __forceinline__ void route_token(const float* __restrict__ logits, int* __restrict__ ids, float* __restrict__ probs, int* __restrict__ pos,
+__device__ __forceinline__ void route_token(const float* logits, int* ids, float* probs, int* pos,
                                             int* cnt, int t, int experts, int topk, int lane) {
   float v[PER_LANE];
   float mx = -INFINITY;
@@ -838,8 +838,8 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, in
 // shared memory and draws its share of each expert's rows with one global atomic; an atomic per assignment (32768 of them on
 // 32 words at 4096 tokens, top-8) took three quarters of the kernel's time: 22 -> 7 us.
 template <int PER_LANE>
-__global__ void __launch_bounds__(1024) moe_route_kernel(const float* __restrict__ logits, int* __restrict__ ids, float* __restrict__ probs,
-                                                         int* pos, int* __restrict__ counts, int tokens, int experts, int topk) {
+__global__ void __launch_bounds__(1024) moe_route_kernel(const float* logits, int* ids, float* probs,
+                                                         int* pos, int* counts, int tokens, int experts, int topk) {
   extern __shared__ int cnt[];             // [experts] assignments of this block, then the first place of the block
   const int lane = threadIdx.x & 31;
   const int t0 = blockIdx.x * (blockDim.x >> 5), t = t0 + (threadIdx.x >> 5);
@@ -856,8 +856,8 @@ __global__ void __launch_bounds__(1024) moe_route_kernel(const float* __restrict
   for (int i = t0 * topk + threadIdx.x; i < end; i += blockDim.x) pos[i] += cnt[ids[i]];     // both written by this block above
 }
 
-__global__ void __launch_bounds__(256) moe_plan_kernel(const int* __restrict__ counts_all, const int* __restrict__ ids, const int* __restrict__ pos,
-                                                       int* __restrict__ rows, int* __restrict__ row_off, int world, int rank, int experts,
+__global__ void __launch_bounds__(256) moe_plan_kernel(const int* counts_all, const int* ids, const int* pos,
+                                                       int* rows, int* row_off, int world, int rank, int experts,
                                                        int tokens, int topk, int cap) {
   extern __shared__ int first[];           // [experts + 1] rows of the experts before e, over all ranks of the world
   __shared__ int warp_sum[8];

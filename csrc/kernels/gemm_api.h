@@ -24,7 +24,7 @@ enum GemmFlags : uint32_t {
                               // coalescing patch: for comparison runs
   GEMM_SKINNY = 1u << 10,     // few rows (M <= 256, A K-major): weights on the tile's M side, K split over a cluster (gemm_skinny.cu)
   GEMM_DGELU = 1u << 11,      // grouped and all-gather GEMM: D = A*B^T .* gelu_tanh'(D2) (D2 bf16, D's layout, read only)
-  GEMM_GELU_FULL = 1u << 12,  // GEMM_GELU to full fp32 accuracy instead of through the hardware tanh (relative error 2^-11)
+  GEMM_GELU_FULL = 1u << 12,  // GEMM_GELU through exp and a division instead of the hardware tanh (relative error 2^-11)
 };
 
 // D[M,N] (ldd) = A * B^T.  K-major operands: A is [M,K] with row stride lda, B is [N,K] with row
@@ -41,7 +41,7 @@ int gemmSkinnyBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void*
 // D[M,N] = (A * B^T) .* gelu_tanh'(pre[M,N]) in bf16, and colsum[n] += sum_m D[m,n] (fp32, may be null): the
 // backward of "linear -> GELU -> linear" between the second layer's input gradient and the first layer's output
 // gradient, with the first layer's bias gradient as a by-product.  `pre` has D's row stride.  CTA pairs; N a
-// multiple of 32; flags: GEMM_A_MN / GEMM_B_MN only.
+// multiple of 32; flags: GEMM_B_MN only.  gelu' goes through the hardware tanh where M and N are multiples of 256.
 int gemmBf16Dgelu(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, int64_t ldd, const void* pre, float* colsum,
                   int M, int N, int K, uint32_t flags, int sms, uint32_t* status, cudaStream_t stream);
 

@@ -292,11 +292,18 @@ int gemmBf16Dgelu(const void* A, int64_t lda, const void* B, int64_t ldb, void* 
   if (!makeTensorMap2D(&pa, A, TM_BF16, K, M, lda, BK, 128, &g_err)) return static_cast<int>(cudaErrorInvalidValue);
   if (!b_mn ? !makeTensorMap2D(&pb, B, TM_BF16, K, N, ldb, BK, bn / 2, &g_err) : !makeTensorMap2D(&pb, B, TM_BF16, N, K, ldb, 64, BK, &g_err))
     return static_cast<int>(cudaErrorInvalidValue);
-  DgeluEpi epi{static_cast<__nv_bfloat16*>(D), static_cast<const __nv_bfloat16*>(pre), colsum, ldd, M, N, bn};
-  int pair_tiles = ((M + 255) / 256) * ((N + bn - 1) / bn);
-  int grid = 2 * (pair_tiles < n_sm / 2 ? pair_tiles : n_sm / 2);
-  return b_mn ? launchPair<false, true, DgeluEpi>(pa, pb, epi, K, grid, status, stream)
-              : launchPair<false, false, DgeluEpi>(pa, pb, epi, K, grid, status, stream);
+  const int pair_tiles = ((M + 255) / 256) * ((N + bn - 1) / bn);
+  const int grid = 2 * (pair_tiles < n_sm / 2 ? pair_tiles : n_sm / 2);
+  auto go = [&](auto epi) {
+    using Epi = decltype(epi);
+    return b_mn ? launchPair<false, true, Epi>(pa, pb, epi, K, grid, status, stream) : launchPair<false, false, Epi>(pa, pb, epi, K, grid, status, stream);
+  };
+  auto d = static_cast<__nv_bfloat16*>(D);
+  auto x = static_cast<const __nv_bfloat16*>(pre);
+  // Whole 256 x 256 tiles: gelu' through the hardware tanh.  Any other size had an accurate gelu' of its own before this epilogue
+  // took it, and keeps one: 1 - tanh^2 cancels on the negative side, where the hardware tanh's 2^-11 is a fifth of gelu'(-3).
+  if (M % 256 == 0 && N % 256 == 0) return go(DgeluEpiT<false>{d, x, colsum, ldd, M, N, bn});
+  return go(DgeluEpiT<true>{d, x, colsum, ldd, M, N, bn});
 }
 
 int gemmBf16Dual(const GemmProblem& p0, const GemmProblem& p1, int K, uint32_t flags, int sms, uint32_t* status, cudaStream_t stream) {

@@ -207,6 +207,24 @@ def test_gemm_dgelu_ragged_rows(M):
     assert (sums - ref.sum(0)).abs().max().item() <= 2e-2 * max(1.0, ref.sum(0).abs().max().item())
 
 
+@pytest.mark.parametrize("M,N", [(40, 256), (256, 288), (513, 1056)])
+def test_gemm_dgelu_off_the_tiles_is_accurate_on_the_negative_side(M, N):
+    """gelu' where 1 - tanh^2 cancels: within the bf16 rounding of every single value, against fp64.  The product is exact (one
+    nonzero per row of a), so 2^-8 is the rounding; 1e-4 of |gelu'| <= 1.2 covers the exponential's and the division's error."""
+    from pccl_b200.ops import check_status
+    from pccl_b200.ops.gemm import gemm_dgelu
+    K = 64
+    a = torch.zeros((M, K), dtype=torch.bfloat16, device="cuda")
+    a[torch.arange(M), torch.arange(M) % K] = 1.0
+    b = _rand((K, N), 67)
+    pre = (-1.0 - 3.0 * torch.rand((M, N), device="cuda")).bfloat16()
+    out = gemm_dgelu(a, b, pre, b_t=True)
+    check_status("gemm dgelu accuracy")
+    x = pre.double().requires_grad_(True)
+    torch.nn.functional.gelu(x, approximate="tanh").backward(a.double() @ b.double())
+    assert ((out.double() - x.grad).abs() <= (2 ** -8 + 1e-4) * x.grad.abs() + 1e-7).all()
+
+
 @pytest.mark.parametrize("M", [1, 15, 17, 33, 100, 128])
 @pytest.mark.parametrize("N,K", [(40, 72), (1001, 200), (512, 2048), (8200, 520)])
 @pytest.mark.parametrize("b_t", [False, True])

@@ -16,7 +16,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from ..nn.linear import Embedding, Linear, LinearGelu, _LinearFn, mlp, split_qkv
+from ..nn.linear import Embedding, Linear, LinearGelu, _LinearFn, is_plain, mlp, split_qkv
 from ..nn.loss import fused_cross_entropy
 from ..nn.norm import LayerNorm
 
@@ -84,7 +84,8 @@ class Block(nn.Module):
             h = self.ln1(x)
         else:
             x, h = self.ln1.add_norm(x, delta, prev_bias)
-        if (D // self.n_head) % 8 == 0:
+        # split_qkv gives the projection its bias gradient, from gradients of the projection's own output: nothing may sit between
+        if (D // self.n_head) % 8 == 0 and self.qkv.bias is not None and is_plain(self.qkv, Linear):
             q, k, v = split_qkv(self.qkv(h, defer_bias_grad=True), self.n_head, self.qkv.bias)
         else:
             qkv = self.qkv(h).view(B, T, 3, self.n_head, D // self.n_head)

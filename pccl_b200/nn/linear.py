@@ -234,6 +234,13 @@ def split_qkv(qkv: torch.Tensor, heads: int, bias: torch.Tensor):
     return tuple(t.transpose(1, 2) for t in packed.unbind(2))
 
 
+def is_plain(module: nn.Module, cls: type) -> bool:
+    """Whether calling ``module`` runs ``cls.forward`` and nothing else: not a subclass, no forward of its own, no hooks."""
+    return (type(module) is cls and "forward" not in module.__dict__
+            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
+            and not nn.modules.module._has_any_global_hook())
+
+
 class Linear(nn.Module):
     def __init__(self, in_features: int, out_features: int, bias: bool = True, device=None, dtype=torch.bfloat16,
                  init_std: float = 0.02):

@@ -134,7 +134,7 @@ def allreduce(a):
 
 
 def moe(a):
-    w, T, H, Kt, epr = a.world, a.tokens, a.hidden, 8, 4
+    w, T, H, Kt, epr = a.world, a.tokens or 2048, a.hidden, 8, 4
     cap = T * Kt * w
     q_off, s_off = DATA_OFF, DATA_OFF + cap * H
     y_off = s_off + cap * (H // 128) * 4
@@ -160,11 +160,11 @@ def moe(a):
 
 
 def train_kernels(a):
-    """The fused kernels of the training step at the GPT-1.3B shapes (16384 tokens, d = 2048, d_ff = 8192)."""
+    """The fused kernels of the training step at the GPT-1.3B shapes (d = 2048, d_ff = 8192; 16384 tokens, or --tokens)."""
     from .nn.norm import _ln_backward, _ln_forward
     from .ops.elementwise import colsum
     from .ops.gemm import gemm, gemm_dgelu, gemm_dual
-    T, D, H = 16384, 2048, 8192
+    T, D, H = a.tokens or 16384, 2048, 8192
     r = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
     dz, w2, pre = r(T, D), r(D, H) * 0.02, r(T, H)
     out = torch.empty(T, H, device="cuda", dtype=torch.bfloat16)
@@ -179,9 +179,10 @@ def train_kernels(a):
            "us": _timed(lambda: (gemm(dy1, xin, a_t=True, b_t=True, out=dw1), gemm(dz, act, a_t=True, b_t=True, out=dw2)), a.iters)})
     x, delta, g = r(T, D), r(T, D), r(T, D)
     gamma, beta = torch.ones(D, device="cuda", dtype=torch.bfloat16), torch.zeros(D, device="cuda", dtype=torch.bfloat16)
-    s, _, mean, rstd = _ln_forward(x, delta, gamma, beta, 1e-5)
+    s, _, stats = _ln_forward(x, delta, gamma, beta, 1e-5)
+    dgamma, dbeta, dbias = (torch.empty_like(gamma) for _ in range(3))
     print({"op": "ln_fwd_add", "rows": T, "D": D, "us": _timed(lambda: _ln_forward(x, delta, gamma, beta, 1e-5), a.iters)})
-    print({"op": "ln_bwd_add_colsum", "rows": T, "D": D, "us": _timed(lambda: _ln_backward(g, s, gamma, mean, rstd, delta, True), a.iters)})
+    print({"op": "ln_bwd_add_colsum", "rows": T, "D": D, "us": _timed(lambda: _ln_backward(g, s, gamma, stats, delta, dgamma, dbeta, dbias), a.iters)})
     q = r(T, 3 * D)
     print({"op": "colsum", "rows": T, "N": 3 * D, "us": _timed(lambda: colsum(q), a.iters)})
     from .ops import check_status
@@ -192,7 +193,7 @@ def grouped_gemm(a):
     """Expert FFN of the MoE layer: 32 experts, 7168 -> 2048 (GELU) -> 7168; rows spread unevenly, or (--balanced) the way a
     router with many tokens spreads them: the mean per expert give or take a few per cent."""
     from .ops.moe import grouped_gemm as gg
-    E, H, Fd, rows = 32, a.hidden, 2048, a.tokens
+    E, H, Fd, rows = 32, a.hidden, 2048, a.tokens or 2048
     if a.balanced:
         sizes = (torch.randn(E) * 0.04 * rows / E + rows / E).round().clamp(min=1).long()
         sizes[-1] = max(1, rows - int(sizes[:-1].sum()))
@@ -221,7 +222,7 @@ def main():
     ap.add_argument("--n", type=int, default=0)
     ap.add_argument("--n-copy", type=int, default=8)
     ap.add_argument("--mbytes", type=int, default=64)
-    ap.add_argument("--tokens", type=int, default=2048)
+    ap.add_argument("--tokens", type=int, default=0)
     ap.add_argument("--hidden", type=int, default=7168)
     ap.add_argument("--iters", type=int, default=3)
     ap.add_argument("--balanced", action="store_true", help="grouped_gemm: expert sizes near the mean instead of random cuts")

@@ -525,3 +525,14 @@ def test_projections_that_are_not_the_plain_layer(what):
     for (name, p), q in zip(model.named_parameters(), plain.parameters()):
         if "qkv" in name:
             assert (p.grad.float() - q.grad.float()).abs().max().item() <= 0.04 * q.grad.float().abs().max().item(), name
+
+
+def test_profiler_target_of_the_training_kernels_runs():
+    """The documented command, on a small case."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-m", "pccl_b200.profile_targets", "train_kernels", "--tokens", "256", "--iters", "1"],
+                       cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "ln_bwd_add_colsum" in r.stdout, r.stdout + r.stderr

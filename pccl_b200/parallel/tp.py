@@ -15,6 +15,7 @@ import torch
 import torch.nn as nn
 
 from ..engine import Engine
+from ..nn.linear import is_plain
 from ..ops.fused_tp import AllGatherGemm, GemmReduceScatter
 from ..ops.elementwise import colsum
 from ..ops.gemm import gemm, gemm_dual
@@ -133,8 +134,15 @@ class RowParallelLinear(nn.Module):
         self.rs = GemmReduceScatter(eng, tokens, out_features)
         self.ag_bwd = AllGatherGemm(eng, tokens, out_features, n_copy=n_copy, flag_lane=6)
 
+    def bias_in_epilogue(self) -> bool:
+        """Whether the kernel can add the bias (its loads are 16 bytes of bf16); any other one is added by torch."""
+        b = self.bias
+        return b is None or (b.is_cuda and b.dtype == torch.bfloat16 and b.shape == self.weight.shape[:1] and b.is_contiguous() and b.data_ptr() % 16 == 0)
+
     def forward(self, h: torch.Tensor) -> torch.Tensor:
-        return _RowFn.apply(h, self.weight, self.bias, self)
+        if self.bias_in_epilogue():
+            return _RowFn.apply(h, self.weight, self.bias, self)
+        return _RowFn.apply(h, self.weight, None, self) + self.bias
 
 
 class TensorParallelMLP(nn.Module):
@@ -147,8 +155,9 @@ class TensorParallelMLP(nn.Module):
 
     def forward(self, x_local: torch.Tensor) -> torch.Tensor:
         fc1, fc2 = self.fc1, self.fc2
-        # One node where the GELU-backward epilogue fits (CTA pairs: 256 rows per rank; 32 columns) and nobody listens in between.
-        fits = (fc1.ag.M // fc1.eng.world) % 256 == 0 and fc1.weight.shape[0] % 32 == 0 and fc2.ag_bwd.ctas % 2 == 0
-        if fits and not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in (fc1, fc2)):
+        # One node where both layers are this module's own with nobody listening in between, and the GELU-backward epilogue fits
+        # (CTA pairs: 256 rows per rank; 32 columns).
+        if (is_plain(fc1, ColumnParallelLinear) and is_plain(fc2, RowParallelLinear) and fc2.bias_in_epilogue()
+                and (fc1.ag.M // fc1.eng.world) % 256 == 0 and fc1.weight.shape[0] % 32 == 0 and fc2.ag_bwd.ctas % 2 == 0):
             return _MlpFn.apply(x_local, fc1.weight, fc1.bias, fc2.weight, fc2.bias, fc1, fc2)
         return fc2(torch.nn.functional.gelu(fc1(x_local), approximate="tanh"))

@@ -926,3 +926,68 @@ def test_tp_mlp_world_of_one_matches_fp64(native, tokens, ff):
     for got, want in zip((z,) + tuple(grads), (z64,) + tuple(g64)):
         assert ((got.double() - want).norm() / want.norm()).item() < 8e-3
     del mlp, eng
+
+
+@pytest.mark.parametrize("what", ["fp32", "unaligned", "scalar"])
+def test_row_parallel_bias_that_the_kernel_cannot_add(native, what):
+    """A bias of another type, alignment or shape than the epilogue loads is added by torch, as a layer of its own would."""
+    from pccl_b200.engine import Engine
+    from pccl_b200.ops import check_status
+    from pccl_b200.parallel.tp import RowParallelLinear
+    torch.manual_seed(12)
+    eng = Engine(0, 1)
+    eng.initEngine("cuda", 256 << 20)
+    layer = RowParallelLinear(eng, 256, 64, 256)
+    bias = {"fp32": torch.randn(256, device="cuda"), "unaligned": torch.randn(257, device="cuda").bfloat16()[1:],
+            "scalar": torch.randn(1, device="cuda").bfloat16()}[what]
+    h = torch.randn(256, 64, device="cuda").bfloat16().requires_grad_(True)
+    layer.bias = None
+    plain = layer(h).detach()
+    layer.bias = torch.nn.Parameter(bias)
+    z = layer(h)
+    assert torch.equal(z, plain + bias)
+    z.sum().backward()
+    check_status("row parallel bias")
+    assert torch.equal(layer.bias.grad, (torch.full_like(bias, 256.0) if bias.numel() > 1 else torch.full_like(bias, 65536.0)))
+    del layer, eng
+
+
+@pytest.mark.parametrize("what", ["wrapped", "patched", "global hook"])
+def test_tp_mlp_with_layers_that_are_not_plain(native, what):
+    """A layer that is wrapped, has a forward of its own or is seen by a global hook is called, not passed by."""
+    from pccl_b200.engine import Engine
+    from pccl_b200.ops import check_status
+    from pccl_b200.parallel.tp import TensorParallelMLP
+    torch.manual_seed(13)
+    eng = Engine(0, 1)
+    eng.initEngine("cuda", 256 << 20)
+    mlp = TensorParallelMLP(eng, 256, 256, 64)
+    x = torch.randn(256, 256, device="cuda").bfloat16()
+    plain = torch.nn.functional.gelu(mlp.fc1(x), approximate="tanh")
+    calls = []
+    handle = None
+    if what == "wrapped":
+        class Wrapped(torch.nn.Module):
+            def __init__(self, inner):
+                super().__init__()
+                self.inner = inner
+
+            def forward(self, x):
+                calls.append(1)
+                return self.inner(x)
+
+        mlp.fc1 = Wrapped(mlp.fc1)
+    elif what == "patched":
+        forward = mlp.fc2.forward
+        mlp.fc2.forward = lambda h: (calls.append(1), forward(h))[1]
+    else:
+        handle = torch.nn.modules.module.register_module_forward_hook(lambda m, args, out: calls.append(type(m).__name__))
+    try:
+        z = mlp(x)
+    finally:
+        if handle is not None:
+            handle.remove()
+    assert calls and (what != "global hook" or set(calls) == {"TensorParallelMLP", "ColumnParallelLinear", "RowParallelLinear"})
+    assert torch.equal(z, mlp.fc2(plain))
+    check_status("tp mlp")
+    del mlp, eng

@@ -815,7 +815,7 @@ __device__ __forceinline__ void route_token(const float* logits, int* ids, float
     int bi = 0;
 #pragma unroll
     for (int j = 0; j < PER_LANE; ++j)
-      if (v[j] > best) { best = v[j]; bi = j * 32 + lane; }
+      if (j * 32 + lane < experts && v[j] > best) { best = v[j]; bi = j * 32 + lane; }      // without it, NaN logits lose to the padding
     // warp arg-max; ties go to the lower expert id (what a stable top-k returns)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {

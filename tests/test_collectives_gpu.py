@@ -991,3 +991,28 @@ def test_tp_mlp_with_layers_that_are_not_plain(native, what):
     assert torch.equal(z, mlp.fc2(plain))
     check_status("tp mlp")
     del mlp, eng
+
+
+@pytest.mark.parametrize("E,Kt", [(8, 3), (33, 4), (1024, 8)])
+def test_moe_route_with_nan_and_infinite_logits_stays_in_range(native, E, Kt):
+    """Logits of a diverged model still give experts that exist; a row of good logits beside them is not disturbed."""
+    from pccl_b200._native import C
+    from pccl_b200.ops.moe import MoEExchange
+    torch.manual_seed(14)
+    T = 70
+    logits = torch.randn(T, E, device="cuda")
+    logits[1:20] = float("nan")
+    logits[1:10, 2] = 1.0
+    logits[20:30, 1] = float("inf")
+    logits[30:40] = -float("inf")
+    ids = torch.full((T, Kt), -7, dtype=torch.int32, device="cuda")
+    pos, probs = ids.clone(), torch.empty((T, Kt), device="cuda")
+    counts = torch.zeros(E, dtype=torch.int32, device="cuda")
+    C.moe_route(logits.data_ptr(), ids.data_ptr(), probs.data_ptr(), pos.data_ptr(), counts.data_ptr(), T, E, Kt,
+                torch.cuda.current_stream().cuda_stream)
+    assert ((ids >= 0) & (ids < E)).all()
+    assert torch.equal(counts.long(), torch.bincount(ids.view(-1).long(), minlength=E))
+    assert ((pos >= 0) & (pos < counts[ids.long()])).all()
+    good = [0] + list(range(40, T))
+    ref_ids, ref_probs = MoEExchange.route(logits[good], Kt)
+    assert torch.equal(ids[good], ref_ids) and torch.allclose(probs[good], ref_probs, rtol=1e-4, atol=1e-7)

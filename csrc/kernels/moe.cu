@@ -537,7 +537,7 @@ struct GroupedEpi {
       for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
     }
     __nv_bfloat16* d = D + static_cast<long long>(row) * ldd + col;
-    if (col + 32 <= N) {
+    if (col + 32 <= N && reinterpret_cast<uintptr_t>(D) % 16 == 0) {
 #pragma unroll
       for (int i = 0; i < 32; i += 8) st16(d + i, pack<DT_BF16>(v + i));
     } else {

@@ -993,6 +993,32 @@ def test_tp_mlp_with_layers_that_are_not_plain(native, what):
     del mlp, eng
 
 
+@pytest.mark.parametrize("N,shift", [(30, 0), (2, 0), (300, 0), (64, 2), (256, 1)])
+def test_grouped_gemm_into_unaligned_or_odd_outputs(native, N, shift):
+    """Feature counts that are no multiple of four and outputs off the 8-byte boundaries: the row-major form of the grouped kernel.
+    fp32 sums of 128 terms and one bf16 rounding."""
+    from pccl_b200.ops import check_status
+    from pccl_b200.ops.moe import grouped_gemm
+    torch.manual_seed(6)
+    K, sizes = 128, [130, 0, 5, 257]
+    off = torch.tensor([0] + list(torch.tensor(sizes).cumsum(0)), dtype=torch.int32, device="cuda")
+    total = int(off[-1])
+    a = (torch.randn(total + 3, K, device="cuda") * 0.5).bfloat16()
+    b = (torch.randn(len(sizes) * N, K, device="cuda") * 0.1).bfloat16()
+    ld = (N + shift + 7) // 8 * 8
+    store = torch.full((total + 3, ld), 7.0, device="cuda", dtype=torch.bfloat16)
+    out = store[:, shift:shift + N]
+    grouped_gemm(a, b, off, N, out=out, gelu=N == 300)
+    check_status("grouped gemm")
+    for g, n in enumerate(sizes):
+        lo = int(off[g])
+        ref = a[lo:lo + n].double() @ b[g * N:(g + 1) * N].double().t()
+        if N == 300:
+            ref = torch.nn.functional.gelu(ref, approximate="tanh")
+        assert ((out[lo:lo + n].double() - ref).abs() <= 2 ** -8 * ref.abs() + (2e-3 if N == 300 else 1e-5)).all()      # hardware tanh
+    assert (store[:, :shift] == 7.0).all() and (store[:, shift + N:] == 7.0).all() and (store[total:] == 7.0).all()
+
+
 @pytest.mark.parametrize("E,Kt", [(8, 3), (33, 4), (1024, 8)])
 def test_moe_route_with_nan_and_infinite_logits_stays_in_range(native, E, Kt):
     """Logits of a diverged model still give experts that exist; a row of good logits beside them is not disturbed."""

@@ -85,7 +85,7 @@ class Block(nn.Module):
         else:
             x, h = self.ln1.add_norm(x, delta, prev_bias)
         # split_qkv gives the projection its bias gradient, from gradients of the projection's own output: nothing may sit between
-        if (D // self.n_head) % 8 == 0 and self.qkv.bias is not None and is_plain(self.qkv, Linear):
+        if (D // self.n_head) % 8 == 0 and is_plain(self.qkv, Linear) and self.qkv.bias is not None:
             q, k, v = split_qkv(self.qkv(h, defer_bias_grad=True), self.n_head, self.qkv.bias)
         else:
             qkv = self.qkv(h).view(B, T, 3, self.n_head, D // self.n_head)

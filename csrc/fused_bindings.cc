@@ -141,7 +141,7 @@ void bindFused(py::module_& m) {
   // ---- production: this process is one rank -------------------------------------------------------
   m.def("ag_gemm", [](Engine& e, uint64_t x_off, int M, int N, int K, uint64_t w, int64_t ldw, uint64_t d, int64_t ldd,
                       uint64_t bias, uint64_t ready, uint64_t epoch, int n_copy, int ctas, int flag_lane, uint64_t status,
-                      uint64_t stream, bool b_mn, uint32_t flags, uint64_t d2, uint64_t colsum) {
+                      uint64_t stream, bool b_mn, uint32_t flags, uint64_t d2, uint64_t parts, uint64_t colsum, bool colsum_f32) {
     AgGemmArgs A{};
     A.w = e.worldTable();
     A.nvirt = 1;
@@ -150,7 +150,8 @@ void bindFused(py::module_& m) {
     A.spin_ns = kDefaultSpinLimit;
     A.tail_tiles = static_cast<int>(LaunchEnvironments::getInt("PCCL_AG_TAIL", -1));     // -1: from the cost model
     A.flags = flags | (bias ? GEMM_BIAS : 0);
-    A.r[0].D2 = reinterpret_cast<void*>(d2); A.r[0].colsum = reinterpret_cast<float*>(colsum);
+    A.r[0].D2 = reinterpret_cast<void*>(d2);
+    A.r[0].colsum = ColSum{reinterpret_cast<float*>(parts), reinterpret_cast<void*>(colsum), colsum_f32};
     A.r[0].D = reinterpret_cast<void*>(d); A.r[0].ldd = ldd; A.r[0].bias = reinterpret_cast<const void*>(bias);
     A.ready_off = ready; A.r[0].status = reinterpret_cast<uint32_t*>(status);
     A.r[0].rank = e.rank();
@@ -158,7 +159,8 @@ void bindFused(py::module_& m) {
     check(launchAgGemm(A, &h, ctas, reinterpret_cast<cudaStream_t>(stream)), "ag_gemm");
   }, py::arg("engine"), py::arg("x_off"), py::arg("M"), py::arg("N"), py::arg("K"), py::arg("w"), py::arg("ldw"), py::arg("d"), py::arg("ldd"),
      py::arg("bias"), py::arg("ready"), py::arg("epoch"), py::arg("n_copy"), py::arg("ctas"), py::arg("flag_lane"), py::arg("status"),
-     py::arg("stream"), py::arg("b_mn") = false, py::arg("flags") = 0, py::arg("d2") = 0, py::arg("colsum") = 0);
+     py::arg("stream"), py::arg("b_mn") = false, py::arg("flags") = 0, py::arg("d2") = 0, py::arg("parts") = 0,
+     py::arg("colsum") = 0, py::arg("colsum_f32") = false);
   m.def("gemm_rs", [](Engine& e, uint64_t y, int64_t ldy, uint64_t w, int64_t ldw, uint64_t out, int64_t ldo, int M, int N, int K,
                       uint64_t stage_off, uint64_t flag_off2, uint64_t epoch, int ctas, uint64_t status, uint64_t stream, bool b_mn,
                       uint64_t bias) {

@@ -26,10 +26,11 @@ void bindGemm(py::module_& m) {
         py::arg("N"), py::arg("K"), py::arg("flags"), py::arg("bias") = 0, py::arg("d2") = 0, py::arg("sms") = 0,
         py::arg("status") = 0, py::arg("stream") = 0);
   m.def("gemm_bf16_dgelu",
-        [](uint64_t a, int64_t lda, uint64_t b, int64_t ldb, uint64_t d, int64_t ldd, uint64_t pre, uint64_t colsum, int M, int N, int K,
-           uint32_t flags, int sms, uint64_t status, uint64_t stream) {
+        [](uint64_t a, int64_t lda, uint64_t b, int64_t ldb, uint64_t d, int64_t ldd, uint64_t pre, uint64_t parts, uint64_t colsum,
+           bool colsum_f32, int M, int N, int K, uint32_t flags, int sms, uint64_t status, uint64_t stream) {
+          const ColSum sums{reinterpret_cast<float*>(parts), reinterpret_cast<void*>(colsum), colsum_f32};
           int err = gemmBf16Dgelu(reinterpret_cast<const void*>(a), lda, reinterpret_cast<const void*>(b), ldb, reinterpret_cast<void*>(d),
-                                  ldd, reinterpret_cast<const void*>(pre), reinterpret_cast<float*>(colsum), M, N, K, flags, sms,
+                                  ldd, reinterpret_cast<const void*>(pre), sums, M, N, K, flags, sms,
                                   reinterpret_cast<uint32_t*>(status), reinterpret_cast<cudaStream_t>(stream));
           if (err != 0) throw std::runtime_error(std::string("gemm_bf16_dgelu: ") + cudaErrorName(err) + " " + gemmLastError());
         });

@@ -39,6 +39,16 @@ int launchLayerNormBwd(const void* dy, const void* x, const void* gamma, const f
 int colSumParts(long long rows);
 int launchColSum(const void* x, long long ld, long long rows, int N, void* out_bf16, float* partials, cudaStream_t stream);
 
+// Column sums that a GEMM epilogue takes of its output: it leaves the sum of every 32 rows in `parts` (fp32 [ceil(M / 32), N]), and
+// launchColSumParts adds those up in row order, so a run repeats itself exactly (atomic additions from the epilogue did not).
+// `out`: fp32 [N] that grows by the sums, or bf16 [N] that is written.  No sums if `out` is null.
+struct ColSum {
+  float* parts;
+  void* out;
+  bool f32;
+};
+int launchColSumParts(const ColSum& c, int M, int N, cudaStream_t stream);
+
 // Gradients of q, k, v (grads[3], bf16 [batch, heads, seq, hd] with strides[3 i ..] = batch, head, position in elements, multiples
 // of 8; the last dimension contiguous) packed into out [batch * seq, 3, heads, hd], and its column sums as bf16 [3 * heads * hd].
 // `partials`: fp32 scratch of colSumParts(batch * seq) * 3 * heads * hd elements.

@@ -7,6 +7,7 @@
 #include <cstdint>
 
 #include "api.h"
+#include "elementwise_api.h"
 
 namespace pccl {
 
@@ -38,10 +39,10 @@ struct AgGemmRank {
   void* Dq;                   // when set, the output is quantised instead: e4m3 [M, ldq] ...
   float* Ds;                  // ... with fp32 1 x 128 scales [M, N/128]
   long long ldq;
-  // bf16 CTA-pair form, D's layout: GELU of the output (flags GEMM_GELU), or the pre-activation of GEMM_DGELU, which also adds
-  // the column sums of D to `colsum` (fp32 [N], or null)
+  // bf16 CTA-pair form, D's layout: GELU of the output (flags GEMM_GELU), or the pre-activation of GEMM_DGELU, which also takes
+  // the column sums of D
   void* D2;
-  float* colsum;
+  ColSum colsum;
 };
 
 struct AgGemmArgs {

@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(DGELU ? gemm2::NUM_THREADS_WIDE : NUM_THREADS,
               static_cast<uint32_t>(A.epoch) * static_cast<uint32_t>(A.n_copy), A.spin_ns, probe};
   StoreEpi epi{R.D, R.D2, static_cast<const __nv_bfloat16*>(R.bias), R.ldd, A.M, A.N, A.flags, A.bn};
   if constexpr (DGELU) {
-    DgeluEpiT<true> de{static_cast<__nv_bfloat16*>(R.D), static_cast<const __nv_bfloat16*>(R.D2), R.colsum, R.ldd, A.M, A.N, A.bn};
+    DgeluEpiT<true> de{static_cast<__nv_bfloat16*>(R.D), static_cast<const __nv_bfloat16*>(R.D2), R.colsum.out ? R.colsum.parts : nullptr, R.ldd, A.M, A.N, A.bn};
     const int cta = static_cast<int>(tc::cluster_ctarank());
     gemm2::PairEpi<DgeluEpiT<true>> pe{de, cta};
     gemm2::PairGate<AgGate> pg{gate, cta};
@@ -187,7 +187,11 @@ int launchAgGemm(AgGemmArgs& A, const AgGemmHost* host, int ctas, cudaStream_t s
     if (e != cudaSuccess) return static_cast<int>(e);
     set[which] = true;
   }
-  if (pair) return static_cast<int>(gemm2::launch_pairs(kern, grid, dgelu ? gemm2::NUM_THREADS_WIDE : NUM_THREADS, smem_bytes, stream, true, A));
+  if (pair) {
+    int e = static_cast<int>(gemm2::launch_pairs(kern, grid, dgelu ? gemm2::NUM_THREADS_WIDE : NUM_THREADS, smem_bytes, stream, true, A));
+    for (int v = 0; dgelu && v < nv && e == 0; ++v) e = launchColSumParts(A.r[v].colsum, A.M, A.N, stream);
+    return e;
+  }
   void* args[] = {&A};
   return static_cast<int>(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kern), grid, dim3(NUM_THREADS), args, SMEM_BYTES, stream));
 }

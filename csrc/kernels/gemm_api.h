@@ -7,6 +7,7 @@
 #include <string>
 
 #include "api.h"
+#include "elementwise_api.h"
 
 namespace pccl {
 
@@ -38,11 +39,11 @@ int gemmBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, in
 int gemmSkinnyBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, int64_t ldd, int M, int N, int K, uint32_t flags,
                    const void* bias, void* D2, uint32_t* status, cudaStream_t stream, std::string* err);   // gemmBf16 with GEMM_SKINNY
 
-// D[M,N] = (A * B^T) .* gelu_tanh'(pre[M,N]) in bf16, and colsum[n] += sum_m D[m,n] (fp32, may be null): the
+// D[M,N] = (A * B^T) .* gelu_tanh'(pre[M,N]) in bf16, with its column sums (before the rounding to bf16): the
 // backward of "linear -> GELU -> linear" between the second layer's input gradient and the first layer's output
 // gradient, with the first layer's bias gradient as a by-product.  `pre` has D's row stride.  CTA pairs; N a
 // multiple of 32; flags: GEMM_B_MN only.  gelu' goes through the hardware tanh where M and N are multiples of 256.
-int gemmBf16Dgelu(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, int64_t ldd, const void* pre, float* colsum,
+int gemmBf16Dgelu(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, int64_t ldd, const void* pre, const ColSum& colsum,
                   int M, int N, int K, uint32_t flags, int sms, uint32_t* status, cudaStream_t stream);
 
 // Two GEMMs of the same K and operand forms as ONE launch: their tiles form one list for the persistent CTA pairs, so the

@@ -106,8 +106,8 @@ __device__ __forceinline__ void patch_load_bf16(uint8_t* P, int lane, const __nv
 }
 
 // Backward of a GELU that sits between two linear layers, fused into the GEMM that produces the gradient of the
-// activation: D = (A * B^T) .* gelu'(pre), and the column sums of D (the bias gradient of the first layer) are added
-// to `colsum` (fp32, zeroed by the caller).  N % 32 == 0; `pre` has D's layout.  Runs on the CTA-pair kernels (eight epilogue
+// activation: D = (A * B^T) .* gelu'(pre), and the column sums of every 32 rows of D go to `parts` (fp32 [ceil(M / 32), N], or
+// null): added up (launchColSumParts) they are the bias gradient of the first layer.  N % 32 == 0; `pre` has D's layout.  Runs on the CTA-pair kernels (eight epilogue
 // warps, coalescing patch).
 // FULL: gelu' by dgelu_logistic instead of through the hardware tanh.
 template <bool FULL = false>
@@ -115,7 +115,7 @@ struct DgeluEpiT {
   static constexpr bool kRow128 = false;
   __nv_bfloat16* D;
   const __nv_bfloat16* pre;
-  float* colsum;
+  float* parts;
   long long ldd;
   int M, N;
   int bn = BN;
@@ -162,10 +162,10 @@ struct DgeluEpiT {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * (FULL ? dgelu_logistic(x[i]) : dgelu_tanh(x[i]));
     patch_store_bf16(P, lane, D + static_cast<long long>(row0) * ldd + col, ldd, v, M - row0);
-    if (colsum) {
+    if (parts) {
       // an epilogue warp holds 32 consecutive rows, one per lane; rows past M were multiplied from zero fill, so they add 0
       warp_transpose_sum32(v, lane);
-      atomicAdd(colsum + col + lane, v[0]);
+      parts[static_cast<long long>(row0 >> 5) * N + col + lane] = v[0];
     }
   }
 };

@@ -272,7 +272,7 @@ int gemmBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, in
   return b_mn ? launch<false, true>(ta, tb, epi, K, grid, status, stream) : launch<false, false>(ta, tb, epi, K, grid, status, stream);
 }
 
-int gemmBf16Dgelu(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, int64_t ldd, const void* pre, float* colsum,
+int gemmBf16Dgelu(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, int64_t ldd, const void* pre, const ColSum& colsum,
                   int M, int N, int K, uint32_t flags, int sms, uint32_t* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda | ldb | ldd) % 8 || N % 32 ||
@@ -302,8 +302,9 @@ int gemmBf16Dgelu(const void* A, int64_t lda, const void* B, int64_t ldb, void* 
   auto x = static_cast<const __nv_bfloat16*>(pre);
   // Whole 256 x 256 tiles: gelu' through the hardware tanh.  Any other size had an accurate gelu' of its own before this epilogue
   // took it, and keeps one: 1 - tanh^2 cancels on the negative side, where the hardware tanh's 2^-11 is a fifth of gelu'(-3).
-  if (M % 256 == 0 && N % 256 == 0) return go(DgeluEpiT<false>{d, x, colsum, ldd, M, N, bn});
-  return go(DgeluEpiT<true>{d, x, colsum, ldd, M, N, bn});
+  float* parts = colsum.out ? colsum.parts : nullptr;
+  const int e = M % 256 == 0 && N % 256 == 0 ? go(DgeluEpiT<false>{d, x, parts, ldd, M, N, bn}) : go(DgeluEpiT<true>{d, x, parts, ldd, M, N, bn});
+  return e != 0 ? e : launchColSumParts(colsum, M, N, stream);
 }
 
 int gemmBf16Dual(const GemmProblem& p0, const GemmProblem& p1, int K, uint32_t flags, int sms, uint32_t* status, cudaStream_t stream) {

@@ -236,6 +236,7 @@ __global__ void __launch_bounds__(256, VPT == 1 ? 2 : 1) ln_bwd_kernel(const __n
 struct ReduceJob {
   const float* part[3];
   __nv_bfloat16* out[3];
+  float* add;              // fp32 vector that grows by the sums of the first array instead of out[0], or null
 };
 
 __global__ void __launch_bounds__(1024) partial_rows_reduce_kernel(ReduceJob job, int nparts, int D) {
@@ -256,7 +257,8 @@ __global__ void __launch_bounds__(1024) partial_rows_reduce_kernel(ReduceJob job
     float t = 0.f;
 #pragma unroll
     for (int k = 0; k < 32; ++k) t += sm[k][lane];
-    (blockIdx.y == 0 ? job.out[0] : blockIdx.y == 1 ? job.out[1] : job.out[2])[col] = __float2bfloat16_rn(t);
+    if (job.add) job.add[col] += t;
+    else (blockIdx.y == 0 ? job.out[0] : blockIdx.y == 1 ? job.out[1] : job.out[2])[col] = __float2bfloat16_rn(t);
   }
 }
 
@@ -401,7 +403,7 @@ int launchLayerNormBwd(const void* dy, const void* x, const void* gamma, const f
   };
   const int e = D <= 2048 ? go(ln_bwd_kernel<1, 3>, 1, 3, 2) : D <= 4096 ? go(ln_bwd_kernel<2, 2>, 2, 2, 1) : go(ln_bwd_kernel<4, 1>, 4, 1, 1);
   if (e != 0) return e;
-  ReduceJob job{{pg, pb, pc}, {static_cast<__nv_bfloat16*>(dgamma), static_cast<__nv_bfloat16*>(dbeta), static_cast<__nv_bfloat16*>(dcolsum)}};
+  ReduceJob job{{pg, pb, pc}, {static_cast<__nv_bfloat16*>(dgamma), static_cast<__nv_bfloat16*>(dbeta), static_cast<__nv_bfloat16*>(dcolsum)}, nullptr};
   return static_cast<int>(launchOverlapped(partial_rows_reduce_kernel, dim3((D + 31) / 32, dcolsum ? 3 : 2), dim3(1024), 0, stream, 1, job, nparts, D));
 }
 
@@ -422,8 +424,15 @@ int launchColSum(const void* x, long long ld, long long rows, int N, void* out_b
   const int e = static_cast<int>(launchOverlapped(colsum_partial_kernel, dim3(cols, parts), dim3(256), 0, stream, 1,
                                                   static_cast<const __nv_bfloat16*>(x), ld, rows, N, rows_per_part, partials));
   if (e != 0) return e;
-  ReduceJob job{{partials, nullptr, nullptr}, {static_cast<__nv_bfloat16*>(out_bf16), nullptr, nullptr}};
+  ReduceJob job{{partials, nullptr, nullptr}, {static_cast<__nv_bfloat16*>(out_bf16), nullptr, nullptr}, nullptr};
   return static_cast<int>(launchOverlapped(partial_rows_reduce_kernel, dim3((N + 31) / 32, 1), dim3(1024), 0, stream, 1, job, parts, N));
+}
+
+int launchColSumParts(const ColSum& c, int M, int N, cudaStream_t stream) {
+  if (!c.out) return 0;
+  ReduceJob job{{c.parts, nullptr, nullptr}, {c.f32 ? nullptr : static_cast<__nv_bfloat16*>(c.out), nullptr, nullptr},
+                c.f32 ? static_cast<float*>(c.out) : nullptr};
+  return static_cast<int>(launchOverlapped(partial_rows_reduce_kernel, dim3((N + 31) / 32, 1), dim3(1024), 0, stream, 1, job, (M + 31) / 32, N));
 }
 
 int launchQkvPack(const void* const* grads, const long long* strides, void* out, int batch, int seq, int heads, int hd, void* colsum_bf16,
@@ -444,7 +453,7 @@ int launchQkvPack(const void* const* grads, const long long* strides, void* out,
   const int e = static_cast<int>(launchOverlapped(qkv_pack_kernel, dim3((N + 255) / 256, parts), dim3(256), 0, stream, 1, in,
                                                   static_cast<__nv_bfloat16*>(out), rows, seq, heads, hd, rows_per_part, partials));
   if (e != 0) return e;
-  ReduceJob job{{partials, nullptr, nullptr}, {static_cast<__nv_bfloat16*>(colsum_bf16), nullptr, nullptr}};
+  ReduceJob job{{partials, nullptr, nullptr}, {static_cast<__nv_bfloat16*>(colsum_bf16), nullptr, nullptr}, nullptr};
   return static_cast<int>(launchOverlapped(partial_rows_reduce_kernel, dim3((N + 31) / 32, 1), dim3(1024), 0, stream, 1, job, parts, N));
 }
 

@@ -168,9 +168,12 @@ class _MlpFn(torch.autograd.Function):
         dz2 = _as_operand(dz)
         rows, n1 = pre.shape
         if n1 % 32 == 0:
-            sums = torch.zeros(n1, dtype=torch.float32, device=pre.device) if b1 is not None else None
+            direct = _main_grad_out(b1, torch.bfloat16) if b1 is not None else None
+            sums = direct if direct is not None or b1 is None else b1.new_empty(n1)
             dy2 = gemm_dgelu(dz2, w2, pre, b_t=True, colsum=sums)
-            db1 = _deliver_bias(b1, sums) if b1 is not None else None
+            if direct is not None:
+                _finish_main_grad(b1)
+            db1 = _deliver_bias(b1, sums) if b1 is not None and direct is None else None
         else:
             dact = gemm(dz2, w2, b_t=True)
             dy2 = torch.ops.aten.gelu_backward(dact, pre, approximate="tanh")
@@ -188,7 +191,7 @@ def _deliver_bias(bias: torch.Tensor, db: torch.Tensor) -> Optional[torch.Tensor
     if getattr(bias, "_pccl_written", False):
         mg.add_(db.to(bias.dtype))
     else:
-        mg.copy_(db)                       # rounds fp32 sums to the bucket's dtype
+        mg.copy_(db)
     _finish_main_grad(bias)
     return None
 

@@ -12,7 +12,7 @@ import torch
 
 from .._native import C
 from ..engine import Engine
-from .gemm import count_launch, status_words, stream_handle
+from .gemm import column_sums, count_launch, status_words, stream_handle
 
 
 def default_copy_ctas(world: int) -> int:
@@ -51,7 +51,8 @@ class AllGatherGemm:
                  colsum: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``w`` is [N, K]; with ``w_t`` it is stored [K, N] and consumed transposed (no copy).  ``gelu_out`` (out's shape,
         contiguous like it) receives gelu_tanh(out).  ``dgelu`` (a pre-activation of that shape; rows per rank a multiple of
-        256, N of 32) makes it ``out = product * gelu_tanh'(dgelu)``, and ``colsum`` (fp32 [N]) grows by its column sums."""
+        256, N of 32) makes it ``out = product * gelu_tanh'(dgelu)``, and ``colsum`` gets its column sums: fp32 [N] grows by them,
+        bf16 [N] is overwritten."""
         n = w.shape[1] if w_t else w.shape[0]
         if w.dtype != torch.bfloat16 or w.shape[0 if w_t else 1] != self.K or w.stride(1) != 1:
             raise ValueError("AllGatherGemm: w must be bf16 [N, K] (or [K, N] with w_t)")
@@ -61,14 +62,15 @@ class AllGatherGemm:
         if side is not None and (side.dtype != torch.bfloat16 or side.shape != out.shape or side.stride() != out.stride()
                                  or (gelu_out is not None and dgelu is not None)):
             raise ValueError("AllGatherGemm: one of gelu_out and dgelu, bf16 with out's shape and strides")
-        if colsum is not None and (dgelu is None or colsum.dtype != torch.float32 or colsum.numel() != n or not colsum.is_contiguous()):
-            raise ValueError("AllGatherGemm: colsum goes with dgelu and is a contiguous fp32 vector of length N")
+        if colsum is not None and dgelu is None:
+            raise ValueError("AllGatherGemm: colsum goes with dgelu")
+        parts, sums, f32 = column_sums(colsum, self.M, n, "AllGatherGemm")
         self.epoch += 1
         C.ag_gemm(self.eng.raw, self.eng.heap_offset(self.x_full), self.M, n, self.K, w.data_ptr(), w.stride(0), out.data_ptr(),
                   out.stride(0), bias.data_ptr() if bias is not None else 0, self.eng.heap_offset(self.ready), self.epoch, self.n_copy,
                   self.ctas, self.flag_lane, status_words().data_ptr(), stream_handle(), w_t, flags,
-                  side.data_ptr() if side is not None else 0, colsum.data_ptr() if colsum is not None else 0)
-        count_launch()
+                  side.data_ptr() if side is not None else 0, parts.data_ptr() if parts is not None else 0, sums, f32)
+        count_launch(2 if sums else 1)
         return out
 
 

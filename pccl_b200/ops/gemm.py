@@ -173,10 +173,21 @@ def gemm_dual(a0: torch.Tensor, b0: torch.Tensor, out0: torch.Tensor, a1: torch.
     count_launch()
 
 
+def column_sums(out: Optional[torch.Tensor], M: int, N: int, what: str):
+    """(scratch for the sums of every 32 rows or None, address, is fp32) for a kernel that takes the column sums of its [M, N] output."""
+    if out is None:
+        return None, 0, False
+    f32 = out.dtype is torch.float32
+    if not (f32 or out.dtype is torch.bfloat16) or out.numel() != N or not out.is_contiguous():
+        raise ValueError(f"{what}: colsum must be a contiguous fp32 or bf16 vector of length N")
+    return out.new_empty((M + 31) // 32 * N, dtype=torch.float32), out.data_ptr(), f32
+
+
 def gemm_dgelu(a: torch.Tensor, b: torch.Tensor, pre: torch.Tensor, *, b_t: bool = False, colsum: Optional[torch.Tensor] = None,
                out: Optional[torch.Tensor] = None, sms: int = 0) -> torch.Tensor:
     """``out = (a @ op(b)) * gelu_tanh'(pre)`` in one kernel (the GELU derivative is applied in the GEMM epilogue), and,
-    when ``colsum`` (fp32 [N], zeroed by the caller) is given, ``colsum += out.sum(0)``.  This is the step of an MLP's
+    when ``colsum`` is given, its column sums, added up in row order: fp32 [N] grows by them (``colsum += out.sum(0)``), bf16 [N]
+    is overwritten (``colsum = out.sum(0)``).  This is the step of an MLP's
     backward pass that turns the gradient of the second layer's input into the gradient of the first layer's output;
     the column sums are the first layer's bias gradient.  N must be a multiple of 32."""
     _check(a, "a")
@@ -189,12 +200,11 @@ def gemm_dgelu(a: torch.Tensor, b: torch.Tensor, pre: torch.Tensor, *, b_t: bool
         out = torch.empty_strided((M, N), pre.stride(), dtype=torch.bfloat16, device=a.device)
     if out.stride() != pre.stride() or out.dtype != torch.bfloat16:
         raise ValueError("gemm_dgelu: out must have pre's strides")
-    if colsum is not None and (colsum.dtype != torch.float32 or colsum.numel() != N or not colsum.is_contiguous()):
-        raise ValueError("gemm_dgelu: colsum must be a contiguous fp32 vector of length N")
+    parts, sums, f32 = column_sums(colsum, M, N, "gemm_dgelu")
     C.gemm_bf16_dgelu(a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), out.data_ptr(), out.stride(0), pre.data_ptr(),
-                      colsum.data_ptr() if colsum is not None else 0, M, N, K, C.GEMM_B_MN if b_t else 0, sms,
+                      parts.data_ptr() if parts is not None else 0, sums, f32, M, N, K, C.GEMM_B_MN if b_t else 0, sms,
                       _status_of(a), stream_handle())
-    count_launch()
+    count_launch(2 if sums else 1)
     return out
 
 

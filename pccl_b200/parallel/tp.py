@@ -89,13 +89,12 @@ class _MlpFn(torch.autograd.Function):
         n1, d = w1.shape
         dz_local = dz_local.contiguous()
         fc2.ag_bwd.x_local.copy_(dz_local)
-        sums = torch.zeros(n1, dtype=torch.float32, device=w1.device) if ctx.has_bias[0] else None
+        sums = torch.empty(n1, dtype=torch.bfloat16, device=w1.device) if ctx.has_bias[0] else None
         dpre = fc2.ag_bwd(w2, w_t=True, dgelu=pre, colsum=sums)
         dx = fc1.rs_bwd(dpre, w1, w_t=True)
         dw1, dw2 = torch.empty_like(w1, memory_format=torch.contiguous_format), torch.empty_like(w2, memory_format=torch.contiguous_format)
         gemm_dual(dpre, fc1.ag.x_full, dw1, fc2.ag_bwd.x_full, act, dw2, a_t=True, b_t=True)
-        return (dx, dw1, sums.to(torch.bfloat16) if sums is not None else None, dw2, _column_sums(dz_local) if ctx.has_bias[1] else None,
-                None, None)
+        return dx, dw1, sums, dw2, _column_sums(dz_local) if ctx.has_bias[1] else None, None, None
 
 
 class ColumnParallelLinear(nn.Module):

@@ -916,7 +916,9 @@ def test_tp_mlp_world_of_one_matches_fp64(native, tokens, ff):
     params = [x] + list(mlp.parameters())
     z = mlp(x)
     grads = torch.autograd.grad(z, params, dz)
+    again = torch.autograd.grad(mlp(x), params, dz)
     check_status("tp mlp")
+    assert all(torch.equal(g, h) for g, h in zip(grads, again))
     p64 = [p.detach().double().requires_grad_(True) for p in params]
     names = ["x"] + [n for n, _ in mlp.named_parameters()]
     q = dict(zip(names, p64))

@@ -225,6 +225,29 @@ def test_gemm_dgelu_off_the_tiles_is_accurate_on_the_negative_side(M, N):
     assert ((out.double() - x.grad).abs() <= (2 ** -8 + 1e-4) * x.grad.abs() + 1e-7).all()
 
 
+@pytest.mark.parametrize("M,N", [(1, 32), (31, 96), (33, 256), (2048, 512), (9001, 288)])
+def test_gemm_dgelu_column_sums_repeat_exactly(M, N):
+    """The bias gradient is the same from run to run, in both forms; fp32 sums of M values in groups of 32 rows, against fp64 sums of
+    the values themselves, which differ from the summed ones by one bf16 rounding each."""
+    from pccl_b200.ops import check_status
+    from pccl_b200.ops.gemm import gemm_dgelu
+    K = 64
+    a, b, pre = _rand((M, K), 68), _rand((K, N), 69, 0.1), _rand((M, N), 70)
+    runs = []
+    for _ in range(4):
+        f32, b16 = torch.full((N,), 3.0, device="cuda"), torch.full((N,), 9.0, dtype=torch.bfloat16, device="cuda")
+        out = gemm_dgelu(a, b, pre, b_t=True, colsum=f32)
+        gemm_dgelu(a, b, pre, b_t=True, colsum=b16)
+        runs.append((out, f32, b16))
+    check_status("gemm dgelu sums")
+    for r in runs[1:]:
+        assert all(torch.equal(x, y) for x, y in zip(r, runs[0]))
+    out, f32, b16 = runs[0]
+    want, spread = out.double().sum(0), out.double().abs().sum(0)
+    assert ((f32.double() - 3 - want).abs() <= 2 ** -8 * spread + 1e-5).all()
+    assert ((b16.double() - want).abs() <= 2 ** -8 * (spread + want.abs()) + 1e-5).all()
+
+
 @pytest.mark.parametrize("M", [1, 15, 17, 33, 100, 128])
 @pytest.mark.parametrize("N,K", [(40, 72), (1001, 200), (512, 2048), (8200, 520)])
 @pytest.mark.parametrize("b_t", [False, True])

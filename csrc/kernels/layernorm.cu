@@ -12,6 +12,8 @@
 // to dgamma / dbeta.  That removes the separate element-wise add kernels and one pass per bias gradient.
 #include <cuda_bf16.h>
 
+#include <initializer_list>
+
 #include "api.h"
 #include "elementwise_api.h"
 #include "launch.h"
@@ -365,12 +367,19 @@ __global__ void __launch_bounds__(256) qkv_pack_kernel(QkvGrads in, __nv_bfloat1
   }
 }
 
+// The kernels read and write 16 bytes at a time.
+bool aligned16(std::initializer_list<const void*> pointers) {
+  uintptr_t bits = 0;
+  for (const void* p : pointers) bits |= reinterpret_cast<uintptr_t>(p);
+  return bits % 16 == 0;
+}
+
 }  // namespace
 
 int launchLayerNormFwd(const void* x, const void* delta, void* sum_out, const void* gamma, const void* beta, void* y, float* mean,
                        float* rstd, long long rows, int D, float eps, cudaStream_t stream) {
   if (rows <= 0) return 0;
-  if (D % 8 || D > 8192 || (delta && !sum_out)) return static_cast<int>(cudaErrorInvalidValue);
+  if (D % 8 || D > 8192 || (delta && !sum_out) || !aligned16({x, delta, sum_out, gamma, beta, y})) return static_cast<int>(cudaErrorInvalidValue);
   auto X = static_cast<const __nv_bfloat16*>(x); auto G = static_cast<const __nv_bfloat16*>(gamma);
   auto B = static_cast<const __nv_bfloat16*>(beta); auto Y = static_cast<__nv_bfloat16*>(y);
   auto DL = static_cast<const __nv_bfloat16*>(delta); auto S = static_cast<__nv_bfloat16*>(sum_out);
@@ -384,7 +393,7 @@ int layerNormBwdParts(long long rows) { return static_cast<int>(rows < 148 * 2 ?
 int launchLayerNormBwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, const void* dres, void* dx,
                        void* dgamma, void* dbeta, void* dcolsum, float* partials, long long rows, int D, cudaStream_t stream) {
   if (rows <= 0) return 0;
-  if (D % 8 || D > 8192) return static_cast<int>(cudaErrorInvalidValue);
+  if (D % 8 || D > 8192 || !aligned16({dy, x, gamma, dres, dx})) return static_cast<int>(cudaErrorInvalidValue);
   const int most = layerNormBwdParts(rows);
   float* pg = partials;
   float* pb = partials + static_cast<long long>(most) * D;

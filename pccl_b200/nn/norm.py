@@ -91,8 +91,11 @@ def _ln_backward(dy2, x2, weight, stats, dres2, dg, db, dc=None):
 
 
 def _rows(t: torch.Tensor, D: int) -> torch.Tensor:
+    """``t`` as contiguous rows on a 16-byte boundary, as the kernels read them."""
     t2 = t.reshape(-1, D)
-    return t2 if t2.is_contiguous() else t2.contiguous()
+    if not t2.is_contiguous():
+        return t2.contiguous()
+    return t2 if t2.data_ptr() % 16 == 0 else t2.clone()
 
 
 class _LayerNormFn(torch.autograd.Function):

@@ -527,6 +527,25 @@ def test_projections_that_are_not_the_plain_layer(what):
             assert (p.grad.float() - q.grad.float()).abs().max().item() <= 0.04 * q.grad.float().abs().max().item(), name
 
 
+def test_layer_norm_of_rows_off_the_16_byte_boundaries():
+    """Contiguous views that start anywhere are read like aligned ones (same values, same kernel)."""
+    from pccl_b200.nn import LayerNorm
+    torch.manual_seed(11)
+    ln = LayerNorm(64, device="cuda")
+    data = torch.randn(3, 20 * 64 + 8, device="cuda").bfloat16()
+
+    def run(shift):
+        x, d, g = (data[i, 1:1 + 20 * 64].view(20, 64) if shift else data[i, 1:1 + 20 * 64].clone().view(20, 64) for i in range(3))
+        assert (x.data_ptr() % 16 != 0) == shift
+        x.requires_grad_(True)
+        d.requires_grad_(True)
+        s, y = ln.add_norm(x, d, None)
+        out = [s, y, ln(x)] + list(torch.autograd.grad([s, y], [x, d, ln.weight, ln.bias], [g, g]))
+        return [t.detach() for t in out]
+
+    assert all(torch.equal(a, b) for a, b in zip(run(True), run(False)))
+
+
 def test_profiler_target_of_the_training_kernels_runs():
     """The documented command, on a small case."""
     import os

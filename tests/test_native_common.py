@@ -83,3 +83,15 @@ def test_cpu_reduce(native, dtype, name, op):
     d = a.clone()
     assert native.utils.cpu_reduce(d.data_ptr(), b.data_ptr(), d.numel() * d.element_size(), name, op)
     assert torch.equal(d, want)
+
+
+@pytest.mark.parametrize("bad", range(6))
+def test_norm_kernels_refuse_addresses_off_the_16_byte_boundaries(native, bad):
+    """The host refuses before anything is launched (there is no memory at these addresses)."""
+    at = [4096 + 16 * i + (2 if i == bad else 0) for i in range(6)]
+    with pytest.raises(RuntimeError, match="layernorm_fwd: invalid argument"):
+        native.layernorm_fwd(*at, 0, 0, 4, 64, 1e-5, 0)
+    if bad < 5:
+        dy, x, g, dres, dx = at[:5]
+        with pytest.raises(RuntimeError, match="layernorm_bwd: invalid argument"):
+            native.layernorm_bwd(dy, x, g, 4096, 4096, dres, dx, 4096, 4096, 0, 4096, 4, 64, 0)

@@ -23,7 +23,7 @@ enum GemmFlags : uint32_t {
   GEMM_ADD_D2 = 1u << 8,      // D = A*B^T (+bias) + D2 (bf16, D's layout, read only): a residual connection; not with GEMM_GELU
   GEMM_ROW_STORES = 1u << 9,  // epilogue stores straight from the accumulator layout (a row per lane) instead of through the
                               // coalescing patch: for comparison runs
-  GEMM_SKINNY = 1u << 10,     // few rows (M <= 256, A K-major): weights on the tile's M side, K split over a cluster (gemm_skinny.cu)
+  GEMM_SKINNY = 1u << 10,     // few rows (M <= 128, A K-major): weights on the tile's M side, K split over a cluster (gemm_skinny.cu)
   GEMM_DGELU = 1u << 11,      // grouped and all-gather GEMM: D = A*B^T .* gelu_tanh'(D2) (D2 bf16, D's layout, read only)
   GEMM_GELU_FULL = 1u << 12,  // GEMM_GELU through exp and a division instead of the hardware tanh (relative error 2^-11)
 };
@@ -38,6 +38,7 @@ int gemmBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, in
 
 int gemmSkinnyBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, int64_t ldd, int M, int N, int K, uint32_t flags,
                    const void* bias, void* D2, uint32_t* status, cudaStream_t stream, std::string* err);   // gemmBf16 with GEMM_SKINNY
+int gemmSkinnySplits(int N, int K, int sms);     // CTAs per feature tile
 
 // D[M,N] = (A * B^T) .* gelu_tanh'(pre[M,N]) in bf16, with its column sums (before the rounding to bf16): the
 // backward of "linear -> GELU -> linear" between the second layer's input gradient and the first layer's output

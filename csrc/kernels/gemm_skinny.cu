@@ -1,4 +1,4 @@
-// bf16 GEMM for few rows: D[M, N] = A[M, K] * op(B) with M <= 256 (a linear layer at decode-sized token counts, or its input
+// bf16 GEMM for few rows: D[M, N] = A[M, K] * op(B) with M <= 128 (a linear layer at decode-sized token counts, or its input
 // gradient).  The weights are what is read, once, so the kernel is laid out as a stream over them:
 //
 //   * operands exchanged: 128 output features (rows of the weight matrix) are the M side of tcgen05.mma and the input rows,
@@ -13,7 +13,8 @@
 // Device time on one B200, cold L2 (us; single-CTA 128 x 256 tiles -> this kernel): 24 rows 8192 x 8192 71.7 -> 38.8,
 // 128 rows 73.7 -> 43.0, 24 rows 512 -> 8192 inner 59.4 -> 14.3, 24 rows 2048 x 2048 26.7 -> 12.3, 24 rows of 50257 x 2048
 // 61.4 -> 53.3.  With the weights' bytes at the copy rate those take 20, 20, 1.3, 1.3 and 31; an empty launch measures about
-// 8 in the same loop.  From 129 rows on the CTA-pair kernel is as good or better (256 rows 50257 x 2048: 61.5 against 96).
+// 8 in the same loop.  From 129 rows on the CTA-pair kernel is as good or better (256 rows of 50257 x 2048: 61.5 against 96 with
+// a form of this kernel for 256 rows).
 #include <cuda.h>
 
 #include <string>
@@ -34,7 +35,6 @@ constexpr int W_BYTES = TILE_F * BK * 2;              // 16 KiB
 constexpr int MAX_STAGES = 8;
 constexpr int NUM_THREADS = 256;                      // producer warp, MMA warp; all eight read TMEM and reduce
 constexpr int RING_BYTES = 100 * 1024;
-constexpr int P_ROWS = 128;                           // rows per reduction pass: 64 KiB of fp32 partials over the drained ring
 constexpr int SMEM_BYTES = RING_BYTES + 1024 + 256;
 
 struct Barriers {
@@ -129,7 +129,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   const int kb0 = static_cast<int>(static_cast<long long>(A.num_kb) * rank / SPLITS);
   const int kb1 = static_cast<int>(static_cast<long long>(A.num_kb) * (rank + 1) / SPLITS);
   const int stage_bytes = W_BYTES + A.nb * (BK * 2);
-  const uint32_t tmem_cols = A.nb <= 32 ? 32u : A.nb <= 64 ? 64u : A.nb <= 128 ? 128u : 256u;
+  const uint32_t tmem_cols = A.nb <= 32 ? 32u : A.nb <= 64 ? 64u : 128u;
   volatile uint32_t* abort = &bar->abort;
 
   if (threadIdx.x == 0) {
@@ -211,47 +211,43 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __syncthreads();
   const bool failed = *abort != 0;
 
-  float* P = reinterpret_cast<float*>(smem);        // [row][128 features]
+  float* P = reinterpret_cast<float*>(smem);        // [row][128 features], up to 64 KiB over the drained ring
   const uint32_t p_addr = tc::smem_u32(P);
-  for (int r0 = 0; r0 < A.nb; r0 += P_ROWS) {
-    const int rows = min(P_ROWS, A.nb - r0);
-    if (!failed) {                                  // two warps per lane quarter, each half of the rows
-      const int quarter = warp & 3, half = (rows / 16 + 1) / 2 * 16;
-      for (int c = (warp >> 2) ? half : 0; c < ((warp >> 2) ? rows : half); c += 16) {
-        uint32_t r[16];
-        tc::tmem_ld_32x16(tmem + (static_cast<uint32_t>(quarter * 32) << 16) + r0 + c, r);
-        tc::tmem_ld_wait();
+  if (!failed) {                                    // two warps per lane quarter, each half of the rows
+    const int quarter = warp & 3, half = (A.nb / 16 + 1) / 2 * 16;
+    for (int c = (warp >> 2) ? half : 0; c < ((warp >> 2) ? A.nb : half); c += 16) {
+      uint32_t r[16];
+      tc::tmem_ld_32x16(tmem + (static_cast<uint32_t>(quarter * 32) << 16) + c, r);
+      tc::tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 16; ++j) P[(c + j) * TILE_F + quarter * 32 + lane] = __uint_as_float(r[j]);
-      }
+      for (int j = 0; j < 16; ++j) P[(c + j) * TILE_F + quarter * 32 + lane] = __uint_as_float(r[j]);
     }
-    tc::cluster_sync();                             // all partial tiles of the cluster are written
-    const int live = min(rows, A.M - r0);
-    if (!failed) {
-      // a warp takes one row at a time per CTA of the cluster; eight 16-byte loads are in flight per lane
-      constexpr int R = 8 / SPLITS;
-      for (int row = rank + warp * SPLITS; row < live; row += 8 * SPLITS * R) {
-        float4 v[R][SPLITS];
-#pragma unroll
-        for (int i = 0; i < R; ++i) {
-          const int rr = min(row + i * 8 * SPLITS, live - 1);
-          const uint32_t off = p_addr + static_cast<uint32_t>(rr * TILE_F + lane * 4) * 4u;
-#pragma unroll
-          for (int q = 0; q < SPLITS; ++q) v[i][q] = ld_cluster_f4(tc::mapa(off, static_cast<uint32_t>(q)));
-        }
-#pragma unroll
-        for (int i = 0; i < R; ++i) {
-          float4 s = v[i][0];
-#pragma unroll
-          for (int q = 1; q < SPLITS; ++q) {
-            s.x += v[i][q].x; s.y += v[i][q].y; s.z += v[i][q].z; s.w += v[i][q].w;
-          }
-          if (row + i * 8 * SPLITS < live && f0 + lane * 4 < A.N) skinny_store(A, r0 + row + i * 8 * SPLITS, f0 + lane * 4, s);
-        }
-      }
-    }
-    tc::cluster_sync();                             // nobody reads this CTA's partials any more
   }
+  tc::cluster_sync();                               // all partial tiles of the cluster are written
+  if (!failed) {
+    // a warp takes one row at a time per CTA of the cluster; eight 16-byte loads are in flight per lane
+    constexpr int R = 8 / SPLITS;
+    for (int row = rank + warp * SPLITS; row < A.M; row += 8 * SPLITS * R) {
+      float4 v[R][SPLITS];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const int rr = min(row + i * 8 * SPLITS, A.M - 1);
+        const uint32_t off = p_addr + static_cast<uint32_t>(rr * TILE_F + lane * 4) * 4u;
+#pragma unroll
+        for (int q = 0; q < SPLITS; ++q) v[i][q] = ld_cluster_f4(tc::mapa(off, static_cast<uint32_t>(q)));
+      }
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        float4 s = v[i][0];
+#pragma unroll
+        for (int q = 1; q < SPLITS; ++q) {
+          s.x += v[i][q].x; s.y += v[i][q].y; s.z += v[i][q].z; s.w += v[i][q].w;
+        }
+        if (row + i * 8 * SPLITS < A.M && f0 + lane * 4 < A.N) skinny_store(A, row + i * 8 * SPLITS, f0 + lane * 4, s);
+      }
+    }
+  }
+  tc::cluster_sync();                               // nobody reads this CTA's partials any more
   tc::tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -261,6 +257,16 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 }
 
 }  // namespace
+
+// CTAs per feature tile: as many as are resident at once (two per SM), each with at least four k-blocks to stream.  Measured at 24
+// rows with 1 / 2 / 4 / 8 CTAs per tile (us): 8192 x 8192 51 / 41 / 39 / 43, 12288 x 4096 35 / 31 / 37 / 39, 50257 x 2048
+// 53 / 59 / 66 / 84, 512 x 8192 37 / 25 / 16 / 14: the rule takes 4, 2, 1 and 8.
+int gemmSkinnySplits(int N, int K, int sms) {
+  const int tiles = (N + sk::TILE_F - 1) / sk::TILE_F, num_kb = (K + sk::BK - 1) / sk::BK;
+  int splits = 1;
+  while (splits < 8 && tiles * splits * 2 <= 2 * sms && num_kb >= splits * 8) splits *= 2;
+  return splits;
+}
 
 int gemmSkinnyBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, int64_t ldd, int M, int N, int K, uint32_t flags,
                    const void* bias, void* D2, uint32_t* status, cudaStream_t stream, std::string* err) {
@@ -274,11 +280,7 @@ int gemmSkinnyBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void*
   const int tiles = (N + sk::TILE_F - 1) / sk::TILE_F;
   int stages = sk::RING_BYTES / (sk::W_BYTES + nb * sk::BK * 2);
   if (stages > sk::MAX_STAGES) stages = sk::MAX_STAGES;
-  // As many CTAs as are resident at once (two per SM), each with at least four k-blocks to stream.  Measured at 24 rows with
-  // 1 / 2 / 4 / 8 CTAs per tile (us): 8192 x 8192 51 / 41 / 39 / 43, 12288 x 4096 35 / 31 / 37 / 39, 50257 x 2048 53 / 59 / 66 / 84,
-  // 512 x 8192 37 / 25 / 16 / 14: the rule takes 4, 2, 1 and 8.
-  int splits = 1;
-  while (splits < 8 && tiles * splits * 2 <= 2 * deviceSmCount() && num_kb >= splits * 8) splits *= 2;
+  const int splits = gemmSkinnySplits(N, K, deviceSmCount());
   SkinnyArgs args{D, D2, static_cast<const __nv_bfloat16*>(bias), ldd, M, N, num_kb, nb, stages, flags, status};
   static bool set[8] = {false, false, false, false, false, false, false, false};
   auto go = [&](auto kern, bool* done) {

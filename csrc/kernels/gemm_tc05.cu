@@ -239,7 +239,7 @@ int gemmBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void* D, in
     return static_cast<int>(cudaErrorInvalidValue);
   }
   const bool a_mn = flags & GEMM_A_MN, b_mn = flags & GEMM_B_MN;
-  if ((flags & GEMM_SKINNY) && !a_mn && M <= 256 && reinterpret_cast<uintptr_t>(D2) % 8 == 0)
+  if ((flags & GEMM_SKINNY) && !a_mn && M <= 128 && reinterpret_cast<uintptr_t>(D2) % 8 == 0)
     return gemmSkinnyBf16(A, lda, B, ldb, D, ldd, M, N, K, flags, bias, D2, status, stream, &g_err);
   // tensor maps: a K-major operand has dims {K, rows}, an MN-major one {rows, K}
   StoreEpi epi{D, D2, static_cast<const __nv_bfloat16*>(bias), ldd, M, N, flags};

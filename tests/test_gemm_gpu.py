@@ -249,11 +249,13 @@ def test_gemm_dgelu_column_sums_repeat_exactly(M, N):
 
 
 @pytest.mark.parametrize("M", [1, 15, 17, 33, 100, 128])
-@pytest.mark.parametrize("N,K", [(40, 72), (1001, 200), (512, 2048), (8200, 520)])
+@pytest.mark.parametrize("N,K,splits", [(40, 72, 1), (1001, 200, 1), (512, 2048, 8), (8200, 520, 2), (1001, 1032, 4), (8190, 1096, 4)])
 @pytest.mark.parametrize("b_t", [False, True])
-def test_few_row_gemm(M, N, K, b_t):
-    """Weights on the tile's M side, K split over a cluster of 1, 4 or 8 CTAs, with every epilogue."""
+def test_few_row_gemm(M, N, K, splits, b_t):
+    """Weights on the tile's M side, K split over a cluster of 1, 2, 4 or 8 CTAs, with every epilogue."""
+    from pccl_b200._native import C
     from pccl_b200.ops import gemm, check_status
+    assert C.gemm_skinny_splits(N, K, 148) == splits
     ld = (N + 7) // 8 * 8
     a = _rand((M, K), 71)
     b = _rand((K, ld), 72)[:, :N] if b_t else _rand((N, K), 72)

@@ -240,8 +240,11 @@ void bindFused(py::module_& m) {
   m.def("emu_ag_gemm", [](const std::vector<uint64_t>& heaps, uint64_t flag_off, uint64_t x_off, int M, int N, int K,
                           const std::vector<uint64_t>& w, int64_t ldw, const std::vector<uint64_t>& d, int64_t ldd,
                           uint64_t ready_off, uint64_t epoch, int n_copy, int ctas,
-                          const std::vector<uint64_t>& status, uint64_t spin_ns, uint64_t stream, int tail_tiles) {
+                          const std::vector<uint64_t>& status, uint64_t spin_ns, uint64_t stream, int tail_tiles, bool b_mn,
+                          uint32_t flags, const std::vector<uint64_t>& bias, const std::vector<uint64_t>& d2,
+                          const std::vector<uint64_t>& parts, const std::vector<uint64_t>& colsum) {
     AgGemmArgs A{};
+    A.flags = flags | (bias.empty() ? 0 : GEMM_BIAS);
     A.ready_off = ready_off;
     A.w = emuWorld2(heaps, flag_off);
     int n = A.w.world;
@@ -254,19 +257,25 @@ void bindFused(py::module_& m) {
       A.r[r].D = reinterpret_cast<void*>(d.at(r)); A.r[r].ldd = ldd;
       A.r[r].status = reinterpret_cast<uint32_t*>(status.at(r));
       A.r[r].rank = r;
-      h[r] = AgGemmHost{reinterpret_cast<const void*>(w.at(r)), ldw, false};
+      A.r[r].bias = bias.empty() ? nullptr : reinterpret_cast<const void*>(bias.at(r));
+      A.r[r].D2 = d2.empty() ? nullptr : reinterpret_cast<void*>(d2.at(r));
+      if (!colsum.empty()) A.r[r].colsum = ColSum{reinterpret_cast<float*>(parts.at(r)), reinterpret_cast<void*>(colsum.at(r)), false};
+      h[r] = AgGemmHost{reinterpret_cast<const void*>(w.at(r)), ldw, b_mn};
     }
     check(launchAgGemm(A, h.data(), ctas, reinterpret_cast<cudaStream_t>(stream)), "emu_ag_gemm");
   }, py::arg("heaps"), py::arg("flag_off"), py::arg("x_off"), py::arg("M"), py::arg("N"), py::arg("K"), py::arg("w"), py::arg("ldw"),
      py::arg("d"), py::arg("ldd"), py::arg("ready_off"), py::arg("epoch"), py::arg("n_copy"), py::arg("ctas"), py::arg("status"),
-     py::arg("spin_ns"), py::arg("stream"), py::arg("tail_tiles") = -1);
+     py::arg("spin_ns"), py::arg("stream"), py::arg("tail_tiles") = -1, py::arg("b_mn") = false, py::arg("flags") = 0,
+     py::arg("bias") = std::vector<uint64_t>{}, py::arg("d2") = std::vector<uint64_t>{}, py::arg("parts") = std::vector<uint64_t>{},
+     py::arg("colsum") = std::vector<uint64_t>{});
   // time attribution of the fused kernels: a zeroed device buffer of PROBE_WORDS u64 per CTA, or 0 to switch it off
   m.def("fused_set_probe", [](uint64_t ptr) { setFusedProbe(reinterpret_cast<unsigned long long*>(ptr)); });
   m.attr("PROBE_WORDS") = kProbeWords;
   m.def("emu_gemm_rs", [](const std::vector<uint64_t>& heaps, const std::vector<uint64_t>& y, int64_t ldy,
                           const std::vector<uint64_t>& w, int64_t ldw, const std::vector<uint64_t>& out, int64_t ldo, int M,
                           int N, int K, uint64_t stage_off, uint64_t flag_off2, uint64_t epoch, int ctas,
-                          const std::vector<uint64_t>& status, uint64_t spin_ns, uint64_t stream) {
+                          const std::vector<uint64_t>& status, uint64_t spin_ns, uint64_t stream, bool b_mn,
+                          const std::vector<uint64_t>& bias) {
     GemmRsArgs A{};
     A.w = emuWorld2(heaps, 0);
     int n = A.w.world;
@@ -277,8 +286,11 @@ void bindFused(py::module_& m) {
     for (int r = 0; r < n; ++r) {
       A.r[r].out = reinterpret_cast<void*>(out.at(r)); A.r[r].ldo = ldo;
       A.r[r].status = reinterpret_cast<uint32_t*>(status.at(r)); A.r[r].rank = r;
-      h[r] = GemmRsHost{reinterpret_cast<const void*>(y.at(r)), ldy, reinterpret_cast<const void*>(w.at(r)), ldw, false};
+      A.r[r].bias = bias.empty() ? nullptr : reinterpret_cast<const void*>(bias.at(r));
+      h[r] = GemmRsHost{reinterpret_cast<const void*>(y.at(r)), ldy, reinterpret_cast<const void*>(w.at(r)), ldw, b_mn};
     }
     check(launchGemmRs(A, h.data(), ctas, reinterpret_cast<cudaStream_t>(stream)), "emu_gemm_rs");
-  });
+  }, py::arg("heaps"), py::arg("y"), py::arg("ldy"), py::arg("w"), py::arg("ldw"), py::arg("out"), py::arg("ldo"), py::arg("M"), py::arg("N"),
+     py::arg("K"), py::arg("stage_off"), py::arg("flag_off2"), py::arg("epoch"), py::arg("ctas"), py::arg("status"), py::arg("spin_ns"),
+     py::arg("stream"), py::arg("b_mn") = false, py::arg("bias") = std::vector<uint64_t>{});
 }

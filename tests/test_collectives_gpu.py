@@ -1044,3 +1044,83 @@ def test_moe_route_with_nan_and_infinite_logits_stays_in_range(native, E, Kt):
     good = [0] + list(range(40, T))
     ref_ids, ref_probs = MoEExchange.route(logits[good], Kt)
     assert torch.equal(ids[good], ref_ids) and torch.allclose(probs[good], ref_probs, rtol=1e-4, atol=1e-7)
+
+
+@pytest.mark.parametrize("world,M_local,N,w_t", [(2, 256, 520, False), (4, 256, 96, True), (2, 512, 320, True), (2, 4352, 512, False)])
+def test_ag_gemm_gelu_forms_emulated(native, world, M_local, N, w_t):
+    """Bias and GELU, and the GELU-backward form with its column sums, over the gathered rows of several ranks; 4352 rows per rank
+    are a second block of 16 tile rows.  One bf16 rounding (2^-8), fp32 sums of 64 terms; column sums of unrounded values."""
+    K = 64
+    M = M_local * world
+    g = torch.Generator(device="cuda").manual_seed(15)
+    def rand(*shape, scale=1.0):
+        return (torch.randn(*shape, generator=g, device="cuda") * scale).bfloat16()
+    xs = [rand(M_local, K, scale=0.5) for _ in range(world)]
+    ws = [rand(K, N, scale=0.1) if w_t else rand(N, K, scale=0.1) for _ in range(world)]
+    bias = [rand(N) for _ in range(world)]
+    pre_in = [rand(M, N, scale=1.5) for _ in range(world)]
+    ready_off = DATA_OFF + M * K * 2
+    heaps = [torch.zeros(ready_off + 4096, dtype=torch.uint8, device="cuda") for _ in range(world)]
+    st = [torch.zeros(4, dtype=torch.int32, device="cuda") for _ in range(world)]
+    for r in range(world):
+        heaps[r][DATA_OFF:ready_off].view(torch.bfloat16).view(M, K)[r * M_local:(r + 1) * M_local] = xs[r]
+    pre, act, dpre = ([torch.full((M, N), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(world)] for _ in range(3))
+    parts = [torch.empty((M + 31) // 32 * N, device="cuda") for _ in range(world)]
+    sums = [torch.full((N,), 9.0, dtype=torch.bfloat16, device="cuda") for _ in range(world)]
+    at = lambda ts: [t.data_ptr() for t in ts]  # noqa: E731
+    ctas = (148 // world) & ~1
+
+    def run(out, epoch, **kw):
+        native.emu_ag_gemm(at(heaps), FLAG_OFF, DATA_OFF, M, N, K, at(ws), ws[0].stride(0), at(out), N, ready_off, epoch, 4, ctas, at(st), 0,
+                           torch.cuda.current_stream().cuda_stream, b_mn=w_t, **kw)
+
+    run(pre, 1, flags=native.GEMM_GELU | native.GEMM_GELU_FULL, bias=at(bias), d2=at(act))
+    forms = [(pre, lambda p, r: p + bias[r].double()), (act, lambda p, r: torch.nn.functional.gelu(p + bias[r].double(), approximate="tanh"))]
+    if N % 32 == 0:
+        def back(p, r):
+            x = pre_in[r].double().requires_grad_(True)
+            gx, = torch.autograd.grad(torch.nn.functional.gelu(x, approximate="tanh").sum(), x)
+            return p * gx
+        run(dpre, 2, flags=native.GEMM_DGELU, d2=at(pre_in), parts=at(parts), colsum=at(sums))
+        forms.append((dpre, back))
+    torch.cuda.synchronize()
+    assert all(s[0].item() == 0 for s in st), [s.tolist() for s in st]
+    X = torch.cat(xs).double()
+    for r in range(world):
+        prod = X @ (ws[r].double() if w_t else ws[r].double().t())
+        for got, want in forms:
+            ref = want(prod, r)
+            assert ((got[r].double() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-5).all()
+        if N % 32 == 0:
+            ref = back(prod, r)
+            assert ((sums[r].double() - ref.sum(0)).abs() <= 2 ** -8 * ref.sum(0).abs() + 1e-5 * ref.abs().sum(0)).all()
+
+
+@pytest.mark.parametrize("world,M_local,w_t", [(2, 128, False), (2, 256, True), (4, 256, False), (2, 4352, False)])
+def test_gemm_rs_bias_emulated(native, world, M_local, w_t):
+    """Every rank adds its bias to its own rows, once; 4352 rows per rank are a second block of 16 tile rows.  The peers' partial sums
+    are rounded to bf16 on the way: 2^-8 of each, and of the result."""
+    K, N = 64, 512
+    M = M_local * world
+    g = torch.Generator(device="cuda").manual_seed(16)
+    def rand(*shape, scale=1.0):
+        return (torch.randn(*shape, generator=g, device="cuda") * scale).bfloat16()
+    ys = [rand(M, K, scale=0.5) for _ in range(world)]
+    ws = [rand(K, N, scale=0.1) if w_t else rand(N, K, scale=0.1) for _ in range(world)]
+    bias = [rand(N) for _ in range(world)]
+    stage_bytes = world * M_local * N * 2
+    n_flags = world * (M_local // 128) * (N // 256)
+    heaps = [torch.zeros(DATA_OFF + stage_bytes + n_flags * 8, dtype=torch.uint8, device="cuda") for _ in range(world)]
+    st = [torch.zeros(4, dtype=torch.int32, device="cuda") for _ in range(world)]
+    outs = [torch.zeros(M_local, N, dtype=torch.bfloat16, device="cuda") for _ in range(world)]
+    at = lambda ts: [t.data_ptr() for t in ts]  # noqa: E731
+    native.emu_gemm_rs(at(heaps), at(ys), K, at(ws), ws[0].stride(0), at(outs), N, M, N, K, DATA_OFF, DATA_OFF + stage_bytes, 1, 148 // world,
+                       at(st), 0, torch.cuda.current_stream().cuda_stream, b_mn=w_t, bias=at(bias))
+    torch.cuda.synchronize()
+    assert all(s[0].item() == 0 for s in st), [s.tolist() for s in st]
+    parts = [ys[r].double() @ (ws[r].double() if w_t else ws[r].double().t()) for r in range(world)]
+    for r in range(world):
+        rows = slice(r * M_local, (r + 1) * M_local)
+        ref = sum(p[rows] for p in parts) + bias[r].double()
+        spread = sum(p[rows].abs() for p in parts) + ref.abs()
+        assert ((outs[r].double() - ref).abs() <= 2 ** -8 * spread + 1e-5).all()

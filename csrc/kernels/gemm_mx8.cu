@@ -117,7 +117,9 @@ thread_local std::string g_errx;
 
 // Columns per tile: 224 unless narrower tiles fill the last round of CTAs better.  Measured time of a full round relative to
 // 224 columns (148 tiles of 128 rows each, K = 2048 and 8192, one B200, mean of the two): a round is bound by the operands
-// that an SM gets from L2, of which A's 128 rows stay.  1531 x 8192 x 3584: 192 tiles of 224 in two rounds, 276 of 160 in two.
+// that an SM gets from L2, of which A's 128 rows stay.  1531 x 3584 x 8192: 192 tiles of 224 in two rounds, 276 of 160 in two.
+// Against 224 columns (us): 300 x 4096 x 1024 15.3 -> 13.3, 777 x 2048 x 2048 19.5 -> 17.4, 1000 x 1152 x 4096 25.6 -> 21.4,
+// 1531 x 3584 x 8192 60 -> 54 to 58; within 2 % at four larger shapes, which keep 224.
 int pickWidthMx(int tiles_m, int n, int sms) {
   static const struct { int bn; float round; } kWidths[] = {{224, 1.f}, {192, .89f}, {160, .83f}, {128, .78f}, {96, .75f}, {64, .70f}, {32, .68f}};
   int best = gemmx::BN;

@@ -197,6 +197,12 @@ const char* gemmLastError() { return g_err.c_str(); }
 // 224 ... 32).  Measured both ways (us, 256 wide -> chosen): 1531 x 2048 x 8192 53 -> 47 (48 tiles on 74 pairs -> 66),
 // 2331 x 768 x 3072 28.6 -> 22.6, 8192 x 3584 x 8192 328 -> 316 (448 tiles = 6.05 rounds -> 512 = 6.9); 1531 x 6144 x 2048
 // (144 tiles, 1.95 rounds) stays at 256: 40 against 44 at 192.  Two problems (gemmBf16Dual) share one width.
+// With an MN-major B a CTA loads whole 64-column boxes, and a round costs more at the widths that do not fill them (1, .935, .84,
+// .805, .70, .705, .68, .61 for 256 ... 32).  The one table serves that form and the epilogues with arithmetic too, because few
+// choices lie between the two: over 20 shapes x 3 operand forms (768 x 2304 x 2331 to 8192 x 2048 x 16384), cold L2, the rule's width
+// was never more than 4 % behind 256 columns and mostly the best of the eight or within 1 us of it (us, 256 -> rule; MN-major B:
+// 1531 x 2048 x 8192 58 -> 50, 2331 x 768 x 3072 26.7 -> 21.5, 8192 x 3584 x 8192 366 -> 345, 1999 x 1416 x 3000 30.8 -> 31.7; GELU
+// backward: 1000 x 1024 x 256 21.5 -> 15.4, 1531 x 8192 x 2048 51 -> 51 (224: 49), 8192 x 3584 x 8192 329 -> 331).
 int gemmPairTileN(int tiles_m0, int n0, int tiles_m1, int n1, int pairs) {
   static const struct { int bn; float round; } kWidths[] = {{256, 1.f}, {224, .91f}, {192, .80f}, {160, .725f},
                                                             {128, .62f}, {96, .56f}, {64, .53f}, {32, .48f}};

@@ -895,7 +895,7 @@ def test_run_time_compiled_program_launches_and_mixes_with_the_interpreter(nativ
     del ar, ag, eng
 
 
-@pytest.mark.parametrize("tokens,ff", [(256, 320), (768, 64), (256, 328), (384, 320)])
+@pytest.mark.parametrize("tokens,ff", [(256, 320), (768, 64), (256, 328), (384, 320), (768, 4672)])       # the last one: tiles of 224 columns
 def test_tp_mlp_world_of_one_matches_fp64(native, tokens, ff):
     """The MLP as one node (GELU, its derivative and the biases in the fused kernels' epilogues), and the layer-by-layer form that
     a d_ff off the multiples of 32 (328) or rows off the multiples of 256 (384) take.  Against fp64; up to four bf16 roundings

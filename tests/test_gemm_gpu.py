@@ -166,12 +166,15 @@ def test_gemm_residual_epilogue_adds_the_residual_stream():
         assert (out.float() - ref).abs().max().item() <= 2e-2 * max(1.0, ref.abs().max().item())
 
 
-# The CTA-pair kernel picks its tile width per launch: these sizes select 64, 64, 192, 128, 224, 160 and 256 columns, with
-# rows and columns that end inside a tile and (1416, 2056, 3000) inside a 32-column strip.
-@pytest.mark.parametrize("M,N,K", [(257, 40, 72), (300, 1416, 200), (1531, 2056, 136), (2331, 776, 264), (4096, 3576, 128), (1999, 1416, 328), (1531, 6152, 64)])
+# The CTA-pair kernel picks its tile width per launch: every width, with rows and columns that end inside a tile and inside a
+# 32-column strip.
+@pytest.mark.parametrize("M,N,K,width", [(257, 40, 72, 32), (300, 1416, 200, 64), (200, 4808, 72, 96), (2331, 776, 264, 128), (4096, 3576, 128, 160),
+                                         (1999, 1416, 328, 160), (1531, 2056, 136, 192), (1531, 6152, 64, 192), (700, 4664, 136, 224), (700, 5480, 72, 256)])
 @pytest.mark.parametrize("a_t,b_t", [(False, False), (False, True), (True, True)])
-def test_cta_pair_gemm_tile_widths(M, N, K, a_t, b_t):
+def test_cta_pair_gemm_tile_widths(M, N, K, width, a_t, b_t):
+    from pccl_b200._native import C
     from pccl_b200.ops import gemm, check_status
+    assert C.gemm_pair_tile_n((M + 255) // 256, N, 0, 0, 74) == width          # 148 SMs
     if a_t:
         M = (M + 7) // 8 * 8
     a = _rand((K, M) if a_t else (M, K), 61)
@@ -207,7 +210,7 @@ def test_gemm_dgelu_ragged_rows(M):
     assert (sums - ref.sum(0)).abs().max().item() <= 2e-2 * max(1.0, ref.sum(0).abs().max().item())
 
 
-@pytest.mark.parametrize("M,N", [(40, 256), (256, 288), (513, 1056)])
+@pytest.mark.parametrize("M,N", [(40, 256), (256, 288), (513, 1056), (700, 4672)])            # the last one: tiles of 224 columns
 def test_gemm_dgelu_off_the_tiles_is_accurate_on_the_negative_side(M, N):
     """gelu' where 1 - tanh^2 cancels: within the bf16 rounding of every single value, against fp64.  The product is exact (one
     nonzero per row of a), so 2^-8 is the rounding; 1e-4 of |gelu'| <= 1.2 covers the exponential's and the division's error."""

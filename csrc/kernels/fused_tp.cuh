@@ -42,12 +42,6 @@ __device__ __forceinline__ bool cta_peer_barrier(const World& W, int me, int lan
 // =================================================================================================
 // all-gather -> GEMM
 // =================================================================================================
-// Tile order of the all-gather GEMM: the rank's own rows first (they are there), then the remote rows
-// row block by row block -- block b of EVERY peer before block b+1 of any -- which is the order in which
-// the senders emit them, so the data keeps ahead of the tensor cores from the first remote tile on.
-// Within a row block consecutive tiles share the B panel (same n, different source rank).
-// [begin, end) is the slice of that order which this group of CTAs works through (`first` + it * `stride` inside it):
-// the GEMM CTAs take everything but the last `tail` tiles, the copy CTAs take the tail once their rows are sent.
 // Tile r of a panel of tiles_m x tiles_n: 16 rows of tiles at a time, column by column, so that their A rows stay in L2 while the
 // columns go by.  Down whole columns an A of 8192 x 8192 (134 MB) came from memory again for every two or three columns, which
 // a launch at the power limit pays for in clock.
@@ -58,6 +52,12 @@ __device__ __forceinline__ void panel_tile(int r, int tiles_m, int tiles_n, int*
   *n = rr / gm;
 }
 
+// Tile order of the all-gather GEMM: the rank's own rows first (they are there), then the remote rows
+// row block by row block -- block b of EVERY peer before block b+1 of any -- which is the order in which
+// the senders emit them, so the data keeps ahead of the tensor cores from the first remote tile on.
+// Within a row block consecutive tiles share the B panel (same n, different source rank).
+// [begin, end) is the slice of that order which this group of CTAs works through (`first` + it * `stride` inside it):
+// the GEMM CTAs take everything but the last `tail` tiles, the copy CTAs take the tail once their rows are sent.
 struct AgSched {
   int me, world, tiles_ml, tiles_n, first, stride;
   long long begin, end;

@@ -1,9 +1,9 @@
 // CTA-pair variant of the tcgen05 GEMM pipeline: two CTAs of a cluster (cta_group::2) compute one
-// 256 x 256 tile.  Each CTA loads its own 128 rows of A and its own 128 rows of B (half of N) per
-// k-block -- 32 KiB instead of 48 KiB per 128 x 256 of output, which takes a third off the L2 -> SM
-// traffic that bounds the single-CTA kernel -- into a 6-stage ring; the leader CTA issues
+// 256 x 256 tile (or one of fewer columns, see HasWidth and HasVarN below).  Each CTA loads its own 128 rows of A and its
+// own half of the tile's columns of B per k-block -- 32 KiB instead of 48 KiB per 128 x 256 of output, which takes a third
+// off the L2 -> SM traffic that bounds the single-CTA kernel -- into a 6-stage ring; the leader CTA issues
 // tcgen05.mma.cta_group::2 (M = 256) that reads both CTAs' shared memory and writes both CTAs'
-// tensor memory; each CTA runs the epilogue of its own 128 accumulator rows.
+// tensor memory; each CTA runs the epilogue of its own 128 accumulator rows on four or eight warps.
 //
 // No load uses cluster multicast: the operands are not shared between the CTAs, only the completion
 // of both CTAs' loads is counted on the leader's barrier.  tcgen05.commit multicasts the "stage free"

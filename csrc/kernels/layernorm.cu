@@ -1,9 +1,9 @@
-// LayerNorm forward and backward for bf16 activations (fp32 statistics).  One CTA per row; every
-// thread keeps its 8-element vectors of the row in registers, so x is read once in forward and x, dy
-// once in backward.  The backward kernel is persistent: each CTA walks rows with a stride, keeps its
-// share of dgamma / dbeta in registers across all of its rows and writes one partial row at the end;
-// a second small kernel adds the partial rows.  (PyTorch's stock backward takes two kernels and ~230 us
-// per call at 16384 x 2048.)
+// LayerNorm forward and backward for bf16 activations (fp32 statistics).  Forward: one CTA per row; every
+// thread keeps its 8-element vectors of the row in registers, so x is read once.  Backward: a group of warps
+// per row (as many as cover it), several rows at a time, x and dy read once; the kernel is persistent, its
+// threads keep their columns' share of dgamma / dbeta in registers across all of their rows, and each CTA writes
+// one partial row at the end; a second small kernel adds the partial rows.  (PyTorch's stock backward takes two
+// kernels and ~230 us per call at 16384 x 2048.)
 //
 // Both directions can carry the residual connection that surrounds the norm in a pre-norm transformer block:
 // forward takes `delta` and computes s = x + delta (stored, it is the next residual stream) and y = LN(s) in one
@@ -99,8 +99,8 @@ __global__ void __launch_bounds__(256) ln_fwd_kernel(const __nv_bfloat16* x, con
 // rows cross the group in one exchange.  A thread keeps the same columns for all of its rows, so the column sums (dgamma,
 // dbeta, bias gradient) stay in registers; the CTA's groups add theirs up at the end and write one partial row per array.
 // With dres and column sums, 148 or 296 CTAs (us, before -> now): 16384 x 768 89 -> 42, 2331 x 768 32 -> 17, 8192 x 4096 136 -> 83,
-// 4096 x 8192 218 -> 83; 16384 x 2048 77 -> 79 (3.4 TB/s; before, a form of its own for D = 256, 512, 1024 and 2048 with one warp per
-// row and its sums in shared memory).
+// 4096 x 8192 218 -> 83; 16384 x 2048 88 to 91 -> 86 to 90 warm, 77 -> 79 cold (3.4 TB/s; before, a form of its own for D = 256, 512, 1024
+// and 2048 with one warp per row and its sums in shared memory).
 template <int VPT, int R>
 __global__ void __launch_bounds__(256, VPT == 1 ? 2 : 1) ln_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
                                                                        const __nv_bfloat16* gamma, const float* mean,

@@ -558,10 +558,11 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
 // The same product with the operands exchanged: the weights of a group are the M side of the tile (256 output features; the
 // last tile of a group may reach into the next group's weights, its surplus rows are not stored) and the group's rows are the
-// N side, whose extent the MMA instruction takes per tile in steps
-// of 16.  A group of 520 rows then costs 2 + 8/256 tiles of tensor time per weight tile, where the row-major form above pays
-// for 3: with a few hundred rows per expert that is a fifth of the whole product.  The accumulator arrives transposed (lane =
-// output feature, column = row of the group), so a warp stores 32 consecutive features of one row per instruction.
+// N side, whose extent the MMA instruction takes per tile in steps of 16.  A group of 520 rows then costs 2 + 8/256 tiles of
+// tensor time per weight tile, where the row-major form above pays for 3: with a few hundred rows per expert that is a fifth of
+// the whole product.  The accumulator arrives transposed (lane = output feature, column = row of the group), so a warp stores
+// 32 consecutive features of one row per instruction.  The row-major form is left with what the 8-byte stores of this one cannot
+// write: feature counts that are no multiple of four and outputs off the 8-byte boundaries.
 struct RaggedSched {
   const int* row_off;
   int groups, tiles_f, first, stride;        // tiles_f = ceil(N / 256) weight tiles per group

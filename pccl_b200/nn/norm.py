@@ -36,9 +36,10 @@ def _grad_buffer(ctx, param: torch.Tensor) -> torch.Tensor:
     """Where a kernel puts the gradient of a parameter of the norm.  It always goes back to autograd, which knows who else
     contributes to it and which hooks see it; but where it will end in the flat bucket anyway it is written there to begin with,
     and the wrapper's hook finds nothing to copy.  The bucket is lent once per step: a second contribution gets memory of
-    its own, and autograd adds the two."""
-    mg = _writable(param)
-    if mg is None or getattr(param, "_pccl_lent", True) or not _accumulates(ctx, param):
+    its own, and autograd adds the two.  Hooks other than the wrapper's may keep what they see: memory of its own as well."""
+    mg, hooks = _writable(param), param._post_accumulate_grad_hooks
+    if (mg is None or getattr(param, "_pccl_lent", True) or param._backward_hooks or (hooks is not None and len(hooks) > 1)
+            or not _accumulates(ctx, param)):
         return torch.empty_like(param)
     param._pccl_lent = True
     return mg.view(mg.shape)                   # a tensor of its own: autograd keeps it as ``.grad`` without a copy

@@ -477,6 +477,20 @@ def test_norm_weight_that_the_loss_uses_once_more():
     assert all(torch.equal(p.main_grad, g) for p, g in zip(list(net.parameters())[1:], ref[2:]))
 
 
+def test_gradients_that_hooks_keep_are_not_the_bucket():
+    net, dp, x, t, ref = _wrapped_norms()
+    kept = []
+    net.a.weight.register_hook(kept.append)
+    net.b.bias.register_post_accumulate_grad_hook(lambda p: None)
+    net(x, t).backward()
+    dp.optimizer_step()
+    dp.zero_grad()
+    (net(x, t) * 3).backward()
+    torch.cuda.synchronize()
+    assert torch.equal(kept[0], ref[1]) and not torch.equal(kept[1], ref[1])
+    assert kept[0].data_ptr() != net.a.weight.main_grad.data_ptr()
+
+
 def test_norm_bias_may_change_between_forward_and_backward():
     from pccl_b200.nn import LayerNorm
     ln = LayerNorm(64, device="cuda")

@@ -96,18 +96,18 @@ __global__ void __launch_bounds__(256) ln_fwd_kernel(const __nv_bfloat16* x, con
 
 // Backward.  A group of `gw` warps owns a row -- as many as cover it with one 16-byte vector per thread and trip (VPT trips; one
 // up to D = 2048) -- and takes R rows at a time: R x VPT x 3 vectors are in flight per thread, and the row statistics of all R
-// rows cross the group in one exchange.  A thread keeps the same columns for all of its rows, so the column sums (dgamma,
+// rows cross the group in one exchange.  The next R rows are fetched (AHEAD) while these are worked on, as far as that goes without
+// spills, which cost far more than the fetch brings: two vectors per row in the plain form, three and the column sums of dx in the
+// EXTRA one.  A thread keeps the same columns for all of its rows, so the column sums (dgamma,
 // dbeta, bias gradient) stay in registers; the CTA's groups add theirs up at the end and write one partial row per array.
-// With dres and column sums, 148 or 296 CTAs (us, before -> now): 16384 x 768 89 -> 42, 2331 x 768 32 -> 17, 8192 x 4096 136 -> 83,
-// 4096 x 8192 218 -> 83; 16384 x 2048 88 to 91 -> 86 to 90 warm, 77 -> 79 cold (3.4 TB/s; before, a form of its own for D = 256, 512, 1024
-// and 2048 with one warp per row and its sums in shared memory).
-template <int VPT, int R>
-__global__ void __launch_bounds__(256, VPT == 1 ? 2 : 1) ln_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
-                                                                       const __nv_bfloat16* gamma, const float* mean,
-                                                                       const float* rstd, const __nv_bfloat16* dres,
-                                                                       __nv_bfloat16* dx, float* part_g,
-                                                                       float* part_b, float* part_c, long long rows,
-                                                                       int D, int gw) {
+// Times, us, cold L2 (one warp per row with its sums in shared memory for D = 256, 512, 1024 and 2048, a CTA per row for the rest
+// -> now; in brackets three rows on two CTAs per SM without the fetch ahead): EXTRA 16384 x 2048
+// 77 -> 64 [77], 16384 x 1024 44 -> 39 [48], 16384 x 256 28 -> 17 [20], 2331 x 768 32 -> 15 [17], 8192 x 4096 136 -> 64 [83], 4096 x 8192
+// 220 -> 83; plain 16384 x 2048 64 -> 52 [73] (3.9 TB/s), 16384 x 1024 40 -> 32 [44], 8192 x 4096 101 -> 52 [79], 4096 x 8192 153 -> 56 [81].
+template <int VPT, int R, bool EXTRA, bool AHEAD, int CTAS>
+__global__ void __launch_bounds__(256, CTAS) ln_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* gamma,
+                                                           const float* mean, const float* rstd, const __nv_bfloat16* dres, __nv_bfloat16* dx,
+                                                           float* part_g, float* part_b, float* part_c, long long rows, int D, int gw) {
   __shared__ float2 stat[2][8][R];                          // [parity][warp][row]: partial sums of a warp
   extern __shared__ __align__(16) float group_sums[];       // [groups][arrays][D], with more than one group
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -115,34 +115,47 @@ __global__ void __launch_bounds__(256, VPT == 1 ? 2 : 1) ln_bwd_kernel(const __n
   const int nvec = D >> 3, width = gw * 32;
   dev::pdl_launch();
   dev::pdl_wait();
+  const Vec16 zero{{0u, 0u, 0u, 0u}};
   Vec16 g[VPT];
-  float ag[VPT][8], ab[VPT][8], ac[VPT][8];
+  float ag[VPT][8], ab[VPT][8], ac[EXTRA ? VPT : 1][8];
 #pragma unroll
   for (int j = 0; j < VPT; ++j) {
-    g[j] = tid + j * width < nvec ? ld16(gamma + (tid + j * width) * 8) : Vec16{{0u, 0u, 0u, 0u}};
+    g[j] = tid + j * width < nvec ? ld16(gamma + (tid + j * width) * 8) : zero;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) { ag[j][k] = 0.f; ab[j][k] = 0.f; ac[j][k] = 0.f; }
+    for (int k = 0; k < 8; ++k) {
+      ag[j][k] = 0.f;
+      ab[j][k] = 0.f;
+      if (EXTRA) ac[EXTRA ? j : 0][k] = 0.f;
+    }
   }
   const float inv_d = 1.0f / D;
   const long long step = static_cast<long long>(gridDim.x) * groups * R;
-  int parity = 0;
-  for (long long row0 = (static_cast<long long>(blockIdx.x) * groups + group) * R; row0 < rows; row0 += step, parity ^= 1) {
-    Vec16 vx[R][VPT], vd[R][VPT], vr[R][VPT];
-    float mu[R], rs[R], s1[R], s2[R];
+  struct Rows {
+    Vec16 x[R][VPT], d[R][VPT], r[EXTRA ? R : 1][VPT];
+    float mu[R], rs[R];
+  };
+  auto load = [&](Rows& t, long long row0) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const long long at = (row0 + r) * D + tid * 8;
 #pragma unroll
       for (int j = 0; j < VPT; ++j) {
         const bool in = row0 + r < rows && tid + j * width < nvec;
-        const Vec16 zero{{0u, 0u, 0u, 0u}};
-        vx[r][j] = in ? ld16(x + at + j * width * 8) : zero;
-        vd[r][j] = in ? ld16(dy + at + j * width * 8) : zero;
-        vr[r][j] = in && dres ? ld16(dres + at + j * width * 8) : zero;
+        t.x[r][j] = in ? ld16(x + at + j * width * 8) : zero;
+        t.d[r][j] = in ? ld16(dy + at + j * width * 8) : zero;
+        if (EXTRA) t.r[EXTRA ? r : 0][j] = in && dres ? ld16(dres + at + j * width * 8) : zero;
       }
-      mu[r] = row0 + r < rows ? mean[row0 + r] : 0.f;
-      rs[r] = row0 + r < rows ? rstd[row0 + r] : 0.f;
+      t.mu[r] = row0 + r < rows ? mean[row0 + r] : 0.f;
+      t.rs[r] = row0 + r < rows ? rstd[row0 + r] : 0.f;
     }
+  };
+  long long row0 = (static_cast<long long>(blockIdx.x) * groups + group) * R;
+  Rows cur;
+  if (AHEAD) load(cur, row0);
+  int parity = 0;
+  for (; row0 < rows; row0 += step, parity ^= 1) {
+    if (!AHEAD) load(cur, row0);
+    float s1[R], s2[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       s1[r] = 0.f;
@@ -150,16 +163,21 @@ __global__ void __launch_bounds__(256, VPT == 1 ? 2 : 1) ln_bwd_kernel(const __n
 #pragma unroll
       for (int j = 0; j < VPT; ++j) {
         float xf[8], df[8], gf[8];
-        unpack<DT_BF16>(vx[r][j], xf);
-        unpack<DT_BF16>(vd[r][j], df);
+        unpack<DT_BF16>(cur.x[r][j], xf);
+        unpack<DT_BF16>(cur.d[r][j], df);
         unpack<DT_BF16>(g[j], gf);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const float dg = df[k] * gf[k];
           s1[r] += dg;
-          s2[r] += dg * ((xf[k] - mu[r]) * rs[r]);
+          s2[r] += dg * ((xf[k] - cur.mu[r]) * cur.rs[r]);
         }
       }
+    }
+    Rows next;
+    if (AHEAD) load(next, row0 + step);   // on its way behind the exchange, the arithmetic and the stores
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         s1[r] += __shfl_xor_sync(0xffffffffu, s1[r], o);
@@ -190,31 +208,33 @@ __global__ void __launch_bounds__(256, VPT == 1 ? 2 : 1) ln_bwd_kernel(const __n
 #pragma unroll
       for (int j = 0; j < VPT; ++j) {
         float xf[8], df[8], gf[8], rf[8], of[8];
-        unpack<DT_BF16>(vx[r][j], xf);
-        unpack<DT_BF16>(vd[r][j], df);
+        unpack<DT_BF16>(cur.x[r][j], xf);
+        unpack<DT_BF16>(cur.d[r][j], df);
         unpack<DT_BF16>(g[j], gf);
-        unpack<DT_BF16>(vr[r][j], rf);
+        if (EXTRA) unpack<DT_BF16>(cur.r[EXTRA ? r : 0][j], rf);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const float xh = (xf[k] - mu[r]) * rs[r];
-          of[k] = rs[r] * (df[k] * gf[k] - m1 - xh * m2) + rf[k];
+          const float xh = (xf[k] - cur.mu[r]) * cur.rs[r];
+          of[k] = cur.rs[r] * (df[k] * gf[k] - m1 - xh * m2);
+          if (EXTRA) of[k] += rf[k];
           ag[j][k] += df[k] * xh;
           ab[j][k] += df[k];
-          ac[j][k] += of[k];
+          if (EXTRA) ac[EXTRA ? j : 0][k] += of[k];
         }
         if (row0 + r < rows && tid + j * width < nvec) st16(dx + (row0 + r) * D + (tid + j * width) * 8, pack<DT_BF16>(of));
       }
     }
+    if (AHEAD) cur = next;
   }
-  const int arrays = part_c ? 3 : 2;
+  const int arrays = EXTRA && part_c ? 3 : 2;
 #pragma unroll
   for (int j = 0; j < VPT; ++j) {
     const int v = tid + j * width;
     if (v >= nvec) continue;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
+    for (int a = 0; a < (EXTRA ? 3 : 2); ++a) {
       if (a >= arrays) continue;
-      const float* f = a == 0 ? ag[j] : a == 1 ? ab[j] : ac[j];
+      const float* f = a == 0 ? ag[j] : a == 1 ? ab[j] : ac[EXTRA ? j : 0];
       float* dst = groups > 1 ? group_sums + (group * 3 + a) * D + v * 8
                               : (a == 0 ? part_g : a == 1 ? part_b : part_c) + static_cast<long long>(blockIdx.x) * D + v * 8;
       *reinterpret_cast<float4*>(dst) = make_float4(f[0], f[1], f[2], f[3]);
@@ -410,7 +430,13 @@ int launchLayerNormBwd(const void* dy, const void* x, const void* gamma, const f
                                              static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma), mean, rstd,
                                              static_cast<const __nv_bfloat16*>(dres), static_cast<__nv_bfloat16*>(dx), pg, pb, pc, rows, D, gw));
   };
-  const int e = D <= 2048 ? go(ln_bwd_kernel<1, 3>, 1, 3, 2) : D <= 4096 ? go(ln_bwd_kernel<2, 2>, 2, 2, 1) : go(ln_bwd_kernel<4, 1>, 4, 1, 1);
+  int e;
+  if (dres || dcolsum)
+    e = D <= 2048 ? go(ln_bwd_kernel<1, 4, true, true, 1>, 1, 4, 1) : D <= 4096 ? go(ln_bwd_kernel<2, 2, true, true, 1>, 2, 2, 1)
+                                                                                : go(ln_bwd_kernel<4, 1, true, false, 1>, 4, 1, 1);
+  else
+    e = D <= 2048 ? go(ln_bwd_kernel<1, 2, false, true, 2>, 1, 2, 2) : D <= 4096 ? go(ln_bwd_kernel<2, 2, false, true, 1>, 2, 2, 1)
+                                                                                 : go(ln_bwd_kernel<4, 1, false, true, 1>, 4, 1, 1);
   if (e != 0) return e;
   ReduceJob job{{pg, pb, pc}, {static_cast<__nv_bfloat16*>(dgamma), static_cast<__nv_bfloat16*>(dbeta), static_cast<__nv_bfloat16*>(dcolsum)}, nullptr};
   return static_cast<int>(launchOverlapped(partial_rows_reduce_kernel, dim3((D + 31) / 32, dcolsum ? 3 : 2), dim3(1024), 0, stream, 1, job, nparts, D));

@@ -340,10 +340,10 @@ def test_forward_without_gradients_is_the_same_forward():
 
 
 @pytest.mark.parametrize("D", [8, 64, 256, 264, 768, 1544, 2048, 2056, 4096, 8192])
-@pytest.mark.parametrize("rows", [1, 5, 700])
+@pytest.mark.parametrize("rows", [1, 5, 700, 5003])
 def test_layer_norm_backward_over_widths(D, rows):
-    """One to eight warps per row, one to eight rows side by side in a CTA, widths off the vector counts, fewer rows than a trip
-    takes; against fp64 on the same bf16 inputs.  dx is rounded once (2^-8 of its terms), column sums are fp32 sums of `rows`
+    """With and without the residual gradient and the column sums of dx.  One to eight warps per row, one to eight rows side by side
+    in a CTA, widths off the vector counts, fewer rows than a trip takes and several trips; against fp64 on the same bf16 inputs.  dx is rounded once (2^-8 of its terms), column sums are fp32 sums of `rows`
     terms rounded once."""
     import torch
     from pccl_b200.nn import LayerNorm
@@ -359,6 +359,10 @@ def test_layer_norm_backward_over_widths(D, rows):
     w64, b64 = ln.weight.detach().double().requires_grad_(True), torch.zeros(D, device="cuda", dtype=torch.float64, requires_grad=True)
     y64 = F.layer_norm(s64, (D,), w64, b64, ln.eps)
     dx, dw, db = torch.autograd.grad(y64, [s64, w64, b64], gy.double())
+    sr = s.detach().requires_grad_(True)
+    plain = torch.autograd.grad(ln(sr), [sr, ln.weight, ln.bias], gy)
+    for a, b in zip(plain, (dx, dw, db)):
+        assert (a.double() - b).abs().max().item() <= 2 ** -8 * b.abs().max().item() + 1e-4
     dx = dx + gs.double()
     for a, b in zip(got, (dx, dw, db, dx.sum(0))):
         assert (a.double() - b).abs().max().item() <= 2 ** -8 * b.abs().max().item() + 1e-4

@@ -47,19 +47,22 @@ __device__ __forceinline__ uint2 quant8_mx(const float* f, float inv) {
   return make_uint2(w[0], w[1]);
 }
 
-// 16 consecutive lanes own one 1 x 128 block (8 values each); rows are whole blocks, so the matrix is one list of blocks.  Four
-// loads in flight per thread.  A CTA per row took 61 us at 8192 x 8192 (its fp32-scale twin in moe.cu), this form 41: 201 MB at 4.9 TB/s.
+// 16 consecutive lanes own one 1 x 128 block (8 values each); rows are whole blocks, so the matrix is one list of blocks.  PER
+// loads in flight per thread (see quant_rows_kernel in moe.cu, its fp32-scale twin).  A CTA per row took 45 us at 8192 x 8192, this
+// form 41: 201 MB at 4.9 TB/s.
+template <int PER>
 __global__ void __launch_bounds__(256) quant_rows_mx_kernel(const __nv_bfloat16* x, uint8_t* q,
                                                             uint8_t* scales, long long nvec) {
   dev::pdl_launch();
   dev::pdl_wait();
-  for (long long v0 = static_cast<long long>(blockIdx.x) * 1024 + threadIdx.x; v0 - (threadIdx.x & 31) < nvec; v0 += static_cast<long long>(gridDim.x) * 1024) {
-    dev::Vec16 in[4];
+  constexpr int CHUNK = 256 * PER;
+  for (long long v0 = static_cast<long long>(blockIdx.x) * CHUNK + threadIdx.x; v0 - (threadIdx.x & 31) < nvec; v0 += static_cast<long long>(gridDim.x) * CHUNK) {
+    dev::Vec16 in[PER];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < PER; ++j)
       if (v0 + j * 256 < nvec) in[j] = dev::ld16(x + (v0 + j * 256) * 8);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < PER; ++j) {
       const long long v = v0 + j * 256;
       float f[8];
       float amax = 0.f;
@@ -138,9 +141,12 @@ const char* gemmMx8LastError() { return g_errx.c_str(); }
 
 int launchQuantMx8Rows(const void* x, void* q, uint8_t* scales, long long rows, int k, cudaStream_t stream) {
   if (k % 128 || rows <= 0) return static_cast<int>(cudaErrorInvalidValue);
-  const long long nvec = rows * (k >> 3), blocks = (nvec + 1023) / 1024, most = deviceSmCount() * 8ll;
-  return static_cast<int>(launchOverlapped(quant_rows_mx_kernel, dim3(static_cast<unsigned>(blocks < most ? blocks : most)), dim3(256), 0, stream, 1,
-                                           static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scales, nvec));
+  const long long nvec = rows * (k >> 3), most = deviceSmCount() * 8ll;       // 256-thread CTAs resident at once
+  auto go = [&](auto kern, long long blocks) {
+    return static_cast<int>(launchOverlapped(kern, dim3(static_cast<unsigned>(blocks < most ? blocks : most)), dim3(256), 0, stream, 1,
+                                             static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scales, nvec));
+  };
+  return nvec <= most * 256 ? go(quant_rows_mx_kernel<1>, (nvec + 255) / 256) : go(quant_rows_mx_kernel<4>, (nvec + 1023) / 1024);
 }
 
 int launchQuantMx8Blocks(const void* w, void* q, uint8_t* scales, int rows, int cols, cudaStream_t stream) {

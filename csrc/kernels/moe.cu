@@ -414,19 +414,22 @@ __global__ void __launch_bounds__(256) moe_reduce_groups_kernel(const __nv_bfloa
   }
 }
 
-// Rows are whole 128-value blocks, so the matrix is one list of blocks, 16 lanes to each; four loads in flight per thread.
-// 8192 x 8192: 61 -> 41 us (a CTA per row, staged in shared memory, before).
+// Rows are whole 128-value blocks, so the matrix is one list of blocks, 16 lanes to each; PER loads in flight per thread: four,
+// or one where that already puts the whole matrix in flight.  8192 x 8192: 61 -> 41 us (a CTA per row, staged in shared memory,
+// before).
+template <int PER>
 __global__ void __launch_bounds__(256) quant_rows_kernel(const __nv_bfloat16* x, uint8_t* q,
                                                          float* scales, long long nvec) {
   dev::pdl_launch();
   dev::pdl_wait();
-  for (long long v0 = static_cast<long long>(blockIdx.x) * 1024 + threadIdx.x; v0 - (threadIdx.x & 31) < nvec; v0 += static_cast<long long>(gridDim.x) * 1024) {
-    Vec16 in[4];
+  constexpr int CHUNK = 256 * PER;
+  for (long long v0 = static_cast<long long>(blockIdx.x) * CHUNK + threadIdx.x; v0 - (threadIdx.x & 31) < nvec; v0 += static_cast<long long>(gridDim.x) * CHUNK) {
+    Vec16 in[PER];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < PER; ++j)
       if (v0 + j * 256 < nvec) in[j] = ld16(x + (v0 + j * 256) * 8);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < PER; ++j) {
       const long long v = v0 + j * 256;
       float f[8];
       float amax = 0.f;
@@ -951,9 +954,12 @@ int launchMoeReduceGroups(const void* y, void* z, const int* alias, const void* 
 
 int launchQuantFp8Rows(const void* x, void* q, float* scales, long long rows, int hidden, cudaStream_t stream) {
   if (hidden % 128 || rows <= 0) return static_cast<int>(cudaErrorInvalidValue);
-  const long long nvec = rows * (hidden >> 3), blocks = (nvec + 1023) / 1024, most = deviceSmCount() * 8ll;
-  return static_cast<int>(launchOverlapped(quant_rows_kernel, dim3(static_cast<unsigned>(blocks < most ? blocks : most)), dim3(256), 0, stream, 1,
-                                           static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scales, nvec));
+  const long long nvec = rows * (hidden >> 3), most = deviceSmCount() * 8ll;       // 256-thread CTAs resident at once
+  auto go = [&](auto kern, long long blocks) {
+    return static_cast<int>(launchOverlapped(kern, dim3(static_cast<unsigned>(blocks < most ? blocks : most)), dim3(256), 0, stream, 1,
+                                             static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scales, nvec));
+  };
+  return nvec <= most * 256 ? go(quant_rows_kernel<1>, (nvec + 255) / 256) : go(quant_rows_kernel<4>, (nvec + 1023) / 1024);
 }
 
 int launchQuantFp8Blocks(const void* w, void* q, float* scales, int rows, int cols, cudaStream_t stream) {

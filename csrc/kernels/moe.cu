@@ -808,8 +808,9 @@ __device__ __forceinline__ void route_token(const float* logits, int* ids, float
   float sum = 0.f;
 #pragma unroll
   for (int j = 0; j < PER_LANE; ++j) {
-    v[j] = __expf(v[j] - mx);
-    sum += v[j];
+    const float p = __expf(v[j] - mx);
+    sum += p;
+    v[j] = j * 32 + lane < experts ? p : -2.f;       // the padding is never taken, also where all logits left are NaN
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -819,7 +820,7 @@ __device__ __forceinline__ void route_token(const float* logits, int* ids, float
     int bi = 0;
 #pragma unroll
     for (int j = 0; j < PER_LANE; ++j)
-      if (j * 32 + lane < experts && v[j] > best) { best = v[j]; bi = j * 32 + lane; }      // without it, NaN logits lose to the padding
+      if (v[j] > best) { best = v[j]; bi = j * 32 + lane; }
     // warp arg-max; ties go to the lower expert id (what a stable top-k returns)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -838,20 +839,25 @@ __device__ __forceinline__ void route_token(const float* logits, int* ids, float
   }
 }
 
-// One warp per token.  An assignment's place among those of its expert comes from counters: a block of 32 tokens counts in
-// shared memory and draws its share of each expert's rows with one global atomic; an atomic per assignment (32768 of them on
-// 32 words at 4096 tokens, top-8) took three quarters of the kernel's time: 22 -> 7 us.
-template <int PER_LANE>
-__global__ void __launch_bounds__(1024) moe_route_kernel(const float* logits, int* ids, float* probs,
-                                                         int* pos, int* counts, int tokens, int experts, int topk) {
-  extern __shared__ int cnt[];             // [experts] assignments of this block, then the first place of the block
+// One warp per token.  An assignment's place among those of its expert comes from counters.  SHARED: a block of up to 32 tokens
+// counts in shared memory and draws its share of each expert's rows with one global atomic; with an atomic per assignment
+// 4096 tokens, top-8, over 8 / 32 / 64 / 128 / 256 experts take 28 / 27 / 27 / 18 / 19 us instead of 12 / 11 / 12 / 13 / 15, because
+// they queue up behind one another.  Where few assignments meet (64 tokens over 256 experts) or a block would walk hundreds of
+// counters for its handful of assignments, the atomic per assignment is the faster: 10 against 12 us there, 18 against 19 at
+// 4096 x 512, 12 against 20 at 64 x 1024.
+template <int PER_LANE, bool SHARED>
+__global__ void __launch_bounds__(SHARED ? 1024 : 256) moe_route_kernel(const float* logits, int* ids, float* probs, int* pos, int* counts, int tokens,
+                                                                        int experts, int topk) {
+  extern __shared__ int cnt[];             // SHARED: [experts] assignments of this block, then the first place of the block
   const int lane = threadIdx.x & 31;
   const int t0 = blockIdx.x * (blockDim.x >> 5), t = t0 + (threadIdx.x >> 5);
-  for (int e = threadIdx.x; e < experts; e += blockDim.x) cnt[e] = 0;
+  if (SHARED)
+    for (int e = threadIdx.x; e < experts; e += blockDim.x) cnt[e] = 0;
   dev::pdl_launch();
   dev::pdl_wait();
-  __syncthreads();
-  if (t < tokens) route_token<PER_LANE>(logits, ids, probs, pos, cnt, t, experts, topk, lane);
+  if (SHARED) __syncthreads();
+  if (t < tokens) route_token<PER_LANE>(logits, ids, probs, pos, SHARED ? cnt : counts, t, experts, topk, lane);
+  if (!SHARED) return;
   __syncthreads();
   for (int e = threadIdx.x; e < experts; e += blockDim.x)
     if (cnt[e]) cnt[e] = atomicAdd(counts + e, cnt[e]);
@@ -972,17 +978,19 @@ int launchQuantFp8Blocks(const void* w, void* q, float* scales, int rows, int co
 int launchMoeRoute(const float* logits, int* ids, float* probs, int* pos, int* counts, int tokens, int experts, int topk,
                    cudaStream_t stream) {
   if (experts < 1 || experts > 1024 || topk > experts || tokens <= 0) return static_cast<int>(cudaErrorInvalidValue);
-  const int grid = (tokens + 31) / 32;
   const int per = (experts + 31) / 32;
+  const bool shared = experts <= 256 && tokens * static_cast<long long>(topk) > 8ll * experts;
   auto go = [&](auto kern) {
-    return static_cast<int>(launchOverlapped(kern, dim3(grid), dim3(1024), experts * sizeof(int), stream, 1, logits, ids, probs, pos, counts, tokens,
-                                             experts, topk));
+    int warps = shared ? 32 : 8;
+    // few tokens: smaller blocks on more SMs (the 32 warps of a block share the issue slots of one SM)
+    while (warps > 2 && (tokens + warps - 1) / warps < deviceSmCount()) warps /= 2;
+    return static_cast<int>(launchOverlapped(kern, dim3((tokens + warps - 1) / warps), dim3(32 * warps), shared ? experts * sizeof(int) : 0, stream, 1,
+                                             logits, ids, probs, pos, counts, tokens, experts, topk));
   };
-  if (per <= 1) return go(moe_route_kernel<1>);
-  if (per <= 4) return go(moe_route_kernel<4>);
-  if (per <= 8) return go(moe_route_kernel<8>);
-  if (per <= 16) return go(moe_route_kernel<16>);
-  return go(moe_route_kernel<32>);
+  if (per <= 1) return shared ? go(moe_route_kernel<1, true>) : go(moe_route_kernel<1, false>);
+  if (per <= 4) return shared ? go(moe_route_kernel<4, true>) : go(moe_route_kernel<4, false>);
+  if (per <= 8) return shared ? go(moe_route_kernel<8, true>) : go(moe_route_kernel<8, false>);
+  return per <= 16 ? go(moe_route_kernel<16, false>) : go(moe_route_kernel<32, false>);
 }
 
 int launchMoePlan(const int* counts_all, const int* ids, const int* pos, int* rows, int* row_off, int world, int rank, int experts,

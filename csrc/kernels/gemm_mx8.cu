@@ -118,26 +118,31 @@ __global__ void __launch_bounds__(256) quant_blocks_mx_kernel(const __nv_bfloat1
 
 thread_local std::string g_errx;
 
+}  // namespace
+
+const char* gemmMx8LastError() { return g_errx.c_str(); }
+
 // Columns per tile: 224 unless narrower tiles fill the last round of CTAs better.  Measured time of a full round relative to
 // 224 columns (148 tiles of 128 rows each, K = 2048 and 8192, one B200, mean of the two): a round is bound by the operands
 // that an SM gets from L2, of which A's 128 rows stay.  1531 x 3584 x 8192: 192 tiles of 224 in two rounds, 276 of 160 in two.
 // Against 224 columns (us): 300 x 4096 x 1024 15.3 -> 13.3, 777 x 2048 x 2048 19.5 -> 17.4, 1000 x 1152 x 4096 25.6 -> 21.4,
 // 1531 x 3584 x 8192 60 -> 54 to 58; within 2 % at four larger shapes, which keep 224.
-int pickWidthMx(int tiles_m, int n, int sms) {
+// Up to 32 rows all CTAs ask for the same few lines of A at the same time, and more of them queue longer: 1 x 8192 x 3584 takes 20.3
+// with 224 columns, 20.5 with 160 and 24.4 with 64, 16 x 4096 x 7168 26.9, 24.6 and 28.7; from 40 rows on 64 columns are the best
+// (40 x 8192 x 3584 20.2, 18.5, 18.1; 40 x 4096 x 7168 26.6, 24.6, 22.8).
+int gemmMx8TileN(int rows, int n, int sms) {
+  const int tiles_m = (rows + gemmx::BM - 1) / gemmx::BM, least = rows <= 32 ? 160 : 32;
   static const struct { int bn; float round; } kWidths[] = {{224, 1.f}, {192, .89f}, {160, .83f}, {128, .78f}, {96, .75f}, {64, .70f}, {32, .68f}};
   int best = gemmx::BN;
   float best_cost = 0.f;
   for (const auto& w : kWidths) {
+    if (w.bn < least) break;
     const long long tiles = static_cast<long long>(tiles_m) * ((n + w.bn - 1) / w.bn);
     const float cost = static_cast<float>((tiles + sms - 1) / sms) * w.round;
     if (w.bn == gemmx::BN || cost < best_cost * 0.999f) { best = w.bn; best_cost = cost; }
   }
   return best;
 }
-
-}  // namespace
-
-const char* gemmMx8LastError() { return g_errx.c_str(); }
 
 int launchQuantMx8Rows(const void* x, void* q, uint8_t* scales, long long rows, int k, cudaStream_t stream) {
   if (k % 128 || rows <= 0) return static_cast<int>(cudaErrorInvalidValue);
@@ -181,7 +186,7 @@ int gemmMx8(const void* A, int64_t lda, const uint8_t* sa, int ld_sa, const void
   if (!makeTensorMap2D(&ta, A, TM_U8, K, M, lda, gemmx::BK, gemmx::BM, &g_errx)) return static_cast<int>(cudaErrorInvalidValue);
   int n_sm = deviceSmCount();
   if (sms > 0 && sms < n_sm) n_sm = sms;
-  const int bn = pickWidthMx((M + gemmx::BM - 1) / gemmx::BM, N, n_sm);
+  const int bn = gemmMx8TileN(M, N, n_sm);
   if (!makeTensorMap2D(&tb, B, TM_U8, K, N, ldb, gemmx::BK, bn, &g_errx)) return static_cast<int>(cudaErrorInvalidValue);
   gemm::StoreEpi epi{D, D2, static_cast<const __nv_bfloat16*>(bias), ldd, M, N, flags, bn};
   gemmx::Scales sc{sa, sb, ld_sa, ld_sb, M, N};

@@ -346,12 +346,15 @@ def test_colsum_kernel_matches_torch(rows, N):
         assert (colsum(view).float() - view.float().sum(0)).abs().max().item() <= 1e-2 * max(1.0, view.float().sum(0).abs().max().item())
 
 
-@pytest.mark.parametrize("M,N", [(1, 40), (130, 1000), (300, 4104), (1531, 3584), (2000, 520), (19000, 232), (9000, 448)])
-def test_mx8_tile_widths(M, N):
+@pytest.mark.parametrize("M,N,width", [(1, 40, 160), (33, 40, 32), (130, 1000, 32), (300, 4104, 96), (1531, 3584, 160), (2000, 520, 64), (700, 4104, 192),
+                                       (1531, 2400, 224), (19000, 232, 128), (9000, 448, 224)])
+def test_mx8_tile_widths(M, N, width):
     """Sizes over which the launch picks tiles of 32 ... 224 columns, with ragged last tiles and scale blocks that a tile straddles.
     fp32 output against the product of the dequantised operands: the sums differ in their order only."""
+    from pccl_b200._native import C
     from pccl_b200.ops import check_status
     from pccl_b200.ops.gemm import dequant_rows, gemm_mx8, quant_rows_mx, ue8m0_to_float
+    assert C.gemm_mx8_tile_n(M, N, 148) == width
     K = 384
     a, w = _rand((M, K), 81), _rand((N, K), 82)
     aq, a_s = quant_rows_mx(a)

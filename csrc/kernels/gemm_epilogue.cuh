@@ -257,6 +257,10 @@ struct StoreEpi {
         if (full || col + i < N) v[i] += __bfloat162float(bias[col + i]);
     }
     if (flags & GEMM_OUT_F32) {
+      if (flags & GEMM_GELU_INPLACE) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
+      }
       float* d = static_cast<float*>(D) + static_cast<long long>(row) * ldd + col;
       if (full) {
         if (flags & GEMM_ACCUMULATE) {
@@ -276,7 +280,8 @@ struct StoreEpi {
       return;
     }
     __nv_bfloat16* d = static_cast<__nv_bfloat16*>(D) + static_cast<long long>(row) * ldd + col;
-    if (full) {
+    // a second output may start off the 16-byte boundaries that D and the row stride keep
+    if (full && (!(flags & (GEMM_ADD_D2 | GEMM_GELU)) || (reinterpret_cast<uintptr_t>(D2) & 15) == 0)) {
       if (flags & GEMM_ADD_D2) {        // D = A*B^T (+bias) + D2: the residual connection around a linear layer
         const __nv_bfloat16* res = static_cast<const __nv_bfloat16*>(D2) + static_cast<long long>(row) * ldd + col;
 #pragma unroll
@@ -315,6 +320,7 @@ struct StoreEpi {
       for (int i = 0; i < 32; ++i) {
         if (col + i >= N) continue;
         if (flags & GEMM_ADD_D2) v[i] += __bfloat162float((static_cast<const __nv_bfloat16*>(D2) + static_cast<long long>(row) * ldd + col)[i]);
+        if (flags & GEMM_GELU_INPLACE) v[i] = gelu_tanh(v[i]);
         float x = (flags & GEMM_ACCUMULATE) ? v[i] + __bfloat162float(d[i]) : v[i];
         d[i] = __float2bfloat16_rn(x);
         if (flags & GEMM_GELU)

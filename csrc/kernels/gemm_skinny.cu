@@ -73,6 +73,10 @@ __device__ __forceinline__ void skinny_store(const SkinnyArgs& A, int row, int c
       if (full || col + i < A.N) v[i] += __bfloat162float(A.bias[col + i]);
   }
   if (A.flags & GEMM_OUT_F32) {
+    if (A.flags & GEMM_GELU_INPLACE) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = gemm::gelu_tanh(v[i]);
+    }
     float* d = static_cast<float*>(A.D) + at;
     if (full) {
       if (A.flags & GEMM_ACCUMULATE) {

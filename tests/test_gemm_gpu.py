@@ -368,6 +368,44 @@ def test_mx8_tile_widths(M, N, width):
     assert (out.double() - ref).abs().max().item() <= 2e-3 * max(1.0, ref.abs().max().item())      # a wrong scale or tile is off by O(1)
 
 
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N", [(40, 72), (300, 1000)])
+def test_fp8_gelu_in_every_column(M, N, out_dtype):
+    """GELU on the output reaches the columns past the last whole strip of 32 and fp32 outputs as well; against the same product
+    without it (hardware tanh: 2^-11 of the value, 1e-3 on the flat side), and one bf16 rounding."""
+    from pccl_b200.ops import check_status
+    from pccl_b200.ops.gemm import gemm_fp8, gemm_mx8, quant_blocks, quant_blocks_mx, quant_rows, quant_rows_mx
+    K = 256
+    a, w = _rand((M, K), 91), _rand(((N + 127) // 128 * 128, K), 92, 0.1)
+    for g, qr, qb in ((gemm_fp8, quant_rows, quant_blocks), (gemm_mx8, quant_rows_mx, quant_blocks_mx)):
+        aq, a_s = qr(a)
+        wq, w_s = qb(w)
+        plain = g(aq, a_s, wq[:N], w_s, out_dtype=torch.float32)
+        act = g(aq, a_s, wq[:N], w_s, out_dtype=out_dtype, gelu_inplace=True)
+        check_status("fp8 gelu")
+        want = torch.nn.functional.gelu(plain.double(), approximate="tanh")
+        assert ((act.double() - want).abs() <= (2 ** -8 if out_dtype is torch.bfloat16 else 2 ** -10) * want.abs() + 1.5e-3 * plain.abs()).all()
+
+
+@pytest.mark.parametrize("M,pair", [(40, None), (200, False), (200, True)])
+def test_gemm_second_output_off_the_16_byte_boundaries(M, pair):
+    """A second output that starts anywhere (its rows are strided like out's) gets what an aligned one gets."""
+    from pccl_b200.ops import check_status, gemm
+    N, K, ld = 96, 64, 104
+    a, w = _rand((M, K), 93), _rand((N, K), 94, 0.2)
+    def strided(shift):
+        return torch.zeros((M, ld), dtype=torch.bfloat16, device="cuda").view(-1)[shift:shift + M * ld - 8].as_strided((M, N), (ld, 1))
+    got = []
+    for shift in (0, 1, 4):
+        act, pre = strided(shift), strided(0)
+        gemm(a, w, gelu_out=act, out=pre, pair=pair)
+        got.append([pre.clone(), act.clone()])
+    check_status("second output")
+    assert all(torch.equal(x, y) for g in got[1:] for x, y in zip(g, got[0]))
+    ref = a.double() @ w.double().t()
+    assert ((got[0][0].double() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-4).all()
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 8, 128), (127, 136, 256), (129, 264, 640), (260, 1000, 1152), (3000, 128, 384)])
 def test_fp8_gemm_at_the_edges_of_its_tiles(M, N, K):
     """Ragged rows and columns around 128, one to nine K blocks (four accumulators are taken in turn), scales that differ per block;

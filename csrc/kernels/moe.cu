@@ -983,7 +983,7 @@ int launchMoeRoute(const float* logits, int* ids, float* probs, int* pos, int* c
   auto go = [&](auto kern) {
     int warps = shared ? 32 : 8;
     // few tokens: smaller blocks on more SMs (the 32 warps of a block share the issue slots of one SM)
-    while (warps > 2 && (tokens + warps - 1) / warps < deviceSmCount()) warps /= 2;
+    while (shared && warps > 2 && (tokens + warps - 1) / warps < deviceSmCount()) warps /= 2;
     return static_cast<int>(launchOverlapped(kern, dim3((tokens + warps - 1) / warps), dim3(32 * warps), shared ? experts * sizeof(int) : 0, stream, 1,
                                              logits, ids, probs, pos, counts, tokens, experts, topk));
   };

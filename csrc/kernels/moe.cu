@@ -844,7 +844,7 @@ __device__ __forceinline__ void route_token(const float* logits, int* ids, float
 // 4096 tokens, top-8, over 8 / 32 / 64 / 128 / 256 experts take 28 / 27 / 27 / 18 / 19 us instead of 12 / 11 / 12 / 13 / 15, because
 // they queue up behind one another.  Where few assignments meet (64 tokens over 256 experts) or a block would walk hundreds of
 // counters for its handful of assignments, the atomic per assignment is the faster: 10 against 12 us there, 18 against 19 at
-// 4096 x 512, 13 against 20 at 64 x 1024.
+// 4096 x 512, 12 against 20 at 64 x 1024.
 template <int PER_LANE, bool SHARED>
 __global__ void __launch_bounds__(SHARED ? 1024 : 256) moe_route_kernel(const float* logits, int* ids, float* probs, int* pos, int* counts, int tokens,
                                                                         int experts, int topk) {

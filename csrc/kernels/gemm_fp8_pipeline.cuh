@@ -14,8 +14,8 @@
 //                bf16 pipeline's
 //
 // so the same epilogue adapters (plain store, reduce-scatter) serve both precisions.
-// What bounds it: the chain of a K block (see run below), not the tensor cores (28 % busy at 4096 x 4096 x 3584 with 128-column
-// tiles), not TMEM reads and not L2.  Its gain over bf16 is the halved operand traffic and storage.
+// What bounds it with 128-column tiles: the operands from L2 (see run below), not the tensor cores and not TMEM reads.  Its gain over
+// bf16 is the halved operand traffic and storage.
 // All waits are bounded; on a time-out the CTA flags the error, drains its copies, frees TMEM
 // and returns.  No TMA load uses cluster multicast.
 //
@@ -213,19 +213,9 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
       const int gblk = min((epi.b_row0(t) + half * CW) >> 7, sb_rows - 1);
       const float* pa = sc.sa + static_cast<long long>(grow) * sc.ld_sa;
       const float* pb = sc.sb + static_cast<long long>(gblk) * sc.ld_sb;
-      // raw scales travel two K blocks ahead of their use, so that no load latency is exposed
-      // (A's scales may have been written by a peer during this launch: read them past L1)
-      float a0 = dev::ld_cg_f32(pa), b0 = dev::ld_f32(pb);
-      float a1 = num_kb > 1 ? dev::ld_cg_f32(pa + 1) : 0.f, b1 = num_kb > 1 ? dev::ld_f32(pb + 1) : 0.f;
-      for (int kb = 0; kb < num_kb; ++kb) {
-        const float s = a0 * b0;
-        a0 = a1;
-        b0 = b1;
-        if (kb + 2 < num_kb) {
-          a1 = dev::ld_cg_f32(pa + kb + 2);
-          b1 = dev::ld_f32(pb + kb + 2);
-        }
-        if (!tc::mbar_wait(&bar->tmem_full[acc], acc_phase, abort)) { ok = false; break; }
+      // one K block: wait for its partial products, fold them in times s
+      auto fold = [&](float s) {
+        if (!tc::mbar_wait(&bar->tmem_full[acc], acc_phase, abort)) return false;
         tc::tc_fence_after();
         const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BNT + half * CW;
 #pragma unroll
@@ -243,6 +233,45 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&bar->tmem_empty[acc]);
         if (++acc == ACC) { acc = 0; acc_phase ^= 1; }
+        return true;
+      };
+      int kb = 0;
+      if constexpr (BNT == NARROW_BN) {
+        // Four K blocks' row scales in one load.  A load per block touches 32 cache lines per warp, 256 look-ups per K block and CTA: that,
+        // not the chain of the K block, was what the kernel waited for (L1 71 % busy).  8192 x 3584 x 8192 321 -> 264 us, 8192 x 8192 x 3584
+        // 302 -> 271, 16384 x 8192 x 8192 1371 -> 1110 (1.95 PFLOP/s), 1531 x 3584 x 8192 87 -> 68; a round of tiles now takes 540 clocks per K
+        // block, which is the 32 KiB of operands at the 63 bytes per clock that an SM gets from L2.
+        if ((sc.ld_sa & 3) == 0 && (reinterpret_cast<uintptr_t>(sc.sa) & 15) == 0 && num_kb >= 4) {
+          dev::Vec16 a = dev::ld16_cg(pa);
+          float b0 = dev::ld_f32(pb);
+          for (; ok && kb + 4 <= num_kb; kb += 4) {
+            dev::Vec16 an = a;
+            if (kb + 8 <= num_kb) an = dev::ld16_cg(pa + kb + 4);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float s = __uint_as_float(a.w[j]) * b0;
+              if (kb + j + 1 < num_kb) b0 = dev::ld_f32(pb + kb + j + 1);
+              if (!fold(s)) { ok = false; break; }
+            }
+            a = an;
+          }
+        }
+      }
+      // raw scales travel two K blocks ahead of their use, so that no load latency is exposed
+      // (A's scales may have been written by a peer during this launch: read them past L1)
+      if (ok && kb < num_kb) {
+        float a0 = dev::ld_cg_f32(pa + kb), b0 = dev::ld_f32(pb + kb);
+        float a1 = kb + 1 < num_kb ? dev::ld_cg_f32(pa + kb + 1) : 0.f, b1 = kb + 1 < num_kb ? dev::ld_f32(pb + kb + 1) : 0.f;
+        for (; kb < num_kb; ++kb) {
+          const float s = a0 * b0;
+          a0 = a1;
+          b0 = b1;
+          if (kb + 2 < num_kb) {
+            a1 = dev::ld_cg_f32(pa + kb + 2);
+            b1 = dev::ld_f32(pb + kb + 2);
+          }
+          if (!fold(s)) { ok = false; break; }
+        }
       }
       if (!ok) break;
       epi.tile_begin(t);

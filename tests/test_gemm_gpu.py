@@ -421,3 +421,25 @@ def test_fp8_gemm_at_the_edges_of_its_tiles(M, N, K):
     wf = wq.view(torch.float8_e4m3fn).double() * w_s.double().repeat_interleave(128, 1).repeat_interleave(128, 0)[:N]
     ref = dequant_rows(aq, a_s).double() @ wf.t()
     assert (out.double() - ref).abs().max().item() <= 2e-3 * max(1.0, ref.abs().max().item())
+
+
+@pytest.mark.parametrize("K", [512, 640, 1152])
+@pytest.mark.parametrize("shift,stride", [(0, 4), (0, 12), (1, 12), (0, 9)])
+def test_fp8_gemm_row_scales_of_any_stride(K, shift, stride):
+    """Row scales are read four K blocks at a time where their rows allow it: rows of any stride and start give the same bits, with
+    whole and partial groups of four."""
+    from pccl_b200.ops import check_status
+    from pccl_b200.ops.gemm import gemm_fp8, quant_blocks, quant_rows
+    if stride < K // 128 + shift:
+        pytest.skip("rows shorter than their scales")
+    a = (_rand((200, K), 95).float() * torch.logspace(-1, 1, K // 128, device="cuda").repeat_interleave(128)).bfloat16()
+    aq, a_s = quant_rows(a)
+    wq, w_s = quant_blocks(_rand((256, K), 96))
+    ref = (aq.view(torch.float8_e4m3fn).double() * a_s.double().repeat_interleave(128, 1)) @ (
+        wq.view(torch.float8_e4m3fn).double() * w_s.double().repeat_interleave(128, 0).repeat_interleave(128, 1)).t()
+    rows = torch.full((200, stride), float("nan"), device="cuda")
+    rows[:, shift:shift + K // 128] = a_s
+    out = gemm_fp8(aq, rows[:, shift:shift + K // 128], wq, w_s, out_dtype=torch.float32)
+    check_status("gemm_fp8")
+    assert torch.equal(out, gemm_fp8(aq, a_s, wq, w_s, out_dtype=torch.float32))
+    assert (out.double() - ref).abs().max().item() <= 2e-3 * max(1.0, ref.abs().max().item())

@@ -46,6 +46,7 @@ struct Barriers {
   uint64_t inbox_full[SCHED_SLOTS];    // used in the peer: the leader has stored the index into `inbox`
   int32_t sched_tile[SCHED_SLOTS];     // per CTA: tile index, or -1 for "no more tiles"; written by this CTA's producer
   int32_t inbox[SCHED_SLOTS];          // used in the peer: written by the leader's producer, read by the peer's producer
+  uint32_t drained[2];          // per CTA: epilogue warps that are done with the accumulator
   uint32_t tmem_base;
   uint32_t abort;
 };
@@ -115,7 +116,8 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
     }
     for (int a = 0; a < 2; ++a) {
       tc::mbar_init(&bar->tmem_full[a], 1);
-      tc::mbar_init(&bar->tmem_empty[a], 2 * EPI_WARPS);      // the epilogue warps of both CTAs of the pair
+      tc::mbar_init(&bar->tmem_empty[a], 2);                  // the last epilogue warp of either CTA
+      bar->drained[a] = 0;
     }
     tc::mbar_init(&bar->drain, 1);
     for (int q = 0; q < SCHED_SLOTS; ++q) {
@@ -337,7 +339,9 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
       }
       tc::tc_fence_before();
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive_cluster(tc::mapa(tc::smem_u32(&bar->tmem_empty[acc]), 0));   // on the leader's barrier
+      // the CTA's last warp signals the leader: arrivals from another CTA's side are taken one after the other, some 45 clocks each
+      if (lane == 0 && tc::atom_inc_shared(&bar->drained[acc], EPI_WARPS - 1) == EPI_WARPS - 1)
+        tc::mbar_arrive_remote(tc::mapa(tc::smem_u32(&bar->tmem_empty[acc]), 0));
       epi.tile_done(t, abort);
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }

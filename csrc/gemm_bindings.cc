@@ -38,6 +38,7 @@ void bindGemm(py::module_& m) {
   m.def("gemm_skinny_splits", &gemmSkinnySplits);
   m.def("gemm_pair_tile_n", &gemmPairTileN);
   m.def("gemm_mx8_tile_n", &gemmMx8TileN);
+  m.def("gemm_mx8_pair_tile_n", &gemmMx8PairTileN);
   m.def("gemm_reset_tile_counters", &gemmResetTileCounters);
   m.def("gemm_bf16_dual",
         [](uint64_t a0, int64_t lda0, uint64_t b0, int64_t ldb0, uint64_t d0, int64_t ldd0, int M0, int N0, bool acc0, uint64_t a1, int64_t lda1,

@@ -91,7 +91,8 @@ int gemmMx8(const void* A, int64_t lda, const uint8_t* sa, int ld_sa, const void
 int launchQuantMx8Rows(const void* x, void* q, uint8_t* scales, long long rows, int k, cudaStream_t stream);
 int launchQuantMx8Blocks(const void* w, void* q, uint8_t* scales, int rows, int cols, cudaStream_t stream);
 const char* gemmMx8LastError();
-int gemmMx8TileN(int rows, int n, int sms);      // tile width (columns) of a hardware-scaled fp8 launch
+int gemmMx8TileN(int rows, int n, int sms);      // tile width (columns) of a hardware-scaled fp8 launch on single CTAs
+int gemmMx8PairTileN(int rows, int n, int sms);  // ... on CTA pairs, 0 where single CTAs run it
 
 const char* gemmLastError();
 // Tile width (columns) of a CTA-pair launch over up to two problems of `tiles` 256-row tiles and n columns each.

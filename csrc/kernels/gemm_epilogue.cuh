@@ -67,9 +67,9 @@ __device__ __forceinline__ void warp_transpose_sum32(float* v, int lane) {
 // bytes; an epilogue with two outputs (pre-activation and GELU) or a side input is bound by exactly that.
 constexpr int kPatchRowBytes = 80;
 constexpr int kPatchBytes = 32 * kPatchRowBytes;          // per epilogue warp
-constexpr int kPatchBytesPerCta = 8 * kPatchBytes;       // up to eight epilogue warps
-// the calling epilogue warp's patch: warps 2, 3, ... of the CTA are the epilogue warps
-__device__ __forceinline__ uint8_t* my_patch(uint8_t* base) { return base + (((threadIdx.x >> 5) - 2) & 7) * kPatchBytes; }
+constexpr int kPatchBytesPerCta = 8 * kPatchBytes;       // eight epilogue warps (gemm_fp8_pair.cuh has sixteen)
+// the calling epilogue warp's patch: `base` is that of warp 2 (warps 2, 3, ... of the CTA are the epilogue warps as a rule)
+__device__ __forceinline__ uint8_t* my_patch(uint8_t* base) { return base + ((threadIdx.x >> 5) - 2) * kPatchBytes; }
 
 // the lane's 32 values -> bf16 -> rows [0, rows_valid) of the 32 x 32 strip at g0 (row stride ldd elements)
 __device__ __forceinline__ void patch_store_bf16(uint8_t* P, int lane, __nv_bfloat16* g0, long long ldd, const float* v, int rows_valid) {

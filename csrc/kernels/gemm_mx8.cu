@@ -8,6 +8,7 @@
 
 #include "gemm_api.h"
 #include "gemm_epilogue.cuh"
+#include "gemm_mx8_pair.cuh"
 #include "gemm_mx8_pipeline.cuh"
 #include "tensormap.h"
 
@@ -22,6 +23,15 @@ gemm_mx8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                            static_cast<int>(gridDim.x)};
   gemm::NoGate gate;
   gemmx::run(&tmA, &tmB, K, sc, sched, gate, epi, status, epi.bn);
+}
+
+__global__ void __launch_bounds__(gemmxp::NUM_THREADS, 1)
+gemm_mx8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, gemm::StoreEpi epi,
+                     gemmx::Scales sc, int K, uint32_t* status) {
+  gemm::GroupedSched sched{(epi.M + gemmxp::PAIR_M - 1) / gemmxp::PAIR_M, (epi.N + epi.bn - 1) / epi.bn, static_cast<int>(blockIdx.x >> 1),
+                           static_cast<int>(gridDim.x >> 1)};
+  gemm2::PairEpi<gemm::StoreEpi> pe{epi, static_cast<int>(tc::cluster_ctarank())};
+  gemmxp::run(&tmA, &tmB, K, sc, sched, pe, status);
 }
 
 // Smallest power of two >= amax / 448 (so that the scaled block fits e4m3), as a float and as its UE8M0 byte.
@@ -130,18 +140,41 @@ const char* gemmMx8LastError() { return g_errx.c_str(); }
 // Up to 32 rows all CTAs ask for the same few lines of A at the same time, and more of them queue longer: 1 x 8192 x 3584 takes 20.3
 // with 224 columns, 20.5 with 160 and 24.4 with 64, 16 x 4096 x 7168 26.9, 24.6 and 28.7; from 40 rows on 64 columns are the best
 // (40 x 8192 x 3584 20.2, 18.5, 18.1; 40 x 4096 x 7168 26.6, 24.6, 22.8).
-int gemmMx8TileN(int rows, int n, int sms) {
-  const int tiles_m = (rows + gemmx::BM - 1) / gemmx::BM, least = rows <= 32 ? 160 : 32;
-  static const struct { int bn; float round; } kWidths[] = {{224, 1.f}, {192, .89f}, {160, .83f}, {128, .78f}, {96, .75f}, {64, .70f}, {32, .68f}};
-  int best = gemmx::BN;
-  float best_cost = 0.f;
-  for (const auto& w : kWidths) {
-    if (w.bn < least) break;
-    const long long tiles = static_cast<long long>(tiles_m) * ((n + w.bn - 1) / w.bn);
-    const float cost = static_cast<float>((tiles + sms - 1) / sms) * w.round;
-    if (w.bn == gemmx::BN || cost < best_cost * 0.999f) { best = w.bn; best_cost = cost; }
+struct RoundCost { int bn; float round; };
+static int cheapestWidth(const RoundCost* widths, int count, int tiles_m, int n, int slots, int least, float* cost, long long* rounds) {
+  int best = 0;
+  for (int i = 0; i < count && widths[i].bn >= least; ++i) {
+    const long long r = (static_cast<long long>(tiles_m) * ((n + widths[i].bn - 1) / widths[i].bn) + slots - 1) / slots;
+    const float c = static_cast<float>(r) * widths[i].round;
+    if (i == 0 || c < *cost * 0.999f) { best = widths[i].bn; *cost = c; *rounds = r; }
   }
   return best;
+}
+static int singleWidth(int rows, int n, int sms, float* cost, long long* rounds) {
+  static const RoundCost kWidths[] = {{224, 1.f}, {192, .89f}, {160, .83f}, {128, .78f}, {96, .75f}, {64, .70f}, {32, .68f}};
+  return cheapestWidth(kWidths, 7, (rows + gemmx::BM - 1) / gemmx::BM, n, sms, rows <= 32 ? 160 : 32, cost, rounds);
+}
+int gemmMx8TileN(int rows, int n, int sms) {
+  float cost;
+  long long rounds;
+  return singleWidth(rows, n, sms, &cost, &rounds);
+}
+
+// Columns per tile of a CTA-pair launch, or 0 where single CTAs are the better form.  Pairs halve what an SM fetches of B: a full round
+// of 74 pairs of 224 columns took 10.5 us at K = 3584 where 148 single CTAs took 13.0, 21.9 and 26 at K = 8192 (narrower tiles:
+// mean of the two, relative).  A K block of theirs is a longer chain (barriers across the cluster), so what fits into one round of
+// single CTAs stays there: 777 x 2048 x 2048 14.5 us single, 16.4 pairs; 384 x 8192 x 2048 16.4 and 18.5; 512 x 8192 x 8192 36.9 and 37.7.
+// More than a round (us, cold L2, single -> pairs): 8192 x 3584 x 8192 180 -> 150, 8192 x 8192 x 3584 202 -> 159, 16384 x 8192 x 8192
+// 851 -> 711 (3.06 PFLOP/s), 1531 x 8192 x 3584 46 -> 42, 1531 x 3584 x 8192 50 -> 46, 5000 x 1920 x 2048 31.4 -> 26.6, 640 x 7168 x 4096
+// 30.6 -> 29.5, 1000 x 4096 x 4096 28.7 -> 26.7.
+int gemmMx8PairTileN(int rows, int n, int sms) {
+  static const RoundCost kWidths[] = {{224, 1.f}, {192, .90f}, {160, .84f}, {128, .76f}, {96, .69f}, {64, .66f}};
+  float single, pair;
+  long long single_rounds, pair_rounds;
+  singleWidth(rows, n, sms, &single, &single_rounds);
+  if (single_rounds < 2 || sms < 2) return 0;
+  const int bn = cheapestWidth(kWidths, 6, (rows + gemmxp::PAIR_M - 1) / gemmxp::PAIR_M, n, sms / 2, 64, &pair, &pair_rounds);
+  return pair < 1.2f * single ? bn : 0;
 }
 
 int launchQuantMx8Rows(const void* x, void* q, uint8_t* scales, long long rows, int k, cudaStream_t stream) {
@@ -186,6 +219,20 @@ int gemmMx8(const void* A, int64_t lda, const uint8_t* sa, int ld_sa, const void
   if (!makeTensorMap2D(&ta, A, TM_U8, K, M, lda, gemmx::BK, gemmx::BM, &g_errx)) return static_cast<int>(cudaErrorInvalidValue);
   int n_sm = deviceSmCount();
   if (sms > 0 && sms < n_sm) n_sm = sms;
+  if (const int bn = gemmMx8PairTileN(M, N, n_sm)) {
+    if (!makeTensorMap2D(&tb, B, TM_U8, K, N, ldb, gemmxp::BK, bn / 2, &g_errx)) return static_cast<int>(cudaErrorInvalidValue);
+    static bool pair_attr_set = false;
+    if (!pair_attr_set) {
+      cudaError_t e = cudaFuncSetAttribute(gemm_mx8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gemmxp::SMEM_BYTES);
+      if (e != cudaSuccess) return static_cast<int>(e);
+      pair_attr_set = true;
+    }
+    const int pair_tiles = ((M + gemmxp::PAIR_M - 1) / gemmxp::PAIR_M) * ((N + bn - 1) / bn), pairs = n_sm / 2;
+    return static_cast<int>(launchOverlapped(gemm_mx8_pair_kernel, dim3(2 * (pair_tiles < pairs ? pair_tiles : pairs)), dim3(gemmxp::NUM_THREADS),
+                                             gemmxp::SMEM_BYTES, stream, 2, ta, tb,
+                                             gemm::StoreEpi{D, D2, static_cast<const __nv_bfloat16*>(bias), ldd, M, N, flags, bn},
+                                             gemmx::Scales{sa, sb, ld_sa, ld_sb, M, N}, K, status));
+  }
   const int bn = gemmMx8TileN(M, N, n_sm);
   if (!makeTensorMap2D(&tb, B, TM_U8, K, N, ldb, gemmx::BK, bn, &g_errx)) return static_cast<int>(cudaErrorInvalidValue);
   gemm::StoreEpi epi{D, D2, static_cast<const __nv_bfloat16*>(bias), ldd, M, N, flags, bn};

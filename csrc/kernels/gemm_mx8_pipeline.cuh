@@ -93,6 +93,52 @@ __device__ __forceinline__ void mma_mx8(uint32_t d_tmem, uint64_t a_desc, uint64
 // [15]/[16] A/B MN-major, [17,23) N>>3, [23] scale format (1 = UE8M0), [24,29) M>>4, [29,31) A scale id.
 __host__ __device__ constexpr uint32_t make_idesc_mx(uint32_t m, uint32_t n) { return ((n >> 3) << 17) | (1u << 23) | ((m >> 4) << 24); }
 
+// The words of one scale image (128 rows of A, up to 256 columns of B, 512 values of K): a lane of the builder warp holds rows and
+// columns 32 q + lane.
+struct ScaleWords {
+  uint32_t a[4], b[8];
+  // Rows from row0, columns from col0, K blocks from kb0 on; rows and columns past the operands repeat the last one's scales.
+  __device__ __forceinline__ void fetch(const Scales& sc, int row0, int col0, int kb0, int num_kb, int lane) {
+    const int nblk = (sc.N + 127) / 128;
+    const bool aligned4 = ((sc.ld_sa | sc.ld_sb) & 3) == 0 && ((reinterpret_cast<uintptr_t>(sc.sa) | reinterpret_cast<uintptr_t>(sc.sb)) & 3) == 0;
+    const bool wide = aligned4 && kb0 + 4 <= num_kb;     // four scale bytes in one load
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int row = min(row0 + 32 * q + lane, sc.M - 1);
+      const uint8_t* p = sc.sa + static_cast<long long>(row) * sc.ld_sa;
+      uint32_t w = 0;
+      if (wide) {
+        w = dev::ld_cg_u32(p + kb0);     // may have been written by a peer: past L1
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (kb0 + j < num_kb) w |= dev::ld_cg_u8(p + kb0 + j) << (8 * j);
+      }
+      a[q] = w;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int blk = min((col0 + 32 * q + lane) >> 7, nblk - 1);
+      const uint8_t* p = sc.sb + static_cast<long long>(blk) * sc.ld_sb;
+      uint32_t w = 0;
+      if (wide) {
+        w = dev::ld_u32(p + kb0);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (kb0 + j < num_kb) w |= dev::ld_u8(p + kb0 + j) << (8 * j);
+      }
+      b[q] = w;
+    }
+  }
+  __device__ __forceinline__ void store(uint8_t* img, int lane) const {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) *reinterpret_cast<uint32_t*>(img + lane * 16 + q * 4) = a[q];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) *reinterpret_cast<uint32_t*>(img + 512 + (q >> 2) * 512 + lane * 16 + (q & 3) * 4) = b[q];
+  }
+};
+
 // `width` (a multiple of 32, at most BN): columns of a tile.
 template <class Sched, class Gate, class Epi>
 __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* tmB, int K, const Scales& sc, const Sched& sched,
@@ -222,41 +268,8 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
     // ------------------------------------------------------------------ scale builder (whole warp)
     // The words of the NEXT group (also across a tile boundary) are fetched from global memory into registers while
     // the MMAs of the current ones run; once the image buffer is free only the shared-memory writes remain.
-    const int nblk = (sc.N + 127) / 128;
-    const bool aligned4 = ((sc.ld_sa | sc.ld_sb) & 3) == 0 && ((reinterpret_cast<uintptr_t>(sc.sa) | reinterpret_cast<uintptr_t>(sc.sb)) & 3) == 0;
-    uint32_t wa[4], wb[8];
-    auto fetch = [&](const TileCoord& tt, int kg) {
-      const int row0 = tt.m * BM, col0 = tt.n * width, kb0 = kg * 4;
-      const bool wide = aligned4 && kb0 + 4 <= num_kb;     // four scale bytes in one load
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {               // A: rows 32 q + lane
-        const int row = min(row0 + 32 * q + lane, sc.M - 1);
-        const uint8_t* p = sc.sa + static_cast<long long>(row) * sc.ld_sa;
-        uint32_t w = 0;
-        if (wide) {
-          w = dev::ld_cg_u32(p + kb0);     // may have been written by a peer: past L1
-        } else {
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (kb0 + j < num_kb) w |= dev::ld_cg_u8(p + kb0 + j) << (8 * j);
-        }
-        wa[q] = w;
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {               // B: tile columns 32 q + lane
-        const int blk = min((col0 + 32 * q + lane) >> 7, nblk - 1);
-        const uint8_t* p = sc.sb + static_cast<long long>(blk) * sc.ld_sb;
-        uint32_t w = 0;
-        if (wide) {
-          w = dev::ld_u32(p + kb0);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (kb0 + j < num_kb) w |= dev::ld_u8(p + kb0 + j) << (8 * j);
-        }
-        wb[q] = w;
-      }
-    };
+    ScaleWords words;
+    auto fetch = [&](const TileCoord& tt, int kg) { words.fetch(sc, tt.m * BM, tt.n * width, kg * 4, num_kb, lane); };
     auto gate_open = [&](const TileCoord& tt) {   // A's scales arrive with its rows: read them only behind the gate
       int open = 1;
       if (lane == 0) open = gate.wait(tt, abort) ? 1 : 0;
@@ -277,11 +290,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         int open = 1;
         if (lane == 0) open = tc::mbar_wait(&bar->sf_empty[im], ((g / SF_IMAGES) & 1) ^ 1, abort) ? 1 : 0;
         if (!__shfl_sync(0xffffffffu, open, 0)) { ok = false; break; }
-        uint8_t* img = sf_smem + im * SF_BYTES;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) *reinterpret_cast<uint32_t*>(img + lane * 16 + q * 4) = wa[q];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) *reinterpret_cast<uint32_t*>(img + 512 + (q >> 2) * 512 + lane * 16 + (q & 3) * 4) = wb[q];
+        words.store(sf_smem + im * SF_BYTES, lane);
         tc::fence_proxy_async_smem();                // the image is read by tcgen05.cp (async proxy)
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&bar->sf_full[im]);

@@ -443,3 +443,37 @@ def test_fp8_gemm_row_scales_of_any_stride(K, shift, stride):
     check_status("gemm_fp8")
     assert torch.equal(out, gemm_fp8(aq, a_s, wq, w_s, out_dtype=torch.float32))
     assert (out.double() - ref).abs().max().item() <= 2e-3 * max(1.0, ref.abs().max().item())
+
+
+@pytest.mark.parametrize("M,N,K,width", [(12546, 392, 128, 224), (2100, 4360, 640, 192), (18947, 136, 256, 160), (1531, 3584, 1152, 160), (1000, 4096, 256, 128),
+                                         (19000, 112, 384, 128), (9490, 232, 1152, 96), (18965, 40, 512, 64)])
+def test_mx8_cta_pairs(M, N, K, width):
+    """The CTA-pair form at every width the launch picks: ragged rows and columns, tiles that straddle a block of scales, one to nine
+    K blocks (a scale image holds four); fp32 and bf16 outputs, bias, GELU and accumulation in the epilogue."""
+    from pccl_b200._native import C
+    from pccl_b200.ops import check_status
+    from pccl_b200.ops.gemm import dequant_rows, gemm_mx8, quant_rows_mx, ue8m0_to_float
+    assert C.gemm_mx8_pair_tile_n(M, N, 148) == width
+    # magnitudes that differ per K block, per 32 rows and per 128 columns, so that a scale of another place shows
+    a = (_rand((M, K), 97).float() * torch.logspace(-1, 1, K // 128, device="cuda").repeat_interleave(128)
+         * (1.0 + (torch.arange(M, device="cuda") // 32 % 8).float())[:, None]).bfloat16()
+    w = (_rand((N, K), 98, 0.05).float() * (1.0 + (torch.arange(N, device="cuda") // 128 % 5).float())[:, None]).bfloat16()
+    aq, a_s = quant_rows_mx(a)
+    wq, w_rows = quant_rows_mx(w)
+    w_s = w_rows[::128].contiguous()
+    ref = dequant_rows(aq, ue8m0_to_float(a_s)).double() @ (
+        wq.view(torch.float8_e4m3fn).double() * ue8m0_to_float(w_s).double().repeat_interleave(128, 1).repeat_interleave(128, 0)[:N]).t()
+    out = gemm_mx8(aq, a_s, wq, w_s, out_dtype=torch.float32)
+    check_status("gemm_mx8 pairs")
+    top = max(1.0, ref.abs().max().item())
+    assert (out.double() - ref).abs().max().item() <= 2e-3 * top            # sums in another order; a wrong scale or tile is off by O(1)
+    bias = _rand((N,), 99)
+    old = _rand((M, N), 100)
+    got = old.clone()
+    gemm_mx8(aq, a_s, wq, w_s, out=got, bias=bias, accumulate=True)
+    act = gemm_mx8(aq, a_s, wq, w_s, bias=bias, gelu_inplace=True)
+    check_status("gemm_mx8 pairs")
+    full = out.double() + bias.double()
+    assert ((got.double() - full - old.double()).abs() <= 2 ** -8 * (full + old.double()).abs() + 1e-4).all()
+    want = torch.nn.functional.gelu(full, approximate="tanh")
+    assert ((act.double() - want).abs() <= 2 ** -8 * want.abs() + 1.5e-3 * full.abs() + 1e-4).all()

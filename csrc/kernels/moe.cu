@@ -703,13 +703,13 @@ struct RaggedEpi {
 struct RaggedMaps { CUtensorMap x[5]; };     // boxes of 128, 64, 32, 16, 8 rows
 
 template <bool W_MN>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(gemm2::NUM_THREADS_WIDE, 1)
 gemm_grouped_ragged_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ RaggedMaps tmX, RaggedEpi<W_MN> epi, int groups,
                            int K, uint32_t* status) {
   RaggedSched sched{epi.row_off, groups, (epi.N + 255) / 256, static_cast<int>(blockIdx.x >> 1), static_cast<int>(gridDim.x >> 1)};
   NoGate gate;
   epi.cta = static_cast<int>(tc::cluster_ctarank());
-  gemm2::run<W_MN, false>(&tmW, tmX.x, K, sched, gate, epi, status);
+  gemm2::run<W_MN, false, RaggedSched, NoGate, RaggedEpi<W_MN>, gemm2::STAGES, 1, false, 8>(&tmW, tmX.x, K, sched, gate, epi, status);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1028,7 +1028,7 @@ int gemmGroupedBf16(const void* A, int64_t lda, const void* B, int64_t ldb, void
         if (e != cudaSuccess) return static_cast<int>(e);
         *done = true;
       }
-      return static_cast<int>(launchOverlapped(kern, dim3(n_sm & ~1), dim3(NUM_THREADS), gemm2::SMEM_BYTES, stream, 2, tw, tx, epi, groups, K, status));
+      return static_cast<int>(launchOverlapped(kern, dim3(n_sm & ~1), dim3(gemm2::NUM_THREADS_WIDE), gemm2::SMEM_BYTES, stream, 2, tw, tx, epi, groups, K, status));
     };
     if (w_mn)
       return go(gemm_grouped_ragged_kernel<true>,

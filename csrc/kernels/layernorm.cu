@@ -1,4 +1,4 @@
-// LayerNorm forward and backward for bf16 activations (fp32 statistics).  Forward: one CTA per row; every
+// LayerNorm forward and backward for bf16 activations (fp32 statistics).  Forward: a group of warps per row; every
 // thread keeps its 8-element vectors of the row in registers, so x is read once.  Backward: a group of warps
 // per row (as many as cover it), several rows at a time, x and dy read once; the kernel is persistent, its
 // threads keep their columns' share of dgamma / dbeta in registers across all of their rows, and each CTA writes
@@ -25,71 +25,89 @@ namespace {
 
 using namespace dev;
 
-__device__ __forceinline__ float block_sum(float v, float* scratch) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  __syncthreads();
-  if (lane == 0) scratch[warp] = v;
-  __syncthreads();
-  float r = 0.f;
-  for (int w = 0; w < nw; ++w) r += scratch[w];
-  return r;
-}
-
-template <int MAXV>
-__global__ void __launch_bounds__(256) ln_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* delta,
-                                                     __nv_bfloat16* sum_out, const __nv_bfloat16* gamma,
-                                                     const __nv_bfloat16* beta, __nv_bfloat16* y,
-                                                     float* mean, float* rstd, int D, float eps) {
-  __shared__ float scratch[8];
+// Forward.  A group of `gw` warps owns a row with up to four 16-byte vectors per thread (one warp up to D = 1024) and a CTA takes as
+// many rows as its 256 threads hold: all loads of a row are out before the first sum, and a row of one warp takes no barrier.  A row
+// stays in registers as it came, eight values in four registers, and scale and shift are read last (they are in L1 or L2), so that four
+// CTAs fit an SM; with two vectors per thread and six CTAs, with CTAs of 128 threads or with scale and shift ahead of the sums 16384 x 2048
+// takes 53, 55 and 51 us.
+// Memory bounds it.  Times, us, cold L2, plain and with the residual sum (a CTA of 256 threads per row before -> now): 16384 x 2048
+// 39 -> 36, 55 -> 49 (5.5 TB/s); 16384 x 1536 37 -> 32, 49 -> 40; 16384 x 1024 33 -> 21, 43 -> 29; 16384 x 256 29 -> 12, 35 -> 14;
+// 4096 x 1024 14 -> 11, 16 -> 12; 4096 x 8192 41 -> 37, 64 -> 49; 1531 x 2048 unchanged at 10 and 12.
+template <int VPT>
+__global__ void __launch_bounds__(256, VPT == 4 ? 4 : 1) ln_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* delta, __nv_bfloat16* sum_out,
+                                                     const __nv_bfloat16* gamma, const __nv_bfloat16* beta, __nv_bfloat16* y,
+                                                     float* mean, float* rstd, long long rows, int D, float eps, int gw) {
+  __shared__ float part[2][8];                              // [sum, squares][warp]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int group = warp / gw, groups = (blockDim.x >> 5) / gw, tid = threadIdx.x - group * gw * 32;
+  const int nvec = D >> 3, width = gw * 32;
   dev::pdl_launch();
   dev::pdl_wait();
-  const long long row = blockIdx.x;
-  const int nvec = D >> 3;
-  float f[MAXV][8];
+  const long long row = static_cast<long long>(blockIdx.x) * groups + group;
+  if (row >= rows) return;                                  // the whole group: barriers are per group
+  const long long at = row * D + tid * 8;
+  const Vec16 zero{{0u, 0u, 0u, 0u}};
+  Vec16 v[VPT];
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) v[j] = tid + j * width < nvec ? ld16(x + at + j * width * 8) : zero;
+  if (delta) {
+    Vec16 g[VPT];
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) g[j] = tid + j * width < nvec ? ld16(delta + at + j * width * 8) : zero;
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+      // the norm sees the sum as it is stored (rounded to bf16), so that backward, which re-reads it, agrees
+      float f[8], d[8];
+      unpack<DT_BF16>(v[j], f);
+      unpack<DT_BF16>(g[j], d);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) f[k] += d[k];
+      v[j] = pack<DT_BF16>(f);
+      if (tid + j * width < nvec) st16(sum_out + at + j * width * 8, v[j]);
+    }
+  }
+  auto group_sum = [&](float t, int which) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (gw == 1) return t;
+    if (lane == 0) part[which][warp] = t;
+    asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(width) : "memory");
+    t = 0.f;
+    for (int w = 0; w < gw; ++w) t += part[which][group * gw + w];
+    return t;
+  };
   float s = 0.f;
 #pragma unroll
-  for (int j = 0; j < MAXV; ++j) {
-    const int v = threadIdx.x + j * 256;
-    if (v < nvec) {
-      unpack<DT_BF16>(ld16(x + row * D + v * 8), f[j]);
-      if (delta) {
-        // the norm sees the sum as it is stored (rounded to bf16), so that backward, which re-reads it, agrees
-        float d[8];
-        unpack<DT_BF16>(ld16(delta + row * D + v * 8), d);
+  for (int j = 0; j < VPT; ++j) {
+    float f[8];
+    unpack<DT_BF16>(v[j], f);                               // vectors past the row are zeros
 #pragma unroll
-        for (int k = 0; k < 8; ++k) f[j][k] += d[k];
-        const Vec16 r = pack<DT_BF16>(f[j]);
-        st16(sum_out + row * D + v * 8, r);
-        unpack<DT_BF16>(r, f[j]);
-      }
-#pragma unroll
-      for (int k = 0; k < 8; ++k) s += f[j][k];
-    }
+    for (int k = 0; k < 8; ++k) s += f[k];
   }
-  const float mu = block_sum(s, scratch) / D;
+  const float mu = group_sum(s, 0) / D;
   float q = 0.f;
 #pragma unroll
-  for (int j = 0; j < MAXV; ++j) {
-    const int v = threadIdx.x + j * 256;
-    if (v < nvec) {
+  for (int j = 0; j < VPT; ++j) {
+    if (tid + j * width < nvec) {
+      float f[8];
+      unpack<DT_BF16>(v[j], f);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) { const float d = f[j][k] - mu; q += d * d; }
+      for (int k = 0; k < 8; ++k) { const float d = f[k] - mu; q += d * d; }
     }
   }
-  const float rs = rsqrtf(block_sum(q, scratch) / D + eps);
-  if (threadIdx.x == 0 && mean) { mean[row] = mu; rstd[row] = rs; }
+  const float rs = rsqrtf(group_sum(q, 1) / D + eps);
+  if (tid == 0 && mean) { mean[row] = mu; rstd[row] = rs; }
 #pragma unroll
-  for (int j = 0; j < MAXV; ++j) {
-    const int v = threadIdx.x + j * 256;
-    if (v < nvec) {
-      float g[8], b[8], o[8];
-      unpack<DT_BF16>(ld16(gamma + v * 8), g);
-      unpack<DT_BF16>(ld16(beta + v * 8), b);
+  for (int j = 0; j < VPT; ++j) {
+    if (tid + j * width < nvec) {
+      const Vec16 g = ld16(gamma + (tid + j * width) * 8), b = ld16(beta + (tid + j * width) * 8);
+      float f[8], gf[8], bf[8], o[8];
+      unpack<DT_BF16>(v[j], f);
+      unpack<DT_BF16>(g, gf);
+      unpack<DT_BF16>(b, bf);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) o[k] = (f[j][k] - mu) * rs * g[k] + b[k];
-      st16(y + row * D + v * 8, pack<DT_BF16>(o));
+      for (int k = 0; k < 8; ++k) o[k] = (f[k] - mu) * rs * gf[k] + bf[k];
+      st16(y + at + j * width * 8, pack<DT_BF16>(o));
     }
   }
 }
@@ -403,9 +421,22 @@ int launchLayerNormFwd(const void* x, const void* delta, void* sum_out, const vo
   auto X = static_cast<const __nv_bfloat16*>(x); auto G = static_cast<const __nv_bfloat16*>(gamma);
   auto B = static_cast<const __nv_bfloat16*>(beta); auto Y = static_cast<__nv_bfloat16*>(y);
   auto DL = static_cast<const __nv_bfloat16*>(delta); auto S = static_cast<__nv_bfloat16*>(sum_out);
-  const unsigned grid = static_cast<unsigned>(rows);
-  auto go = [&](auto kern) { return static_cast<int>(launchOverlapped(kern, dim3(grid), dim3(256), 0, stream, 1, X, DL, S, G, B, Y, mean, rstd, D, eps)); };
-  return D <= 2048 ? go(ln_fwd_kernel<1>) : D <= 4096 ? go(ln_fwd_kernel<2>) : go(ln_fwd_kernel<4>);
+  const int nvec = D / 8;
+  int gw = (nvec + 127) / 128, vpt = gw > 1 ? 4 : (nvec + 31) / 32;
+  // Up to four million values a thread takes one vector: its chain is the shorter (24 x 2048 9 -> 8 us, 1531 x 2048 equal by itself), and
+  // with 40 registers per thread a CTA finds room beside one of a GEMM, to be in its place when that ends.
+  if (rows * D <= 4ll << 20 && nvec <= 256) {
+    gw = (nvec + 31) / 32;
+    vpt = 1;
+  }
+  // as many rows per CTA as 256 threads hold, fewer where the rows would then leave SMs without work
+  int groups = 8 / gw;
+  while (groups > 1 && (rows + groups - 1) / groups < deviceSmCount()) groups /= 2;
+  const unsigned grid = static_cast<unsigned>((rows + groups - 1) / groups);
+  auto go = [&](auto kern) {
+    return static_cast<int>(launchOverlapped(kern, dim3(grid), dim3(groups * gw * 32), 0, stream, 1, X, DL, S, G, B, Y, mean, rstd, rows, D, eps, gw));
+  };
+  return vpt == 1 ? go(ln_fwd_kernel<1>) : vpt == 2 ? go(ln_fwd_kernel<2>) : vpt == 3 ? go(ln_fwd_kernel<3>) : go(ln_fwd_kernel<4>);
 }
 
 int layerNormBwdParts(long long rows) { return static_cast<int>(rows < 148 * 2 ? rows : 148 * 2); }

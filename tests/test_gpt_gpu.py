@@ -368,6 +368,29 @@ def test_layer_norm_backward_over_widths(D, rows):
         assert (a.double() - b).abs().max().item() <= 2 ** -8 * b.abs().max().item() + 1e-4
 
 
+@pytest.mark.parametrize("D", [8, 248, 264, 512, 520, 776, 1024, 1032, 2048, 2056, 4104, 8192])
+@pytest.mark.parametrize("rows", [1, 297, 5003, 17001])
+def test_layer_norm_forward_over_widths(D, rows):
+    """One to eight warps per row with one to four vectors per thread, rows that do not fill the last CTA, and the row counts at which
+    the launch goes from one vector per thread to as many as fit.  Against fp64 on the same bf16 inputs: the sum is rounded to bf16
+    once and compared exactly, the statistics are fp32 sums (1e-5), the result is rounded once."""
+    import torch
+    from pccl_b200.nn.norm import _ln_forward
+    torch.manual_seed(D + rows)
+    x, d = ((torch.randn(rows, D, device="cuda") + 3.0).bfloat16() for _ in range(2))
+    w, b = (torch.randn(D, device="cuda").bfloat16() for _ in range(2))
+    for delta in (None, d):
+        s, y, stats = _ln_forward(x, delta, w, b, 1e-5)
+        total = x if delta is None else (x.float() + d.float()).bfloat16()
+        assert s is None or torch.equal(s, total)
+        t = total.double()
+        var = t.var(1, unbiased=False)
+        assert torch.allclose(stats[0].double(), t.mean(1), rtol=1e-5, atol=1e-6)
+        assert torch.allclose(stats[1].double(), (var + 1e-5).rsqrt(), rtol=1e-4)
+        ref = F.layer_norm(t, (D,), w.double(), b.double(), 1e-5)
+        assert ((y.double() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-4 * (1 + ref.abs().max())).all()
+
+
 @pytest.mark.parametrize("vocab", [7, 1001, 50257])
 def test_cross_entropy_with_masked_and_large_logits(vocab):
     """Logits of -inf (masked classes, whole stretches of them), of the type's lowest value and of +-3e4: the running maximum starts

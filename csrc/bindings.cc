@@ -196,6 +196,7 @@ py::dict layoutDict(const Engine& e) {
 
 void bindGemm(py::module_& m);    // gemm_bindings.cc
 void bindFused(py::module_& m);   // fused_bindings.cc
+void bindBlock(py::module_& m);   // block_bindings.cc
 
 PYBIND11_MODULE(_C, m) {
   m.doc() = "pccl_b200 native runtime";
@@ -311,6 +312,7 @@ PYBIND11_MODULE(_C, m) {
 
   bindGemm(m);
   bindFused(m);
+  bindBlock(m);
 
   auto utils = m.def_submodule("utils");
   py::class_<LaunchEnvironments, std::unique_ptr<LaunchEnvironments, py::nodelete>>(utils, "LaunchEnvironments")

@@ -16,6 +16,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from ..nn.block import attn_in, halves_apply, mlp_out
 from ..nn.linear import Embedding, Linear, LinearGelu, _LinearFn, is_plain, mlp, split_qkv
 from ..nn.loss import fused_cross_entropy
 from ..nn.norm import LayerNorm
@@ -80,6 +81,10 @@ class Block(nn.Module):
             a = F.scaled_dot_product_attention(q, k, v, is_causal=True)
             x = x + self.proj(a.transpose(1, 2).reshape(B, T, D))
             return x + self.fc2(self.fc1(self.ln2(x))), None, None
+        if halves_apply(self, x):
+            x, q, k, v = attn_in(self, x, delta, prev_bias)
+            x, out = mlp_out(self, F.scaled_dot_product_attention(q, k, v, is_causal=True), x)
+            return x, out, self.fc2.bias
         if delta is None:
             h = self.ln1(x)
         else:

@@ -596,3 +596,56 @@ def test_profiler_target_of_the_training_kernels_runs():
     r = subprocess.run([sys.executable, "-m", "pccl_b200.profile_targets", "train_kernels", "--tokens", "256", "--iters", "1"],
                        cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "ln_bwd_add_colsum" in r.stdout, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("batch,seq", [(2, 64), (3, 77), (2, 256)])
+@pytest.mark.parametrize("what", ["autograd", "bucket", "frozen", "saved on cpu", "no grad", "grad"])
+def test_block_halves_are_their_layers(batch, seq, what, monkeypatch):
+    """A block's halves issue the launches of its layers, so loss, logits and every gradient are the same bits as with the layers called
+    one by one: up to and above 128 rows, with gradients returned by autograd, written to the bucket, for some parameters or inputs only,
+    and with saved tensors that leave the GPU in between."""
+    import torch
+    from pccl_b200.models import gpt
+    cfg = gpt.GPTConfig(n_layer=3, n_head=4, d_model=128, seq_len=seq, vocab_size=264)
+    ids = torch.randint(0, 264, (batch, seq), device="cuda")
+    got = []
+    for halves in (True, False):
+        if not halves:
+            monkeypatch.setattr(gpt, "halves_apply", lambda block, x: False)
+        torch.manual_seed(3)
+        model = gpt.GPT(cfg, device="cuda")
+        for p in model.parameters():
+            if p.dim() == 1:
+                p.data.copy_((torch.randn(p.shape, device="cuda") * 0.3 + (1.0 if p.data.mean() > 0.5 else 0.0)).bfloat16())
+        if what == "frozen":
+            for m in (model.blocks[0].ln1, model.blocks[1].ln2, model.blocks[1].proj):
+                m.requires_grad_(False)
+            model.blocks[2].fc2.bias.requires_grad_(False)
+        if what == "no grad":
+            with torch.no_grad():
+                got.append([model.logits(ids)])
+            continue
+        if what == "grad":
+            blk = model.blocks[1]
+            wanted = [blk.ln1.weight, blk.qkv.bias, blk.proj.bias, blk.fc1.weight, model.blocks[0].fc2.bias, model.wpe.weight]
+            got.append(list(torch.autograd.grad(model(ids, ids.roll(-1, 1)), wanted)))
+            continue
+        if what == "bucket":
+            from pccl_b200.parallel.dp import ShardedDataParallel
+            dp = ShardedDataParallel(model, lr=1e-3, heap_bytes=256 << 20)
+            losses = [dp.train_step(ids, ids.roll(-1, 1)).clone() for _ in range(2)]
+            got.append(losses + [dp.flat_grads.clone(), dp.flat_params.clone()])
+            continue
+        hooks = torch.autograd.graph.save_on_cpu() if what == "saved on cpu" else torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t)
+        with hooks:
+            loss = model(ids, ids.roll(-1, 1))
+        loss.backward()
+        got.append([loss.detach()] + [p.grad for p in model.parameters() if p.requires_grad])
+    # the embedding's gradient is a sum in no fixed order (index_add_), and everything else does not depend on it
+    for a, b in zip(*got):
+        if what in ("autograd", "frozen", "saved on cpu") and a.shape == (264, 128) or a.shape == (seq, 128) and what != "no grad":
+            assert torch.allclose(a.float(), b.float(), rtol=2e-2, atol=1e-4)
+        elif what == "bucket" and a.dim() == 1:
+            assert (a != b).float().mean().item() < 0.2 and torch.allclose(a.float(), b.float(), rtol=5e-2, atol=2e-3)
+        else:
+            assert torch.equal(a, b)

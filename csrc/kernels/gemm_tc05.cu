@@ -80,10 +80,11 @@ struct DualSched {
     const long long n0 = static_cast<long long>(tiles_m[0]) * tiles_n[0];
     const int q = idx >= n0 ? 1 : 0;
     if (q) idx -= n0;
-    if (idx >= static_cast<long long>(tiles_m[q]) * tiles_n[q]) return false;
-    const int per_group = GroupedSched::GROUP_M * tiles_n[q];
+    const int tm = q ? tiles_m[1] : tiles_m[0], tn = q ? tiles_n[1] : tiles_n[0];       // no variable index: the arrays would live in local memory
+    if (idx >= static_cast<long long>(tm) * tn) return false;
+    const int per_group = GroupedSched::GROUP_M * tn;
     const int g = static_cast<int>(idx / per_group), r = static_cast<int>(idx % per_group);
-    const int gm = min(GroupedSched::GROUP_M, tiles_m[q] - g * GroupedSched::GROUP_M);
+    const int gm = min(GroupedSched::GROUP_M, tm - g * GroupedSched::GROUP_M);
     t->m = g * GroupedSched::GROUP_M + r % gm;
     t->n = r / gm;
     t->extra = q;
@@ -94,14 +95,18 @@ struct DualSched {
 struct DualEpi {
   static constexpr bool kRow128 = false;
   StoreEpi e[2];
+  StoreEpi cur;          // the tile's problem, picked once per tile: indexed with a variable the two would live in local memory
   __device__ __forceinline__ int width() const { return e[0].bn; }        // one width for both problems
-  __device__ __forceinline__ int a_row0(const TileCoord& t) const { return e[t.extra].a_row0(t); }
-  __device__ __forceinline__ int b_row0(const TileCoord& t) const { return e[t.extra].b_row0(t); }
+  __device__ __forceinline__ int a_row0(const TileCoord& t) const { return e[0].a_row0(t); }
+  __device__ __forceinline__ int b_row0(const TileCoord& t) const { return e[0].b_row0(t); }
   __device__ __forceinline__ void attach_smem(uint8_t*) {}
   __device__ __forceinline__ void attach_patch(uint8_t* p) { e[0].attach_patch(p); e[1].attach_patch(p); }
-  __device__ __forceinline__ void tile_begin(const TileCoord&) {}
+  __device__ __forceinline__ void tile_begin(const TileCoord& t) {
+    cur = e[0];
+    if (t.extra) cur = e[1];
+  }
   __device__ __forceinline__ void tile_done(const TileCoord&, const volatile uint32_t*) {}
-  __device__ __forceinline__ void strip(const TileCoord& t, int row, int col, uint32_t* r) { e[t.extra].strip(t, row, col, r); }
+  __device__ __forceinline__ void strip(const TileCoord& t, int row, int col, uint32_t* r) { cur.strip(t, row, col, r); }
 };
 
 template <bool A_MN, bool B_MN, bool DYN>

@@ -6,9 +6,9 @@ kernel is queued on a high-priority side stream: each rank reduces its 1/world s
 (multimem.ld_reduce through the switch, or loads from every peer over NVLink), multiplies by
 1/world and applies AdamW to its fp32 master slice -- reduction, scaling, cast and optimizer in one
 pass -- and writes the new bf16 parameters, which the bucket's all-gather kernel then pushes to
-every rank (ZeRO-1).  The kernels run as short, wide bursts (64 to 128 CTAs) that slip in between
-two GEMM kernels of backward.  With a world of one the same kernels run (the reduce-scatter
-degenerates to the scale/cast/update pass), so single-GPU and multi-GPU steps share one code path.
+every rank (ZeRO-1).  The kernels run as short, wide bursts (64 CTAs) that slip in between
+two GEMM kernels of backward.  With a world of one the reduce-scatter is a flat scale/cast/update pass
+over the bucket, whose small CTAs run beside the GEMMs' on the same SMs.
 ``fuse_optimizer=False`` keeps the reduce-scatter (with scale and fp32 cast) and the optimizer apart.
 """
 from __future__ import annotations
@@ -81,7 +81,8 @@ class ShardedDataParallel:
         # Communication kernels run as short, wide bursts on a high-priority stream: they slip in at the
         # boundary between two GEMM kernels and delay the next one by their own (tens of microseconds)
         # duration.  A narrow long-running kernel would instead hold a few SMs for the whole GEMM and make
-        # the persistent GEMM's last CTAs start a full wave late.
+        # the persistent GEMM's last CTAs start a full wave late.  (A world of one exchanges nothing and has a kernel of its own,
+        # which runs beside the GEMMs and takes no block count.)
         self.comm_blocks = comm_blocks if comm_blocks else (128 if engine.world == 1 else 64)
         self.comm_stream = torch.cuda.Stream(priority=-1)
         self.step_count = 0

@@ -111,6 +111,33 @@ def test_adamw_kernel_matches_torch():
     assert torch.equal(out, p.bfloat16())
 
 
+@pytest.mark.parametrize("n", [8, 504, 520, 2048, 2056, 303112, (32 << 20) + 24])
+def test_bucket_update_in_a_world_of_one(n):
+    """Whole and partial trips of a warp, more trips than CTAs, and the size from which more CTAs run; two steps against the formula in
+    fp64 (each step rounds master and moments to fp32 a few times: 1e-5), parameters one bf16 rounding of the masters."""
+    import torch
+    from pccl_b200.engine import Engine
+    from pccl_b200.ops import collectives as coll
+    torch.manual_seed(n % 1000)
+    eng = Engine(0, 1)
+    eng.initEngine("cuda", 2 * n + (640 << 20))
+    g = eng.symmetric_tensor((n,), torch.bfloat16, align=256)
+    pad = torch.full((n + 64,), 7.0, dtype=torch.bfloat16, device="cuda")
+    out = pad[32:32 + n]
+    p, m, v = torch.randn(n, device="cuda"), torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda")
+    p64, m64, v64 = p.double(), m.double(), v.double()
+    for step in (1, 2):
+        g.copy_(torch.randn(n, device="cuda"))
+        coll.reduce_scatter_adamw(eng, g, p, m, v, out, lr=1e-2, betas=(0.9, 0.95), eps=1e-8, weight_decay=0.1, step=step, scale=0.5)
+        g64 = g.double() * 0.5
+        m64, v64 = 0.9 * m64 + 0.1 * g64, 0.95 * v64 + 0.05 * g64 * g64
+        p64 = p64 * (1 - 1e-2 * 0.1) - 1e-2 * (m64 / (1 - 0.9 ** step)) / ((v64 / (1 - 0.95 ** step)).sqrt() + 1e-8)
+    for got, want in ((p, p64), (m, m64), (v, v64)):
+        assert (got.double() - want).abs().max().item() <= 1e-5 * max(1.0, want.abs().max().item())
+    assert torch.equal(out, p.bfloat16())
+    assert (pad[:32] == 7).all() and (pad[32 + n:] == 7).all()
+
+
 def test_sharded_dp_world_of_one_trains_and_matches_plain_adamw():
     from pccl_b200.models import GPT, GPTConfig
     from pccl_b200.models.gpt import smoke_step
@@ -633,8 +660,8 @@ def test_block_halves_are_their_layers(batch, seq, what, monkeypatch):
         if what == "bucket":
             from pccl_b200.parallel.dp import ShardedDataParallel
             dp = ShardedDataParallel(model, lr=1e-3, heap_bytes=256 << 20)
-            losses = [dp.train_step(ids, ids.roll(-1, 1)).clone() for _ in range(2)]
-            got.append(losses + [dp.flat_grads.clone(), dp.flat_params.clone()])
+            loss = dp.train_step(ids, ids.roll(-1, 1)).clone()
+            got.append([loss] + [p.main_grad.clone() for p in model.parameters()])
             continue
         hooks = torch.autograd.graph.save_on_cpu() if what == "saved on cpu" else torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t)
         with hooks:
@@ -643,9 +670,7 @@ def test_block_halves_are_their_layers(batch, seq, what, monkeypatch):
         got.append([loss.detach()] + [p.grad for p in model.parameters() if p.requires_grad])
     # the embedding's gradient is a sum in no fixed order (index_add_), and everything else does not depend on it
     for a, b in zip(*got):
-        if what in ("autograd", "frozen", "saved on cpu") and a.shape == (264, 128) or a.shape == (seq, 128) and what != "no grad":
+        if what != "no grad" and a.shape in ((264, 128), (seq, 128)):
             assert torch.allclose(a.float(), b.float(), rtol=2e-2, atol=1e-4)
-        elif what == "bucket" and a.dim() == 1:
-            assert (a != b).float().mean().item() < 0.2 and torch.allclose(a.float(), b.float(), rtol=5e-2, atol=2e-3)
         else:
             assert torch.equal(a, b)

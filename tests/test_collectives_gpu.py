@@ -1124,3 +1124,39 @@ def test_gemm_rs_bias_emulated(native, world, M_local, w_t):
         ref = sum(p[rows] for p in parts) + bias[r].double()
         spread = sum(p[rows].abs() for p in parts) + ref.abs()
         assert ((outs[r].double() - ref).abs() <= 2 ** -8 * spread + 1e-5).all()
+
+
+@pytest.mark.parametrize("T,H,E,topk", [(40, 128, 8, 1), (41, 2176, 8, 3), (300, 1024, 16, 8), (97, 7168, 32, 8), (33, 16512, 4, 4)])
+def test_moe_exchange_group_sizes(native, T, H, E, topk):
+    """Tokens handled by groups of 64 and of 256 threads (the launch picks by tokens per block): the same bytes, scales and combined
+    rows; the gate gradients add up in another order (fp32 sums of H products: 1e-5 of the sum of magnitudes)."""
+    from pccl_b200.engine import Engine
+    from pccl_b200.ops import check_status
+    from pccl_b200.ops.moe import MoEExchange
+    torch.manual_seed(T)
+    eng = Engine(0, 1)
+    cap = 2 * T * topk + 256
+    eng.initEngine("cuda", 2 * cap * (H * 5 + H // 32 + 256) + (640 << 20))
+    x, logits = torch.randn(T, H, device="cuda").bfloat16(), torch.randn(T, E, device="cuda")
+    y = torch.randn(cap, H, device="cuda").bfloat16()
+    got = []
+    for blocks in (1, 148):
+        ex = MoEExchange(eng, T, H, E, topk, blocks=blocks)
+        if not got:
+            ids, probs, plan = ex.route_and_plan(logits)
+        n = T * topk
+        ex.dispatch(x, ids, plan)
+        plain = (ex.recv_q[:n].clone(), ex.recv_s[:n].clone())
+        ex.dispatch(x, ids, plan, probs=probs)
+        scaled = (ex.recv_q[:n].clone(), ex.recv_s[:n].clone())
+        ex.y.copy_(y[:ex.cap])
+        got.append(plain + scaled + (ex.combine(ids, probs, plan), ex.combine_dot(x, ids, plan)))
+        check_status("moe exchange")
+    for a, b in zip(got[0][:5], got[1][:5]):
+        assert torch.equal(a, b)
+    rows = plan["rows"].long()
+    products = x.double()[:, None, :] * y.double()[rows]
+    for g in got:
+        assert ((g[5].double() - products.sum(-1)).abs() <= 1e-5 * products.abs().sum(-1)).all()
+    want = (probs.double()[:, :, None] * y.double()[rows]).sum(1)
+    assert ((got[0][4].double() - want).abs() <= 2 ** -8 * want.abs() + 1e-4).all()

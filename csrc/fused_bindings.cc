@@ -90,6 +90,10 @@ void bindFused(py::module_& m) {
                          reinterpret_cast<int*>(pos), reinterpret_cast<int*>(counts), tokens, experts, topk,
                          reinterpret_cast<cudaStream_t>(stream)), "moe_route");
   });
+  m.def("moe_route_backward", [](uint64_t logits, uint64_t ids, uint64_t dprobs, uint64_t dlogits, int tokens, int experts, int topk, uint64_t stream) {
+    check(launchMoeRouteBackward(reinterpret_cast<const float*>(logits), reinterpret_cast<const int*>(ids), reinterpret_cast<const float*>(dprobs),
+                                 reinterpret_cast<float*>(dlogits), tokens, experts, topk, reinterpret_cast<cudaStream_t>(stream)), "moe_route_backward");
+  });
   m.def("moe_plan", [](uint64_t counts_all, uint64_t ids, uint64_t pos, uint64_t rows, uint64_t row_off, int world, int rank, int experts,
                        int tokens, int topk, int cap, uint64_t stream) {
     check(launchMoePlan(reinterpret_cast<const int*>(counts_all), reinterpret_cast<const int*>(ids), reinterpret_cast<const int*>(pos),

@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(GT * kCombineSubs<GT>) moe_combine_kernel(cons
     const Assignment a = next;
     next.fetch(A, slot, t + step, lane, A.probs[slot]);       // in flight behind this token's rows
     const char* src_l = a.dest >= 0 ? A.w.heap[a.dest] + A.y_off + static_cast<long long>(a.row) * H * 2 : nullptr;
-    float p_l = a.p;
+    float p_l = A.probs[slot] ? a.p : 1.0f;                 // without weights a plain sum
     const uint32_t peers = __match_any_sync(0xffffffffu, a.dest);
     if (A.dedupe && A.z_off && a.dest >= 0) {
       // one row per (token, rank): the first assignment to a rank stands for the token's whole group there; a group of two
@@ -932,6 +932,57 @@ __global__ void __launch_bounds__(256) moe_plan_kernel(const int* counts_all, co
   }
 }
 
+// Gradient of the routing logits of one token per warp: with p = softmax(logits) over all experts and d the gradients of the weights
+// of the experts taken (zero for the others), p .* (d - <p, d>).  The exponentials are taken in fp64, a few per lane: the fast
+// ones of this file are good to 1e-6 only.  One launch of 3 us for eight of tensor operations (25 us, 2001 tokens, 32 experts).
+template <int PER_LANE>
+__global__ void __launch_bounds__(256) moe_route_backward_kernel(const float* logits, const int* ids, const float* dprobs, float* dlogits, int tokens,
+                                                                 int experts, int topk) {
+  dev::pdl_launch();
+  dev::pdl_wait();
+  const int lane = threadIdx.x & 31, t = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (t >= tokens) return;
+  float p[PER_LANE], d[PER_LANE];
+  float mx = -INFINITY;
+#pragma unroll
+  for (int j = 0; j < PER_LANE; ++j) {
+    const int e = j * 32 + lane;
+    p[j] = e < experts ? ld_f32(logits + static_cast<long long>(t) * experts + e) : -INFINITY;
+    d[j] = 0.f;
+    mx = fmaxf(mx, p[j]);
+  }
+  for (int k = 0; k < topk; ++k) {
+    const int e = static_cast<int>(ld_u32(ids + t * topk + k));
+    const float g = ld_f32(dprobs + t * topk + k);
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j)
+      if (j * 32 + lane == e) d[j] = g;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  float sum = 0.f;
+#pragma unroll
+  for (int j = 0; j < PER_LANE; ++j) {
+    p[j] = j * 32 + lane < experts ? static_cast<float>(exp(static_cast<double>(p[j]) - mx)) : 0.f;
+    sum += p[j];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  float dot = 0.f;
+#pragma unroll
+  for (int j = 0; j < PER_LANE; ++j) {
+    p[j] = __fdiv_rn(p[j], sum);
+    dot += p[j] * d[j];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+#pragma unroll
+  for (int j = 0; j < PER_LANE; ++j) {
+    const int e = j * 32 + lane;
+    if (e < experts) dlogits[static_cast<long long>(t) * experts + e] = p[j] * (d[j] - dot);
+  }
+}
+
 template <typename K>
 int coop(K kernel, const MoeArgs& a, int blocks, size_t smem, cudaStream_t stream, int threads, int subs, int ctas_per_sm) {
   if (blocks < 1) blocks = 1;
@@ -1028,6 +1079,17 @@ int launchMoeRoute(const float* logits, int* ids, float* probs, int* pos, int* c
   if (per <= 4) return shared ? go(moe_route_kernel<4, true>) : go(moe_route_kernel<4, false>);
   if (per <= 8) return shared ? go(moe_route_kernel<8, true>) : go(moe_route_kernel<8, false>);
   return per <= 16 ? go(moe_route_kernel<16, false>) : go(moe_route_kernel<32, false>);
+}
+
+int launchMoeRouteBackward(const float* logits, const int* ids, const float* dprobs, float* dlogits, int tokens, int experts, int topk,
+                           cudaStream_t stream) {
+  if (experts < 1 || experts > 1024 || topk > experts || tokens <= 0) return static_cast<int>(cudaErrorInvalidValue);
+  auto go = [&](auto kern) {
+    return static_cast<int>(launchOverlapped(kern, dim3((tokens + 7) / 8), dim3(256), 0, stream, 1, logits, ids, dprobs, dlogits, tokens, experts, topk));
+  };
+  const int per = (experts + 31) / 32;
+  return per <= 1 ? go(moe_route_backward_kernel<1>) : per <= 4 ? go(moe_route_backward_kernel<4>) : per <= 8 ? go(moe_route_backward_kernel<8>)
+                                                                                              : go(moe_route_backward_kernel<32>);
 }
 
 int launchMoePlan(const int* counts_all, const int* ids, const int* pos, int* rows, int* row_off, int world, int rank, int experts,

@@ -44,7 +44,7 @@ struct MoeArgs {
 int launchMoeDispatch(const MoeArgs& a, int blocks, cudaStream_t stream);
 // out (fp32 [tokens, topk]) = <x[t], y[rank of expert (t,k)][dst_rows[t,k]]>: gradients of the gate weights.
 int launchMoeCombineDot(const MoeArgs& a, int blocks, cudaStream_t stream);
-// out[t] = sum_k probs[t,k] * y[rank of expert (t,k)][dst_rows[t,k]]: pulls the rows over NVLink.
+// out[t] = sum_k probs[t,k] * y[rank of expert (t,k)][dst_rows[t,k]]: pulls the rows over NVLink.  Without probs a plain sum.
 int launchMoeCombine(const MoeArgs& a, int blocks, cudaStream_t stream);
 // bf16 rows from fp8 rows + scales, for rows [0, *n_rows) (device count).  `alias` (or null): row r is read from alias[r].
 int launchMoeDequant(const void* q, const float* scales, void* out, const int* n_rows, int max_rows, int hidden, const int* alias,
@@ -62,6 +62,9 @@ int launchQuantFp8Blocks(const void* w, void* q, float* scales, int rows, int co
 // rank's assignments to the same expert (counts[experts] must be zero on entry and holds the totals afterwards).
 int launchMoeRoute(const float* logits, int* ids, float* probs, int* pos, int* counts, int tokens, int experts, int topk,
                    cudaStream_t stream);
+// Its backward: gradient of the logits from those of the k probabilities taken (fp32 [tokens, k]), through the softmax over all experts.
+int launchMoeRouteBackward(const float* logits, const int* ids, const float* dprobs, float* dlogits, int tokens, int experts, int topk,
+                           cudaStream_t stream);
 // Placement: from the counts of all ranks ([world, experts]) compute, for every assignment, its row in the receive
 // buffer of the expert's rank (-1 when the buffer of `cap` rows is full), and for this rank row_off[experts_per_rank+1].
 int launchMoePlan(const int* counts_all, const int* ids, const int* pos, int* rows, int* row_off, int world, int rank, int experts,

@@ -162,6 +162,15 @@ class MoEExchange:
         count_launch(2)
         return ids, probs, {"rows": rows, "row_off": row_off, "n_rows": row_off[-1:]}
 
+    def route_backward(self, gate_logits: torch.Tensor, ids: torch.Tensor, dprobs: torch.Tensor) -> torch.Tensor:
+        """Gradient (fp32) of the gate logits from the gradients ``dprobs`` (fp32 [tokens, topk]) of the probabilities of the experts
+        ``ids``: the chain rule through the softmax over all experts."""
+        lg = gate_logits.float().contiguous()
+        out = torch.empty_like(lg)
+        C.moe_route_backward(lg.data_ptr(), ids.data_ptr(), dprobs.data_ptr(), out.data_ptr(), lg.shape[0], self.E, self.K, stream_handle())
+        count_launch()
+        return out
+
     # ---- kernels ----------------------------------------------------------------------------
     def _exchange(self, kind: str, x, ids, rows, probs, out, gate=None, dedupe: bool = False, groups: bool = True) -> None:
         self.epoch += 1
@@ -204,7 +213,7 @@ class MoEExchange:
     def combine_dot(self, g: torch.Tensor, ids: torch.Tensor, plan: Dict[str, torch.Tensor]) -> torch.Tensor:
         """``dot[t, k] = <g[t], y row of assignment (t, k)>`` (fp32 [tokens, topk]): with ``g`` the upstream gradient and
         the expert outputs of the forward pass still in ``self.y``, the gradient of the gate weights."""
-        out = torch.zeros((self.T, self.K), dtype=torch.float32, device="cuda")
+        out = torch.empty((self.T, self.K), dtype=torch.float32, device="cuda")
         self._exchange("combine_dot", g, ids, plan["rows"], None, out)
         return out
 
@@ -217,9 +226,9 @@ class MoEExchange:
         h = grouped_gemm(self.x_bf16, w1, plan["row_off"], d_ff, gelu=True)
         grouped_gemm(h, w2, plan["row_off"], self.H, out=self.y)
 
-    def combine(self, ids: torch.Tensor, probs: torch.Tensor, plan: Dict[str, torch.Tensor], out: Optional[torch.Tensor] = None,
+    def combine(self, ids: torch.Tensor, probs: Optional[torch.Tensor], plan: Dict[str, torch.Tensor], out: Optional[torch.Tensor] = None,
                 grouped: bool = False) -> torch.Tensor:
-        """``out[t] = sum_k probs[t, k] * (expert output of assignment (t, k))``, the rows pulled over NVLink.
+        """``out[t] = sum_k probs[t, k] * (expert output of assignment (t, k))``, the rows pulled over NVLink; without ``probs`` the plain sum.
 
         ``grouped`` (after a dispatch with ``gate=probs``): every rank first adds up, locally, the weighted outputs of
         the assignments that one token has on it, and the token then pulls one row per rank instead of one per expert."""

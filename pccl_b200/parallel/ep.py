@@ -56,11 +56,8 @@ class _MoEFn(torch.autograd.Function):
         grouped_gemm(dh_pre, w1, row_off, H, b_t=True, out=ex.y)
         dw1, dw2 = grouped_wgrad(dh_pre, xr, g, h, row_off)
         # input gradients back to the tokens: a plain sum over the k assignments (the gate weight went out with dout)
-        dx = ex.combine(ids, torch.ones_like(probs), plan)
-        # softmax over all experts, top-k taken: chain rule through the softmax for the selected probabilities
-        pf = torch.softmax(gate_logits.float(), dim=-1)
-        dfull = torch.zeros_like(pf).scatter_(1, ids.long(), dp)
-        dlogits = pf * (dfull - (dfull * pf).sum(-1, keepdim=True))
+        dx = ex.combine(ids, None, plan)
+        dlogits = ex.route_backward(gate_logits, ids, dp)
         return dx, dlogits.to(gate_logits.dtype), dw1, dw2, None
 
 

@@ -1160,3 +1160,24 @@ def test_moe_exchange_group_sizes(native, T, H, E, topk):
         assert ((g[5].double() - products.sum(-1)).abs() <= 1e-5 * products.abs().sum(-1)).all()
     want = (probs.double()[:, :, None] * y.double()[rows]).sum(1)
     assert ((got[0][4].double() - want).abs() <= 2 ** -8 * want.abs() + 1e-4).all()
+
+
+@pytest.mark.parametrize("T,E,topk", [(1, 1, 1), (9, 31, 2), (64, 32, 8), (33, 100, 4), (17, 256, 8), (5, 1024, 8)])
+def test_moe_route_backward(native, T, E, topk):
+    """One to 32 experts per lane, experts that fill no lane count, against autograd in fp64 (fp32 sums of E terms: 1e-5 of the largest
+    gradient); logits far apart and a plain combine without weights."""
+    from pccl_b200.engine import Engine
+    from pccl_b200.ops.moe import MoEExchange
+    torch.manual_seed(E)
+    eng = Engine(0, 1)
+    eng.initEngine("cuda", 640 << 20)
+    ex = MoEExchange(eng, T, 128, E, topk)
+    logits = torch.randn(T, E, device="cuda") * 6
+    ids, probs, plan = ex.route_and_plan(logits)
+    dp = torch.randn(T, topk, device="cuda")
+    l64 = logits.double().requires_grad_(True)
+    (torch.softmax(l64, -1).gather(1, ids.long()) * dp.double()).sum().backward()
+    got = ex.route_backward(logits, ids, dp)
+    assert (got.double() - l64.grad).abs().max().item() <= 1e-5 * max(1e-3, l64.grad.abs().max().item())
+    ex.y.copy_(torch.randn(ex.y.shape, device="cuda"))
+    assert torch.equal(ex.combine(ids, None, plan), ex.combine(ids, torch.ones_like(probs), plan))

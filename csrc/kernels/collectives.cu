@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(512) reduce_scatter_adamw_kernel(const __grid_
 // the GEMM's arithmetic.  A warp takes 4 x 128 parameters at a time, four of each 128 per lane, so that every access of a warp is one
 // stretch of memory; the 16 loads of a trip are out before the first is used (28 KiB per SM).  A bucket of 13.1 M parameters alone: 95 ->
 // 87 us (4.2 TB/s), of 0.26 M 25 -> 10; the training step of GPT-1.3B, 16384 tokens, 133.1 -> 128.9 ms (two CTAs per SM: the same).
-constexpr int kLocalAdamThreads = 128, kLocalAdamTrip = 512;
+constexpr int kLocalAdamThreads = 128, kLocalAdamTrip = 512, kLocalAdamTrips = 4;
 __global__ void __launch_bounds__(kLocalAdamThreads, 6) local_adamw_kernel(const __nv_bfloat16* grads, const AdamArgs O, long long count, float scale) {
   const int lane = threadIdx.x & 31;
   const float one_m_b1 = 1.f - O.b1, one_m_b2 = 1.f - O.b2, decay = 1.f - O.lr * O.wd;
@@ -578,13 +578,24 @@ int launchReduceScatterAdamW(const CollArgs& a, const AdamArgs& o, int blocks, i
   if (blocks < 1) blocks = 1;
   if (blocks > kMaxBlocksPerColl) blocks = kMaxBlocksPerColl;
   if (a.w.world == 1 && a.algo != ALGO_NVLS) {
-    const long long trips = (static_cast<long long>(a.count) + kLocalAdamTrip * (kLocalAdamThreads / 32) - 1) / (kLocalAdamTrip * (kLocalAdamThreads / 32));
-    // One CTA per SM beside the backward pass; four for a bucket above 32 Mi parameters, an embedding or a head, which as a rule is the last
-    // (102.9 M parameters alone: 610 -> 481 us, 6.0 TB/s).
-    const long long most = static_cast<long long>(deviceSmCount()) * (a.count > (32u << 20) ? 4 : 1);
-    if (trips == 0) return 0;
-    local_adamw_kernel<<<static_cast<unsigned>(trips < most ? trips : most), kLocalAdamThreads, 0, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(a.w.heap[a.rank] + a.in_off), o, static_cast<long long>(a.count), a.scale);
+    // One CTA per SM beside the backward pass, in launches of kLocalAdamTrips trips (some 25 us): attention and the norms' backward take
+    // whole SMs, and a CTA that stays for the bucket keeps them from its SM for 300 us (GPT-1.3B: 137.8 -> 135.4 ms on a GPU that ran
+    // slow, on a stream of the backward pass's own priority; 2 or 8 trips the same, 136.1 with a higher priority).  A bucket above 32 Mi
+    // parameters, an embedding or a head, which as a rule is the last, is one launch of four CTAs per SM (102.9 M parameters alone:
+    // 610 -> 481 us, 6.0 TB/s).
+    const long long count = static_cast<long long>(a.count), per_cta = kLocalAdamTrip * (kLocalAdamThreads / 32);
+    const bool last = count > (32ll << 20);
+    const long long sms = deviceSmCount(), part = last ? count : sms * kLocalAdamTrips * per_cta;
+    const __nv_bfloat16* grads = reinterpret_cast<const __nv_bfloat16*>(a.w.heap[a.rank] + a.in_off);
+    for (long long at = 0; at < count; at += part) {
+      const long long n = count - at < part ? count - at : part, trips = (n + per_cta - 1) / per_cta, most = last ? 4 * sms : sms;
+      AdamArgs q = o;
+      q.p += at;
+      q.m += at;
+      q.v += at;
+      q.p_bf16 = static_cast<__nv_bfloat16*>(o.p_bf16) + at;
+      local_adamw_kernel<<<static_cast<unsigned>(trips < most ? trips : most), kLocalAdamThreads, 0, stream>>>(grads + at, q, n, a.scale);
+    }
     return static_cast<int>(cudaGetLastError());
   }
   void* args[] = {const_cast<CollArgs*>(&a), const_cast<AdamArgs*>(&o)};

@@ -84,7 +84,8 @@ class ShardedDataParallel:
         # the persistent GEMM's last CTAs start a full wave late.  (A world of one exchanges nothing and has a kernel of its own,
         # which runs beside the GEMMs and takes no block count.)
         self.comm_blocks = comm_blocks if comm_blocks else (128 if engine.world == 1 else 64)
-        self.comm_stream = torch.cuda.Stream(priority=-1)
+        # A world of one has no peers to keep waiting: its update stands back behind the backward pass's kernels.
+        self.comm_stream = torch.cuda.Stream(priority=-1 if engine.world > 1 else 0)
         self.step_count = 0
         self._plan_schedule(int(bucket_mb * (1 << 20)), schedule, topology)
         self._build_buckets(params, int(bucket_mb * (1 << 20)) // 2)

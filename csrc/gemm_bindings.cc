@@ -99,6 +99,16 @@ void bindGemm(py::module_& m) {
                                  reinterpret_cast<uint32_t*>(status), reinterpret_cast<cudaStream_t>(stream));
     if (err != 0) throw std::runtime_error(std::string("cross_entropy: ") + cudaErrorName(err));
   });
+  m.def("embed_fwd", [](uint64_t ids, uint64_t tok, uint64_t pos, uint64_t out, long long n_ids, int seq, long long vocab, int D, uint64_t stream) {
+    int err = launchEmbedFwd(reinterpret_cast<const long long*>(ids), reinterpret_cast<const void*>(tok), reinterpret_cast<const void*>(pos),
+                             reinterpret_cast<void*>(out), n_ids, seq, vocab, D, reinterpret_cast<cudaStream_t>(stream));
+    if (err != 0) throw std::runtime_error(std::string("embed_fwd: ") + cudaErrorName(err));
+  });
+  m.def("embed_bwd", [](uint64_t dy, uint64_t ids, uint64_t d_tok, uint64_t d_pos, int batch, int seq, long long vocab, int D, bool add_pos, uint64_t stream) {
+    int err = launchEmbedBwd(reinterpret_cast<const void*>(dy), reinterpret_cast<const long long*>(ids), reinterpret_cast<void*>(d_tok),
+                             reinterpret_cast<void*>(d_pos), batch, seq, vocab, D, add_pos, reinterpret_cast<cudaStream_t>(stream));
+    if (err != 0) throw std::runtime_error(std::string("embed_bwd: ") + cudaErrorName(err));
+  });
   m.def("layernorm_fwd", [](uint64_t x, uint64_t delta, uint64_t sum_out, uint64_t g, uint64_t b, uint64_t y, uint64_t mean, uint64_t rstd,
                             long long rows, int D, float eps, uint64_t stream) {
     int err = launchLayerNormFwd(reinterpret_cast<const void*>(x), reinterpret_cast<const void*>(delta), reinterpret_cast<void*>(sum_out),

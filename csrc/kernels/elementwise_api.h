@@ -20,6 +20,16 @@ int launchAdamW(float* p, float* m, float* v, const float* g, void* p_bf16, long
 int launchCrossEntropy(void* logits, const long long* targets, float* loss, long long rows, int vocab, long long ld,
                        float grad_scale, long long ignore_index, uint32_t* status, cudaStream_t stream);
 
+// out[b, t] = tok[ids[b, t]] + pos[t] for bf16 tables tok [vocab, D], pos [>= seq, D] (D % 8 == 0, 16-byte aligned); n_ids = batch * seq,
+// n_ids * D / 8 < 2^31.
+// Negative indices count from the end; one outside the table is a device assertion, as in the index kernels of the framework underneath.
+int launchEmbedFwd(const long long* ids, const void* tok, const void* pos, void* out, long long n_ids, int seq, long long vocab, int D,
+                   cudaStream_t stream);
+// Backward: rows of dy [batch, seq, D] are added to d_tok (bf16 [vocab, D], may be null) and summed over the batch into d_pos (bf16,
+// may be null), written or, with `add_pos`, added.
+int launchEmbedBwd(const void* dy, const long long* ids, void* d_tok, void* d_pos, int batch, int seq, long long vocab, int D, bool add_pos,
+                   cudaStream_t stream);
+
 // LayerNorm over the last dimension D (multiple of 8, <= 8192) of bf16 [rows, D]; mean / rstd are fp32 [rows], or both
 // null where no backward pass follows.
 // With `delta` (bf16 [rows, D], may be null) the norm is taken of s = x + delta and s is stored to `sum_out`:

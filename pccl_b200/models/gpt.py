@@ -17,6 +17,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..nn.block import attn_in, halves_apply, mlp_out
+from ..nn.embedding import token_position
 from ..nn.linear import Embedding, Linear, LinearGelu, _LinearFn, is_plain, mlp, split_qkv
 from ..nn.loss import fused_cross_entropy
 from ..nn.norm import LayerNorm
@@ -115,9 +116,7 @@ class GPT(nn.Module):
             self.lm_head = Linear(cfg.d_model, cfg.vocab_size, bias=False, device=device)
 
     def logits(self, ids: torch.Tensor) -> torch.Tensor:
-        B, T = ids.shape
-        pos = torch.arange(T, device=ids.device)
-        x = self.wte(ids) + self.wpe(pos)[None]
+        x = token_position(ids, self.wte, self.wpe)
         delta, prev_bias = None, None
         for blk in self.blocks:
             x, delta, prev_bias = blk(x, delta, prev_bias)

@@ -674,3 +674,51 @@ def test_block_halves_are_their_layers(batch, seq, what, monkeypatch):
             assert torch.allclose(a.float(), b.float(), rtol=2e-2, atol=1e-4)
         else:
             assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,T,D,V,extra,bucket", [(1, 1, 8, 3, 0, "none"), (3, 7, 40, 5, 4, "none"), (5, 33, 264, 1001, 1, "new"), (32, 3, 768, 50, 0, "added to"),
+                                                  (4, 129, 2048, 517, 2, "new"), (33, 5, 64, 9, 0, "none"), (2, 9, 64, 9, 3, "tok frozen"),
+                                                  (2, 9, 64, 9, 3, "pos frozen")])
+def test_token_and_position_embedding(B, T, D, V, extra, bucket):
+    """One kernel per direction against the layers' own calls: the values are the same, the positions' gradient is a sum in fp32 rounded
+    once, the tokens' a sum of bf16 values in no fixed order."""
+    from pccl_b200.nn.embedding import _fused, token_position
+    from pccl_b200.nn.linear import Embedding
+    torch.manual_seed(B + T)
+    wte, wpe = Embedding(V, D, device="cuda"), Embedding(T + extra, D, device="cuda")
+    ids = torch.randint(-V, V, (B, T), device="cuda")               # negative ones count from the end
+    assert _fused(ids, wte, wpe) == (B <= 32)
+    with torch.no_grad():
+        want = wte.weight[ids] + wpe.weight[:T][None]
+        assert torch.equal(token_position(ids, wte, wpe), want)
+    if bucket == "none" and B > 32:
+        ids = ids % V                                               # the layers' own backward takes no negative index
+    before = [torch.zeros_like(m.weight) for m in (wte, wpe)]
+    if bucket in ("new", "added to"):
+        for m, b in zip((wte, wpe), before):
+            m.weight.main_grad = torch.randn_like(m.weight)
+            m.weight._pccl_written = bucket == "added to"
+            if bucket == "added to":
+                b.copy_(m.weight.main_grad)
+    wte.weight.requires_grad_(bucket != "tok frozen")
+    wpe.weight.requires_grad_(bucket != "pos frozen")
+    y = token_position(ids, wte, wpe)
+    assert torch.equal(y, wte.weight[ids] + wpe.weight[:T][None])
+    dy = torch.randn(T, B, D, device="cuda").bfloat16().transpose(0, 1)      # not as the kernel reads it
+    y.backward(dy)
+    pos = dy.float().sum(0).bfloat16()
+    want_pos = before[1].clone()
+    want_pos[:T] = want_pos[:T] + pos if bucket == "added to" else pos
+    tok, mag = before[0].double(), before[0].double().abs()
+    tok.index_add_(0, ids.flatten() % V, dy.reshape(-1, D).double())
+    mag.index_add_(0, ids.flatten() % V, dy.reshape(-1, D).double().abs())
+    n = torch.bincount(ids.flatten() % V, minlength=V)[:, None]
+    for m, frozen in ((wte, "tok frozen"), (wpe, "pos frozen")):
+        g = getattr(m.weight, "main_grad", None) if bucket in ("new", "added to") else m.weight.grad
+        if bucket == frozen:
+            assert g is None
+        elif m is wte:          # n additions, each off by 2^-8 (half a unit in the last place of 8 bits) of a partial sum, which earlier ones moved
+            assert ((g.double() - tok).abs() <= n * 2.0 ** -8 * (1 + 2.0 ** -8) ** n * mag).all()
+        else:                   # B fp32 additions in another order may round to the other neighbour: one unit (2^-7) of the sum, one of the total
+            assert ((g.float() - want_pos.float()).abs() <= 2.0 ** -7 * ((g - before[1]).float().abs() + g.float().abs()) + B * 2.0 ** -22).all()

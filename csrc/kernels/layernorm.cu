@@ -112,21 +112,103 @@ __global__ void __launch_bounds__(256, VPT == 4 ? 4 : 1) ln_fwd_kernel(const __n
   }
 }
 
-// Backward.  A group of `gw` warps owns a row -- as many as cover it with one 16-byte vector per thread and trip (VPT trips; one
-// up to D = 2048) -- and takes R rows at a time: R x VPT x 3 vectors are in flight per thread, and the row statistics of all R
-// rows cross the group in one exchange.  The next R rows are fetched (AHEAD) while these are worked on, as far as that goes without
-// spills, which cost far more than the fetch brings: two vectors per row in the plain form, three and the column sums of dx in the
-// EXTRA one.  A thread keeps the same columns for all of its rows, so the column sums (dgamma,
-// dbeta, bias gradient) stay in registers; the CTA's groups add theirs up at the end and write one partial row per array.
-// Times, us, cold L2 (one warp per row with its sums in shared memory for D = 256, 512, 1024 and 2048, a CTA per row for the rest
-// -> now; in brackets three rows on two CTAs per SM without the fetch ahead): EXTRA 16384 x 2048
-// 77 -> 64 [77], 16384 x 1024 44 -> 39 [48], 16384 x 256 28 -> 17 [20], 2331 x 768 32 -> 15 [17], 8192 x 4096 136 -> 64 [83], 4096 x 8192
-// 220 -> 83; plain 16384 x 2048 64 -> 52 [73] (3.9 TB/s), 16384 x 1024 40 -> 32 [44], 8192 x 4096 101 -> 52 [79], 4096 x 8192 153 -> 56 [81].
-template <int VPT, int R, bool EXTRA, bool AHEAD, int CTAS>
-__global__ void __launch_bounds__(256, CTAS) ln_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* gamma,
+// Sums of N values (a power of two) over a group of `gw` warps (those from `first` on); every thread gets them.  The lanes of a warp halve
+// the values among them as they add up, so eight values take 9 shuffles where a butterfly each takes 40, and a warp reads each word of
+// `stat` ([warp][N]) once where every thread did.  `bar` is the group's barrier.
+template <int N>
+__device__ __forceinline__ void group_sum(float (&v)[N], float (*stat)[N], int warp, int lane, int gw, int first, int bar) {
+  int idx = 0;
+#pragma unroll
+  for (int n = N / 2, o = 1; n > 0; n /= 2, o *= 2) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+    idx += up ? n : 0;
+  }
+  float t = v[0];
+#pragma unroll
+  for (int o = N; o < 32; o *= 2) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (gw == 1) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      int from = 0;                                          // the lane below N whose idx is i
+#pragma unroll
+      for (int n = N / 2, o = 1; n > 0; n /= 2, o *= 2) from += i & n ? o : 0;
+      v[i] = __shfl_sync(0xffffffffu, t, from);
+    }
+    return;
+  }
+  if (lane < N) stat[warp][idx] = t;
+  asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(gw * 32) : "memory");
+  t = 0.f;
+  for (int w = lane / N; w < gw; w += 32 / N) t += stat[first + w][lane & (N - 1)];
+#pragma unroll
+  for (int o = N; o < 32; o *= 2) t += __shfl_xor_sync(0xffffffffu, t, o);
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = __shfl_sync(0xffffffffu, t, i);
+}
+
+// Two fp32 values in one 64-bit register pair: one instruction adds or multiplies both.
+__device__ __forceinline__ uint64_t pair(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 split(uint64_t p) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t pair_of(uint32_t bf16x2) {
+  return pair(__uint_as_float(bf16x2 << 16), __uint_as_float(bf16x2 & 0xffff0000u));
+}
+__device__ __forceinline__ uint32_t bf16x2_of(uint64_t p) {
+  const float2 f = split(p);
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(f.y), "f"(f.x));
+  return r;
+}
+
+// 16 bytes to shared memory behind the thread's back; only the first `n` of them are read, the rest become zeros.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int n) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src), "r"(n) : "memory");
+}
+
+// Backward.  A group of `gw` warps owns a row -- as many as cover it with VPT 16-byte vectors per thread (one up to D = 2048) -- and takes
+// R rows at a time: R x VPT x 3 vectors are in flight per thread, and the row statistics of all R rows cross the group in one exchange.
+// The next R rows are fetched into registers while these are worked on (STAGES = 0), as far as that goes without spills, which cost
+// far more than the fetch brings.  Beyond D = 2048 the EXTRA form has no registers for that: its rows come through a ring in shared
+// memory, STAGES - 1 trips ahead.  A thread copies only what it reads itself, so no barrier guards the ring, and a slot is filled again
+// one trip after its values were used.  (Where the registers hold the next rows a ring brings nothing: 16384 x 2048 52 with either.)
+// A thread keeps the same columns for all of its rows, so the column sums (dgamma, dbeta, bias gradient) stay in registers; the CTA's
+// groups add theirs up at the end and write one partial row per array.
+// With eight warps per SM the instructions count beside the memory: the arithmetic is on pairs (f32x2) and the exchange is group_sum.
+// Times, us, 20 calls in a row (a butterfly per sum, one value per instruction, no ring -> now): EXTRA 16384 x 2048 57.7 -> 51.7 (5.2 TB/s),
+// 16384 x 1536 57.3 -> 46.0, 16384 x 512 18.9 -> 15.4, 2331 x 768 9.5 -> 8.6, 20000 x 2560 115 -> 90, 8192 x 4096 57.7 -> 55.1, 4096 x 8192
+// 74.3 -> 60.4, 256 x 8192 15.2 -> 16.1; plain 16384 x 2048 46.6 -> 44.1, 16384 x 1536 40.2 -> 37.7, 8192 x 4096 44.7 -> 43.9.
+template <int VPT, int R, bool EXTRA, int CTAS, int STAGES, int THREADS>
+__global__ void __launch_bounds__(THREADS, CTAS) ln_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* gamma,
                                                            const float* mean, const float* rstd, const __nv_bfloat16* dres, __nv_bfloat16* dx,
                                                            float* part_g, float* part_b, float* part_c, long long rows, int D, int gw) {
-  __shared__ float2 stat[2][8][R];                          // [parity][warp][row]: partial sums of a warp
+  __shared__ float stat[2][THREADS / 32][2 * R];                       // [parity][warp][value]: partial sums of a warp
   extern __shared__ __align__(16) float group_sums[];       // [groups][arrays][D], with more than one group
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = warp / gw, groups = (blockDim.x >> 5) / gw, tid = threadIdx.x - group * gw * 32;
@@ -135,15 +217,15 @@ __global__ void __launch_bounds__(256, CTAS) ln_bwd_kernel(const __nv_bfloat16* 
   dev::pdl_wait();
   const Vec16 zero{{0u, 0u, 0u, 0u}};
   Vec16 g[VPT];
-  float ag[VPT][8], ab[VPT][8], ac[EXTRA ? VPT : 1][8];
+  uint64_t ag[VPT][4], ab[VPT][4], ac[EXTRA ? VPT : 1][4];
 #pragma unroll
   for (int j = 0; j < VPT; ++j) {
     g[j] = tid + j * width < nvec ? ld16(gamma + (tid + j * width) * 8) : zero;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      ag[j][k] = 0.f;
-      ab[j][k] = 0.f;
-      if (EXTRA) ac[EXTRA ? j : 0][k] = 0.f;
+    for (int k = 0; k < 4; ++k) {
+      ag[j][k] = 0;
+      ab[j][k] = 0;
+      if (EXTRA) ac[EXTRA ? j : 0][k] = 0;
     }
   }
   const float inv_d = 1.0f / D;
@@ -169,80 +251,107 @@ __global__ void __launch_bounds__(256, CTAS) ln_bwd_kernel(const __nv_bfloat16* 
   };
   long long row0 = (static_cast<long long>(blockIdx.x) * groups + group) * R;
   Rows cur;
-  if (AHEAD) load(cur, row0);
-  int parity = 0;
-  for (; row0 < rows; row0 += step, parity ^= 1) {
-    if (!AHEAD) load(cur, row0);
-    float s1[R], s2[R];
+  constexpr int ARR = EXTRA ? 3 : 2, SLOTS = STAGES ? STAGES : 1;
+  Vec16* ring = reinterpret_cast<Vec16*>(group_sums);       // [STAGES][R][ARR][VPT][THREADS]
+  auto slot_of = [&](int slot, int r, int a, int j) { return ring + (((slot * R + r) * ARR + a) * VPT + j) * THREADS + threadIdx.x; };
+  auto fetch = [&](int slot, long long row0) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      s1[r] = 0.f;
-      s2[r] = 0.f;
 #pragma unroll
       for (int j = 0; j < VPT; ++j) {
-        float xf[8], df[8], gf[8];
-        unpack<DT_BF16>(cur.x[r][j], xf);
-        unpack<DT_BF16>(cur.d[r][j], df);
-        unpack<DT_BF16>(g[j], gf);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float dg = df[k] * gf[k];
-          s1[r] += dg;
-          s2[r] += dg * ((xf[k] - cur.mu[r]) * cur.rs[r]);
-        }
+        const bool in = row0 + r < rows && tid + j * width < nvec;
+        const long long at = in ? (row0 + r) * D + (tid + j * width) * 8 : 0;
+        const int n = in ? 16 : 0;                          // nothing is read where this is 0, the slot becomes zeros
+        cp_async16(slot_of(slot, r, 0, j), x + at, n);
+        cp_async16(slot_of(slot, r, 1, j), dy + at, n);
+        if (EXTRA) cp_async16(slot_of(slot, r, ARR - 1, j), dres ? dres + at : x, dres ? n : 0);
       }
     }
-    Rows next;
-    if (AHEAD) load(next, row0 + step);   // on its way behind the exchange, the arithmetic and the stores
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float mu_next[R], rs_next[R];
+  auto stats = [&](long long row0) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        s1[r] += __shfl_xor_sync(0xffffffffu, s1[r], o);
-        s2[r] += __shfl_xor_sync(0xffffffffu, s2[r], o);
-      }
+      mu_next[r] = row0 + r < rows ? mean[row0 + r] : 0.f;
+      rs_next[r] = row0 + r < rows ? rstd[row0 + r] : 0.f;
     }
-    if (gw > 1) {
-      if (lane == 0) {
+  };
+  if (STAGES) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) stat[parity][warp][r] = make_float2(s1[r], s2[r]);
-      }
-      // the other parity's slots are not written again before every warp of the group has passed this barrier once more
-      asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(width) : "memory");
+    for (int i = 0; i < STAGES - 1; ++i) fetch(i, row0 + i * step);
+    stats(row0);
+  } else {
+    load(cur, row0);
+  }
+  int parity = 0, slot = 0;
+  for (; row0 < rows; row0 += step, parity ^= 1, slot = slot + 1 == SLOTS ? 0 : slot + 1) {
+    if (STAGES) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(STAGES > 1 ? STAGES - 2 : 0) : "memory");
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        s1[r] = 0.f;
-        s2[r] = 0.f;
-        for (int w = 0; w < gw; ++w) {
-          const float2 p = stat[parity][group * gw + w][r];
-          s1[r] += p.x;
-          s2[r] += p.y;
+        cur.mu[r] = mu_next[r];
+        cur.rs[r] = rs_next[r];
+#pragma unroll
+        for (int j = 0; j < VPT; ++j) {
+          cur.x[r][j] = *slot_of(slot, r, 0, j);
+          cur.d[r][j] = *slot_of(slot, r, 1, j);
+          if (EXTRA) cur.r[EXTRA ? r : 0][j] = *slot_of(slot, r, ARR - 1, j);
         }
       }
+      fetch(slot == 0 ? SLOTS - 1 : slot - 1, row0 + (STAGES - 1) * step);     // the slot of the trip before
+      stats(row0 + step);
     }
+    float sums[2 * R];                     // per row: of dy * gamma, and of that times the normalised x
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const float m1 = s1[r] * inv_d, m2 = s2[r] * inv_d;
+      uint64_t s1 = 0, s2 = 0;
+      const uint64_t nmu = pair(-cur.mu[r], -cur.mu[r]), rs = pair(cur.rs[r], cur.rs[r]);
 #pragma unroll
       for (int j = 0; j < VPT; ++j) {
-        float xf[8], df[8], gf[8], rf[8], of[8];
-        unpack<DT_BF16>(cur.x[r][j], xf);
-        unpack<DT_BF16>(cur.d[r][j], df);
-        unpack<DT_BF16>(g[j], gf);
-        if (EXTRA) unpack<DT_BF16>(cur.r[EXTRA ? r : 0][j], rf);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float xh = (xf[k] - cur.mu[r]) * cur.rs[r];
-          of[k] = cur.rs[r] * (df[k] * gf[k] - m1 - xh * m2);
-          if (EXTRA) of[k] += rf[k];
-          ag[j][k] += df[k] * xh;
-          ab[j][k] += df[k];
-          if (EXTRA) ac[EXTRA ? j : 0][k] += of[k];
+        for (int k = 0; k < 4; ++k) {
+          const uint64_t dg = mul2(pair_of(cur.d[r][j].w[k]), pair_of(g[j].w[k])), xh = mul2(add2(pair_of(cur.x[r][j].w[k]), nmu), rs);
+          s1 = add2(s1, dg);
+          s2 = fma2(dg, xh, s2);
         }
-        if (row0 + r < rows && tid + j * width < nvec) st16(dx + (row0 + r) * D + (tid + j * width) * 8, pack<DT_BF16>(of));
+      }
+      sums[2 * r] = split(s1).x + split(s1).y;
+      sums[2 * r + 1] = split(s2).x + split(s2).y;
+    }
+    Rows next;
+    if (!STAGES) load(next, row0 + step);  // on its way behind the exchange, the arithmetic and the stores
+    // the other parity's slots are not written again before every warp of the group has passed this barrier once more
+    group_sum<2 * R>(sums, stat[parity], warp, lane, gw, group * gw, group + 1);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float m1 = sums[2 * r] * inv_d, m2 = sums[2 * r + 1] * inv_d;
+      const uint64_t nm1 = pair(-m1, -m1), nm2 = pair(-m2, -m2), nmu = pair(-cur.mu[r], -cur.mu[r]), rs = pair(cur.rs[r], cur.rs[r]);
+#pragma unroll
+      for (int j = 0; j < VPT; ++j) {
+        Vec16 out;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint64_t d = pair_of(cur.d[r][j].w[k]), xh = mul2(add2(pair_of(cur.x[r][j].w[k]), nmu), rs);
+          uint64_t o = fma2(xh, nm2, fma2(d, pair_of(g[j].w[k]), nm1));
+          if (EXTRA) {
+            o = fma2(o, rs, pair_of(cur.r[EXTRA ? r : 0][j].w[k]));
+            ac[EXTRA ? j : 0][k] = add2(ac[EXTRA ? j : 0][k], o);
+          } else {
+            o = mul2(o, rs);
+          }
+          ag[j][k] = fma2(d, xh, ag[j][k]);
+          ab[j][k] = add2(ab[j][k], d);
+          out.w[k] = bf16x2_of(o);
+        }
+        if (row0 + r < rows && tid + j * width < nvec) st16(dx + (row0 + r) * D + (tid + j * width) * 8, out);
       }
     }
-    if (AHEAD) cur = next;
+    if (!STAGES) cur = next;
+  }
+  if (STAGES) {
+    asm volatile("cp.async.wait_all;" ::: "memory");        // the last trips fetched zeros
+    __syncthreads();
   }
   const int arrays = EXTRA && part_c ? 3 : 2;
 #pragma unroll
@@ -252,11 +361,11 @@ __global__ void __launch_bounds__(256, CTAS) ln_bwd_kernel(const __nv_bfloat16* 
 #pragma unroll
     for (int a = 0; a < (EXTRA ? 3 : 2); ++a) {
       if (a >= arrays) continue;
-      const float* f = a == 0 ? ag[j] : a == 1 ? ab[j] : ac[EXTRA ? j : 0];
+      const uint64_t* f = a == 0 ? ag[j] : a == 1 ? ab[j] : ac[EXTRA ? j : 0];
       float* dst = groups > 1 ? group_sums + (group * 3 + a) * D + v * 8
                               : (a == 0 ? part_g : a == 1 ? part_b : part_c) + static_cast<long long>(blockIdx.x) * D + v * 8;
-      *reinterpret_cast<float4*>(dst) = make_float4(f[0], f[1], f[2], f[3]);
-      *reinterpret_cast<float4*>(dst + 4) = make_float4(f[4], f[5], f[6], f[7]);
+      *reinterpret_cast<float4*>(dst) = make_float4(split(f[0]).x, split(f[0]).y, split(f[1]).x, split(f[1]).y);
+      *reinterpret_cast<float4*>(dst + 4) = make_float4(split(f[2]).x, split(f[2]).y, split(f[3]).x, split(f[3]).y);
     }
   }
   if (groups > 1) {
@@ -450,24 +559,30 @@ int launchLayerNormBwd(const void* dy, const void* x, const void* gamma, const f
   float* pb = partials + static_cast<long long>(most) * D;
   float* pc = dcolsum ? partials + 2ll * most * D : nullptr;
   int nparts = 0;
-  // VPT vectors per thread, R rows per trip, `sms` CTAs resident per SM
-  auto go = [&](auto kern, int vpt, int r, int sms) {
-    const int gw = (D / 8 + 32 * vpt - 1) / (32 * vpt), groups = 8 / gw;
+  // VPT vectors per thread, R rows per trip, `sms` CTAs resident per SM, a ring of `slots` bytes
+  auto go = [&](auto kern, int vpt, int r, int sms, int threads, size_t slots) {
+    const int gw = (D / 8 + 32 * vpt - 1) / (32 * vpt), groups = threads / 32 / gw;
     const long long want = (rows + static_cast<long long>(groups) * r - 1) / (static_cast<long long>(groups) * r);
     const int limit = deviceSmCount() * sms < most ? deviceSmCount() * sms : most;
     nparts = static_cast<int>(want < limit ? want : limit);
-    const size_t smem = groups > 1 ? static_cast<size_t>(groups) * 3 * D * sizeof(float) : 0;         // at most 24 KiB
-    return static_cast<int>(launchOverlapped(kern, dim3(nparts), dim3(groups * gw * 32), smem, stream, 1, static_cast<const __nv_bfloat16*>(dy),
-                                             static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma), mean, rstd,
-                                             static_cast<const __nv_bfloat16*>(dres), static_cast<__nv_bfloat16*>(dx), pg, pb, pc, rows, D, gw));
+    const size_t sums = groups > 1 ? static_cast<size_t>(groups) * 3 * D * sizeof(float) : 0;         // at most 24 KiB per 256 threads
+    if (slots) {
+      const cudaError_t set = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(slots));
+      if (set != cudaSuccess) return static_cast<int>(set);
+    }
+    return static_cast<int>(launchOverlapped(kern, dim3(nparts), dim3(groups * gw * 32), slots > sums ? slots : sums, stream, 1,
+                                             static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
+                                             static_cast<const __nv_bfloat16*>(gamma), mean, rstd, static_cast<const __nv_bfloat16*>(dres),
+                                             static_cast<__nv_bfloat16*>(dx), pg, pb, pc, rows, D, gw));
   };
+  constexpr size_t kRing = 192 * 1024;    // four stages of two rows of up to 4096 values and three arrays, or of one row of up to 8192
   int e;
   if (dres || dcolsum)
-    e = D <= 2048 ? go(ln_bwd_kernel<1, 4, true, true, 1>, 1, 4, 1) : D <= 4096 ? go(ln_bwd_kernel<2, 2, true, true, 1>, 2, 2, 1)
-                                                                                : go(ln_bwd_kernel<4, 1, true, false, 1>, 4, 1, 1);
+    e = D <= 2048 ? go(ln_bwd_kernel<1, 4, true, 1, 0, 256>, 1, 4, 1, 256, 0) : D <= 4096 ? go(ln_bwd_kernel<1, 2, true, 1, 4, 512>, 1, 2, 1, 512, kRing)
+                                                                                        : go(ln_bwd_kernel<4, 1, true, 1, 4, 256>, 4, 1, 1, 256, kRing);
   else
-    e = D <= 2048 ? go(ln_bwd_kernel<1, 2, false, true, 2>, 1, 2, 2) : D <= 4096 ? go(ln_bwd_kernel<2, 2, false, true, 1>, 2, 2, 1)
-                                                                                 : go(ln_bwd_kernel<4, 1, false, true, 1>, 4, 1, 1);
+    e = D <= 2048 ? go(ln_bwd_kernel<1, 2, false, 2, 0, 256>, 1, 2, 2, 256, 0) : D <= 4096 ? go(ln_bwd_kernel<2, 2, false, 1, 0, 256>, 2, 2, 1, 256, 0)
+                                                                                         : go(ln_bwd_kernel<4, 1, false, 1, 0, 256>, 4, 1, 1, 256, 0);
   if (e != 0) return e;
   ReduceJob job{{pg, pb, pc}, {static_cast<__nv_bfloat16*>(dgamma), static_cast<__nv_bfloat16*>(dbeta), static_cast<__nv_bfloat16*>(dcolsum)}, nullptr};
   return static_cast<int>(launchOverlapped(partial_rows_reduce_kernel, dim3((D + 31) / 32, dcolsum ? 3 : 2), dim3(1024), 0, stream, 1, job, nparts, D));

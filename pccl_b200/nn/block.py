@@ -117,16 +117,17 @@ class _AttnInFn(torch.autograd.Function):
         return dxv, (dxv if ctx.summed else None), dg, dbeta, (_deliver(ctx.prev_bias, dc) if dc is not None else None), dw, db, None, None
 
 
-def _mlp_out_forward(a, x, wp, bp, gamma, beta, w1, b1, w2, b2, eps, want_stats):
+def _mlp_out_forward(a, x, wp, bp, gamma, beta, w1, b1, w2, b2, eps, for_backward):
     B, heads, T, hd = a.shape
     D, F = heads * hd, w1.shape[0]
     a2, x2 = _as_operand(a.transpose(1, 2).reshape(B * T, D)), _rows(x, D)
     rows = B * T
     d, s, h, out = torch.empty_like(x2), torch.empty_like(x2), torch.empty_like(x2), torch.empty_like(x2)
-    pre, act = x2.new_empty((rows, F)), x2.new_empty((rows, F))
-    stats = x2.new_empty((2, rows), dtype=torch.float32) if want_stats else None
+    act = x2.new_empty((rows, F))
+    pre = torch.empty_like(act) if for_backward else None
+    stats = x2.new_empty((2, rows), dtype=torch.float32) if for_backward else None
     C.block_mlp_out(a2.data_ptr(), a2.stride(0), wp.data_ptr(), bp.data_ptr(), d.data_ptr(), x2.data_ptr(), s.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
-                    eps, h.data_ptr(), 0 if stats is None else stats.data_ptr(), w1.data_ptr(), b1.data_ptr(), pre.data_ptr(), act.data_ptr(), w2.data_ptr(),
+                    eps, h.data_ptr(), 0 if stats is None else stats.data_ptr(), w1.data_ptr(), b1.data_ptr(), 0 if pre is None else pre.data_ptr(), act.data_ptr(), w2.data_ptr(),
                     b2.data_ptr(), out.data_ptr(), rows, D, F, _form(rows), _status_of(x2), stream_handle())
     count_launch(4)
     return a2, s, h, stats, pre, act, out

@@ -269,8 +269,7 @@ def mlp(x: torch.Tensor, fc1: "Linear", fc2: "Linear", defer_fc2_bias_grad: bool
     if records_graph():
         return _MlpFn.apply(x, w1, fc1.bias, w2, fc2.bias, defer_fc2_bias_grad)
     x2 = _as_operand(x)
-    act = x2.new_empty((x2.shape[0], w1.shape[0]))
-    gemm(x2, w1, bias=fc1.bias, gelu_out=act)
+    act = gemm(x2, w1, bias=fc1.bias, gelu_inplace=True)    # no backward pass: the pre-activation is not kept
     return gemm(act, w2, bias=fc2.bias).view(*x.shape[:-1], w2.shape[0])
 
 

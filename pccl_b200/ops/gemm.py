@@ -91,10 +91,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
          out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.bfloat16,
          bias: Optional[torch.Tensor] = None, gelu_out: Optional[torch.Tensor] = None,
          accumulate: bool = False, sms: int = 0, pair: Optional[bool] = None,
-         residual: Optional[torch.Tensor] = None, row_stores: bool = False) -> torch.Tensor:
+         residual: Optional[torch.Tensor] = None, row_stores: bool = False, gelu_inplace: bool = False) -> torch.Tensor:
     """``out = op(a) @ op(b)`` with ``op(a) = a.T if a_t else a`` (a: [M,K] or [K,M]) and
     ``op(b) = b if b_t else b.T`` (b: [N,K], or [K,N] when ``b_t``).  So the default is the linear
-    layer form ``a @ b.T``.  ``bias`` (bf16 [N]) is added; ``gelu_out`` receives gelu_tanh(out).
+    layer form ``a @ b.T``.  ``bias`` (bf16 [N]) is added; ``gelu_out`` receives gelu_tanh(out);
+    with ``gelu_inplace`` ``out`` itself does, and the pre-activation is not kept.
     ``pair`` selects the CTA-pair kernel (cta_group::2, tiles of 256 rows); default: up to 128 rows of a K-major ``a`` take
     the few-row kernel, more the CTA pairs (PCCL_GEMM_PAIR).
     ``residual`` (bf16, out's shape and strides) is added in the epilogue: ``out = a @ b.T + bias + residual``.
@@ -134,6 +135,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
         flags |= C.GEMM_BIAS
         bias_ptr = bias.data_ptr()
     d2 = 0
+    if gelu_inplace:
+        if gelu_out is not None or accumulate:
+            raise ValueError("gemm: gelu_inplace excludes gelu_out and accumulate")
+        flags |= C.GEMM_GELU_INPLACE
     if gelu_out is not None:
         if gelu_out.shape != out.shape or gelu_out.stride() != out.stride() or gelu_out.dtype != torch.bfloat16:
             raise ValueError("gemm: gelu_out must match out")

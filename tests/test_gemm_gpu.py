@@ -477,3 +477,18 @@ def test_mx8_cta_pairs(M, N, K, width):
     assert ((got.double() - full - old.double()).abs() <= 2 ** -8 * (full + old.double()).abs() + 1e-4).all()
     want = torch.nn.functional.gelu(full, approximate="tanh")
     assert ((act.double() - want).abs() <= 2 ** -8 * want.abs() + 1.5e-3 * full.abs() + 1e-4).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 64), (17, 200, 72), (128, 512, 256), (129, 264, 64), (130, 200, 136), (777, 3072, 768), (1531, 1000, 264)])
+@pytest.mark.parametrize("pair", [None, False, True])
+def test_gelu_in_place_is_the_side_output(M, N, K, pair):
+    """With ``gelu_inplace`` the output is what ``gelu_out`` gets, bit for bit, whichever kernel the row count picks."""
+    from pccl_b200.ops.gemm import check_status, gemm
+    torch.manual_seed(M)
+    a, b, bias = (torch.randn(*s, device="cuda").bfloat16() for s in ((M, K), (N, K), (N,)))
+    act = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    gemm(a, b, bias=bias, gelu_out=act, pair=pair)
+    assert torch.equal(gemm(a, b, bias=bias, gelu_inplace=True, pair=pair), act)
+    check_status()
+    with pytest.raises(ValueError):
+        gemm(a, b, bias=bias, gelu_out=act, gelu_inplace=True)

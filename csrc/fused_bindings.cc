@@ -106,6 +106,11 @@ void bindFused(py::module_& m) {
                            reinterpret_cast<cudaStream_t>(stream)), "moe_dequant");
   }, py::arg("q"), py::arg("scales"), py::arg("out"), py::arg("n_rows"), py::arg("max_rows"), py::arg("hidden"), py::arg("stream"),
      py::arg("alias") = 0);
+  m.def("moe_expand", [](uint64_t x, uint64_t ids, uint64_t rows, uint64_t probs, uint64_t out, int tokens, int topk, int hidden, uint64_t stream) {
+    check(launchMoeExpand(reinterpret_cast<const void*>(x), reinterpret_cast<const int*>(ids), reinterpret_cast<const int*>(rows),
+                          reinterpret_cast<const float*>(probs), reinterpret_cast<void*>(out), tokens, topk, hidden,
+                          reinterpret_cast<cudaStream_t>(stream)), "moe_expand");
+  });
   m.def("moe_reduce_groups", [](uint64_t y, uint64_t z, uint64_t alias, uint64_t groups, uint64_t n_rows, int max_rows, int hidden,
                                 uint64_t stream) {
     check(launchMoeReduceGroups(reinterpret_cast<const void*>(y), reinterpret_cast<void*>(z), reinterpret_cast<const int*>(alias),

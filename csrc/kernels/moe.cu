@@ -380,6 +380,58 @@ __global__ void __launch_bounds__(256) moe_dequant_kernel(const uint8_t* q, cons
   }
 }
 
+// Dispatch and conversion in one, for a world of one: nothing travels, so the rows that the experts read are written at once, without
+// the e4m3 rows and scales in between (the values are those: quantised and converted back).  A warp takes 256 values of a token, 16 lanes a
+// block of 128, with nothing kept from one to the next: the many short chains keep the memory busy better than longer ones (four vectors
+// per thread 89 us, one 85), and a store is 512 consecutive bytes of one row.  The stores bound it.  Times, us, dispatch and conversion
+// -> this (scaled by gate weights in brackets): 4096 x 7168, top-8 131 -> 85, 5.5 TB/s stored [183 -> 84]; 64 x 7168 10.8 -> 3.7;
+// 2001 x 2048, top-4 14.1 -> 7.4 [17.4 -> 7.9]; 512 x 4096, top-2 15.0 -> 4.1; 128 x 1024, top-2 5.5 -> 2.5.
+__global__ void __launch_bounds__(256) moe_expand_kernel(const __nv_bfloat16* x, const int* ids, const int* dst_rows, const float* probs, __nv_bfloat16* out,
+                                                         int tokens, int topk, int hidden) {
+  dev::pdl_launch();
+  dev::pdl_wait();
+  const int nvec = hidden >> 3, chunks = (nvec + 31) >> 5, lane = threadIdx.x & 31;
+  const long long item = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  const int t = static_cast<int>(item / chunks), v = static_cast<int>(item % chunks) * 32 + lane;
+  if (t >= tokens) return;
+  const bool in = v < nvec;                                 // the last chunk may be one block
+  float f[16], amax = 0.f;
+  if (in) unpack<DT_BF16>(ld16(x + static_cast<long long>(t) * hidden + v * 8), f);
+  int row_l = -1;                                           // negative: dropped (receive buffer full), or no assignment of this lane
+  float p_l = 1.f;
+  if (lane < topk) {
+    const long long at = static_cast<long long>(t) * topk + lane;
+    if (ids[at] >= 0) row_l = dst_rows[at];
+    if (probs) p_l = probs[at];
+  }
+  if (in) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(f[k]));
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  const float scale = amax > 0.f ? amax * (1.0f / 448.0f) : 1.0f;
+  if (in) {
+    const uint2 q = quant8(f, 1.0f / scale);
+    unpack<DT_FP8_E4M3>(Vec16{{q.x, q.y, 0u, 0u}}, f);
+  }
+  Vec16 o;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int row = __shfl_sync(0xffffffffu, row_l, k);
+    const float p = __shfl_sync(0xffffffffu, p_l, k);
+    if (!in) continue;
+    if (k == 0 || probs) {
+      const float s = probs ? scale * p : scale;
+      float g[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) g[j] = f[j] * s;
+      o = pack<DT_BF16>(g);
+    }
+    if (row >= 0) st16(out + static_cast<long long>(row) * hidden + v * 8, o);
+  }
+}
+
 // z[r] = sum_j weight_j * y[row_j] over the group record of primary row r, for groups of two or more (a group of one stays in y
 // and gets its weight in the combine).  Element-wise over the row, accumulated in fp32.
 __global__ void __launch_bounds__(256) moe_reduce_groups_kernel(const __nv_bfloat16* y, __nv_bfloat16* z,
@@ -1036,6 +1088,15 @@ int launchMoeDequant(const void* q, const float* scales, void* out, const int* n
   if (hidden % 128) return static_cast<int>(cudaErrorInvalidValue);
   return static_cast<int>(launchOverlapped(moe_dequant_kernel, dim3(deviceSmCount() * 8), dim3(256), 0, stream, 1, static_cast<const uint8_t*>(q),
                                            scales, static_cast<__nv_bfloat16*>(out), n_rows, max_rows, hidden, alias));
+}
+
+int launchMoeExpand(const void* x, const int* ids, const int* dst_rows, const float* probs, void* out, int tokens, int topk, int hidden,
+                    cudaStream_t stream) {
+  if (tokens <= 0) return 0;
+  if (hidden % 128 || topk < 1 || topk > 8) return static_cast<int>(cudaErrorInvalidValue);
+  const long long items = static_cast<long long>(tokens) * ((hidden / 8 + 31) / 32);
+  return static_cast<int>(launchOverlapped(moe_expand_kernel, dim3(static_cast<unsigned>((items + 7) / 8)), dim3(256), 0, stream, 1,
+                                           static_cast<const __nv_bfloat16*>(x), ids, dst_rows, probs, static_cast<__nv_bfloat16*>(out), tokens, topk, hidden));
 }
 
 int launchMoeReduceGroups(const void* y, void* z, const int* alias, const void* groups, const int* n_rows, int max_rows, int hidden,

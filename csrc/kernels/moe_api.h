@@ -49,6 +49,10 @@ int launchMoeCombine(const MoeArgs& a, int blocks, cudaStream_t stream);
 // bf16 rows from fp8 rows + scales, for rows [0, *n_rows) (device count).  `alias` (or null): row r is read from alias[r].
 int launchMoeDequant(const void* q, const float* scales, void* out, const int* n_rows, int max_rows, int hidden, const int* alias,
                      cudaStream_t stream);
+// Dispatch and conversion for a world of one: out[dst_rows[t,k]] = what the dispatch of token t would deliver there and launchMoeDequant
+// turn into bf16, times probs[t,k] if given.  Assignments with a negative expert or row are dropped; every row is below out's.
+int launchMoeExpand(const void* x, const int* ids, const int* dst_rows, const float* probs, void* out, int tokens, int topk, int hidden,
+                    cudaStream_t stream);
 // z[r] = sum over the group of primary row r of weight x y[row], for groups of two or more rows (local; after the experts).
 int launchMoeReduceGroups(const void* y, void* z, const int* alias, const void* groups, const int* n_rows, int max_rows, int hidden,
                           cudaStream_t stream);

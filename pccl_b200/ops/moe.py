@@ -172,7 +172,7 @@ class MoEExchange:
         return out
 
     # ---- kernels ----------------------------------------------------------------------------
-    def _exchange(self, kind: str, x, ids, rows, probs, out, gate=None, dedupe: bool = False, groups: bool = True) -> None:
+    def _exchange(self, kind: str, x, ids, rows, probs, out, gate=None, dedupe: bool = False) -> None:
         self.epoch += 1
         st = status_words()
         off = self.eng.heap_offset
@@ -181,7 +181,7 @@ class MoEExchange:
                        [x.data_ptr()] if x is not None else [], [ids.data_ptr()], [rows.data_ptr()],
                        [probs.data_ptr()] if probs is not None else [], [out.data_ptr()] if out is not None else [],
                        [st.data_ptr()], self.blocks, 0, stream_handle(),
-                       alias_off=off(self.alias), group_off=off(self.groups) if groups else 0, z_off=off(self.z),
+                       alias_off=off(self.alias), group_off=off(self.groups), z_off=off(self.z),
                        gate=[gate.data_ptr()] if gate is not None else [], dedupe=dedupe)
         count_launch()
 
@@ -210,6 +210,20 @@ class MoEExchange:
         count_launch()
         return out
 
+    def deliver(self, x: torch.Tensor, ids: torch.Tensor, plan: Dict[str, torch.Tensor], probs: Optional[torch.Tensor] = None,
+                out: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """``dispatch`` and ``received`` in one.  In a world of one nothing travels and one kernel writes the rows; the receive
+        buffers stay as they are."""
+        if self.eng.world > 1:
+            self.dispatch(x, ids, plan, probs=probs)
+            return self.received(plan, out)
+        if out is None:
+            out = torch.empty((self.cap, self.H), dtype=torch.bfloat16, device="cuda")
+        C.moe_expand(x.data_ptr(), ids.data_ptr(), plan["rows"].data_ptr(), 0 if probs is None else probs.data_ptr(), out.data_ptr(), self.T, self.K,
+                     self.H, stream_handle())
+        count_launch()
+        return out
+
     def combine_dot(self, g: torch.Tensor, ids: torch.Tensor, plan: Dict[str, torch.Tensor]) -> torch.Tensor:
         """``dot[t, k] = <g[t], y row of assignment (t, k)>`` (fp32 [tokens, topk]): with ``g`` the upstream gradient and
         the expert outputs of the forward pass still in ``self.y``, the gradient of the gate weights."""
@@ -219,9 +233,10 @@ class MoEExchange:
 
     def experts(self, w1: torch.Tensor, w2: torch.Tensor, plan: Dict[str, torch.Tensor]) -> None:
         """w1: [experts_per_rank * d_ff, hidden], w2: [experts_per_rank * hidden, d_ff]; result in self.y."""
-        C.moe_dequant(self.recv_q.data_ptr(), self.recv_s.data_ptr(), self.x_bf16.data_ptr(), plan["n_rows"].data_ptr(), self.cap,
-                      self.H, stream_handle(), alias=self.alias.data_ptr())
-        count_launch()
+        self.received(plan, self.x_bf16)
+        self._experts(w1, w2, plan)
+
+    def _experts(self, w1: torch.Tensor, w2: torch.Tensor, plan: Dict[str, torch.Tensor]) -> None:
         d_ff = w1.shape[0] // self.epr
         h = grouped_gemm(self.x_bf16, w1, plan["row_off"], d_ff, gelu=True)
         grouped_gemm(h, w2, plan["row_off"], self.H, out=self.y)
@@ -246,6 +261,10 @@ class MoEExchange:
         # Adding up a token's rows on each rank before they travel saves NVLink traffic.  In a world of one nothing travels and it
         # would be a second pass over the sums: the combine weighs the expert rows itself (the same fp32 sum in the same order).
         grouped = self.eng.world > 1
-        self._exchange("dispatch", x, ids, plan["rows"], None, None, gate=probs, dedupe=True, groups=grouped)
-        self.experts(w1, w2, plan)
+        if grouped:
+            self._exchange("dispatch", x, ids, plan["rows"], None, None, gate=probs, dedupe=True)
+            self.experts(w1, w2, plan)
+        else:
+            self.deliver(x, ids, plan, out=self.x_bf16)
+            self._experts(w1, w2, plan)
         return self.combine(ids, probs, plan, grouped=grouped)

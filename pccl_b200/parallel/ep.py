@@ -27,8 +27,7 @@ class _MoEFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, gate_logits, w1, w2, ex: MoEExchange):
         ids, probs, plan = ex.route_and_plan(gate_logits)
-        ex.dispatch(x, ids, plan)
-        xr = ex.received(plan)                                   # what the experts see (after the e4m3 round trip)
+        xr = ex.deliver(x, ids, plan)                            # what the experts see (after the e4m3 round trip)
         d_ff = w1.shape[0] // ex.epr
         h = torch.empty((xr.shape[0], d_ff), dtype=torch.bfloat16, device=xr.device)
         h_pre = grouped_gemm(xr, w1, plan["row_off"], d_ff, gelu_out=h)
@@ -49,8 +48,7 @@ class _MoEFn(torch.autograd.Function):
         # gate weights: d p[t,k] = <dout[t], expert output row>, while the forward outputs are still in ex.y
         dp = ex.combine_dot(dout, ids, plan)
         # output gradients to the experts, each weighted by its gate probability
-        ex.dispatch(dout, ids, plan, probs=probs)
-        g = ex.received(plan)
+        g = ex.deliver(dout, ids, plan, probs=probs)
         # experts: the same grouped kernel on the weights as they lie, gelu' in its epilogue, then all weight gradients at once
         dh_pre = grouped_gemm(g, w2, row_off, d_ff, b_t=True, dgelu=h_pre)
         grouped_gemm(dh_pre, w1, row_off, H, b_t=True, out=ex.y)

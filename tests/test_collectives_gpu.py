@@ -1181,3 +1181,39 @@ def test_moe_route_backward(native, T, E, topk):
     assert (got.double() - l64.grad).abs().max().item() <= 1e-5 * max(1e-3, l64.grad.abs().max().item())
     ex.y.copy_(torch.randn(ex.y.shape, device="cuda"))
     assert torch.equal(ex.combine(ids, None, plan), ex.combine(ids, torch.ones_like(probs), plan))
+
+
+@pytest.mark.parametrize("T,H,E,topk,drop", [(1, 128, 8, 1, 0), (7, 128, 8, 2, 5), (41, 2176, 8, 3, 0), (130, 1024, 16, 8, 40), (97, 7168, 32, 8, 0), (9, 16512, 4, 4, 3)])
+def test_moe_deliver_in_a_world_of_one(native, T, H, E, topk, drop):
+    """The rows that one kernel writes are those of dispatch and conversion, bit for bit, plain and scaled, for widths off the 256 values of
+    a warp, blocks of zeros and infinities, and with assignments dropped by row and by expert; nothing else is written."""
+    from pccl_b200.engine import Engine
+    from pccl_b200.ops import check_status
+    from pccl_b200.ops.moe import MoEExchange
+    torch.manual_seed(T)
+    eng = Engine(0, 1)
+    cap = 2 * T * topk + 256
+    eng.initEngine("cuda", 2 * cap * (H * 5 + H // 32 + 256) + (640 << 20))
+    ex = MoEExchange(eng, T, H, E, topk)
+    x = torch.randn(T, H, device="cuda").bfloat16() * torch.logspace(-8, 8, T, device="cuda")[:, None].bfloat16()
+    x[T // 2, :128] = 0
+    if T > 8:
+        x[3, 5] = float("inf")
+    ids, probs, plan = ex.route_and_plan(torch.randn(T, E, device="cuda"))
+    rows = plan["rows"].flatten().long()
+    if drop:
+        plan["rows"].view(-1)[:drop] = -1
+        ids.view(-1)[-1] = -1
+    kept = torch.ones(T * topk, dtype=torch.bool, device="cuda")
+    if drop:
+        kept[:drop] = False
+        kept[-1] = False
+    for p in (None, probs):
+        ex.dispatch(x, ids, plan, probs=p)
+        want = ex.received(plan)
+        got = ex.deliver(x, ids, plan, probs=p, out=torch.full((ex.cap, H), 3.0, device="cuda").bfloat16())
+        assert torch.equal(got[rows[kept]].view(torch.int16), want[rows[kept]].view(torch.int16))
+        rest = torch.ones(ex.cap, dtype=torch.bool, device="cuda")
+        rest[rows[kept]] = False
+        assert (got[rest] == 3.0).all()
+    check_status("moe deliver")

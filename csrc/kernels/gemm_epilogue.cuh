@@ -67,7 +67,7 @@ __device__ __forceinline__ void warp_transpose_sum32(float* v, int lane) {
 // bytes; an epilogue with two outputs (pre-activation and GELU) or a side input is bound by exactly that.
 constexpr int kPatchRowBytes = 80;
 constexpr int kPatchBytes = 32 * kPatchRowBytes;          // per epilogue warp
-constexpr int kPatchBytesPerCta = 8 * kPatchBytes;       // eight epilogue warps (gemm_fp8_pair.cuh has sixteen)
+constexpr int kPatchBytesPerCta = 8 * kPatchBytes;       // eight epilogue warps
 // the calling epilogue warp's patch: `base` is that of warp 2 (warps 2, 3, ... of the CTA are the epilogue warps as a rule)
 __device__ __forceinline__ uint8_t* my_patch(uint8_t* base) { return base + ((threadIdx.x >> 5) - 2) * kPatchBytes; }
 

@@ -83,12 +83,10 @@ __device__ __forceinline__ void ffma2(float& acc0, float& acc1, uint32_t r0, uin
 }
 
 // STAGES (<= 4) operand stages of 48 KiB; an epilogue that needs shared memory of its own runs with three.
-// BNT = 128 (up to six stages of 32 KiB): a K block is a chain MMA -> commit -> tcgen05.ld -> fold -> accumulator free -> MMA, about
-// 2900 clocks long at 256 columns, and with two accumulators in turn half of that is what a block takes, whatever the tensor
-// cores and TMEM could do (eight warps read TMEM at 880 bytes per clock and SM: 150 clocks per block).  128 columns leave room for
-// four accumulators, and the 64 sums per thread no longer spill: 8192 x 8192 x 3584 372 -> 320 us, 1531 x 8192 x 3584 117 -> 80,
-// 128 x 8192 x 3584 66 -> 31, 18944 x 8192 x 1024 (whole rounds) 218 -> 203.  The fused kernels keep 256 columns: their epilogues
-// quantise or stage whole 128-column halves.
+// BNT = 128 (up to six stages of 32 KiB): a K block is a chain MMA -> commit -> tcgen05.ld -> fold -> accumulator free -> MMA.  128 columns
+// leave room for four accumulators where 256 have two, and the 64 sums per thread no longer spill: 8192 x 8192 x 3584 322 us at 256
+// columns, 260 at 128.  What is left is the operands' way from L2 (see the scales below).  The fused kernels keep 256 columns: their
+// epilogues quantise or stage whole 128-column halves.
 template <int STAGES = MAX_STAGES, int BNT = BN, class Sched, class Gate, class Epi>
 __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* tmB, int K, const Scales& sc, const Sched& sched,
                                     const Gate& gate, Epi& epi, uint32_t* status) {

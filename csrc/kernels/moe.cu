@@ -336,8 +336,8 @@ __global__ void __launch_bounds__(GT * kCombineSubs<GT>) moe_combine_dot_kernel(
 }
 
 // One warp per row, eight values per lane and step (a warp stores 512 consecutive bytes), four steps in flight, the next row's
-// alias fetched behind this row.  The stores bound it (the e4m3 rows of a de-duplicated exchange come out of L2): 32768 rows of
-// 7168 take 110 us, 470 MB at 4.3 TB/s (a CTA per row and half-filled second trips: 167).
+// alias fetched behind this row.  The e4m3 rows of a de-duplicated exchange come out of L2: 32768 rows of
+// 7168 take 110 us, 470 MB stored at 4.3 TB/s (a CTA per row and half-filled second trips: 167).
 __global__ void __launch_bounds__(256) moe_dequant_kernel(const uint8_t* q, const float* scales,
                                                           __nv_bfloat16* out, const int* n_rows,
                                                           int max_rows, int hidden, const int* alias) {

@@ -81,7 +81,8 @@ def reduce_scatter_adamw(eng: Engine, grads: torch.Tensor, master: torch.Tensor,
                          lane: int = 0, stream=None) -> None:
     """Gradient-bucket reduce-scatter fused with the sharded AdamW step.  ``grads`` is the symmetric bf16
     bucket (world * n elements); ``master`` / ``exp_avg`` / ``exp_avg_sq`` are this rank's fp32 slices (n
-    elements, n % 8 == 0); the updated parameters are written to ``param_bf16`` (bf16, n elements)."""
+    elements, n % 8 == 0); the updated parameters are written to ``param_bf16`` (bf16, n elements).  A world of one has a kernel of
+    its own with a grid of its own; ``blocks`` and ``threads`` are for the exchange."""
     n = master.numel()
     if grads.dtype != torch.bfloat16 or grads.numel() != n * eng.world or n % 8:
         raise ValueError("reduce_scatter_adamw: bf16 bucket of world * n elements with n % 8 == 0 expected")

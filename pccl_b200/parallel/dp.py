@@ -2,13 +2,13 @@
 
 Gradients live in flat bf16 buckets (25 MB by default) inside the symmetric heap.  The moment the
 last gradient of a bucket has been written (the weight-gradient GEMMs write there directly), ONE
-kernel is queued on a high-priority side stream: each rank reduces its 1/world slice of the bucket
+kernel is queued on a side stream (of high priority where ranks wait for it): each rank reduces its 1/world slice of the bucket
 (multimem.ld_reduce through the switch, or loads from every peer over NVLink), multiplies by
 1/world and applies AdamW to its fp32 master slice -- reduction, scaling, cast and optimizer in one
 pass -- and writes the new bf16 parameters, which the bucket's all-gather kernel then pushes to
 every rank (ZeRO-1).  The kernels run as short, wide bursts (64 CTAs) that slip in between
 two GEMM kernels of backward.  With a world of one the reduce-scatter is a flat scale/cast/update pass
-over the bucket, whose small CTAs run beside the GEMMs' on the same SMs.
+over the bucket in short launches, whose small CTAs run beside the GEMMs' on the same SMs.
 ``fuse_optimizer=False`` keeps the reduce-scatter (with scale and fp32 cast) and the optimizer apart.
 """
 from __future__ import annotations
@@ -78,7 +78,7 @@ class ShardedDataParallel:
             engine.initEngine("cuda", max(heap_bytes, need + (512 << 20)))
         self.engine = engine
         self.world, self.rank = engine.world, engine.rank
-        # Communication kernels run as short, wide bursts on a high-priority stream: they slip in at the
+        # With ranks to exchange with, communication kernels run as short, wide bursts on a high-priority stream: they slip in at the
         # boundary between two GEMM kernels and delay the next one by their own (tens of microseconds)
         # duration.  A narrow long-running kernel would instead hold a few SMs for the whole GEMM and make
         # the persistent GEMM's last CTAs start a full wave late.  (A world of one exchanges nothing and has a kernel of its own,

@@ -84,9 +84,9 @@ __device__ __forceinline__ void ffma2(float& acc0, float& acc1, uint32_t r0, uin
 
 // STAGES (<= 4) operand stages of 48 KiB; an epilogue that needs shared memory of its own runs with three.
 // BNT = 128 (up to six stages of 32 KiB): a K block is a chain MMA -> commit -> tcgen05.ld -> fold -> accumulator free -> MMA.  128 columns
-// leave room for four accumulators where 256 have two, and the 64 sums per thread no longer spill: 8192 x 8192 x 3584 322 us at 256
-// columns, 260 at 128.  What is left is the operands' way from L2 (see the scales below).  The fused kernels keep 256 columns: their
-// epilogues quantise or stage whole 128-column halves.
+// leave room for four accumulators where 256 have two, and the 64 sums per thread no longer spill: 8192 x 8192 x 3584 372 -> 320 us, and
+// 260 with the scales read as below.  What is left is the operands' way from L2.  The fused kernels keep 256 columns: their epilogues
+// quantise or stage whole 128-column halves.
 template <int STAGES = MAX_STAGES, int BNT = BN, class Sched, class Gate, class Epi>
 __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* tmB, int K, const Scales& sc, const Sched& sched,
                                     const Gate& gate, Epi& epi, uint32_t* status) {

@@ -68,7 +68,7 @@ def _fused(ids: torch.Tensor, wte: torch.nn.Module, wpe: torch.nn.Module) -> boo
     if not (is_plain(wte, Embedding) and is_plain(wpe, Embedding) and wte.weight is not wpe.weight):
         return False
     (B, T), D = ids.shape, wte.weight.shape[1]
-    return (B <= _MAX_BATCH and ids.dtype is torch.int64 and ids.device == wte.weight.device == wpe.weight.device and ids.is_contiguous()
+    return (B <= _MAX_BATCH and ids.dtype is torch.int64 and ids.device == wte.weight.device == wpe.weight.device
             and 0 < ids.numel() * D < 1 << 34 and D % 8 == 0 and T <= wpe.weight.shape[0] and _fits(wte.weight, D) and _fits(wpe.weight, D))
 
 
@@ -76,5 +76,6 @@ def token_position(ids: torch.Tensor, wte: torch.nn.Module, wpe: torch.nn.Module
     """``wte(ids) + wpe(arange(T))`` for ids [B, T].  Two plain ``Embedding`` layers with bf16 tables run as one kernel; anything else as
     the layers' own calls."""
     if _fused(ids, wte, wpe):
+        ids = ids.contiguous()                # token windows are often slices of longer rows
         return _TokenPositionFn.apply(ids, wte.weight, wpe.weight) if records_graph() else _forward(ids, wte.weight, wpe.weight)
     return wte(ids) + wpe(torch.arange(ids.shape[1], device=ids.device))[None]

@@ -124,6 +124,10 @@ void bindGemm(py::module_& m) {
                             reinterpret_cast<float*>(partials), reinterpret_cast<cudaStream_t>(stream));
     if (err != 0) throw std::runtime_error(std::string("qkv_pack: ") + cudaErrorName(err));
   });
+  m.def("layernorm_fwd_form", [](long long rows, int D, int sms) {
+    const LayerNormFwdForm f = layerNormFwdForm(rows, D, sms);
+    return py::make_tuple(f.warps, f.vectors, f.rows, f.one_row);
+  });
   m.def("layernorm_bwd_parts", &layerNormBwdParts);
   m.def("layernorm_bwd", [](uint64_t dy, uint64_t x, uint64_t g, uint64_t mean, uint64_t rstd, uint64_t dres, uint64_t dx, uint64_t dg,
                             uint64_t db, uint64_t dcolsum, uint64_t partials, long long rows, int D, uint64_t stream) {

@@ -34,6 +34,19 @@ int launchEmbedBwd(const void* dy, const long long* ids, void* d_tok, void* d_po
 // null where no backward pass follows.
 // With `delta` (bf16 [rows, D], may be null) the norm is taken of s = x + delta and s is stored to `sum_out`:
 // the residual connection of a pre-norm block and the norm in one pass.
+//
+// How a launch divides its rows: warps per row, 16-byte vectors per thread, rows per CTA, and whether the CTA is one row's by construction (a
+// kernel with one barrier; the other one names its barriers at run time and takes all 16, so an SM holds fewer CTAs of it).
+// Measured on 148 SMs behind a GEMM that writes the rows (us; a CTA of as many rows as fit / one row per CTA):
+//   1531 x 2048 5.6 / 3.8, 1000 x 1536 3.9 / 2.7, 128 x 1536 2.3 / 2.1, 1 x 2560 3.0 / 2.2, 128 x 4096 2.8 / 2.3, 1531 x 3072 6.2 / 5.1, 3000 x
+//   2560 9.2 / 6.9, 4096 x 5120 23 / 16, but 300 x 2048 2.4 / 2.4 (with the residual sum 2.6 / 2.9), 300 x 4096 3.2 / 3.8, 2331 x 2048 4.7 / 5.3:
+// one row per CTA up to one row per SM and, beyond D = 1024, from more than three on, but not for large inputs of up to 2048 columns.
+// One vector per thread (two beyond 2048, three beyond 4096, four beyond 6144) is the shorter chain, which few rows need; four per thread
+// leave more rows in flight on an SM: from 7 Mi values on up to D = 5120 (4096 x 3072 11.4 -> 9.5, but 1531 x 4096, 6 Mi, 6.0 -> 6.6).
+// Eight warps of two vectors fit an SM six times: the seventh and eighth row of an SM would be a second round (1000 x 4096 4.5 / 4.8).
+// Up to eight rows per SM eight warps spread more evenly than the five to seven that narrower rows need (800 x 1032 3.7 -> 3.4).
+struct LayerNormFwdForm { int warps, vectors, rows; bool one_row; };
+LayerNormFwdForm layerNormFwdForm(long long rows, int D, int sms);
 int launchLayerNormFwd(const void* x, const void* delta, void* sum_out, const void* gamma, const void* beta, void* y, float* mean,
                        float* rstd, long long rows, int D, float eps, cudaStream_t stream);
 // Backward: dx bf16 [rows, D] = d(norm input) + dres (bf16 [rows, D], may be null: the gradient on the residual stream);

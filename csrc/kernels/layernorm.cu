@@ -25,21 +25,19 @@ namespace {
 
 using namespace dev;
 
-// Forward.  A group of `gw` warps owns a row with up to four 16-byte vectors per thread (one warp up to D = 1024) and a CTA takes as
-// many rows as its 256 threads hold: all loads of a row are out before the first sum, and a row of one warp takes no barrier.  A row
-// stays in registers as it came, eight values in four registers, and scale and shift are read last (they are in L1 or L2), so that four
-// CTAs fit an SM; with two vectors per thread and six CTAs, with CTAs of 128 threads or with scale and shift ahead of the sums 16384 x 2048
-// takes 53, 55 and 51 us.
-// Memory bounds it.  Times, us, cold L2, plain and with the residual sum (a CTA of 256 threads per row before -> now): 16384 x 2048
-// 39 -> 36, 55 -> 49 (5.5 TB/s); 16384 x 1536 37 -> 32, 49 -> 40; 16384 x 1024 33 -> 21, 43 -> 29; 16384 x 256 29 -> 12, 35 -> 14;
-// 4096 x 1024 14 -> 11, 16 -> 12; 4096 x 8192 41 -> 37, 64 -> 49; 1531 x 2048 unchanged at 10 and 12.
-template <int VPT>
-__global__ void __launch_bounds__(256, VPT == 4 ? 4 : 1) ln_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* delta, __nv_bfloat16* sum_out,
-                                                     const __nv_bfloat16* gamma, const __nv_bfloat16* beta, __nv_bfloat16* y,
-                                                     float* mean, float* rstd, long long rows, int D, float eps, int gw) {
+// Forward.  A group of `gw` warps owns a row with up to four 16-byte vectors per thread: all loads of a row are out before the first sum, and a
+// row of one warp (D <= 1024) takes no barrier.  A row stays in registers as it came, eight values in four registers, and scale and shift
+// are read last (they are in L1 or L2).  A CTA is ONE_ROW, or as many rows as its 256 threads hold; the groups' barriers of the latter are named
+// at run time, for which a CTA sets all 16 barriers aside, and an SM then holds few of them.  layerNormFwdForm (below) says which runs where.
+// Memory bounds it: cold L2, us, plain and with the residual sum, 16384 x 2048 36, 49 (5.5 TB/s); 16384 x 1024 21, 29; 16384 x 256 12, 14;
+// 4096 x 8192 33, 50.  With two vectors per thread, CTAs of 128 threads or scale and shift ahead of the sums 16384 x 2048 takes 53, 55 and 51.
+template <int VPT, bool ONE_ROW>
+__global__ void __launch_bounds__(256, ONE_ROW ? (VPT == 1 ? 8 : VPT == 2 ? 6 : 5) : VPT == 4 ? 4 : 1)
+ln_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* delta, __nv_bfloat16* sum_out, const __nv_bfloat16* gamma, const __nv_bfloat16* beta,
+              __nv_bfloat16* y, float* mean, float* rstd, long long rows, int D, float eps, int gw) {
   __shared__ float part[2][8];                              // [sum, squares][warp]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int group = warp / gw, groups = (blockDim.x >> 5) / gw, tid = threadIdx.x - group * gw * 32;
+  const int group = ONE_ROW ? 0 : warp / gw, groups = ONE_ROW ? 1 : (blockDim.x >> 5) / gw, tid = threadIdx.x - group * gw * 32;
   const int nvec = D >> 3, width = gw * 32;
   dev::pdl_launch();
   dev::pdl_wait();
@@ -69,9 +67,10 @@ __global__ void __launch_bounds__(256, VPT == 4 ? 4 : 1) ln_fwd_kernel(const __n
   auto group_sum = [&](float t, int which) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (gw == 1) return t;
+    if (!ONE_ROW && gw == 1) return t;
     if (lane == 0) part[which][warp] = t;
-    asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(width) : "memory");
+    if (ONE_ROW) __syncthreads();
+    else asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(width) : "memory");
     t = 0.f;
     for (int w = 0; w < gw; ++w) t += part[which][group * gw + w];
     return t;
@@ -523,6 +522,29 @@ bool aligned16(std::initializer_list<const void*> pointers) {
 
 }  // namespace
 
+LayerNormFwdForm layerNormFwdForm(long long rows, int D, int sms) {
+  const int nvec = D / 8;
+  const long long values = rows * D, mi = 1ll << 20;
+  LayerNormFwdForm f{(nvec + 127) / 128, 4, 1, false};
+  if (f.warps == 1) f.vectors = (nvec + 31) / 32;
+  const bool short_chain = D <= 2048 ? values <= 4 * mi : values <= 7 * mi || D > 5120;
+  if (short_chain) {
+    f.vectors = (nvec + 255) / 256;
+    f.warps = (nvec + 32 * f.vectors - 1) / (32 * f.vectors);
+  }
+  if (f.warps > 1 && (D > 2048 || short_chain)) f.one_row = rows <= sms || (D > 1024 && rows > 3 * sms);
+  if (f.one_row && f.vectors == 2 && f.warps == 8 && rows > 6 * sms && rows <= 8 * sms) f.one_row = false;
+  if (!f.one_row && D > 2048) {
+    f.vectors = 4;
+    f.warps = (nvec + 127) / 128;
+  }
+  if (f.one_row && f.vectors == 1 && D > 1024 && rows <= 8 * sms) f.warps = 8;
+  if (f.one_row) return f;
+  f.rows = 8 / f.warps;
+  while (f.rows > 1 && (rows + f.rows - 1) / f.rows < sms) f.rows /= 2;
+  return f;
+}
+
 int launchLayerNormFwd(const void* x, const void* delta, void* sum_out, const void* gamma, const void* beta, void* y, float* mean,
                        float* rstd, long long rows, int D, float eps, cudaStream_t stream) {
   if (rows <= 0) return 0;
@@ -530,23 +552,21 @@ int launchLayerNormFwd(const void* x, const void* delta, void* sum_out, const vo
   auto X = static_cast<const __nv_bfloat16*>(x); auto G = static_cast<const __nv_bfloat16*>(gamma);
   auto B = static_cast<const __nv_bfloat16*>(beta); auto Y = static_cast<__nv_bfloat16*>(y);
   auto DL = static_cast<const __nv_bfloat16*>(delta); auto S = static_cast<__nv_bfloat16*>(sum_out);
-  const int nvec = D / 8;
-  int gw = (nvec + 127) / 128, vpt = gw > 1 ? 4 : (nvec + 31) / 32;
-  // Up to four million values a thread takes one vector: its chain is the shorter (24 x 2048 9 -> 8 us, 1531 x 2048 equal by itself), and
-  // with 40 registers per thread a CTA finds room beside one of a GEMM, to be in its place when that ends.
-  if (rows * D <= 4ll << 20 && nvec <= 256) {
-    gw = (nvec + 31) / 32;
-    vpt = 1;
-  }
-  // as many rows per CTA as 256 threads hold, fewer where the rows would then leave SMs without work
-  int groups = 8 / gw;
-  while (groups > 1 && (rows + groups - 1) / groups < deviceSmCount()) groups /= 2;
-  const unsigned grid = static_cast<unsigned>((rows + groups - 1) / groups);
+  const LayerNormFwdForm form = layerNormFwdForm(rows, D, deviceSmCount());
+  const unsigned grid = static_cast<unsigned>((rows + form.rows - 1) / form.rows);
   auto go = [&](auto kern) {
-    return static_cast<int>(launchOverlapped(kern, dim3(grid), dim3(groups * gw * 32), 0, stream, 1, X, DL, S, G, B, Y, mean, rstd, rows, D, eps, gw));
+    return static_cast<int>(launchOverlapped(kern, dim3(grid), dim3(form.rows * form.warps * 32), 0, stream, 1, X, DL, S, G, B, Y, mean, rstd, rows, D, eps,
+                                             form.warps));
   };
-  return vpt == 1 ? go(ln_fwd_kernel<1>) : vpt == 2 ? go(ln_fwd_kernel<2>) : vpt == 3 ? go(ln_fwd_kernel<3>) : go(ln_fwd_kernel<4>);
+  if (form.one_row) {
+    return form.vectors == 1 ? go(ln_fwd_kernel<1, true>) : form.vectors == 2 ? go(ln_fwd_kernel<2, true>)
+         : form.vectors == 3 ? go(ln_fwd_kernel<3, true>) : go(ln_fwd_kernel<4, true>);
+  }
+  return form.vectors == 1 ? go(ln_fwd_kernel<1, false>) : form.vectors == 2 ? go(ln_fwd_kernel<2, false>)
+       : form.vectors == 3 ? go(ln_fwd_kernel<3, false>) : go(ln_fwd_kernel<4, false>);
 }
+
+bool layerNormBwdRing(long long rows, int D, int sms) { return D > 2048 && rows > (D <= 4096 ? 16 : 7) * sms; }
 
 int layerNormBwdParts(long long rows) { return static_cast<int>(rows < 148 * 2 ? rows : 148 * 2); }
 

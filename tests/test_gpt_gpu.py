@@ -290,6 +290,27 @@ def test_fused_residual_add_layernorm_matches_fp32_reference(rows, D):
         assert (got.float() - ref).abs().max().item() <= 2e-2 * max(1.0, ref.abs().max().item())
 
 
+# edges of the rules that pick the forward kernel's form (148 SMs): one row per CTA up to one row per SM and from three on, the widths at which a
+# thread takes another vector, 6 and 8 rows per SM with eight warps, 4 and 7 Mi values
+@pytest.mark.parametrize("rows,D", [(148, 264), (149, 1032), (444, 1032), (445, 1032), (2048, 2048), (2049, 2048), (3, 2056), (445, 2056), (889, 4096), (1185, 4096),
+                                    (2389, 3072), (2390, 3072), (5, 4104), (445, 5120), (448, 5128), (148, 6152), (149, 8192), (445, 8192)])
+def test_layernorm_forward_at_the_edges_of_its_forms(rows, D):
+    from pccl_b200.nn.norm import _ln_forward
+    torch.manual_seed(rows + D)
+    x, delta = (torch.randn(rows, D, device="cuda") * 2 + 0.5).bfloat16(), torch.randn(rows, D, device="cuda").bfloat16()
+    w, b = (torch.randn(D, device="cuda") * 0.5 + 1).bfloat16(), torch.randn(D, device="cuda").bfloat16()
+    for d in (None, delta):
+        s, y, stats = _ln_forward(x, d, w, b, 1e-5)
+        base = x if d is None else (x.float() + d.float()).bfloat16()      # the norm sees the sum as it is stored
+        assert d is None or torch.equal(s, base)
+        ref = F.layer_norm(base.double(), (D,), w.double(), b.double(), 1e-5)
+        # a bf16 result is rounded by half of 2^-8; fp32 sums of up to 8192 terms and rsqrt leave some 1e-6 of a normalised value (at most 6 here) times w
+        assert ((y.double() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-4).all()
+        assert (stats[0].double() - base.double().mean(1)).abs().max().item() < 1e-5
+        rstd = (base.double().var(1, unbiased=False) + 1e-5).rsqrt()
+        assert (stats[1].double() / rstd - 1).abs().max().item() < 1e-5
+
+
 def test_fused_mlp_backward_matches_fp32_reference():
     """fc2(gelu(fc1(x))) as one autograd node (GELU derivative and first bias gradient inside the GEMM epilogue)."""
     from pccl_b200.nn import Linear, mlp

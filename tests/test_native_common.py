@@ -95,3 +95,17 @@ def test_norm_kernels_refuse_addresses_off_the_16_byte_boundaries(native, bad):
         dy, x, g, dres, dx = at[:5]
         with pytest.raises(RuntimeError, match="layernorm_bwd: invalid argument"):
             native.layernorm_bwd(dy, x, g, 4096, 4096, dres, dx, 4096, 4096, 0, 4096, 4, 64, 0)
+
+
+
+def test_layernorm_forward_forms(native):
+    """One row per CTA (one barrier, as many CTAs as registers allow) where a CTA of several rows was slower; every form covers its row."""
+    form = lambda rows, D: native.layernorm_fwd_form(rows, D, 148)  # noqa: E731   (warps, vectors, rows per CTA, one row by construction)
+    for rows, D in ((1531, 2048), (600, 2048), (1000, 1536), (128, 1536), (1, 2560), (128, 4096), (1531, 3072), (3000, 2560), (4096, 5120), (600, 8192)):
+        assert form(rows, D)[3], (rows, D)
+    for rows, D in ((300, 2048), (444, 2048), (300, 4096), (2331, 2048), (16384, 2048), (1531, 768), (16384, 1024)):
+        assert not form(rows, D)[3], (rows, D)
+    for D in range(8, 8193, 8):
+        for rows in (1, 148, 149, 444, 445, 888, 889, 1184, 1185, 1531, 4096, 70000):
+            warps, vectors, per_cta, one_row = form(rows, D)
+            assert warps * vectors * 32 >= D // 8 and 1 <= vectors <= 4 and 1 <= warps * per_cta <= 8 and (per_cta == 1 or not one_row), (rows, D)

@@ -129,6 +129,7 @@ void bindGemm(py::module_& m) {
     return py::make_tuple(f.warps, f.vectors, f.rows, f.one_row);
   });
   m.def("layernorm_bwd_parts", &layerNormBwdParts);
+  m.def("layernorm_bwd_ring", &layerNormBwdRing);
   m.def("layernorm_bwd", [](uint64_t dy, uint64_t x, uint64_t g, uint64_t mean, uint64_t rstd, uint64_t dres, uint64_t dx, uint64_t dg,
                             uint64_t db, uint64_t dcolsum, uint64_t partials, long long rows, int D, uint64_t stream) {
     int err = launchLayerNormBwd(reinterpret_cast<const void*>(dy), reinterpret_cast<const void*>(x), reinterpret_cast<const void*>(g),

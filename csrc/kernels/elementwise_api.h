@@ -54,6 +54,9 @@ int launchLayerNormFwd(const void* x, const void* delta, void* sum_out, const vo
 // the linear layer that fed the residual sum.  `x` is the norm's input (the stored sum when forward had a delta).
 // `partials` is fp32 scratch of 3 * layerNormBwdParts(rows) * D elements.
 int layerNormBwdParts(long long rows);
+// Whether a backward pass with a residual gradient or column sums takes its rows through the ring in shared memory: from 16 rows per SM on
+// beyond 2048 columns, from 7 on beyond 4096 (the kernel has both sides' times).
+bool layerNormBwdRing(long long rows, int D, int sms);
 int launchLayerNormBwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, const void* dres, void* dx,
                        void* dgamma, void* dbeta, void* dcolsum, float* partials, long long rows, int D, cudaStream_t stream);
 

@@ -194,9 +194,12 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, int n) {
 // Backward.  A group of `gw` warps owns a row -- as many as cover it with VPT 16-byte vectors per thread (one up to D = 2048) -- and takes
 // R rows at a time: R x VPT x 3 vectors are in flight per thread, and the row statistics of all R rows cross the group in one exchange.
 // The next R rows are fetched into registers while these are worked on (STAGES = 0), as far as that goes without spills, which cost
-// far more than the fetch brings.  Beyond D = 2048 the EXTRA form has no registers for that: its rows come through a ring in shared
-// memory, STAGES - 1 trips ahead.  A thread copies only what it reads itself, so no barrier guards the ring, and a slot is filled again
-// one trip after its values were used.  (Where the registers hold the next rows a ring brings nothing: 16384 x 2048 52 with either.)
+// far more than the fetch brings.  Beyond D = 2048 many rows of the EXTRA form come through a ring in shared memory, STAGES - 1 trips ahead.
+// A thread copies only what it reads itself, so no barrier guards the ring, and a slot is filled again one trip after its values were
+// used.  (Where the registers hold the next rows a ring brings nothing: 16384 x 2048 52 with either.)  Few rows gain nothing from a ring and
+// pay for its filling: they come straight into registers, beyond D = 4096 each trip's own (STAGES = -1: no registers for the next).
+// us, ring / without: 1 x 3072 5.7 / 4.6, 600 x 4096 12.4 / 11.3, 1531 x 4096 17.2 / 15.5, 2331 x 3072 16.4 / 15.8, 3000 x 2560 18.4 / 19.4; 1 x 8192
+// 9.9 / 9.1, 600 x 5120 14.8 / 13.6, 1000 x 6144 18.9 / 17.8, 1531 x 5120 23.0 / 23.9, 4096 x 8192 60 / 79.
 // A thread keeps the same columns for all of its rows, so the column sums (dgamma, dbeta, bias gradient) stay in registers; the CTA's
 // groups add theirs up at the end and write one partial row per array.
 // With eight warps per SM the instructions count beside the memory: the arithmetic is on pairs (f32x2) and the exchange is group_sum.
@@ -250,7 +253,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) ln_bwd_kernel(const __nv_bfloat
   };
   long long row0 = (static_cast<long long>(blockIdx.x) * groups + group) * R;
   Rows cur;
-  constexpr int ARR = EXTRA ? 3 : 2, SLOTS = STAGES ? STAGES : 1;
+  constexpr int ARR = EXTRA ? 3 : 2, SLOTS = STAGES > 0 ? STAGES : 1;
   Vec16* ring = reinterpret_cast<Vec16*>(group_sums);       // [STAGES][R][ARR][VPT][THREADS]
   auto slot_of = [&](int slot, int r, int a, int j) { return ring + (((slot * R + r) * ARR + a) * VPT + j) * THREADS + threadIdx.x; };
   auto fetch = [&](int slot, long long row0) {
@@ -276,16 +279,17 @@ __global__ void __launch_bounds__(THREADS, CTAS) ln_bwd_kernel(const __nv_bfloat
       rs_next[r] = row0 + r < rows ? rstd[row0 + r] : 0.f;
     }
   };
-  if (STAGES) {
+  if (STAGES > 0) {
 #pragma unroll
     for (int i = 0; i < STAGES - 1; ++i) fetch(i, row0 + i * step);
     stats(row0);
-  } else {
+  } else if (STAGES == 0) {
     load(cur, row0);
   }
   int parity = 0, slot = 0;
   for (; row0 < rows; row0 += step, parity ^= 1, slot = slot + 1 == SLOTS ? 0 : slot + 1) {
-    if (STAGES) {
+    if (STAGES < 0) load(cur, row0);
+    if (STAGES > 0) {
       asm volatile("cp.async.wait_group %0;" ::"n"(STAGES > 1 ? STAGES - 2 : 0) : "memory");
 #pragma unroll
       for (int r = 0; r < R; ++r) {
@@ -319,7 +323,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) ln_bwd_kernel(const __nv_bfloat
       sums[2 * r + 1] = split(s2).x + split(s2).y;
     }
     Rows next;
-    if (!STAGES) load(next, row0 + step);  // on its way behind the exchange, the arithmetic and the stores
+    if (STAGES == 0) load(next, row0 + step);  // on its way behind the exchange, the arithmetic and the stores
     // the other parity's slots are not written again before every warp of the group has passed this barrier once more
     group_sum<2 * R>(sums, stat[parity], warp, lane, gw, group * gw, group + 1);
 #pragma unroll
@@ -346,9 +350,9 @@ __global__ void __launch_bounds__(THREADS, CTAS) ln_bwd_kernel(const __nv_bfloat
         if (row0 + r < rows && tid + j * width < nvec) st16(dx + (row0 + r) * D + (tid + j * width) * 8, out);
       }
     }
-    if (!STAGES) cur = next;
+    if (STAGES == 0) cur = next;
   }
-  if (STAGES) {
+  if (STAGES > 0) {
     asm volatile("cp.async.wait_all;" ::: "memory");        // the last trips fetched zeros
     __syncthreads();
   }
@@ -596,13 +600,17 @@ int launchLayerNormBwd(const void* dy, const void* x, const void* gamma, const f
                                              static_cast<__nv_bfloat16*>(dx), pg, pb, pc, rows, D, gw));
   };
   constexpr size_t kRing = 192 * 1024;    // four stages of two rows of up to 4096 values and three arrays, or of one row of up to 8192
+  const bool ring = layerNormBwdRing(rows, D, deviceSmCount());
   int e;
-  if (dres || dcolsum)
-    e = D <= 2048 ? go(ln_bwd_kernel<1, 4, true, 1, 0, 256>, 1, 4, 1, 256, 0) : D <= 4096 ? go(ln_bwd_kernel<1, 2, true, 1, 4, 512>, 1, 2, 1, 512, kRing)
-                                                                                        : go(ln_bwd_kernel<4, 1, true, 1, 4, 256>, 4, 1, 1, 256, kRing);
-  else
+  if (!dres && !dcolsum)
     e = D <= 2048 ? go(ln_bwd_kernel<1, 2, false, 2, 0, 256>, 1, 2, 2, 256, 0) : D <= 4096 ? go(ln_bwd_kernel<2, 2, false, 1, 0, 256>, 2, 2, 1, 256, 0)
                                                                                          : go(ln_bwd_kernel<4, 1, false, 1, 0, 256>, 4, 1, 1, 256, 0);
+  else if (D <= 2048)
+    e = go(ln_bwd_kernel<1, 4, true, 1, 0, 256>, 1, 4, 1, 256, 0);
+  else if (D <= 4096)
+    e = ring ? go(ln_bwd_kernel<1, 2, true, 1, 4, 512>, 1, 2, 1, 512, kRing) : go(ln_bwd_kernel<2, 2, true, 1, 0, 256>, 2, 2, 1, 256, 0);
+  else
+    e = ring ? go(ln_bwd_kernel<4, 1, true, 1, 4, 256>, 4, 1, 1, 256, kRing) : go(ln_bwd_kernel<4, 1, true, 1, -1, 256>, 4, 1, 1, 256, 0);
   if (e != 0) return e;
   ReduceJob job{{pg, pb, pc}, {static_cast<__nv_bfloat16*>(dgamma), static_cast<__nv_bfloat16*>(dbeta), static_cast<__nv_bfloat16*>(dcolsum)}, nullptr};
   return static_cast<int>(launchOverlapped(partial_rows_reduce_kernel, dim3((D + 31) / 32, dcolsum ? 3 : 2), dim3(1024), 0, stream, 1, job, nparts, D));

@@ -311,6 +311,26 @@ def test_layernorm_forward_at_the_edges_of_its_forms(rows, D):
         assert (stats[1].double() / rstd - 1).abs().max().item() < 1e-5
 
 
+# edges of the rule for the ring (7 and 16 rows per SM) and of the widths at which the kernel changes
+@pytest.mark.parametrize("rows,D", [(1, 2056), (3, 4096), (2368, 2056), (2369, 2056), (300, 3080), (1, 8192), (1036, 4104), (1037, 4104), (149, 6152)])
+def test_layernorm_backward_with_and_without_its_ring(rows, D):
+    from pccl_b200.nn.norm import _ln_backward, _ln_forward
+    torch.manual_seed(rows + D)
+    x, dy, dres = (torch.randn(rows, D, device="cuda").bfloat16() for _ in range(3))
+    w, b = (torch.randn(D, device="cuda") * 0.5 + 1).bfloat16(), torch.zeros(D, device="cuda", dtype=torch.bfloat16)
+    stats = _ln_forward(x, None, w, b, 1e-5)[2]
+    dg, db, dc = (torch.empty_like(w) for _ in range(3))
+    dx = _ln_backward(dy, x, w, stats, dres, dg, db, dc).double()
+    xd, g = x.double(), dy.double() * w.double()
+    xh = (xd - xd.mean(1, keepdim=True)) * (xd.var(1, unbiased=False, keepdim=True) + 1e-5).rsqrt()
+    rs = (xd.var(1, unbiased=False, keepdim=True) + 1e-5).rsqrt()
+    ref = rs * (g - g.mean(1, keepdim=True) - xh * (g * xh).mean(1, keepdim=True)) + dres.double()
+    assert ((dx - ref).abs() <= 2 ** -8 * ref.abs() + 1e-4).all()              # the rounding of bf16, and fp32 arithmetic on values of some 20
+    # column sums in fp32, rounded to bf16: 2^-8 of the sum and some 1e-6 of the terms' sizes
+    for got, terms in ((dg, dy.double() * xh), (db, dy.double()), (dc, ref)):
+        assert ((got.double() - terms.sum(0)).abs() <= 2 ** -8 * terms.sum(0).abs() + 1e-5 * terms.abs().sum(0) + 1e-6).all()
+
+
 def test_fused_mlp_backward_matches_fp32_reference():
     """fc2(gelu(fc1(x))) as one autograd node (GELU derivative and first bias gradient inside the GEMM epilogue)."""
     from pccl_b200.nn import Linear, mlp

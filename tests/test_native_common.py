@@ -109,3 +109,10 @@ def test_layernorm_forward_forms(native):
         for rows in (1, 148, 149, 444, 445, 888, 889, 1184, 1185, 1531, 4096, 70000):
             warps, vectors, per_cta, one_row = form(rows, D)
             assert warps * vectors * 32 >= D // 8 and 1 <= vectors <= 4 and 1 <= warps * per_cta <= 8 and (per_cta == 1 or not one_row), (rows, D)
+
+
+def test_layernorm_backward_ring_is_for_many_rows(native):
+    ring = lambda rows, D: native.layernorm_bwd_ring(rows, D, 148)  # noqa: E731
+    assert not any(ring(1 << 20, D) for D in (8, 1024, 2048))
+    assert not any(ring(rows, D) for rows, D in ((1, 2056), (600, 4096), (2368, 4096), (1, 8192), (600, 5120), (1036, 4104)))
+    assert all(ring(rows, D) for rows, D in ((2369, 2056), (4096, 4096), (1037, 4104), (4096, 8192)))

@@ -5,6 +5,7 @@ GEMM reads the per-expert row ranges from device memory, so no step needs the ho
 """
 from __future__ import annotations
 
+import weakref
 from typing import Dict, Optional, Tuple
 
 import torch
@@ -78,6 +79,10 @@ def grouped_wgrad(a0: torch.Tensor, b0: torch.Tensor, a1: torch.Tensor, b1: torc
     return outs[0], outs[1]
 
 
+def _version(t: torch.Tensor) -> Optional[int]:
+    return None if t.is_inference() else t._version        # tensors made in inference mode count no versions
+
+
 class MoEExchange:
     """Buffers and kernels of one expert-parallel MoE layer shape."""
 
@@ -100,6 +105,7 @@ class MoEExchange:
         self.z = eng.symmetric_tensor((self.cap, hidden), torch.bfloat16)
         self.alias.copy_(torch.arange(self.cap, dtype=torch.int32, device="cuda"))
         self.epoch = 0
+        self._delivered = None             # (weak reference, version) of the rows if ``deliver`` wrote them past the receive buffers
         self.blocks = blocks or min(C.sm_count(), C.MAX_BLOCKS_PER_COLL)
         self.flag_lane = flag_lane
 
@@ -174,6 +180,8 @@ class MoEExchange:
     # ---- kernels ----------------------------------------------------------------------------
     def _exchange(self, kind: str, x, ids, rows, probs, out, gate=None, dedupe: bool = False) -> None:
         self.epoch += 1
+        if kind == "dispatch":
+            self._delivered = None
         st = status_words()
         off = self.eng.heap_offset
         C.moe_exchange(kind, self.eng.raw, [], 0, self.T, self.H, self.K, self.epr, off(self.recv_q),
@@ -201,8 +209,10 @@ class MoEExchange:
         self._exchange("dispatch", x, ids, plan["rows"], probs, None, gate=gate, dedupe=gate is not None)
 
     def received(self, plan: Dict[str, torch.Tensor], out: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """The rows that the last dispatch delivered to this rank, as bf16 [cap, hidden] (rows past the plan's count are
-        not written)."""
+        """The rows that were last delivered to this rank, by ``dispatch`` or inside ``forward`` or a layer's pass, as bf16 [cap, hidden]
+        (rows past the plan's count are not written)."""
+        if self._delivered is not None:
+            return self._received_past_buffers(plan, out)
         if out is None:
             out = torch.empty((self.cap, self.H), dtype=torch.bfloat16, device="cuda")
         C.moe_dequant(self.recv_q.data_ptr(), self.recv_s.data_ptr(), out.data_ptr(), plan["n_rows"].data_ptr(), self.cap,
@@ -210,10 +220,24 @@ class MoEExchange:
         count_launch()
         return out
 
+    def _received_past_buffers(self, plan: Dict[str, torch.Tensor], out: Optional[torch.Tensor]) -> torch.Tensor:
+        """``received`` where ``deliver`` wrote the rows at once: ``recv_q`` and ``recv_s`` hold those of an earlier dispatch."""
+        ref, version = self._delivered
+        rows = ref()
+        if rows is None or version != _version(rows):
+            raise RuntimeError("MoEExchange.received: the rows that were last delivered are gone (their tensor was released or written to); "
+                               "dispatch them again")
+        if out is None:
+            return rows.clone()
+        if out.data_ptr() != rows.data_ptr():
+            taken = torch.arange(self.cap, device=rows.device)[:, None] < plan["n_rows"]
+            out.copy_(torch.where(taken, rows, out))
+        return out
+
     def deliver(self, x: torch.Tensor, ids: torch.Tensor, plan: Dict[str, torch.Tensor], probs: Optional[torch.Tensor] = None,
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """``dispatch`` and ``received`` in one.  In a world of one nothing travels and one kernel writes the rows; the receive
-        buffers stay as they are."""
+        """``dispatch`` and ``received`` in one.  In a world of one nothing travels and one kernel writes the rows; ``recv_q`` and
+        ``recv_s`` stay as they are, and ``received`` finds the rows in the tensor returned here as long as that lives unchanged."""
         if self.eng.world > 1:
             self.dispatch(x, ids, plan, probs=probs)
             return self.received(plan, out)
@@ -222,6 +246,7 @@ class MoEExchange:
         C.moe_expand(x.data_ptr(), ids.data_ptr(), plan["rows"].data_ptr(), 0 if probs is None else probs.data_ptr(), out.data_ptr(), self.T, self.K,
                      self.H, stream_handle())
         count_launch()
+        self._delivered = weakref.ref(out), _version(out)
         return out
 
     def combine_dot(self, g: torch.Tensor, ids: torch.Tensor, plan: Dict[str, torch.Tensor]) -> torch.Tensor:

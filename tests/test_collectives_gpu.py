@@ -1217,3 +1217,57 @@ def test_moe_deliver_in_a_world_of_one(native, T, H, E, topk, drop):
         rest[rows[kept]] = False
         assert (got[rest] == 3.0).all()
     check_status("moe deliver")
+
+
+def test_moe_received_after_a_pass_in_a_world_of_one(native):
+    """``received`` (and ``experts``) behind ``forward`` or a layer's pass give that pass's rows and not those of an earlier dispatch; rows past
+    the count are left alone; rows that are gone are refused."""
+    from pccl_b200.engine import Engine
+    from pccl_b200.ops.moe import MoEExchange
+    torch.manual_seed(12)
+    T, H, F, E, topk = 33, 256, 128, 8, 2
+    eng = Engine(0, 1)
+    eng.initEngine("cuda", 640 << 20)
+    ex, fresh = MoEExchange(eng, T, H, E, topk), MoEExchange(eng, T, H, E, topk)
+    w1, w2 = (torch.randn(E * F, H, device="cuda") * 0.1).bfloat16(), (torch.randn(E * H, F, device="cuda") * 0.1).bfloat16()
+    logits, old, x = torch.randn(T, E, device="cuda"), torch.randn(T, H, device="cuda").bfloat16(), torch.randn(T, H, device="cuda").bfloat16()
+    ids, probs, plan = ex.route_and_plan(logits)
+    n = T * topk
+
+    def want(t):                                       # one row per expert, whatever order the routing gave its tokens
+        fresh.dispatch(t, ids, plan)
+        return fresh.received(plan)[:n]
+
+    def rows_of(t, p):                                 # the same by token: a pass of its own may place an expert's tokens in another order
+        return t[p["rows"].flatten().long()]
+
+    ex.dispatch(old, ids, plan)
+    with torch.no_grad():
+        ex.forward(x, logits, w1, w2)
+    for mode in (torch.no_grad, torch.inference_mode):
+        with mode():
+            ex.deliver(x, ids, plan, out=ex.x_bf16)
+            out = torch.full((ex.cap, H), 3.0, device="cuda").bfloat16()
+            assert ex.received(plan, out) is out
+            assert torch.equal(out[:n], want(x)) and (out[n:] == 3.0).all()
+            assert torch.equal(rows_of(ex.received(plan), plan), rows_of(want(x), plan))
+            ex.experts(w1, w2, plan)
+            fresh.dispatch(x, ids, plan)
+            fresh.experts(w1, w2, plan)
+            assert torch.equal(ex.y[:n], fresh.y[:n])
+    ex.dispatch(old, ids, plan)
+    assert torch.equal(ex.received(plan)[:n], want(old))
+    with torch.no_grad():                              # forward's own routing: the multiset of rows is the new tokens'
+        ex.forward(x, logits, w1, w2)
+    got = ex.received(plan)[:n].float().sum(1).sort().values
+    assert torch.equal(got, want(x).float().sum(1).sort().values)
+    kept = ex.deliver(old, ids, plan)
+    assert torch.equal(ex.received(plan)[:n], want(old))
+    kept.add_(1)
+    with pytest.raises(RuntimeError, match="gone"):
+        ex.received(plan)
+    ex.deliver(x, ids, plan)
+    with pytest.raises(RuntimeError, match="gone"):
+        ex.received(plan)
+    ex.dispatch(x, ids, plan)
+    assert torch.equal(ex.received(plan)[:n], want(x))

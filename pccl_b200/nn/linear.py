@@ -278,6 +278,11 @@ class LinearGelu(Linear):
         return _LinearGeluFn.apply(x, self.weight, self.bias)
 
 
+def row_indices(ids: torch.Tensor, rows: int) -> torch.Tensor:
+    """Flat indices of a table's rows for ``index_add_``, which takes no negative ones: those count from the end, as in the lookup."""
+    return ids.reshape(-1).remainder(rows)
+
+
 class _EmbeddingFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, ids, weight):
@@ -288,7 +293,7 @@ class _EmbeddingFn(torch.autograd.Function):
     def backward(ctx, dy):
         ids, weight = ctx.saved_tensors
         mg = _grad_target(weight)
-        flat_ids, flat_dy = ids.reshape(-1), dy.reshape(-1, dy.shape[-1])
+        flat_ids, flat_dy = row_indices(ids, weight.shape[0]), dy.reshape(-1, dy.shape[-1])
         if mg is None:
             g = torch.zeros_like(weight)
             g.index_add_(0, flat_ids, flat_dy.to(weight.dtype))

@@ -116,3 +116,19 @@ def test_layernorm_backward_ring_is_for_many_rows(native):
     assert not any(ring(1 << 20, D) for D in (8, 1024, 2048))
     assert not any(ring(rows, D) for rows, D in ((1, 2056), (600, 4096), (2368, 4096), (1, 8192), (600, 5120), (1036, 4104)))
     assert all(ring(rows, D) for rows, D in ((2369, 2056), (4096, 4096), (1037, 4104), (4096, 8192)))
+
+
+@pytest.mark.parametrize("bucket", [False, True])
+def test_embedding_backward_counts_negative_ids_from_the_end(bucket):
+    """As its forward pass does, and as the fused token and position embedding does in both."""
+    from pccl_b200.nn.linear import Embedding
+    emb, V = Embedding(7, 8), 7
+    ids = torch.tensor([[0, -1, 3], [-7, 6, -2]])
+    if bucket:
+        emb.weight.main_grad, emb.weight._pccl_written = torch.randn_like(emb.weight), False
+    y = emb(ids)
+    assert torch.equal(y, emb.weight[ids % V])
+    dy = torch.randn(y.shape).bfloat16()
+    y.backward(dy)
+    want = torch.zeros_like(emb.weight).index_add_(0, ids.flatten() % V, dy.view(-1, 8))
+    assert torch.equal(emb.weight.main_grad if bucket else emb.weight.grad, want)

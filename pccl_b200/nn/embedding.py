@@ -5,7 +5,7 @@ import torch
 
 from .._native import C
 from ..ops.gemm import count_launch, records_graph, stream_handle
-from .linear import Embedding, _finish_main_grad, _grad_target, is_plain
+from .linear import Embedding, _finish_main_grad, _grad_target, is_plain, row_indices
 from .norm import _rows
 
 
@@ -43,9 +43,15 @@ class _TokenPositionFn(torch.autograd.Function):
                 d_pos = torch.empty_like(pos)
             if not add_pos and pos.shape[0] > T:
                 d_pos[T:].zero_()
-        C.embed_bwd(dy2.data_ptr(), ids.data_ptr(), 0 if d_tok is None else d_tok.data_ptr(), 0 if d_pos is None else d_pos.data_ptr(), B, T,
-                    tok.shape[0], tok.shape[1], add_pos, stream_handle())
-        count_launch()
+        # the kernel adds the tokens' rows in no fixed order; index_add_ honours torch.use_deterministic_algorithms
+        by_kernel = d_tok
+        if d_tok is not None and torch.are_deterministic_algorithms_enabled():
+            d_tok.index_add_(0, row_indices(ids, tok.shape[0]), dy2)
+            by_kernel = None
+        if by_kernel is not None or d_pos is not None:
+            C.embed_bwd(dy2.data_ptr(), ids.data_ptr(), 0 if by_kernel is None else by_kernel.data_ptr(), 0 if d_pos is None else d_pos.data_ptr(), B, T,
+                        tok.shape[0], tok.shape[1], add_pos, stream_handle())
+            count_launch()
         for there, p in zip(in_bucket, (tok, pos)):
             if there:
                 _finish_main_grad(p)

@@ -763,3 +763,36 @@ def test_token_and_position_embedding(B, T, D, V, extra, bucket):
             assert ((g.double() - tok).abs() <= n * 2.0 ** -8 * (1 + 2.0 ** -8) ** n * mag).all()
         else:                   # B fp32 additions in another order may round to the other neighbour: one unit (2^-7) of the sum, one of the total
             assert ((g.float() - want_pos.float()).abs() <= 2.0 ** -7 * ((g - before[1]).float().abs() + g.float().abs()) + B * 2.0 ** -22).all()
+
+
+@pytest.mark.parametrize("bucket", [False, True])
+def test_embedding_gradient_repeats_itself_in_deterministic_mode(bucket):
+    """Some 1500 bf16 additions to each of three rows: any other order gives other sums.  The mode counts when the backward pass runs."""
+    from pccl_b200.nn.embedding import _fused, token_position
+    from pccl_b200.nn.linear import Embedding
+    torch.manual_seed(3)
+    wte, wpe = Embedding(3, 64, device="cuda"), Embedding(600, 64, device="cuda")
+    ids = torch.randint(-3, 3, (8, 577), device="cuda")
+    assert _fused(ids, wte, wpe)
+    dy = torch.randn(8, 577, 64, device="cuda").bfloat16()
+    got, pos = [], []
+    for step in range(6):
+        if bucket:
+            for m in (wte, wpe):
+                m.weight.main_grad, m.weight._pccl_written = torch.randn_like(m.weight), False
+        wte.weight.grad = wpe.weight.grad = None
+        y = token_position(ids, wte, wpe)
+        torch.use_deterministic_algorithms(step < 5)
+        try:
+            y.backward(dy)
+        finally:
+            torch.use_deterministic_algorithms(False)
+        got.append(wte.weight.main_grad if bucket else wte.weight.grad)
+        pos.append(wpe.weight.main_grad if bucket else wpe.weight.grad)
+    assert all(torch.equal(g, got[0]) for g in got[:5]) and all(torch.equal(p, pos[0]) for p in pos)
+    torch.use_deterministic_algorithms(True)
+    try:
+        want = torch.zeros_like(wte.weight).index_add_(0, ids.flatten() % 3, dy.view(-1, 64))
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert torch.equal(got[0], want)

@@ -10,7 +10,7 @@
 //               B's scales in full on either side)
 //   warps 4..11 epilogue: two per TMEM lane quarter, each half of the tile's strips
 //
-// TMEM columns, waits and the absence of multicast loads as in the single-CTA form.
+// TMEM columns, bounded waits (and the wait for loads in flight when a role gives up) and the absence of multicast loads as in the single-CTA form.
 #pragma once
 #include "gemm_mx8_pipeline.cuh"
 #include "gemm_pipeline2.cuh"
@@ -43,6 +43,7 @@ struct Barriers {
   uint64_t drain;
   uint32_t tmem_base;
   uint32_t abort;
+  uint32_t stopped;             // used in the leader: where its producer stopped in the ring, stage and phase << 16
 };
 static_assert(sizeof(Barriers) <= BAR_BYTES, "barriers overrun their area");
 
@@ -125,6 +126,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         }
       }
       if (!ok && atomicExch(const_cast<uint32_t*>(&bar->abort), 1u) == 0) dev::report(status, ST_TIMEOUT, blockIdx.x, 0, 0);
+      bar->stopped = static_cast<uint32_t>(stage) | phase << 16;
       dev::pdl_launch();                // the last load is on its way: the next kernel of the stream may move in
     }
   } else if (warp == 1) {
@@ -233,6 +235,10 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
 
   tc::tc_fence_before();
   __syncthreads();
+  if (warp == 0) {                    // a role gave up: the peer is held by the barrier below meanwhile
+    if (leader && lane == 0 && *abort) tc::drain_pair_loads(bar->full, STAGES, bar->stopped & 0xffff, bar->stopped >> 16);
+    __syncwarp();
+  }
   tc::cluster_sync();                 // the leader's MMAs no longer read the peer's shared memory
   if (warp == 1) {
     tc::tc_fence_after();

@@ -252,7 +252,9 @@ class MoEExchange:
     def combine_dot(self, g: torch.Tensor, ids: torch.Tensor, plan: Dict[str, torch.Tensor]) -> torch.Tensor:
         """``dot[t, k] = <g[t], y row of assignment (t, k)>`` (fp32 [tokens, topk]): with ``g`` the upstream gradient and
         the expert outputs of the forward pass still in ``self.y``, the gradient of the gate weights."""
-        out = torch.empty((self.T, self.K), dtype=torch.float32, device="cuda")
+        # a barrier between ranks that gives up leaves the rows unwritten: zeros then; a world of one has none and writes every value
+        make = torch.zeros if self.eng.world > 1 else torch.empty
+        out = make((self.T, self.K), dtype=torch.float32, device=g.device)
         self._exchange("combine_dot", g, ids, plan["rows"], None, out)
         return out
 

@@ -132,3 +132,16 @@ def test_embedding_backward_counts_negative_ids_from_the_end(bucket):
     y.backward(dy)
     want = torch.zeros_like(emb.weight).index_add_(0, ids.flatten() % V, dy.view(-1, 8))
     assert torch.equal(emb.weight.main_grad if bucket else emb.weight.grad, want)
+
+
+def test_moe_gate_gradients_are_zeros_where_the_exchange_gives_up(native, monkeypatch):
+    """Between ranks the kernel's entry barrier may run out, and then nothing is written."""
+    from types import SimpleNamespace
+    from pccl_b200.ops.moe import MoEExchange
+    ex = MoEExchange.__new__(MoEExchange)
+    ex.eng, ex.T, ex.K = SimpleNamespace(world=2), 64, 8
+    monkeypatch.setattr(ex, "_exchange", lambda *a, **k: None, raising=False)
+    made = []
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: made.append(a) or torch.full(*a, float("nan"), **k))
+    assert torch.equal(ex.combine_dot(torch.zeros(64, 128), None, {"rows": None}), torch.zeros(64, 8))
+    assert not made

@@ -289,6 +289,10 @@ PYBIND11_MODULE(_C, m) {
     o.inv_sqrt_bc2 = 1.0f / std::sqrt(1.0f - std::pow(b2, static_cast<float>(step)));
     throwIfCuda(launchReduceScatterAdamW(a, o, blocks, threads, reinterpret_cast<cudaStream_t>(stream)), "reduce_scatter_adamw");
   });
+  m.def("local_adamw_plan", [](long long count, int blocks, int threads, int sms) {
+    const LocalAdamPlan plan = localAdamPlan(count, blocks, threads, sms);
+    return py::make_tuple(plan.ctas, plan.part);
+  });
   m.def("emu_collective", &emuCollective, py::arg("kind"), py::arg("heaps"), py::arg("signal_off"), py::arg("flag_off"), py::arg("dtype"),
         py::arg("redop"), py::arg("in_off"), py::arg("out_off"), py::arg("count"), py::arg("epoch"), py::arg("flag_lane"), py::arg("scale"),
         py::arg("out_dtype"), py::arg("blocks"), py::arg("threads"), py::arg("stream"), py::arg("status"), py::arg("local_in"),

@@ -572,32 +572,43 @@ int launchReduceScatter(const CollArgs& a, int blocks, int threads, cudaStream_t
   return static_cast<int>(cudaErrorNotSupported);
 }
 
+// One CTA per SM beside the backward pass, in launches of kLocalAdamTrips trips (some 25 us): attention and the norms' backward take
+// whole SMs, and a CTA that stays for the bucket keeps them from its SM for 300 us (GPT-1.3B: 137.8 -> 135.4 ms on a GPU that ran
+// slow, on a stream of the backward pass's own priority; 2 or 8 trips the same, 136.1 with a higher priority).  A bucket above 32 Mi
+// parameters, an embedding or a head, which as a rule is the last, is one launch of four CTAs per SM (102.9 M parameters alone:
+// 610 -> 481 us, 6.0 TB/s).  A caller's `blocks` CTAs of `threads` threads are a limit on the threads of a launch.
+LocalAdamPlan localAdamPlan(long long count, int blocks, int threads, int sms) {
+  const long long per_cta = kLocalAdamTrip * (kLocalAdamThreads / 32);
+  const bool last = count > (32ll << 20);
+  LocalAdamPlan plan{last ? 4 * sms : sms, 0};
+  if (blocks > 0) {
+    const long long limit = static_cast<long long>(blocks) * threads / kLocalAdamThreads;
+    if (limit < plan.ctas) plan.ctas = limit < 1 ? 1 : static_cast<int>(limit);
+  }
+  plan.part = last ? count : plan.ctas * kLocalAdamTrips * per_cta;
+  return plan;
+}
+
 int launchReduceScatterAdamW(const CollArgs& a, const AdamArgs& o, int blocks, int threads, cudaStream_t stream) {
   if (a.dtype != DT_BF16 || a.nvirt > 1 || a.count % 8 || a.flag_lane < 0 || a.flag_lane >= 8) return static_cast<int>(cudaErrorInvalidValue);
   if (a.algo == ALGO_NVLS && !a.w.mc_heap) return static_cast<int>(cudaErrorInvalidValue);
-  if (blocks < 1) blocks = 1;
-  if (blocks > kMaxBlocksPerColl) blocks = kMaxBlocksPerColl;
   if (a.w.world == 1 && a.algo != ALGO_NVLS) {
-    // One CTA per SM beside the backward pass, in launches of kLocalAdamTrips trips (some 25 us): attention and the norms' backward take
-    // whole SMs, and a CTA that stays for the bucket keeps them from its SM for 300 us (GPT-1.3B: 137.8 -> 135.4 ms on a GPU that ran
-    // slow, on a stream of the backward pass's own priority; 2 or 8 trips the same, 136.1 with a higher priority).  A bucket above 32 Mi
-    // parameters, an embedding or a head, which as a rule is the last, is one launch of four CTAs per SM (102.9 M parameters alone:
-    // 610 -> 481 us, 6.0 TB/s).
     const long long count = static_cast<long long>(a.count), per_cta = kLocalAdamTrip * (kLocalAdamThreads / 32);
-    const bool last = count > (32ll << 20);
-    const long long sms = deviceSmCount(), part = last ? count : sms * kLocalAdamTrips * per_cta;
+    const LocalAdamPlan plan = localAdamPlan(count, blocks, threads, deviceSmCount());
     const __nv_bfloat16* grads = reinterpret_cast<const __nv_bfloat16*>(a.w.heap[a.rank] + a.in_off);
-    for (long long at = 0; at < count; at += part) {
-      const long long n = count - at < part ? count - at : part, trips = (n + per_cta - 1) / per_cta, most = last ? 4 * sms : sms;
+    for (long long at = 0; at < count; at += plan.part) {
+      const long long n = count - at < plan.part ? count - at : plan.part, trips = (n + per_cta - 1) / per_cta;
       AdamArgs q = o;
       q.p += at;
       q.m += at;
       q.v += at;
       q.p_bf16 = static_cast<__nv_bfloat16*>(o.p_bf16) + at;
-      local_adamw_kernel<<<static_cast<unsigned>(trips < most ? trips : most), kLocalAdamThreads, 0, stream>>>(grads + at, q, n, a.scale);
+      local_adamw_kernel<<<static_cast<unsigned>(trips < plan.ctas ? trips : plan.ctas), kLocalAdamThreads, 0, stream>>>(grads + at, q, n, a.scale);
     }
     return static_cast<int>(cudaGetLastError());
   }
+  if (blocks < 1) blocks = 1;
+  if (blocks > kMaxBlocksPerColl) blocks = kMaxBlocksPerColl;
   void* args[] = {const_cast<CollArgs*>(&a), const_cast<AdamArgs*>(&o)};
   void* kern = a.algo == ALGO_NVLS ? reinterpret_cast<void*>(reduce_scatter_adamw_kernel<true>)
                                    : reinterpret_cast<void*>(reduce_scatter_adamw_kernel<false>);

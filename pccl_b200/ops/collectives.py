@@ -81,16 +81,17 @@ def reduce_scatter_adamw(eng: Engine, grads: torch.Tensor, master: torch.Tensor,
                          lane: int = 0, stream=None) -> None:
     """Gradient-bucket reduce-scatter fused with the sharded AdamW step.  ``grads`` is the symmetric bf16
     bucket (world * n elements); ``master`` / ``exp_avg`` / ``exp_avg_sq`` are this rank's fp32 slices (n
-    elements, n % 8 == 0); the updated parameters are written to ``param_bf16`` (bf16, n elements).  A world of one has a kernel of
-    its own with a grid of its own; ``blocks`` and ``threads`` are for the exchange."""
+    elements, n % 8 == 0); the updated parameters are written to ``param_bf16`` (bf16, n elements).  In a world of one
+    nothing is exchanged and a kernel with a grid of its own runs; ``blocks``, if given, is a limit of ``blocks * threads`` threads on it."""
     n = master.numel()
     if grads.dtype != torch.bfloat16 or grads.numel() != n * eng.world or n % 8:
         raise ValueError("reduce_scatter_adamw: bf16 bucket of world * n elements with n % 8 == 0 expected")
     a = _algo(eng, algo, "bf16", "sum", n * 2)
+    ctas = 0 if eng.world == 1 and a != "nvls" and not blocks else _blocks(n * 2, blocks)
     s = stream.cuda_stream if stream is not None else stream_handle()
     C.reduce_scatter_adamw(eng.raw, a, eng.heap_offset(grads), n, lane, float(scale), master.data_ptr(), exp_avg.data_ptr(),
                            exp_avg_sq.data_ptr(), param_bf16.data_ptr(), lr, betas[0], betas[1], eps, weight_decay, step,
-                           _blocks(n * 2, blocks), threads, s)
+                           ctas, threads, s)
     count_launch()
 
 

@@ -81,9 +81,10 @@ class ShardedDataParallel:
         # With ranks to exchange with, communication kernels run as short, wide bursts on a high-priority stream: they slip in at the
         # boundary between two GEMM kernels and delay the next one by their own (tens of microseconds)
         # duration.  A narrow long-running kernel would instead hold a few SMs for the whole GEMM and make
-        # the persistent GEMM's last CTAs start a full wave late.  (A world of one exchanges nothing and has a kernel of its own,
-        # which runs beside the GEMMs and takes no block count.)
+        # the persistent GEMM's last CTAs start a full wave late.  (The fused update of a world of one exchanges nothing; it has a kernel of
+        # its own that runs beside the GEMMs, with a grid of its own unless the caller set a count.)
         self.comm_blocks = comm_blocks if comm_blocks else (128 if engine.world == 1 else 64)
+        self._update_blocks = None if engine.world == 1 and not comm_blocks else self.comm_blocks
         # A world of one has no peers to keep waiting: its update stands back behind the backward pass's kernels.
         self.comm_stream = torch.cuda.Stream(priority=-1 if engine.world > 1 else 0)
         self.step_count = 0
@@ -233,7 +234,7 @@ class ShardedDataParallel:
         dst = b.values[self.rank * shard:(self.rank + 1) * shard]
         coll.reduce_scatter_adamw(self.engine, b.grads, b.master, b.exp_avg, b.exp_avg_sq, dst, lr=self.lr, betas=self.betas,
                                   eps=self.eps, weight_decay=self.weight_decay if b.decay else 0.0, step=self.step_count,
-                                  scale=1.0 / self.world, algo=self.algo, blocks=self.comm_blocks, lane=1, stream=self.comm_stream)
+                                  scale=1.0 / self.world, algo=self.algo, blocks=self._update_blocks, lane=1, stream=self.comm_stream)
         if reduced_mark is not None:
             reduced_mark.record(self.comm_stream)
         if self.world > 1:

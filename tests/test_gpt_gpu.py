@@ -138,6 +138,29 @@ def test_bucket_update_in_a_world_of_one(n):
     assert (pad[:32] == 7).all() and (pad[32 + n:] == 7).all()
 
 
+def test_bucket_update_with_a_block_count_of_the_callers(monkeypatch):
+    """A wrapper hands its own count on, none otherwise; any count gives the same bits."""
+    from pccl_b200.models import GPT, GPTConfig
+    from pccl_b200.ops import collectives as coll
+    from pccl_b200.parallel.dp import ShardedDataParallel
+    seen, update = [], coll.reduce_scatter_adamw
+    monkeypatch.setattr(coll, "reduce_scatter_adamw", lambda *a, **k: (seen.append(k["blocks"]), update(*a, **k)))
+    masters = []
+    for blocks in (None, 3):
+        torch.manual_seed(1)
+        model = GPT(GPTConfig.tiny(), device="cuda")
+        dp = ShardedDataParallel(model, heap_bytes=256 << 20, comm_blocks=blocks)
+        seen.clear()
+        dp.zero_grad()
+        for b in dp.buckets:                                   # the update alone: gradients made here
+            b.grads.copy_(torch.randn(b.numel, device="cuda"))
+            dp._launch_reduce(b)
+        torch.cuda.synchronize()
+        assert seen and set(seen) == {blocks}
+        masters.append([b.master.clone() for b in dp.buckets])
+    assert all(torch.equal(a, b) for a, b in zip(*masters))
+
+
 def test_sharded_dp_world_of_one_trains_and_matches_plain_adamw():
     from pccl_b200.models import GPT, GPTConfig
     from pccl_b200.models.gpt import smoke_step

@@ -145,3 +145,12 @@ def test_moe_gate_gradients_are_zeros_where_the_exchange_gives_up(native, monkey
     monkeypatch.setattr(torch, "empty", lambda *a, **k: made.append(a) or torch.full(*a, float("nan"), **k))
     assert torch.equal(ex.combine_dot(torch.zeros(64, 128), None, {"rows": None}), torch.zeros(64, 8))
     assert not made
+
+
+def test_bucket_update_of_a_world_of_one_keeps_to_the_callers_blocks(native):
+    plan = lambda count, blocks=0, threads=512: native.local_adamw_plan(count, blocks, threads, 148)  # noqa: E731   (CTAs of 128 threads, parameters)
+    trip = 4 * 4 * 512                                         # parameters of a CTA in a launch: four trips of four warps
+    assert plan(13 << 20) == (148, 148 * trip)
+    assert plan(13 << 20, 8) == (32, 32 * trip) and plan(13 << 20, 1, 32) == (1, trip) and plan(13 << 20, 128) == (148, 148 * trip)
+    big = 102_900_000
+    assert plan(big) == (592, big) and plan(big, 8) == (32, big) and plan(big, 148) == (592, big)

@@ -2,12 +2,12 @@
 
 Gradients live in flat bf16 buckets (25 MB by default) inside the symmetric heap.  The moment the
 last gradient of a bucket has been written (the weight-gradient GEMMs write there directly), ONE
-kernel is queued on a side stream (of high priority where ranks wait for it): each rank reduces its 1/world slice of the bucket
+kernel is queued on a side stream (of high priority, but for the fused update of a world of one): each rank reduces its 1/world slice of the bucket
 (multimem.ld_reduce through the switch, or loads from every peer over NVLink), multiplies by
 1/world and applies AdamW to its fp32 master slice -- reduction, scaling, cast and optimizer in one
 pass -- and writes the new bf16 parameters, which the bucket's all-gather kernel then pushes to
 every rank (ZeRO-1).  The kernels run as short, wide bursts (64 CTAs) that slip in between
-two GEMM kernels of backward.  With a world of one the reduce-scatter is a flat scale/cast/update pass
+two GEMM kernels of backward.  With a world of one the fused reduce-scatter is a flat scale/cast/update pass
 over the bucket in short launches, whose small CTAs run beside the GEMMs' on the same SMs.
 ``fuse_optimizer=False`` keeps the reduce-scatter (with scale and fp32 cast) and the optimizer apart.
 """
@@ -85,8 +85,8 @@ class ShardedDataParallel:
         # its own that runs beside the GEMMs, with a grid of its own unless the caller set a count.)
         self.comm_blocks = comm_blocks if comm_blocks else (128 if engine.world == 1 else 64)
         self._update_blocks = None if engine.world == 1 and not comm_blocks else self.comm_blocks
-        # A world of one has no peers to keep waiting: its update stands back behind the backward pass's kernels.
-        self.comm_stream = torch.cuda.Stream(priority=-1 if engine.world > 1 else 0)
+        # The fused update of a world of one keeps no peers waiting: its short launches take their turn among the backward pass's kernels.
+        self.comm_stream = torch.cuda.Stream(priority=0 if engine.world == 1 and fuse_optimizer else -1)
         self.step_count = 0
         self._plan_schedule(int(bucket_mb * (1 << 20)), schedule, topology)
         self._build_buckets(params, int(bucket_mb * (1 << 20)) // 2)

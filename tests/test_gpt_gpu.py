@@ -161,6 +161,19 @@ def test_bucket_update_with_a_block_count_of_the_callers(monkeypatch):
     assert all(torch.equal(a, b) for a, b in zip(*masters))
 
 
+@pytest.mark.parametrize("fused", [True, False])
+def test_stream_priority_in_a_world_of_one(fused):
+    """The plain reduce-scatter and optimizer of the unfused mode go first; the fused update's short launches do not."""
+    from pccl_b200.models import GPT, GPTConfig
+    from pccl_b200.parallel.dp import ShardedDataParallel
+    torch.manual_seed(1)
+    dp = ShardedDataParallel(GPT(GPTConfig.tiny(), device="cuda"), heap_bytes=256 << 20, fuse_optimizer=fused)
+    assert dp.comm_stream.priority == (0 if fused else -1)
+    ids = torch.randint(0, 1001, (2, 128), device="cuda")
+    losses = [dp.train_step(ids, ids.roll(-1, 1)).item() for _ in range(3)]
+    assert losses[-1] < losses[0]
+
+
 def test_sharded_dp_world_of_one_trains_and_matches_plain_adamw():
     from pccl_b200.models import GPT, GPTConfig
     from pccl_b200.models.gpt import smoke_step

@@ -90,6 +90,7 @@ void bindFused(py::module_& m) {
                          reinterpret_cast<int*>(pos), reinterpret_cast<int*>(counts), tokens, experts, topk,
                          reinterpret_cast<cudaStream_t>(stream)), "moe_route");
   });
+  m.def("moe_group_threads", &moeGroupThreads);
   m.def("moe_route_backward", [](uint64_t logits, uint64_t ids, uint64_t dprobs, uint64_t dlogits, int tokens, int experts, int topk, uint64_t stream) {
     check(launchMoeRouteBackward(reinterpret_cast<const float*>(logits), reinterpret_cast<const int*>(ids), reinterpret_cast<const float*>(dprobs),
                                  reinterpret_cast<float*>(dlogits), tokens, experts, topk, reinterpret_cast<cudaStream_t>(stream)), "moe_route_backward");

@@ -1064,23 +1064,28 @@ int dispatchGroups(const MoeArgs& a, int blocks, cudaStream_t stream) {
   return coop(moe_dispatch_kernel<GT>, a, blocks, smem, stream, GT * subs, subs, 1);
 }
 
-// Tokens from which groups of 64 threads are taken: two for every group of 256 that the blocks hold (64 tokens x 7168 stay as they were,
-// 700 x 1024 takes 5.6 -> 3.6 us in the combine).
-bool smallGroups(const MoeArgs& a, int blocks, int subs256) { return a.tokens >= 2 * subs256 * (blocks < 1 ? 1 : blocks); }
-
 }  // namespace
 
+// Groups of 64 threads are taken in a world of one, from two tokens on for every group of 256 that the blocks hold (64 tokens x 7168 stay as
+// they were, 700 x 1024 takes 5.6 -> 3.6 us in the combine).  Between ranks, where rows cross NVLink and barriers frame the kernel, groups
+// of 256 are what was measured.
+int moeGroupThreads(bool dispatch, int tokens, int blocks, int world) {
+  return world == 1 && tokens >= 2 * (dispatch ? kDispatchSubs<256> : kCombineSubs<256>) * (blocks < 1 ? 1 : blocks) ? 64 : 256;
+}
+
 int launchMoeDispatch(const MoeArgs& a, int blocks, cudaStream_t stream) {
-  return smallGroups(a, blocks, kDispatchSubs<256>) ? dispatchGroups<64>(a, blocks, stream) : dispatchGroups<256>(a, blocks, stream);
+  return moeGroupThreads(true, a.tokens, blocks, a.w.world) == 64 ? dispatchGroups<64>(a, blocks, stream) : dispatchGroups<256>(a, blocks, stream);
 }
 
 int launchMoeCombine(const MoeArgs& a, int blocks, cudaStream_t stream) {
-  return smallGroups(a, blocks, kCombineSubs<256>) ? coop(moe_combine_kernel<64>, a, blocks, 0, stream, 64 * kCombineSubs<64>, kCombineSubs<64>, 1)
-                                                   : coop(moe_combine_kernel<256>, a, blocks, 0, stream, 256 * kCombineSubs<256>, kCombineSubs<256>, 1);
+  return moeGroupThreads(false, a.tokens, blocks, a.w.world) == 64
+             ? coop(moe_combine_kernel<64>, a, blocks, 0, stream, 64 * kCombineSubs<64>, kCombineSubs<64>, 1)
+             : coop(moe_combine_kernel<256>, a, blocks, 0, stream, 256 * kCombineSubs<256>, kCombineSubs<256>, 1);
 }
 int launchMoeCombineDot(const MoeArgs& a, int blocks, cudaStream_t stream) {
-  return smallGroups(a, blocks, kCombineSubs<256>) ? coop(moe_combine_dot_kernel<64>, a, blocks, 0, stream, 64 * kCombineSubs<64>, kCombineSubs<64>, 1)
-                                                   : coop(moe_combine_dot_kernel<256>, a, blocks, 0, stream, 256 * kCombineSubs<256>, kCombineSubs<256>, 2);
+  return moeGroupThreads(false, a.tokens, blocks, a.w.world) == 64
+             ? coop(moe_combine_dot_kernel<64>, a, blocks, 0, stream, 64 * kCombineSubs<64>, kCombineSubs<64>, 1)
+             : coop(moe_combine_dot_kernel<256>, a, blocks, 0, stream, 256 * kCombineSubs<256>, kCombineSubs<256>, 2);
 }
 
 int launchMoeDequant(const void* q, const float* scales, void* out, const int* n_rows, int max_rows, int hidden, const int* alias,

@@ -42,6 +42,7 @@ struct MoeArgs {
 // fp8 (e4m3, one fp32 scale per 128 values) quantisation fused with the push to the experts' ranks.  With `probs` set,
 // destination k of token t receives probs[t,k] * x[t] (the backward pass sends gate-weighted output gradients this way).
 int launchMoeDispatch(const MoeArgs& a, int blocks, cudaStream_t stream);
+int moeGroupThreads(bool dispatch, int tokens, int blocks, int world);   // threads that work on one token in the dispatch, or the combines
 // out (fp32 [tokens, topk]) = <x[t], y[rank of expert (t,k)][dst_rows[t,k]]>: gradients of the gate weights.
 int launchMoeCombineDot(const MoeArgs& a, int blocks, cudaStream_t stream);
 // out[t] = sum_k probs[t,k] * y[rank of expert (t,k)][dst_rows[t,k]]: pulls the rows over NVLink.  Without probs a plain sum.

@@ -560,11 +560,12 @@ def test_grouped_weight_gradients(native, M, N, sizes):
             assert (d[g].double() - ref).abs().le(2 ** -8 * ref.abs() + 1e-4).all()
 
 
-def test_moe_dispatch_combine_emulated(native):
+@pytest.mark.parametrize("T,blocks", [(64, 8), (20, 8), (300, 2)])      # one token per group of threads, groups without a token, many trips
+def test_moe_dispatch_combine_emulated(native, T, blocks):
     """Two emulated ranks: fp8 dispatch lands in the right rows with the right scales; combine pulls
     rows back from both ranks and weights them."""
-    world, T, H, Kt, epr = 2, 64, 256, 2, 2
-    cap = 512
+    world, H, Kt, epr = 2, 256, 2, 2
+    cap = max(512, world * T * Kt)
     q_off, s_off, y_off = DATA_OFF, DATA_OFF + cap * H, DATA_OFF + cap * H + cap * (H // 128) * 4
     heaps = [torch.zeros(y_off + cap * H * 2, dtype=torch.uint8, device="cuda") for _ in range(world)]
     st = [torch.zeros(4, dtype=torch.int32, device="cuda") for _ in range(world)]
@@ -578,7 +579,7 @@ def test_moe_dispatch_combine_emulated(native):
     stream = torch.cuda.current_stream().cuda_stream
     native.moe_exchange("dispatch", None, [h.data_ptr() for h in heaps], FLAG_OFF, T, H, Kt, epr, q_off, s_off, y_off, 1, 0,
                         [x.data_ptr() for x in xs], [i.data_ptr() for i in ids], [r.data_ptr() for r in rows], [], [],
-                        [s.data_ptr() for s in st], 8, 0, stream)
+                        [s.data_ptr() for s in st], blocks, 0, stream)
     torch.cuda.synchronize()
     assert all(s[0].item() == 0 for s in st)
     from pccl_b200.ops.moe import quant_fp8_rows
@@ -598,7 +599,7 @@ def test_moe_dispatch_combine_emulated(native):
         ys.append(y)
     native.moe_exchange("combine", None, [h.data_ptr() for h in heaps], FLAG_OFF, T, H, Kt, epr, q_off, s_off, y_off, 2, 0,
                         [], [i.data_ptr() for i in ids], [r.data_ptr() for r in rows], [p.data_ptr() for p in probs],
-                        [o.data_ptr() for o in outs], [s.data_ptr() for s in st], 8, 0, stream)
+                        [o.data_ptr() for o in outs], [s.data_ptr() for s in st], blocks, 0, stream)
     torch.cuda.synchronize()
     assert all(s[0].item() == 0 for s in st)
     for r in range(world):
@@ -610,12 +611,13 @@ def test_moe_dispatch_combine_emulated(native):
         assert (outs[r].float() - ref).abs().max().item() < 0.05
 
 
-def test_moe_deduplicated_exchange_emulated(native):
+@pytest.mark.parametrize("T,blocks", [(64, 8), (20, 8), (300, 2)])
+def test_moe_deduplicated_exchange_emulated(native, T, blocks):
     """Two emulated ranks, four assignments per token over four experts: most tokens have several assignments on one
     rank.  The dispatch sends the row once per rank and tells the others where it is; the conversion to bf16 fills every
     row; the ranks add up each token's weighted expert outputs locally and the combine pulls one row per rank."""
-    world, T, H, Kt, epr = 2, 64, 256, 4, 2
-    cap = 1024
+    world, H, Kt, epr = 2, 256, 4, 2
+    cap = max(1024, world * T * Kt)
     G = H // 128
     q_off = DATA_OFF
     s_off = q_off + cap * H
@@ -636,7 +638,7 @@ def test_moe_deduplicated_exchange_emulated(native):
     hp = [h.data_ptr() for h in heaps]
     native.moe_exchange("dispatch", None, hp, FLAG_OFF, T, H, Kt, epr, q_off, s_off, y_off, 1, 0,
                         [x.data_ptr() for x in xs], [i.data_ptr() for i in ids], [r.data_ptr() for r in rows], [], [],
-                        [s.data_ptr() for s in st], 8, 0, stream, alias_off=alias_off, group_off=group_off, z_off=z_off,
+                        [s.data_ptr() for s in st], blocks, 0, stream, alias_off=alias_off, group_off=group_off, z_off=z_off,
                         gate=[p.data_ptr() for p in probs], dedupe=True)
     torch.cuda.synchronize()
     assert all(s[0].item() == 0 for s in st)
@@ -679,7 +681,7 @@ def test_moe_deduplicated_exchange_emulated(native):
                                  heaps[d].data_ptr() + group_off, n_rows.data_ptr(), cap, H, stream)
     native.moe_exchange("combine", None, hp, FLAG_OFF, T, H, Kt, epr, q_off, s_off, y_off, 2, 0,
                         [], [i.data_ptr() for i in ids], [r.data_ptr() for r in rows], [p.data_ptr() for p in probs],
-                        [o.data_ptr() for o in outs], [s.data_ptr() for s in st], 8, 0, stream, alias_off=alias_off,
+                        [o.data_ptr() for o in outs], [s.data_ptr() for s in st], blocks, 0, stream, alias_off=alias_off,
                         group_off=group_off, z_off=z_off, dedupe=True)
     torch.cuda.synchronize()
     assert all(s[0].item() == 0 for s in st)

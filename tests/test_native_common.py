@@ -154,3 +154,10 @@ def test_bucket_update_of_a_world_of_one_keeps_to_the_callers_blocks(native):
     assert plan(13 << 20, 8) == (32, 32 * trip) and plan(13 << 20, 1, 32) == (1, trip) and plan(13 << 20, 128) == (148, 148 * trip)
     big = 102_900_000
     assert plan(big) == (592, big) and plan(big, 8) == (32, big) and plan(big, 148) == (592, big)
+
+
+def test_moe_exchange_between_ranks_keeps_the_groups_that_were_measured(native):
+    for dispatch, per_block in ((True, 6), (False, 4)):
+        assert native.moe_group_threads(dispatch, 148 * per_block, 148, 1) == 64
+        assert native.moe_group_threads(dispatch, 148 * per_block - 1, 148, 1) == 256
+        assert all(native.moe_group_threads(dispatch, 1 << 20, blocks, world) == 256 for blocks in (1, 148) for world in (2, 4, 8))

@@ -288,6 +288,9 @@ PYBIND11_MODULE(_C, m) {
     o.inv_bc1 = 1.0f / (1.0f - std::pow(b1, static_cast<float>(step)));
     o.inv_sqrt_bc2 = 1.0f / std::sqrt(1.0f - std::pow(b2, static_cast<float>(step)));
     throwIfCuda(launchReduceScatterAdamW(a, o, blocks, threads, reinterpret_cast<cudaStream_t>(stream)), "reduce_scatter_adamw");
+    if (a.w.world > 1 || a.algo == ALGO_NVLS) return 1ll;
+    const long long n = static_cast<long long>(count), part = localAdamPlan(n, blocks, threads, deviceSmCount()).part;
+    return (n + part - 1) / part;       // kernels launched
   });
   m.def("local_adamw_plan", [](long long count, int blocks, int threads, int sms) {
     const LocalAdamPlan plan = localAdamPlan(count, blocks, threads, sms);

@@ -89,10 +89,9 @@ def reduce_scatter_adamw(eng: Engine, grads: torch.Tensor, master: torch.Tensor,
     a = _algo(eng, algo, "bf16", "sum", n * 2)
     ctas = 0 if eng.world == 1 and a != "nvls" and not blocks else _blocks(n * 2, blocks)
     s = stream.cuda_stream if stream is not None else stream_handle()
-    C.reduce_scatter_adamw(eng.raw, a, eng.heap_offset(grads), n, lane, float(scale), master.data_ptr(), exp_avg.data_ptr(),
-                           exp_avg_sq.data_ptr(), param_bf16.data_ptr(), lr, betas[0], betas[1], eps, weight_decay, step,
-                           ctas, threads, s)
-    count_launch()
+    count_launch(C.reduce_scatter_adamw(eng.raw, a, eng.heap_offset(grads), n, lane, float(scale), master.data_ptr(), exp_avg.data_ptr(),
+                                        exp_avg_sq.data_ptr(), param_bf16.data_ptr(), lr, betas[0], betas[1], eps, weight_decay, step,
+                                        ctas, threads, s))
 
 
 def all_reduce_fp8(eng: Engine, q: torch.Tensor, s: torch.Tensor, out_q: Optional[torch.Tensor] = None,

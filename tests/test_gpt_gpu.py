@@ -138,6 +138,23 @@ def test_bucket_update_in_a_world_of_one(n):
     assert (pad[:32] == 7).all() and (pad[32 + n:] == 7).all()
 
 
+def test_launches_of_the_bucket_update_are_counted():
+    from pccl_b200.engine import Engine
+    from pccl_b200.ops import collectives as coll, launch_count
+    n = 303112
+    eng = Engine(0, 1)
+    eng.initEngine("cuda", 640 << 20)
+    g = eng.symmetric_tensor((n,), torch.bfloat16, align=256)
+    g.zero_()
+    p, m, v = (torch.zeros(n, device="cuda") for _ in range(3))
+    out = torch.empty(n, device="cuda", dtype=torch.bfloat16)
+    for blocks, threads, launches in ((None, 512, 1), (1, 128, 38), (2, 128, 19)):        # 8192 parameters per CTA of 128 threads and launch; 148 CTAs
+        before = launch_count()
+        coll.reduce_scatter_adamw(eng, g, p, m, v, out, lr=1e-2, blocks=blocks, threads=threads)
+        assert launch_count() - before == launches
+    torch.cuda.synchronize()
+
+
 def test_bucket_update_with_a_block_count_of_the_callers(monkeypatch):
     """A wrapper hands its own count on, none otherwise; any count gives the same bits."""
     from pccl_b200.models import GPT, GPTConfig

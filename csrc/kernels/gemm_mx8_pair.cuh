@@ -43,7 +43,6 @@ struct Barriers {
   uint64_t drain;
   uint32_t tmem_base;
   uint32_t abort;
-  uint32_t stopped;             // used in the leader: where its producer stopped in the ring, stage and phase << 16
 };
 static_assert(sizeof(Barriers) <= BAR_BYTES, "barriers overrun their area");
 
@@ -126,7 +125,6 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         }
       }
       if (!ok && atomicExch(const_cast<uint32_t*>(&bar->abort), 1u) == 0) dev::report(status, ST_TIMEOUT, blockIdx.x, 0, 0);
-      bar->stopped = static_cast<uint32_t>(stage) | phase << 16;
       dev::pdl_launch();                // the last load is on its way: the next kernel of the stream may move in
     }
   } else if (warp == 1) {
@@ -172,7 +170,10 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         tc::mma_commit_pair(&bar->tmem_full[acc], 3);          // accumulator ready in both CTAs
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
-      if (!ok && atomicExch(const_cast<uint32_t*>(&bar->abort), 1u) == 0) dev::report(status, ST_TIMEOUT, blockIdx.x, 1, 0);
+      if (!ok) {
+        if (atomicExch(const_cast<uint32_t*>(&bar->abort), 1u) == 0) dev::report(status, ST_TIMEOUT, blockIdx.x, 1, 0);
+        tc::drain_pair_loads(bar->full, STAGES, stage, phase);
+      }
       tc::mma_commit_pair(&bar->drain, 1);
       for (uint32_t i = 0; i < (1u << 20) && !tc::mbar_try_wait(&bar->drain, 0); ++i) {}
     }
@@ -235,10 +236,6 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
 
   tc::tc_fence_before();
   __syncthreads();
-  if (warp == 0) {                    // a role gave up: the peer is held by the barrier below meanwhile
-    if (leader && lane == 0 && *abort) tc::drain_pair_loads(bar->full, STAGES, bar->stopped & 0xffff, bar->stopped >> 16);
-    __syncwarp();
-  }
   tc::cluster_sync();                 // the leader's MMAs no longer read the peer's shared memory
   if (warp == 1) {
     tc::tc_fence_after();

@@ -49,7 +49,6 @@ struct Barriers {
   uint32_t drained[2];          // per CTA: epilogue warps that are done with the accumulator
   uint32_t tmem_base;
   uint32_t abort;
-  uint32_t stopped;             // used in the leader: where its producer stopped in the ring, stage and phase << 16
 };
 static_assert(sizeof(Barriers) <= BAR_BYTES, "barriers overrun their area");
 
@@ -263,7 +262,6 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         }
       }
       if (!ok && atomicExch(const_cast<uint32_t*>(&bar->abort), 1u) == 0) dev::report(status, ST_TIMEOUT, blockIdx.x, 0, 0);
-      bar->stopped = static_cast<uint32_t>(stage) | phase << 16;
       // The last load is on its way: the next kernel of the stream may move in.  Not earlier: its CTAs would wait on the SMs for
       // the whole of this kernel, in the places that a kernel of another stream (the optimizer's) could work in.
       dev::pdl_launch();
@@ -307,7 +305,10 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         tc::mma_commit_pair(&bar->tmem_full[acc], 3);       // accumulator ready in both CTAs
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
-      if (!ok && atomicExch(const_cast<uint32_t*>(&bar->abort), 1u) == 0) dev::report(status, ST_TIMEOUT, blockIdx.x, 1, 0);
+      if (!ok) {
+        if (atomicExch(const_cast<uint32_t*>(&bar->abort), 1u) == 0) dev::report(status, ST_TIMEOUT, blockIdx.x, 1, 0);
+        tc::drain_pair_loads(bar->full, NSTAGES, stage, phase);
+      }
       tc::mma_commit_pair(&bar->drain, 1);
       for (uint32_t i = 0; i < (1u << 20) && !tc::mbar_try_wait(&bar->drain, 0); ++i) {}
     }
@@ -352,10 +353,6 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
 
   tc::tc_fence_before();
   __syncthreads();
-  if (warp == 0) {                    // a role gave up: the peer is held by the barrier below meanwhile
-    if (leader && lane == 0 && *abort) tc::drain_pair_loads(bar->full, NSTAGES, bar->stopped & 0xffff, bar->stopped >> 16);
-    __syncwarp();
-  }
   tc::cluster_sync();                 // the leader's MMAs no longer read the peer's shared memory
   if (warp == 1) {
     tc::tc_fence_after();

@@ -222,18 +222,16 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
     }
   }
 }
-// What the leader of a CTA pair does with the pair's loads when the kernel gives up: they write shared memory of both CTAs, so neither may leave
-// before they have landed.  `stage` and `phase` are where the producer stopped: the slots below `stage` were armed in this lap of the ring, the
-// others in the lap before (or never: a new barrier passes for the phase before its first).  Not longer than two milliseconds: a slot for which the
-// other CTA issued nothing does not complete, and what was issued takes microseconds.
+// What the MMA thread of a CTA pair does with the pair's loads when it gives up: they write shared memory of both CTAs, so neither may leave
+// before they have landed, and the pair's last barrier holds both until this thread is there.  From `stage` on (in `phase`, and in the next
+// lap below `stage`) lie the slots that it has not consumed.  For some two milliseconds at most: a slot for which nothing, or one CTA's half only,
+// was issued does not complete, and what was issued takes microseconds.
 __device__ __forceinline__ void drain_pair_loads(uint64_t* full, int stages, int stage, uint32_t phase) {
-  uint64_t t0, t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+  int tries = 100;                    // of 20 us each
+#pragma unroll 1
   for (int s = 0; s < stages; ++s) {
-    while (!mbar_try_wait_for(&full[s], s < stage ? phase : phase ^ 1, 20 * 1000)) {
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      if (t - t0 > 2000 * 1000) return;
-    }
+#pragma unroll 1
+    while (tries > 0 && !mbar_try_wait_for(&full[s], s < stage ? phase ^ 1 : phase, 20 * 1000)) --tries;
   }
 }
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {

@@ -42,17 +42,17 @@ def test_kernels_that_start_early_promise_nothing_about_their_inputs():
 
 def test_kernels_that_give_up_wait_for_their_loads():
     """A TMA load writes shared memory whenever it lands: a kernel whose waits have run out stays, for a bounded time, until its loads have landed.
-    One CTA waits for the slots that it armed; a CTA pair's loads are counted in the leader, which waits before the pair's last barrier."""
+    One CTA waits for the slots that it armed; a CTA pair's loads are counted in the leader, whose MMA thread waits for those it has not used."""
     found = {"single": 0, "pair": 0}
     for path in sorted(KERNELS.glob("*.cu*")):
         for signature, body in _functions(_code(path)):
             where = f"{path.name}: {' '.join(signature.split())}"
             if "tma_load_2d_pair(" in body:
                 found["pair"] += 1
-                tail = body[body.rindex("tma_load_2d_pair("):]
-                assert re.search(r"bar->stopped\s*=.*stage.*phase", tail), where
-                assert re.search(r"\*abort\)\s*tc::drain_pair_loads\(bar->full, \w*STAGES,", tail), where
-                assert tail.index("drain_pair_loads(") < tail.rindex("cluster_sync()"), where
+                issuer = body[body.rindex("tma_load_2d_pair("):]
+                gave_up = issuer[issuer.index("if (!ok) {"):]
+                assert re.match(r"if \(!ok\) \{[^}]*drain_pair_loads\(bar->full, \w*STAGES, stage, phase\);\s*\}", gave_up), where
+                assert issuer.index("drain_pair_loads(") < issuer.rindex("cluster_sync()"), where
             elif "tma_load_2d(" in body:
                 found["single"] += 1
                 assert re.search(r"if \(armed & \(1u << s\)\)", body), where

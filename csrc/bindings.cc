@@ -277,7 +277,7 @@ PYBIND11_MODULE(_C, m) {
         py::arg("s_in_off") = 0, py::arg("s_out_off") = 0);
   m.def("reduce_scatter_adamw", [](Engine& e, const std::string& algo, uint64_t in_off, uint64_t count, int flag_lane, float scale,
                                    uint64_t p, uint64_t mm, uint64_t v, uint64_t p_bf16, float lr, float b1, float b2, float eps,
-                                   float wd, int step, int blocks, int threads, uint64_t stream) {
+                                   float wd, int step, int blocks, int threads, bool beside, uint64_t stream) {
     CollArgs a = makeCollArgs(e.worldTable(), 1, e.rank(), algo, "bf16", "sum", in_off, 0, count, e.nextEpoch(flag_lane), flag_lane,
                               scale, "", 0);
     a.status[0] = reinterpret_cast<uint32_t*>(e.statusPtr(8 + flag_lane));
@@ -287,13 +287,13 @@ PYBIND11_MODULE(_C, m) {
     o.lr = lr; o.b1 = b1; o.b2 = b2; o.eps = eps; o.wd = wd;
     o.inv_bc1 = 1.0f / (1.0f - std::pow(b1, static_cast<float>(step)));
     o.inv_sqrt_bc2 = 1.0f / std::sqrt(1.0f - std::pow(b2, static_cast<float>(step)));
-    throwIfCuda(launchReduceScatterAdamW(a, o, blocks, threads, reinterpret_cast<cudaStream_t>(stream)), "reduce_scatter_adamw");
+    throwIfCuda(launchReduceScatterAdamW(a, o, blocks, threads, beside, reinterpret_cast<cudaStream_t>(stream)), "reduce_scatter_adamw");
     if (a.w.world > 1 || a.algo == ALGO_NVLS) return 1ll;
-    const long long n = static_cast<long long>(count), part = localAdamPlan(n, blocks, threads, deviceSmCount()).part;
+    const long long n = static_cast<long long>(count), part = localAdamPlan(n, blocks, threads, beside, deviceSmCount()).part;
     return (n + part - 1) / part;       // kernels launched
   });
-  m.def("local_adamw_plan", [](long long count, int blocks, int threads, int sms) {
-    const LocalAdamPlan plan = localAdamPlan(count, blocks, threads, sms);
+  m.def("local_adamw_plan", [](long long count, int blocks, int threads, bool beside, int sms) {
+    const LocalAdamPlan plan = localAdamPlan(count, blocks, threads, beside, sms);
     return py::make_tuple(plan.ctas, plan.part);
   });
   m.def("emu_collective", &emuCollective, py::arg("kind"), py::arg("heaps"), py::arg("signal_off"), py::arg("flag_off"), py::arg("dtype"),

@@ -171,10 +171,10 @@ struct AdamArgs {
   float lr, b1, b2, eps, wd, inv_bc1, inv_sqrt_bc2;
 };
 // How the step of a world of one (without NVLS) is launched: CTAs of 128 threads and parameters per launch.  `blocks` > 0 with `threads` limits the
-// threads of a launch, 0 leaves it to the kernel.
+// threads of a launch, 0 leaves it to the kernel; `beside`: other kernels run at the same time and come first.
 struct LocalAdamPlan { int ctas; long long part; };
-LocalAdamPlan localAdamPlan(long long count, int blocks, int threads, int sms);
-int launchReduceScatterAdamW(const CollArgs& a, const AdamArgs& o, int blocks, int threads, cudaStream_t stream);
+LocalAdamPlan localAdamPlan(long long count, int blocks, int threads, bool beside, int sms);
+int launchReduceScatterAdamW(const CollArgs& a, const AdamArgs& o, int blocks, int threads, bool beside, cudaStream_t stream);
 // Block-scaled fp8 (e4m3 payload + one fp32 scale per 128 values) all-reduce and reduce-scatter: every 128-value block is
 // dequantised, accumulated in fp32 over the ranks and re-quantised with a fresh scale (block maximum / 448), all inside
 // the transfer.  `count` = elements (AR: whole vector; RS: per shard), a multiple of 128.  Sum or max.  P2P only.

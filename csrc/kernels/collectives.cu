@@ -446,10 +446,10 @@ __global__ void __launch_bounds__(512) reduce_scatter_adamw_kernel(const __grid_
 
 // The same step in a world of one, where nothing is exchanged: a flat pass over the bucket.  The kernel above has CTAs of 512 threads that
 // find no room on an SM that runs a GEMM's CTA (320 threads of 168 registers), so an update took the SMs from the backward pass in
-// bursts of 114 us; one CTA of 128 threads with at most 80 registers fits beside it, and the update's memory traffic then passes behind
+// bursts of 93 us; one CTA of 128 threads with at most 80 registers fits beside it, and the update's memory traffic then passes behind
 // the GEMM's arithmetic.  A warp takes 4 x 128 parameters at a time, four of each 128 per lane, so that every access of a warp is one
-// stretch of memory; the 16 loads of a trip are out before the first is used (28 KiB per SM).  A bucket of 13.1 M parameters alone: 95 ->
-// 87 us (4.2 TB/s), of 0.26 M 25 -> 10; the training step of GPT-1.3B, 16384 tokens, 133.1 -> 128.9 ms (two CTAs per SM: the same).
+// stretch of memory; the 16 loads of a trip are out before the first is used (28 KiB per SM).  By itself, in one launch of four CTAs per SM, us
+// (the kernel above): 0.26 M parameters 7.6 (23), 5.2 M 17 (36), 13.6 M 68 (93), 5.6 TB/s, 102.9 M 474 (602).
 constexpr int kLocalAdamThreads = 128, kLocalAdamTrip = 512, kLocalAdamTrips = 4;
 __global__ void __launch_bounds__(kLocalAdamThreads, 6) local_adamw_kernel(const __nv_bfloat16* grads, const AdamArgs O, long long count, float scale) {
   const int lane = threadIdx.x & 31;
@@ -578,10 +578,11 @@ int launchReduceScatter(const CollArgs& a, int blocks, int threads, cudaStream_t
 // parameters, an embedding or a head, is one launch of four CTAs per SM (102.9 M parameters: 610 -> 481 us, 6.0 TB/s), also where it is an
 // untied head's, whose gradient is the first of the backward pass: in short launches there, the step of 24 layers of 2048 with 16384 tokens
 // takes the same 131.0 ms and that of 6 layers with 2048 tokens 8.70 ms instead of 8.25.
+// A call that runs by itself is one such launch at any size (13.6 M parameters 68 us, 142 in short launches).
 // A caller's `blocks` CTAs of `threads` threads are a limit on the threads of a launch.
-LocalAdamPlan localAdamPlan(long long count, int blocks, int threads, int sms) {
+LocalAdamPlan localAdamPlan(long long count, int blocks, int threads, bool beside, int sms) {
   const long long per_cta = kLocalAdamTrip * (kLocalAdamThreads / 32);
-  const bool wide = count > (32ll << 20);
+  const bool wide = !beside || count > (32ll << 20);
   LocalAdamPlan plan{wide ? 4 * sms : sms, 0};
   if (blocks > 0) {
     const long long limit = static_cast<long long>(blocks) * threads / kLocalAdamThreads;
@@ -591,12 +592,12 @@ LocalAdamPlan localAdamPlan(long long count, int blocks, int threads, int sms) {
   return plan;
 }
 
-int launchReduceScatterAdamW(const CollArgs& a, const AdamArgs& o, int blocks, int threads, cudaStream_t stream) {
+int launchReduceScatterAdamW(const CollArgs& a, const AdamArgs& o, int blocks, int threads, bool beside, cudaStream_t stream) {
   if (a.dtype != DT_BF16 || a.nvirt > 1 || a.count % 8 || a.flag_lane < 0 || a.flag_lane >= 8) return static_cast<int>(cudaErrorInvalidValue);
   if (a.algo == ALGO_NVLS && !a.w.mc_heap) return static_cast<int>(cudaErrorInvalidValue);
   if (a.w.world == 1 && a.algo != ALGO_NVLS) {
     const long long count = static_cast<long long>(a.count), per_cta = kLocalAdamTrip * (kLocalAdamThreads / 32);
-    const LocalAdamPlan plan = localAdamPlan(count, blocks, threads, deviceSmCount());
+    const LocalAdamPlan plan = localAdamPlan(count, blocks, threads, beside, deviceSmCount());
     const __nv_bfloat16* grads = reinterpret_cast<const __nv_bfloat16*>(a.w.heap[a.rank] + a.in_off);
     for (long long at = 0; at < count; at += plan.part) {
       const long long n = count - at < plan.part ? count - at : plan.part, trips = (n + per_cta - 1) / per_cta;

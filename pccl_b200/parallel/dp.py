@@ -234,7 +234,7 @@ class ShardedDataParallel:
         dst = b.values[self.rank * shard:(self.rank + 1) * shard]
         coll.reduce_scatter_adamw(self.engine, b.grads, b.master, b.exp_avg, b.exp_avg_sq, dst, lr=self.lr, betas=self.betas,
                                   eps=self.eps, weight_decay=self.weight_decay if b.decay else 0.0, step=self.step_count,
-                                  scale=1.0 / self.world, algo=self.algo, blocks=self._update_blocks, lane=1, stream=self.comm_stream)
+                                  scale=1.0 / self.world, algo=self.algo, blocks=self._update_blocks, lane=1, stream=self.comm_stream, beside=True)
         if reduced_mark is not None:
             reduced_mark.record(self.comm_stream)
         if self.world > 1:

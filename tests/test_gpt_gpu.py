@@ -111,9 +111,10 @@ def test_adamw_kernel_matches_torch():
     assert torch.equal(out, p.bfloat16())
 
 
-@pytest.mark.parametrize("n", [8, 504, 520, 2048, 2056, 303112, (32 << 20) + 24])
-def test_bucket_update_in_a_world_of_one(n):
-    """Whole and partial trips of a warp, more trips than CTAs, and the size from which more CTAs run; two steps against the formula in
+@pytest.mark.parametrize("n", [8, 504, 520, 2048, 2056, 303112, 1212424, (32 << 20) + 24])
+@pytest.mark.parametrize("beside", [False, True])
+def test_bucket_update_in_a_world_of_one(n, beside):
+    """Whole and partial trips of a warp, more trips than CTAs, one launch and several, and the size from which more CTAs run; two steps against the formula in
     fp64 (each step rounds master and moments to fp32 a few times: 1e-5), parameters one bf16 rounding of the masters."""
     import torch
     from pccl_b200.engine import Engine
@@ -128,7 +129,7 @@ def test_bucket_update_in_a_world_of_one(n):
     p64, m64, v64 = p.double(), m.double(), v.double()
     for step in (1, 2):
         g.copy_(torch.randn(n, device="cuda"))
-        coll.reduce_scatter_adamw(eng, g, p, m, v, out, lr=1e-2, betas=(0.9, 0.95), eps=1e-8, weight_decay=0.1, step=step, scale=0.5)
+        coll.reduce_scatter_adamw(eng, g, p, m, v, out, lr=1e-2, betas=(0.9, 0.95), eps=1e-8, weight_decay=0.1, step=step, scale=0.5, beside=beside)
         g64 = g.double() * 0.5
         m64, v64 = 0.9 * m64 + 0.1 * g64, 0.95 * v64 + 0.05 * g64 * g64
         p64 = p64 * (1 - 1e-2 * 0.1) - 1e-2 * (m64 / (1 - 0.9 ** step)) / ((v64 / (1 - 0.95 ** step)).sqrt() + 1e-8)
@@ -150,7 +151,7 @@ def test_launches_of_the_bucket_update_are_counted():
     out = torch.empty(n, device="cuda", dtype=torch.bfloat16)
     for blocks, threads, launches in ((None, 512, 1), (1, 128, 38), (2, 128, 19)):        # 8192 parameters per CTA of 128 threads and launch; 148 CTAs
         before = launch_count()
-        coll.reduce_scatter_adamw(eng, g, p, m, v, out, lr=1e-2, blocks=blocks, threads=threads)
+        coll.reduce_scatter_adamw(eng, g, p, m, v, out, lr=1e-2, blocks=blocks, threads=threads, beside=True)
         assert launch_count() - before == launches
     torch.cuda.synchronize()
 

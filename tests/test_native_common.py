@@ -148,12 +148,18 @@ def test_moe_gate_gradients_are_zeros_where_the_exchange_gives_up(native, monkey
 
 
 def test_bucket_update_of_a_world_of_one_keeps_to_the_callers_blocks(native):
-    plan = lambda count, blocks=0, threads=512: native.local_adamw_plan(count, blocks, threads, 148)  # noqa: E731   (CTAs of 128 threads, parameters)
+    plan = lambda count, blocks=0, threads=512: native.local_adamw_plan(count, blocks, threads, True, 148)  # noqa: E731   (CTAs of 128 threads, parameters)
     trip = 4 * 4 * 512                                         # parameters of a CTA in a launch: four trips of four warps
     assert plan(13 << 20) == (148, 148 * trip)
     assert plan(13 << 20, 8) == (32, 32 * trip) and plan(13 << 20, 1, 32) == (1, trip) and plan(13 << 20, 128) == (148, 148 * trip)
     big = 102_900_000
     assert plan(big) == (592, big) and plan(big, 8) == (32, big) and plan(big, 148) == (592, big)
+
+
+def test_bucket_update_by_itself_is_one_launch(native):
+    for count in (8, 5 << 20, 13 << 20, 102_900_000):
+        assert native.local_adamw_plan(count, 0, 512, False, 148) == (592, count)
+        assert native.local_adamw_plan(count, 4, 512, False, 148) == (16, count)
 
 
 def test_moe_exchange_between_ranks_keeps_the_groups_that_were_measured(native):

@@ -85,7 +85,7 @@ __device__ __forceinline__ void ffma2(float& acc0, float& acc1, uint32_t r0, uin
 // STAGES (<= 4) operand stages of 48 KiB; an epilogue that needs shared memory of its own runs with three.
 // BNT = 128 (up to six stages of 32 KiB): a K block is a chain MMA -> commit -> tcgen05.ld -> fold -> accumulator free -> MMA.  128 columns
 // leave room for four accumulators where 256 have two, and the 64 sums per thread no longer spill: 8192 x 8192 x 3584 372 -> 320 us, and
-// 260 with the scales read as below.  What is left is the operands' way from L2.  The fused kernels keep 256 columns: their epilogues
+// 271 with the scales read as below.  What is left is the operands' way from L2.  The fused kernels keep 256 columns: their epilogues
 // quantise or stage whole 128-column halves.
 template <int STAGES = MAX_STAGES, int BNT = BN, class Sched, class Gate, class Epi>
 __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* tmB, int K, const Scales& sc, const Sched& sched,
@@ -238,20 +238,28 @@ __device__ __forceinline__ void run(const CUtensorMap* tmA, const CUtensorMap* t
         // Four K blocks' row scales in one load.  A load per block touches 32 cache lines per warp, 256 look-ups per K block and CTA: that,
         // not the chain of the K block, was what the kernel waited for (L1 71 % busy).  8192 x 3584 x 8192 321 -> 264 us, 8192 x 8192 x 3584
         // 302 -> 271, 16384 x 8192 x 8192 1371 -> 1110 (1.95 PFLOP/s), 1531 x 3584 x 8192 87 -> 68; a round of tiles now takes 540 clocks per K
-        // block, which is the 32 KiB of operands at the 63 bytes per clock that an SM gets from L2.
-        if ((sc.ld_sa & 3) == 0 && (reinterpret_cast<uintptr_t>(sc.sa) & 15) == 0 && num_kb >= 4) {
+        // block, which is the 32 KiB of operands at the 63 bytes per clock that an SM gets from L2.  The weights' scales come four blocks
+        // ahead as well (the two GEMMs of 8192 tokens, 8192 <-> 3584, with their quantisers: one block ahead 720 us, four 707).  Below eight K
+        // blocks there is nothing to fetch ahead, and a load per block is the quicker (16 x 2048 x 512 4.1 us, 3.9).
+        if ((sc.ld_sa & 3) == 0 && (reinterpret_cast<uintptr_t>(sc.sa) & 15) == 0 && num_kb >= 8) {
           dev::Vec16 a = dev::ld16_cg(pa);
-          float b0 = dev::ld_f32(pb);
+          float b[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) b[j] = dev::ld_f32(pb + j);
           for (; ok && kb + 4 <= num_kb; kb += 4) {
             dev::Vec16 an = a;
-            if (kb + 8 <= num_kb) an = dev::ld16_cg(pa + kb + 4);
+            float bn[4] = {0.f, 0.f, 0.f, 0.f};
+            if (kb + 8 <= num_kb) {
+              an = dev::ld16_cg(pa + kb + 4);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float s = __uint_as_float(a.w[j]) * b0;
-              if (kb + j + 1 < num_kb) b0 = dev::ld_f32(pb + kb + j + 1);
-              if (!fold(s)) { ok = false; break; }
+              for (int j = 0; j < 4; ++j) bn[j] = dev::ld_f32(pb + kb + 4 + j);
             }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (!fold(__uint_as_float(a.w[j]) * b[j])) { ok = false; break; }
             a = an;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = bn[j];
           }
         }
       }

@@ -423,11 +423,11 @@ def test_fp8_gemm_at_the_edges_of_its_tiles(M, N, K):
     assert (out.double() - ref).abs().max().item() <= 2e-3 * max(1.0, ref.abs().max().item())
 
 
-@pytest.mark.parametrize("K", [512, 640, 1152])
+@pytest.mark.parametrize("K", [512, 640, 896, 1024, 1152, 1408, 1536])
 @pytest.mark.parametrize("shift,stride", [(0, 4), (0, 12), (1, 12), (0, 9)])
 def test_fp8_gemm_row_scales_of_any_stride(K, shift, stride):
-    """Row scales are read four K blocks at a time where their rows allow it: rows of any stride and start give the same bits, with
-    whole and partial groups of four."""
+    """Row scales are read four K blocks at a time where their rows allow it and there are eight blocks: rows of any stride and start give the
+    same bits, with whole and partial groups of four."""
     from pccl_b200.ops import check_status
     from pccl_b200.ops.gemm import gemm_fp8, quant_blocks, quant_rows
     if stride < K // 128 + shift:

@@ -224,6 +224,27 @@ def test_fused_and_unfused_optimizer_paths_agree():
     assert (flats[0] == flats[1]).float().mean().item() > 0.9       # identical except where atomics order / bf16 rounding of a gradient differs
 
 
+def test_an_untied_head_above_32_mi_parameters_is_updated_while_backward_runs():
+    """Its bucket is the first to complete and goes out as one wide launch: the same parameters as with the optimizer behind the backward pass."""
+    from pccl_b200.models import GPT, GPTConfig
+    from pccl_b200.parallel import ShardedDataParallel
+    cfg = GPTConfig(n_layer=1, n_head=16, d_model=2048, seq_len=64, vocab_size=16401, tie_embeddings=False)
+    ids = torch.randint(0, cfg.vocab_size, (2, 64), device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    got = []
+    for fused in (True, False):
+        torch.manual_seed(0)
+        dp = ShardedDataParallel(GPT(cfg, device="cuda"), lr=1e-3, fuse_optimizer=fused)
+        assert dp.buckets[0].numel > 32 << 20 and dp.buckets[0].params[0] is dp.model.lm_head.weight
+        dp.train_step(ids, ids.roll(-1, 1))
+        torch.cuda.synchronize()
+        got.append({n: p.detach().clone() for n, p in dp.model.named_parameters()})
+    for name, p in got[0].items():
+        if name == "wte.weight":                               # its gradient is a sum in no fixed order
+            assert (p == got[1][name]).float().mean().item() > 0.99
+        else:
+            assert torch.equal(p, got[1][name]), name
+
+
 def test_timed_step_reports_every_bucket_and_trains_like_train_step():
     """The opt-in per-bucket timing takes the same step as train_step and returns ordered, non-negative spans."""
     from pccl_b200.engine import Engine

@@ -204,7 +204,7 @@ int gemmMx8(const void* A, int64_t lda, const uint8_t* sa, int ld_sa, const void
     return static_cast<int>(cudaErrorInvalidValue);
   }
   if (flags & (GEMM_A_MN | GEMM_B_MN | GEMM_PAIR)) {
-    g_errx = "gemmMx8: operands are K-major and tiles belong to single CTAs";
+    g_errx = "gemmMx8: operands are K-major, and the launch itself picks single CTAs or pairs";
     return static_cast<int>(cudaErrorInvalidValue);
   }
   if ((flags & GEMM_GELU) && (!D2 || (flags & GEMM_OUT_F32))) {

@@ -64,9 +64,9 @@ def _fits(p: torch.Tensor, D: int) -> bool:
             and (mg is None or (mg.dtype is torch.bfloat16 and mg.is_contiguous() and mg.data_ptr() % 16 == 0)))
 
 
-# The backward walks the batch in one thread per eight columns of a position.  That pays at any batch where there are positions enough to fill
-# the device (64 x 256 x 2048: 52 us against the layers' 294) and loses where they are few (64 x 1 x 256: 23.6 against 19.5; 1024 x 16 x 2048:
-# 500 against 305).  The line lies where the shortest sequences still gain.
+# The backward walks the batch in one thread per eight columns of a position.  Up to 32 sequences it gains whatever their length.  Beyond that it
+# depends on the positions as well: where they fill the device it would still gain (64 x 256 x 2048: 52 us against the layers' 294), where they are
+# few it loses (64 x 1 x 256: 23.6 against 19.5; 1024 x 16 x 2048: 500 against 305).  The line is drawn by the batch alone, on the safe side.
 _MAX_BATCH = 32
 
 

@@ -84,7 +84,7 @@ def _version(t: torch.Tensor) -> Optional[int]:
 
 
 class MoEExchange:
-    """Buffers and kernels of one expert-parallel MoE layer shape."""
+    """Buffers and kernels of one expert-parallel MoE layer shape.  ``recv_q`` and ``recv_s`` hold what the last ``dispatch`` brought."""
 
     def __init__(self, eng: Engine, tokens: int, hidden: int, n_experts: int, topk: int, capacity_factor: float = 2.0,
                  blocks: Optional[int] = None, flag_lane: int = 5):
